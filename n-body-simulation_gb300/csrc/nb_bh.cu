@@ -135,12 +135,23 @@ __device__ uint64_t key_word_quantized(const double* __restrict__ box, double px
     return (spread3(hy) << 2) | (spread3(~hz & m) << 1) | spread3(~hx & m);
 }
 
+// Box entries beyond the AABB, by the first threads of the keys kernels: the centre, for the node
+// records, and the scale exponent of the fixed-point records.
+__device__ __forceinline__ void box_extras(double* __restrict__ box, uint32_t i) {
+    if (i < 3) box[7 + i] = box[i] + box[6] / 2;
+    if (i == 3) {
+        double v = 0.0;
+        for (int k = 0; k < 6; ++k) v = fmax(v, fabs(box[k]));
+        box[10] = (double)nbfix::k_of(v);
+    }
+}
+
 __global__ void keys_quantized_kernel(const double* __restrict__ x, const double* __restrict__ y,
                                       const double* __restrict__ z, uint32_t n,
                                       double* __restrict__ box, uint64_t* __restrict__ key0,
                                       uint32_t* __restrict__ ids) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 3) box[7 + i] = box[i] + box[6] / 2;  // box centre, for the node records
+    box_extras(box, i);
     if (i >= n) return;
     key0[i] = key_word_quantized(box, x[i], y[i], z[i], 0);
     ids[i] = i;
@@ -193,7 +204,7 @@ keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
             uint64_t* __restrict__ key0, uint32_t* __restrict__ ids) {
     __shared__ FixedGrid grid_s;  // once per block: it takes an FP64 division
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 3) box[7 + i] = box[i] + box[6] / 2;  // box centre, for the node records
+    box_extras(box, i);
     if (threadIdx.x == 0) grid_s = fixed_grid(box);
     __syncthreads();
     if (i >= n) return;
@@ -415,6 +426,8 @@ struct ComArgs {
     uint32_t* node_count;
     double *comx, *comy, *comz, *mass, *q;
     NodeRec64* rec64;
+    nbfix::FixHi* fix_hi;
+    uint4* fix_lo;
     NodeRec32* rec32;
     float4* rec32lo;
     float4* rec32lo2;
@@ -453,6 +466,14 @@ __device__ __forceinline__ double leaf_quotient(double x, double m, double c) {
     return __ddiv_rn(c, m);
 }
 
+// Fixed-point record of a node with centre (cx, cy, cz) and mass m.
+__device__ __forceinline__ void write_fix(const ComArgs& A, uint32_t idx, double cx, double cy,
+                                          double cz, double m) {
+    const nbfix::FixRec r = nbfix::make_rec(cx, cy, cz, m, (int)A.box[10]);
+    A.fix_hi[idx] = nbfix::FixHi{r.x2, r.y2, r.z2, r.mh, r.x1, r.y1, r.z1, r.e};
+    A.fix_lo[idx] = make_uint4(r.x0, r.y0, r.z0, r.ml);
+}
+
 __device__ void write_records(const ComArgs& A, uint32_t idx, double cx, double cy, double cz,
                               double sm, double qsum, uint32_t count, int level, uint32_t skip,
                               uint32_t body) {
@@ -487,6 +508,7 @@ __device__ void write_records(const ComArgs& A, uint32_t idx, double cx, double 
         r.skip = skip;
         r.body = body;
         A.rec64[idx] = r;
+        write_fix(A, idx, rcx, rcy, rcz, sm);
     }
     NodeRec32 q;
     const double gx = rcx - ox, gy = rcy - oy, gz = rcz - oz;
@@ -635,6 +657,7 @@ __device__ void leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32_t b
         r.skip = skip;
         r.body = b;
         A.rec64[idx] = r;
+        write_fix(A, idx, rcx, rcy, rcz, mb);
     }
     const double gx = rcx - ox, gy = rcy - oy, gz = rcz - oz;
     NodeRec32 q;
@@ -903,6 +926,8 @@ void carve(nb_bh_tree* t, Carver& c) {
     t->node_comz = c.take<double>(cap);
     t->node_mass = c.take<double>(cap);
     t->rec64 = c.take<NodeRec64>(cap);
+    t->fix_hi = c.take<nbfix::FixHi>(cap);
+    t->fix_lo = c.take<uint4>(cap);
     t->rec32 = c.take<NodeRec32>(cap);
     t->rec32lo = c.take<float4>(cap);
     t->rec32lo2 = c.take<float4>(cap);
@@ -1098,6 +1123,8 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     A.comz = t->node_comz;
     A.mass = t->node_mass;
     A.rec64 = t->rec64;
+    A.fix_hi = t->fix_hi;
+    A.fix_lo = t->fix_lo;
     A.rec32 = t->rec32;
     A.rec32lo = t->rec32lo;
     A.rec32lo2 = t->rec32lo2;

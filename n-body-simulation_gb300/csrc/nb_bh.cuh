@@ -8,9 +8,11 @@
 //  per node (DFS pre-order, children in the reference's visit order 2,0,3,1,6,4,7,5):
 //    level, first/last sorted position, skip (DFS index after the subtree), parent, body,
 //    child count, centre-of-mass numerators and mass (FP64, the reference's sums), and the
-//    traversal records rec64 (FP64 centre, mass, edge, skip, body: 48 B) and rec32 (FP32 centre
+//    traversal records rec64 (FP64 centre, mass, edge, skip, body: 48 B), fix_hi (the same centre
+//    and mass in fixed point: 48 B) and rec32 (FP32 centre
 //    relative to the box centre, G*mass, edge^2, skip, body: 32 B).
 #pragma once
+#include "nb_fix.cuh"
 #include "nb_internal.cuh"
 
 constexpr uint32_t NB_NONE = 0xffffffffu;
@@ -46,7 +48,8 @@ struct nb_bh_tree {
     double G = 0;
     int device = 0;
 
-    double* box = nullptr;  // [0..6] AABB (min xyz, max xyz, edge), [7..9] box centre
+    double* box = nullptr;  // [0..6] AABB (min xyz, max xyz, edge), [7..9] box centre, [10] the
+                            // scale exponent K of the fixed-point records (nb_fix.cuh)
     uint32_t* info = nullptr;  // [0] node count (copy of base[n])
     uint2* tier_cells[2] = {};      // centre-of-mass tiers: cells passed up, (node, level)
     uint32_t* tier_count[2] = {};   // their count per chunk
@@ -83,6 +86,9 @@ struct nb_bh_tree {
     uint32_t* node_count = nullptr;
     double *node_comx = nullptr, *node_comy = nullptr, *node_comz = nullptr, *node_mass = nullptr;
     NodeRec64* rec64 = nullptr;
+    // rec64's centre and mass in fixed point (nb_fix.cuh): 32 + 16 B
+    nbfix::FixHi* fix_hi = nullptr;
+    uint4* fix_lo = nullptr;
     NodeRec32* rec32 = nullptr;
     float4* rec32lo = nullptr;   // second FP32 terms of rec32's centre and G*mass
     float4* rec32lo2 = nullptr;  // third FP32 terms of the centre (triple-float: exact FP64)

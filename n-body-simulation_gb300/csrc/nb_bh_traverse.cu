@@ -6,12 +6,14 @@
 // "Accept" (or skip) continues at the skip link and "open" continues at the next node, so a
 // traversal needs no stack at all and visits nodes in exactly the reference's order.
 //
-//  * per-body rule (NB_OPEN_THETA), default schedule (bh_theta_lane_kernel, FP64; and
-//    bh_theta_df_kernel, double-float): each lane walks its own body's DFS sequence, deciding each
+//  * per-body rule (NB_OPEN_THETA), default schedule (bh_theta_fix_kernel, NB_F64 with fixed-point
+//    monopoles (nb_fix.cuh), and bh_theta_team_kernel, the same with several lanes per body for
+//    small systems; bh_theta_lane_kernel, NB_F64_IEEE; bh_theta_df_kernel, double-float): each lane
+//    walks its own body's DFS sequence, deciding each
 //    cell with an FP32 pre-test whose rounding margin is proven and the reference's FP64
 //    expression only inside that margin; find-then-compute, so the FP64 monopoles of all lanes
 //    that found one run together. Warps take groups of 32 bodies close together in the tree, after
-//    the first traversal of a tree sorted within windows of 1,024 by the length of their last
+//    the first traversal of a tree sorted within windows of 512 by the length of their last
 //    walk, so that the lanes of a warp finish together.
 //  * per-body rule, lockstep schedule (bh_theta_f64_kernel, nb_bh_set_schedule(1)): the 32 lanes
 //    of a warp hold 32 bodies adjacent in tree order, each with its own position in the DFS
@@ -71,37 +73,88 @@ struct Arith<FAST64> {
     __device__ static double rsqrt(double v) { return nb_rsqrt_f64(v); }
     __device__ static double mul(double a, double b) { return a * b; }
     __device__ static double add(double a, double b) { return a + b; }
-    __device__ static double accum(double acc, double m, double d, double inv) {
-        return fma(m * inv, d, acc);
-    }
-    // m (d2 + eps2)^(-3/2) by nb_m_rinv3_f64: 7 FP64 operations instead of cubing den and
-    // refining its rsqrt (8).
-    __device__ static void monopole(double m, double dx, double dy, double dz, double d2,
-                                    double eps2, double& ax, double& ay, double& az) {
-        monopole_den(m, dx, dy, dz, d2 + eps2, ax, ay, az);
-    }
-    __device__ static void monopole_xyz(double m, double dx, double dy, double dz, double eps2,
-                                        double& ax, double& ay, double& az) {
-        monopole_den(m, dx, dy, dz, fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))), ax, ay, az);
-    }
-    __device__ static void monopole_den(double m, double dx, double dy, double dz, double den,
-                                        double& ax, double& ay, double& az) {
-        const double w = nb_m_rinv3_f64(m, den);
-        ax = fma(w, dx, ax);
-        ay = fma(w, dy, ay);
-        az = fma(w, dz, az);
-    }
 };
+
+using nbfix::FixRec;
+
+// 32-byte loads (one instruction of the load pipe instead of two).
+__device__ __forceinline__ NodeRec32 load_rec32(const NodeRec32* __restrict__ p) {
+    NodeRec32 r;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.cx), "=f"(r.cy), "=f"(r.cz), "=f"(r.gm), "=f"(r.edge2), "=r"(r.skip),
+          "=r"(r.body), "=r"(r.level)
+        : "l"(p));
+    return r;
+}
+__device__ __forceinline__ FixRec load_fix(const nbfix::FixHi* __restrict__ hi,
+                                           const uint4* __restrict__ lo, uint32_t k) {
+    FixRec r;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r.x2), "=r"(r.y2), "=r"(r.z2), "=r"(r.mh), "=r"(r.x1), "=r"(r.y1), "=r"(r.z1),
+          "=r"(r.e)
+        : "l"(hi + k));
+    const uint4 l = lo[k];
+    r.x0 = l.x;
+    r.y0 = l.y;
+    r.z0 = l.z;
+    r.ml = l.w;
+    return r;
+}
+
+// A body in the fixed point of the node records (nb_fix.cuh); sh_max < 0: FP64 pairs only.
+struct FixBody {
+    nbfix::Fix3 p;
+    int sh_max;
+};
+template <int MODE>
+__device__ __forceinline__ FixBody fix_body(double px, double py, double pz, int K,
+                                            const nbfix::Eps2Table& e2) {
+    FixBody b{};
+    if constexpr (MODE == FAST64) b.sh_max = nbfix::split3(px, py, pz, K, b.p) ? e2.sh_max : -1;
+    return b;
+}
+
+// Adds the monopole of node k to a body's sums: NB_F64's arithmetic, in every schedule.
+__device__ __forceinline__ void fix_monopole(const FixRec& f, const NodeRec64* __restrict__ rec64,
+                                             uint32_t k, const FixBody& b, int K,
+                                             const nbfix::Eps2Table& e2,
+                                             const double* __restrict__ x,
+                                             const double* __restrict__ y,
+                                             const double* __restrict__ z, uint32_t me,
+                                             double eps2, double& acx, double& acy, double& acz) {
+    double w, dx, dy, dz;
+    if (b.sh_max < 0 || !nbfix::term(f, b.p, K, e2, b.sh_max, w, dx, dy, dz)) {
+        const NodeRec64 q = rec64[k];
+        if (q.mass == 0) return;
+        dx = q.cx - x[me];
+        dy = q.cy - y[me];
+        dz = q.cz - z[me];
+        w = nb_m_rinv3_f64(q.mass, fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+    }
+    acx = fma(w, dx, acx);
+    acy = fma(w, dy, acy);
+    acz = fma(w, dz, acz);
+}
 
 // Per-body reference rule, FP64 (IEEE64 bit-identical to the host evaluation; FAST64 with FMAs).
 template <int MODE>
 __global__ void __launch_bounds__(TR_THREADS)
-bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const uint32_t* __restrict__ info,
+bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const nbfix::FixHi* __restrict__ fix_hi,
+                    const uint4* __restrict__ fix_lo,
+                    const uint32_t* __restrict__ info,
                     const uint32_t* __restrict__ ids, const double* __restrict__ x,
-                    const double* __restrict__ y, const double* __restrict__ z, uint32_t n,
-                    double theta, double eps2, double G, double* __restrict__ ax,
+                    const double* __restrict__ y, const double* __restrict__ z,
+                    const double* __restrict__ box, uint32_t n,
+                    double theta, double eps2, double G, int team,
+                    double* __restrict__ ax,
                     double* __restrict__ ay, double* __restrict__ az) {
     using A = Arith<MODE>;
+    __shared__ nbfix::Eps2Table e2;
+    const int K = (int)box[10];
+    if (MODE == FAST64) {
+        nbfix::fill_eps2(e2, eps2, K);
+        __syncthreads();
+    }
     const uint32_t p = blockIdx.x * TR_THREADS + threadIdx.x;
     const bool valid = p < n;
     const uint32_t nn = info[0];
@@ -112,7 +165,11 @@ bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const uint32_t* __restric
         py = y[me];
         pz = z[me];
     }
-    double acx = 0, acy = 0, acz = 0;
+    const FixBody me_fix = fix_body<MODE>(px, py, pz, K, e2);
+    // NB_F64: `team` partial sums in turn, as bh_theta_team_kernel
+    constexpr int TEAM_MAX = MODE == FAST64 ? 32 : 1;
+    double acx[TEAM_MAX] = {}, acy[TEAM_MAX] = {}, acz[TEAM_MAX] = {};
+    uint32_t ord = 0;
     uint32_t kl = valid ? 0u : nn;
     for (;;) {
         const uint32_t k = __reduce_min_sync(0xffffffffu, kl);
@@ -124,7 +181,13 @@ bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const uint32_t* __restric
             const double d2 = A::norm2(dx, dy, dz);
             const double cur = A::mul(r.edge, A::rsqrt(d2));  // :355-357
             if (cur < theta || r.body != NB_NONE) {           // :359
-                A::monopole(r.mass, dx, dy, dz, d2, eps2, acx, acy, acz);
+                if constexpr (MODE == FAST64) {
+                    const uint32_t c = ord++ & (uint32_t)(team - 1);
+                    fix_monopole(load_fix(fix_hi, fix_lo, k), rec, k, me_fix, K, e2, x, y, z, me,
+                                 eps2, acx[c], acy[c], acz[c]);
+                } else {
+                    A::monopole(r.mass, dx, dy, dz, d2, eps2, acx[0], acy[0], acz[0]);
+                }
                 kl = r.skip;
             } else {
                 kl = k + 1;
@@ -133,10 +196,18 @@ bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const uint32_t* __restric
             kl = r.skip;
         }
     }
+    if constexpr (MODE == FAST64) {
+        for (int o = team / 2; o > 0; o >>= 1)
+            for (int c = 0; c < o; ++c) {
+                acx[c] += acx[c + o];
+                acy[c] += acy[c + o];
+                acz[c] += acz[c + o];
+            }
+    }
     if (valid) {
-        ax[me] = A::mul(acx, G);
-        ay[me] = A::mul(acy, G);
-        az[me] = A::mul(acz, G);
+        ax[me] = A::mul(acx[0], G);
+        ay[me] = A::mul(acy[0], G);
+        az[me] = A::mul(acz[0], G);
     }
 }
 
@@ -150,7 +221,6 @@ bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const uint32_t* __restric
 // positions; with `order` != nullptr the bodies of the positions come from it (the previous
 // walk's lengths regrouped within windows, regroup_kernel) instead of from ids. Each body's
 // accepted-cell count goes to walk_len[body].
-template <int MODE>
 __global__ void __launch_bounds__(TR_THREADS)
 bh_theta_lane_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __restrict__ rec64,
                      const uint32_t* __restrict__ info, const uint32_t* __restrict__ ids,
@@ -160,7 +230,7 @@ bh_theta_lane_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
                      double* __restrict__ ay, double* __restrict__ az,
                      uint32_t* __restrict__ next_group, const uint32_t* __restrict__ order,
                      uint32_t* __restrict__ walk_len) {
-    using A = Arith<MODE>;
+    using A = Arith<IEEE64>;
     const uint32_t n_groups = (n + 31) / 32;
     const int lane = threadIdx.x & 31;
     // persistent warps: each takes the next 32 bodies until none are left, so no warp waits for
@@ -241,12 +311,224 @@ bh_theta_lane_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
     }
 }
 
+// Decision of the reference's opening rule for node `idx` seen from a body: true = accepted (a
+// leaf, or certainly below theta), by the FP32 test where its margin allows (see
+// bh_theta_lane_kernel), else by the FP64 expression.
+struct Pretest {
+    float px, py, pz, th2, edge;  // body relative to the box centre, theta^2, box edge
+};
+__device__ __forceinline__ bool accepts(const NodeRec32& r, const Pretest& b,
+                                        const NodeRec64* __restrict__ rec64, uint32_t idx,
+                                        const double* __restrict__ x,
+                                        const double* __restrict__ y,
+                                        const double* __restrict__ z, uint32_t me, double theta) {
+    using A = Arith<FAST64>;
+    const float u4 = 4.0f * 5.9604645e-8f;  // 4 * 2^-24
+    const float dx = r.cx - b.px, dy = r.cy - b.py, dz = r.cz - b.pz;
+    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    const float t = b.th2 * d2;
+    const float rel = u4 * (3.5f * b.edge * nb_rsqrt_f32(d2) + 8.0f);
+    const float margin = t * rel + u4 * r.edge2;
+    if (r.body != NB_NONE || r.edge2 < t - margin) return true;
+    if (r.edge2 > t + margin) return false;
+    const NodeRec64 q = rec64[idx];
+    const double ex = A::sub(q.cx, x[me]), ey = A::sub(q.cy, y[me]), ez = A::sub(q.cz, z[me]);
+    return A::mul(q.edge, A::rsqrt(A::norm2(ex, ey, ez))) < theta;
+}
+
+__device__ __forceinline__ Pretest pretest_of(const double* __restrict__ box, double px, double py,
+                                              double pz, double theta) {
+    const double E = box[6];
+    return Pretest{(float)(px - (box[0] + E / 2)), (float)(py - (box[1] + E / 2)),
+                   (float)(pz - (box[2] + E / 2)), (float)(theta * theta), (float)E};
+}
+
+// Per-body reference rule, NB_F64: one lane per body. Each lane walks its body's DFS sequence and
+// lists up to FIX_LIST accepted cells, then the warp evaluates its lanes' lists together, the next
+// cell's record loaded while the current one is computed.
+//  Bound: the load pipe (75% of its wavefronts: every lane reads its own 32-byte walk record per
+//  visited and 48-byte fixed-point record per accepted cell) and issue (61% of cycles, integer
+//  pipe 57%, FP64 pipe 41%). The monopole is ~190 instructions with 3 FP64 ones (nb_fix.cuh)
+//  against 16 FP64 operations before, whose pipe was 82% busy; 256-bit loads halve the load
+//  instructions (14.6 -> 13.45 ms), the lists (against one accepted cell at a time) keep 30.9 of
+//  32 lanes active (17.2 -> 14.6 ms with the record prefetch). 1,048,576-body disc, theta = 0.5:
+//  35.5 -> 13.5 ms per step. 24 warps per SM at 80 registers: 28 or 32 warps at 72 or 64 registers
+//  measured 1% and 6% slower.
+constexpr int FIX_LIST = 16;
+constexpr int FIX_BLOCKS_PER_SM = 6;
+
+__global__ void __launch_bounds__(TR_THREADS, FIX_BLOCKS_PER_SM)
+bh_theta_fix_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __restrict__ rec64,
+                    const nbfix::FixHi* __restrict__ fix_hi, const uint4* __restrict__ fix_lo,
+                    const uint32_t* __restrict__ info, const uint32_t* __restrict__ ids,
+                    const double* __restrict__ x, const double* __restrict__ y,
+                    const double* __restrict__ z, const double* __restrict__ box, uint32_t n,
+                    double theta, double eps2, double G, double* __restrict__ ax,
+                    double* __restrict__ ay, double* __restrict__ az,
+                    uint32_t* __restrict__ next_group, const uint32_t* __restrict__ order,
+                    uint32_t* __restrict__ walk_len) {
+    __shared__ nbfix::Eps2Table e2;
+    __shared__ uint32_t list[FIX_LIST][TR_THREADS];
+    const int K = (int)box[10];
+    nbfix::fill_eps2(e2, eps2, K);
+    __syncthreads();
+    const uint32_t n_groups = (n + 31) / 32, nn = info[0];
+    const int lane = threadIdx.x & 31, tid = threadIdx.x;
+    for (;;) {  // persistent warps, as bh_theta_lane_kernel
+        uint32_t grp = 0;
+        if (lane == 0) grp = atomicAdd(next_group, 1u);
+        grp = __shfl_sync(0xffffffffu, grp, 0);
+        if (grp >= n_groups) break;
+        const uint32_t p = grp * 32 + lane;
+        const bool valid = p < n;
+        const uint32_t me = valid ? (order != nullptr ? order[p] : ids[p]) : 0u;
+        Pretest pre;
+        FixBody body;
+        {
+            const double px = x[me], py = y[me], pz = z[me];
+            pre = pretest_of(box, px, py, pz, theta);
+            body = fix_body<FAST64>(px, py, pz, K, e2);
+        }
+        uint32_t accepted = 0, k = valid ? 0u : nn;
+        double acx = 0, acy = 0, acz = 0;
+        for (;;) {
+            int cnt = 0;
+            while (cnt < FIX_LIST && k < nn) {
+                const NodeRec32 r = load_rec32(rec32 + k);
+                const bool accept = accepts(r, pre, rec64, k, x, y, z, me, theta);
+                if (accept && r.body != me) {
+                    list[cnt][tid] = k;
+                    ++cnt;
+                }
+                k = accept ? r.skip : k + 1;
+            }
+            accepted += cnt;
+            const int most = __reduce_max_sync(0xffffffffu, cnt);
+            if (most == 0) break;
+            FixRec next = load_fix(fix_hi, fix_lo, cnt > 0 ? list[0][tid] : 0u);
+            for (int i = 0; i < most; ++i) {
+                const FixRec f = next;
+                if (i + 1 < cnt) next = load_fix(fix_hi, fix_lo, list[i + 1][tid]);
+                if (i < cnt)
+                    fix_monopole(f, rec64, list[i][tid], body, K, e2, x, y, z, me, eps2, acx, acy,
+                                 acz);
+            }
+        }
+        if (valid) {
+            ax[me] = acx * G;
+            ay[me] = acy * G;
+            az[me] = acz * G;
+            walk_len[me] = accepted;
+        }
+    }
+}
+
+// Per-body reference rule, NB_F64, T lanes per body, for systems too small to fill the chip with
+// one lane per body. A body's lanes test T consecutive nodes of its DFS sequence at once (aligned
+// windows: one coalesced load). Within a window a node is visited exactly when no accepted node
+// before it covers it (an accepted node's subtree ends at its skip link, and whatever covers an
+// unvisited node covers its subtree too), which a prefix maximum of the accepted nodes' skip links
+// decides. The accepted cells go to the body's list in DFS order; cell number c belongs to lane
+// c mod T, and the lanes' sums are added pairwise at the end.
+//  Bound: the latency of a walk of dependent windows and of ~accepted / T monopoles by one warp.
+//  Traversal at theta = 0.5 (disc), one lane per body -> T lanes: 777 bodies 135 -> 31 us (T = 32),
+//  4,000 273 -> 77 us (16), 16,411 471 -> 300 us (4), 32,768 625 -> 540 us (2).
+template <int T>
+__global__ void __launch_bounds__(TR_THREADS, FIX_BLOCKS_PER_SM)
+bh_theta_team_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __restrict__ rec64,
+                     const nbfix::FixHi* __restrict__ fix_hi, const uint4* __restrict__ fix_lo,
+                     const uint32_t* __restrict__ info, const uint32_t* __restrict__ ids,
+                     const double* __restrict__ x, const double* __restrict__ y,
+                     const double* __restrict__ z, const double* __restrict__ box, uint32_t n,
+                     double theta, double eps2, double G, double* __restrict__ ax,
+                     double* __restrict__ ay, double* __restrict__ az,
+                     uint32_t* __restrict__ walk_len) {
+    constexpr int B = 32 / T;                     // bodies per warp
+    constexpr int CAP = T * 8 > 64 ? T * 8 : 64;  // listed cells per body and round
+    constexpr int WARPS = TR_THREADS / 32;
+    __shared__ nbfix::Eps2Table e2;
+    __shared__ uint32_t lists[WARPS][B][CAP];
+    const int K = (int)box[10];
+    nbfix::fill_eps2(e2, eps2, K);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, seg = lane / T, j = lane % T;
+    const uint32_t seg_mask = T == 32 ? 0xffffffffu : (1u << (T & 31)) - 1u;
+    uint32_t* list = lists[warp][seg];
+    const uint32_t p = (blockIdx.x * WARPS + warp) * B + seg, nn = info[0];
+    const bool valid = p < n;
+    const uint32_t me = valid ? ids[p] : 0u;
+    Pretest pre;
+    FixBody body;
+    {
+        const double px = x[me], py = y[me], pz = z[me];
+        pre = pretest_of(box, px, py, pz, theta);
+        body = fix_body<FAST64>(px, py, pz, K, e2);
+    }
+    double acx = 0, acy = 0, acz = 0;
+    uint32_t k = valid ? 0u : nn;  // the same in a body's lanes, like cnt and ord
+    int ord = 0;                   // cells accepted in earlier rounds
+    for (;;) {
+        int cnt = 0;
+        for (;;) {
+            const bool active = k < nn && cnt <= CAP - T;
+            if (!__any_sync(0xffffffffu, active)) break;
+            const uint32_t base = k & ~(uint32_t)(T - 1), idx = base + j;
+            bool take = false;
+            uint32_t end = 0;  // inclusive prefix maximum of the accepted nodes' skip links
+            if (active && idx >= k && idx < nn) {
+                const NodeRec32 r = load_rec32(rec32 + idx);
+                const bool accept = accepts(r, pre, rec64, idx, x, y, z, me, theta);
+                take = accept && r.body != me;
+                if (accept) end = r.skip;
+            }
+#pragma unroll
+            for (int o = 1; o < T; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, end, o, T);
+                if (j >= o) end = max(end, v);
+            }
+            uint32_t before = __shfl_up_sync(0xffffffffu, end, 1, T);
+            if (j == 0) before = 0;
+            take = take && before <= idx;
+            const uint32_t taken = (__ballot_sync(0xffffffffu, take) >> (seg * T)) & seg_mask;
+            if (take) list[cnt + __popc(taken & ((1u << j) - 1u))] = idx;
+            end = __shfl_sync(0xffffffffu, end, T - 1, T);
+            if (active) k = max(base + T, end);
+            cnt += __popc(taken);
+        }
+        const int most = __reduce_max_sync(0xffffffffu, cnt);
+        if (most == 0) break;
+        __syncwarp();
+        int i = (j - ord) & (T - 1);
+        FixRec next = load_fix(fix_hi, fix_lo, i < cnt ? list[i] : 0u);
+        for (int c = 0; c < most; c += T, i += T) {
+            const FixRec f = next;
+            if (i + T < cnt) next = load_fix(fix_hi, fix_lo, list[i + T]);
+            if (i < cnt)
+                fix_monopole(f, rec64, list[i], body, K, e2, x, y, z, me, eps2, acx, acy, acz);
+        }
+        ord += cnt;
+        __syncwarp();
+    }
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) {
+        acx += __shfl_xor_sync(0xffffffffu, acx, o);
+        acy += __shfl_xor_sync(0xffffffffu, acy, o);
+        acz += __shfl_xor_sync(0xffffffffu, acz, o);
+    }
+    if (valid && j == 0) {
+        ax[me] = acx * G;
+        ay[me] = acy * G;
+        az[me] = acz * G;
+        walk_len[me] = ord;
+    }
+}
+
 // Walk order of the next per-body traversal: within each window of RG_WINDOW sorted positions
 // (bodies close together in the tree), the bodies by decreasing length of their last walk (ties
 // by position), so that the 32 lanes of a warp walk sequences of similar length and fewer lanes
 // sit idle while the FP64 monopoles of the others run (a warp instruction costs the FP64 pipe the
 // same however few lanes are active). Bitonic sort of (length, position) keys in shared memory.
-constexpr int RG_WINDOW = 1024;
+constexpr int RG_WINDOW = 512;
 
 __global__ void __launch_bounds__(RG_WINDOW)
 regroup_kernel(const uint32_t* __restrict__ ids, const uint32_t* __restrict__ walk_len, uint32_t n,
@@ -616,20 +898,34 @@ bh_count_kernel(const NodeRec64* __restrict__ rec, const uint32_t* __restrict__ 
 // walk (bh_theta_f64_kernel). Both produce identical results; the switch exists for comparison.
 int g_lockstep = 0;
 
-// Resident blocks per SM of the two lane-kernel instantiations (queried once, before any
-// stream capture uses them).
+// Resident blocks per SM of the persistent kernels (queried once, before any stream capture uses
+// them): the IEEE lane kernel, the fixed-point kernel.
 int g_lane_per_sm[2] = {0, 0};
 
-template <int MODE>
-nb_status lane_per_sm(int* out) {
-    int& ps = g_lane_per_sm[MODE == IEEE64 ? 0 : 1];
+nb_status lane_per_sm(bool ieee, int* out) {
+    int& ps = g_lane_per_sm[ieee ? 0 : 1];
     if (ps == 0) {
-        NB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, bh_theta_lane_kernel<MODE>,
-                                                                  TR_THREADS, 0));
+        NB_CUDA_TRY(ieee ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, bh_theta_lane_kernel,
+                                                                         TR_THREADS, 0)
+                         : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, bh_theta_fix_kernel,
+                                                                         TR_THREADS, 0));
         if (ps < 1) ps = 1;
     }
     *out = ps;
     return NB_OK;
+}
+
+// Lanes per body of the NB_F64 traversal: the largest power of two that keeps the launch within
+// TEAM_LANES_PER_SM lanes per SM. Beyond one wave of resident warps (768 lanes per SM) every extra
+// lane only adds walk work; measured on the 152-SM part the fastest T is 32 up to 2,000 bodies, 16
+// at 4,000, 8 at 8,000, 4 at 16,411, 2 at 32,768 and 1 at 65,536 (disc theta 0.5 and 1.05,
+// Plummer 0.7), next to which half or twice the T is 2 to 25% slower.
+constexpr long long TEAM_LANES_PER_SM = 480;
+
+int team_lanes(const nb_ctx* ctx, uint32_t n) {
+    int t = 32;
+    while (t > 1 && (long long)n * t > TEAM_LANES_PER_SM * ctx->sm_count) t >>= 1;
+    return t;
 }
 
 // The walk lengths of the last per-body traversal of the same bodies order this one's groups
@@ -652,22 +948,51 @@ nb_status walk_order(const nb_bh_tree* t, cudaStream_t s, const uint32_t** order
 // 1,048,576 bodies than 40, 0.2% faster than 24 or 16).
 constexpr int LANE_BLOCKS_PER_SM = 5;
 
-template <int MODE>
-nb_status launch_lane(nb_ctx* ctx, const nb_bh_tree* t, const double* x, const double* y,
-                      const double* z, double* ax, double* ay, double* az, double G, double eps2,
-                      cudaStream_t s) {
+nb_status launch_lane(nb_ctx* ctx, const nb_bh_tree* t, bool ieee, const double* x,
+                      const double* y, const double* z, double* ax, double* ay, double* az,
+                      double G, double eps2, cudaStream_t s) {
     int ps = 0;
-    NB_TRY(lane_per_sm<MODE>(&ps));
-    ps = std::min(ps, LANE_BLOCKS_PER_SM);
+    NB_TRY(lane_per_sm(ieee, &ps));
+    if (ieee) ps = std::min(ps, LANE_BLOCKS_PER_SM);
     int grid = nb::ceil_div(t->n, TR_THREADS);
     if (grid > ctx->sm_count * ps) grid = ctx->sm_count * ps;
     NB_CUDA_TRY(cudaMemsetAsync(t->work + 1, 0, sizeof(uint32_t), s));
     const uint32_t* order = nullptr;
     NB_TRY(walk_order(t, s, &order));
-    bh_theta_lane_kernel<MODE><<<grid, TR_THREADS, 0, s>>>(
-        t->rec32, t->rec64, t->info, t->ids, x, y, z, t->box, t->n, t->params.theta, eps2, G, ax,
-        ay, az, t->work + 1, order, t->walk_len);
-    NB_TRY(nb::check_launch(MODE == IEEE64 ? "bh_theta_lane_kernel<ieee>" : "bh_theta_lane_kernel"));
+    if (ieee)
+        bh_theta_lane_kernel<<<grid, TR_THREADS, 0, s>>>(
+            t->rec32, t->rec64, t->info, t->ids, x, y, z, t->box, t->n, t->params.theta, eps2, G,
+            ax, ay, az, t->work + 1, order, t->walk_len);
+    else
+        bh_theta_fix_kernel<<<grid, TR_THREADS, 0, s>>>(
+            t->rec32, t->rec64, t->fix_hi, t->fix_lo, t->info, t->ids, x, y, z, t->box, t->n,
+            t->params.theta, eps2, G, ax, ay, az, t->work + 1, order, t->walk_len);
+    NB_TRY(nb::check_launch(ieee ? "bh_theta_lane_kernel" : "bh_theta_fix_kernel"));
+    t->walk_n = t->n;
+    return NB_OK;
+}
+
+// NB_F64 under the per-body rule: teams of lanes for small systems (in tree order: neighbouring
+// bodies share their windows' loads), one lane per body otherwise.
+nb_status launch_f64(nb_ctx* ctx, const nb_bh_tree* t, const double* x, const double* y,
+                     const double* z, double* ax, double* ay, double* az, double G, double eps2,
+                     cudaStream_t s) {
+    const int team = team_lanes(ctx, t->n);
+    if (team == 1) return launch_lane(ctx, t, false, x, y, z, ax, ay, az, G, eps2, s);
+    const int grid = nb::ceil_div((long long)t->n * team, TR_THREADS);
+    auto go = [&](auto kernel) {
+        kernel<<<grid, TR_THREADS, 0, s>>>(t->rec32, t->rec64, t->fix_hi, t->fix_lo, t->info,
+                                           t->ids, x, y, z, t->box, t->n, t->params.theta, eps2, G,
+                                           ax, ay, az, t->walk_len);
+    };
+    switch (team) {
+        case 2: go(bh_theta_team_kernel<2>); break;
+        case 4: go(bh_theta_team_kernel<4>); break;
+        case 8: go(bh_theta_team_kernel<8>); break;
+        case 16: go(bh_theta_team_kernel<16>); break;
+        default: go(bh_theta_team_kernel<32>); break;
+    }
+    NB_TRY(nb::check_launch("bh_theta_team_kernel"));
     t->walk_n = t->n;
     return NB_OK;
 }
@@ -700,24 +1025,27 @@ nb_status nb_bh_accel(nb_ctx* ctx, const nb_bh_tree* t, const double* x, const d
     const uint32_t n = t->n;
     const int grid = nb::ceil_div(n, TR_THREADS);
     const double theta = t->params.theta;
+    const int team = team_lanes(ctx, n);
     if (opening == NB_OPEN_THETA) {
         switch (prec) {
             case NB_F64_IEEE:
                 NB_TRY(nb_need_records(t, NB_REC_FP64, "nb_bh_accel"));
                 if (g_lockstep) {
                     bh_theta_f64_kernel<IEEE64><<<grid, TR_THREADS, 0, s>>>(
-                        t->rec64, t->info, t->ids, x, y, z, n, theta, eps2, G, ax, ay, az);
+                        t->rec64, t->fix_hi, t->fix_lo, t->info, t->ids, x, y, z, t->box, n, theta,
+                        eps2, G, team, ax, ay, az);
                     return nb::check_launch("bh_theta_f64_kernel<ieee>");
                 }
-                return launch_lane<IEEE64>(ctx, t, x, y, z, ax, ay, az, G, eps2, s);
+                return launch_lane(ctx, t, true, x, y, z, ax, ay, az, G, eps2, s);
             case NB_F64:
                 NB_TRY(nb_need_records(t, NB_REC_FP64, "nb_bh_accel"));
                 if (g_lockstep) {
                     bh_theta_f64_kernel<FAST64><<<grid, TR_THREADS, 0, s>>>(
-                        t->rec64, t->info, t->ids, x, y, z, n, theta, eps2, G, ax, ay, az);
+                        t->rec64, t->fix_hi, t->fix_lo, t->info, t->ids, x, y, z, t->box, n, theta,
+                        eps2, G, team, ax, ay, az);
                     return nb::check_launch("bh_theta_f64_kernel");
                 }
-                return launch_lane<FAST64>(ctx, t, x, y, z, ax, ay, az, G, eps2, s);
+                return launch_f64(ctx, t, x, y, z, ax, ay, az, G, eps2, s);
             case NB_DF64:
                 NB_TRY(nb_need_records(t, NB_REC_FP64 | NB_REC_DF, "nb_bh_accel"));
                 if (t->G == 0)
@@ -814,8 +1142,8 @@ nb_status nb_bh_graph_create(nb_ctx* ctx, nb_bh_tree* t, const double* m, double
         return nb::set_error(NB_ERR_INVALID_ARG, "nb_bh_graph_create: phase timing is on");
     *out = nullptr;
     int ps = 0;  // one-time queries happen here, outside the capture
-    NB_TRY(lane_per_sm<IEEE64>(&ps));
-    NB_TRY(lane_per_sm<FAST64>(&ps));
+    NB_TRY(lane_per_sm(true, &ps));
+    NB_TRY(lane_per_sm(false, &ps));
     NB_TRY(nb::learned_per_sm(&ps));
     cudaStream_t s;
     NB_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));

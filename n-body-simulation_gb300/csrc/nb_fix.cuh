@@ -1,0 +1,391 @@
+// nb_fix.cuh -- FP64-accurate pair arithmetic on the integer pipes.
+//
+// This part runs an FP64 instruction 75 times slower than an FP32 one (1.67 lanes per clock and SM
+// measured, against 64 for 32-bit integer operations and 32 for 32 x 32 -> 64-bit multiply-adds),
+// so a pair's separation, r^2 + eps^2 and m r^-3 are computed in fixed point and only the sums
+// (one DFMA per axis) stay on the FP64 pipe.
+//
+//  * Coordinates: 96-bit two's complement multiples of 2^(K - 93), K chosen so that every
+//    coordinate is below 2^K. A double above 2^(K - 40) is represented exactly, a smaller one to
+//    2^(K - 94).
+//  * A pair: the three exact differences are shifted left by a common `sh` until the largest has
+//    its top bit in place; r^2 + eps^2 as a 64-bit integer D in [2^60, 2^64) (relative error below
+//    2^-57); r^-3 from the MUFU estimate Y of D^(-1/2), the exact residual e = 1 - D Y^2 and
+//    Y^3 (1 + 3e/2 + 15e^2/8) (the binomial series; |e| < 2^-20, dropped terms below 2^-60),
+//    times the mass's 53 bits, rounded once to a double (relative error below 2^-53 + 2^-55).
+//  * What the integers cannot hold is left to the caller's FP64 expressions: a pair closer than
+//    2^(K - 30), masses that are not positive normal numbers, coordinates outside 2^K, scales
+//    beyond the exponent range, eps^2 too large for the scale.
+//
+// Everything up to the device-only part also compiles as plain C++, for the CPU tests.
+#pragma once
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#ifdef __CUDACC__
+#define NB_FIX_FN __host__ __device__ __forceinline__
+#else
+#define NB_FIX_FN inline
+#endif
+#ifdef __CUDA_ARCH__
+#define NB_FIX_DEV 1
+#else
+#define NB_FIX_DEV 0
+#endif
+
+namespace nbfix {
+
+constexpr int NO_EXP = INT32_MIN;   // FixRec::e of a source the FP64 expressions must handle
+constexpr int K_MAX = 300;          // |K| beyond this: FP64 expressions for everything
+constexpr int SH_MAX = 30;          // largest common shift
+
+// A source: coordinate words (most significant first), the mass's mantissa (64 bits, top bit set)
+// and its biased exponent - 3 K.
+struct alignas(16) FixRec {
+    uint32_t x2, y2, z2, mh;
+    uint32_t x1, y1, z1, ml;
+    uint32_t x0, y0, z0;
+    int e;
+};
+
+// The same as it is stored: a 32-byte half (one load) and a 16-byte half {x0, y0, z0, ml}.
+struct alignas(32) FixHi {
+    uint32_t x2, y2, z2, mh, x1, y1, z1;
+    int e;
+};
+
+struct Fix3 {
+    uint32_t x2, y2, z2, x1, y1, z1, x0, y0, z0;
+};
+
+NB_FIX_FN uint64_t bits_of(double v) {
+#if NB_FIX_DEV
+    return (uint64_t)__double_as_longlong(v);
+#else
+    uint64_t u;
+    std::memcpy(&u, &v, 8);
+    return u;
+#endif
+}
+NB_FIX_FN double double_of(uint32_t hi, uint32_t lo) {
+#if NB_FIX_DEV
+    return __hiloint2double((int)hi, (int)lo);
+#else
+    const uint64_t u = ((uint64_t)hi << 32) | lo;
+    double v;
+    std::memcpy(&v, &u, 8);
+    return v;
+#endif
+}
+// the high word of (hi:lo) << (s & 31)
+NB_FIX_FN uint32_t fsl(uint32_t lo, uint32_t hi, uint32_t s) {
+#if NB_FIX_DEV
+    return __funnelshift_l(lo, hi, s);
+#else
+    s &= 31;
+    return s ? (hi << s) | (lo >> (32 - s)) : hi;
+#endif
+}
+NB_FIX_FN int clz32(uint32_t v) {
+#if NB_FIX_DEV
+    return __clz((int)v);
+#else
+    return v ? __builtin_clz(v) : 32;
+#endif
+}
+NB_FIX_FN float rsqrt_est(float v) {
+#if NB_FIX_DEV
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
+    return y;
+#else
+    return 1.0f / sqrtf(v);
+#endif
+}
+// a - b over three words
+NB_FIX_FN void sub96(uint32_t a2, uint32_t a1, uint32_t a0, uint32_t b2, uint32_t b1, uint32_t b0,
+                     uint32_t& d2, uint32_t& d1, uint32_t& d0) {
+#if NB_FIX_DEV
+    asm("sub.cc.u32 %0, %3, %6;\n\tsubc.cc.u32 %1, %4, %7;\n\tsubc.u32 %2, %5, %8;"
+        : "=r"(d0), "=r"(d1), "=r"(d2)
+        : "r"(a0), "r"(a1), "r"(a2), "r"(b0), "r"(b1), "r"(b2));
+#else
+    const uint64_t l = (uint64_t)a0 - b0;
+    const uint64_t m = (uint64_t)a1 - b1 - (l >> 63);
+    d0 = (uint32_t)l;
+    d1 = (uint32_t)m;
+    d2 = a2 - b2 - (uint32_t)(m >> 63);
+#endif
+}
+
+// K of a set of coordinates: the smallest with every |v| below 2^K (v_max = the largest |v|).
+// Outside +-K_MAX the scale is unusable.
+NB_FIX_FN int k_of(double v_max) { return (int)((bits_of(v_max) >> 52) & 0x7ff) - 1022; }
+NB_FIX_FN bool k_usable(int K) { return K >= -K_MAX && K <= K_MAX; }
+
+// The words of v as a multiple of 2^(K - 93) (rounded to nearest where v has lower bits); false
+// when v is not finite or beyond 2^K.
+NB_FIX_FN bool split96(double v, int K, uint32_t& w2, uint32_t& w1, uint32_t& w0) {
+    const uint64_t u = bits_of(v);
+    const int be = (int)((u >> 52) & 0x7ff);
+    const uint64_t frac = u & 0xfffffffffffffull;
+    const int s = be - 982 - K;  // v = mantissa * 2^(be - 1075) = mantissa * 2^s units
+    w2 = w1 = w0 = 0;
+    if (be == 0 || s < -53) return be != 0x7ff;
+    if (be == 0x7ff || s > 41 || (s == 41 && frac != 0)) return false;
+    const uint64_t mant = frac | (1ull << 52);
+    uint64_t lo, hi;  // 96 bits: hi = bits 32.., lo = bits 0..31
+    if (s >= 32) {
+        lo = 0;
+        hi = mant << (s - 32);
+    } else if (s >= 0) {
+        lo = (mant << s) & 0xffffffffull;
+        hi = mant >> (32 - s);
+    } else {
+        const uint64_t r = (mant + (1ull << (-s - 1))) >> -s;
+        lo = r & 0xffffffffull;
+        hi = r >> 32;
+    }
+    w0 = (uint32_t)lo;
+    w1 = (uint32_t)hi;
+    w2 = (uint32_t)(hi >> 32);
+    if (u >> 63) {  // two's complement
+        w0 = ~w0 + 1u;
+        w1 = ~w1 + (w0 == 0);
+        w2 = ~w2 + (w0 == 0 && w1 == 0);
+    }
+    return true;
+}
+
+NB_FIX_FN bool split3(double x, double y, double z, int K, Fix3& f) {
+    const bool a = split96(x, K, f.x2, f.x1, f.x0);
+    const bool b = split96(y, K, f.y2, f.y1, f.y0);
+    const bool c = split96(z, K, f.z2, f.z1, f.z0);
+    return a && b && c && k_usable(K);
+}
+
+// The mantissa and exponent of a mass; false when it is not a positive normal number.
+NB_FIX_FN bool split_mass(double m, uint32_t& mh, uint32_t& ml, int& biased) {
+    const uint64_t u = bits_of(m);
+    biased = (int)(u >> 52);
+    const uint64_t mant = (u << 11) | (1ull << 63);
+    mh = (uint32_t)(mant >> 32);
+    ml = (uint32_t)mant;
+    return biased >= 1 && biased < 0x7ff;
+}
+
+NB_FIX_FN FixRec make_rec(double x, double y, double z, double m, int K) {
+    FixRec r;
+    Fix3 f;
+    int be;
+    const bool ok = split3(x, y, z, K, f);
+    const bool mk = split_mass(m, r.mh, r.ml, be);
+    r.x2 = f.x2;
+    r.y2 = f.y2;
+    r.z2 = f.z2;
+    r.x1 = f.x1;
+    r.y1 = f.y1;
+    r.z1 = f.z1;
+    r.x0 = f.x0;
+    r.y0 = f.y0;
+    r.z0 = f.z0;
+    r.e = ok && mk ? be - 3 * K : NO_EXP;
+    return r;
+}
+
+// eps^2 in units of D at shift sh: D counts 4^(K - 29 - sh).
+NB_FIX_FN double eps2_units(double eps2, int K, int sh) {
+#if NB_FIX_DEV
+    return scalbn(eps2, 2 * (sh + 29 - K));
+#else
+    return std::scalbn(eps2, 2 * (sh + 29 - K));
+#endif
+}
+constexpr double EPS2_LIMIT = 4611686018427387904.0;  // 2^62: eps^2 in units of D stays below
+
+// A pair's separation, shifted: words (most significant first) of dx, dy, dz and the shift.
+struct Sep {
+    uint32_t xh, yh, zh, xl, yl, zl, xe, ye, ze;
+    int sh;
+};
+
+// c - p, normalised; false when the pair is too close for the integers (the caller's FP64
+// expressions then).
+NB_FIX_FN bool separation(const Fix3& c, const Fix3& p, int sh_max, Sep& s) {
+    uint32_t x2, x1, x0, y2, y1, y0, z2, z1, z0;
+    sub96(c.x2, c.x1, c.x0, p.x2, p.x1, p.x0, x2, x1, x0);
+    sub96(c.y2, c.y1, c.y0, p.y2, p.y1, p.y0, y2, y1, y0);
+    sub96(c.z2, c.z1, c.z0, p.z2, p.z1, p.z0, z2, z1, z0);
+    const uint32_t t = (x2 ^ (uint32_t)((int)x2 >> 31)) | (y2 ^ (uint32_t)((int)y2 >> 31)) |
+                       (z2 ^ (uint32_t)((int)z2 >> 31));
+    const int n = clz32(t) - 1;
+    const int sh = n < sh_max ? n : sh_max;
+    s.sh = sh;
+    s.xh = fsl(x1, x2, sh);
+    s.yh = fsl(y1, y2, sh);
+    s.zh = fsl(z1, z2, sh);
+    s.xl = fsl(x0, x1, sh);
+    s.yl = fsl(y0, y1, sh);
+    s.zl = fsl(z0, z1, sh);
+    s.xe = x0 << sh;
+    s.ye = y0 << sh;
+    s.ze = z0 << sh;
+    return t != 0;
+}
+
+// r^2 in units 4^(K - 29 - sh): the high 64 bits of the squares' sum.
+NB_FIX_FN uint64_t norm2(const Sep& s) {
+    const int xh = (int)s.xh, yh = (int)s.yh, zh = (int)s.zh;
+    int64_t r = (int64_t)xh * xh;
+    int64_t q = (int64_t)xh * (int)(s.xl >> 2);
+    r = (int64_t)((uint64_t)r + (uint64_t)((int64_t)yh * yh));
+    q += (int64_t)yh * (int)(s.yl >> 2);
+    r = (int64_t)((uint64_t)r + (uint64_t)((int64_t)zh * zh));
+    q += (int64_t)zh * (int)(s.zl >> 2);
+    return (uint64_t)r + (uint64_t)(q >> 29);
+}
+
+// Y ~ 2^61 D^(-1/2) and the residual e = 1 - D Y^2 / 2^122 in units 2^-58; W = Y^2.
+NB_FIX_FN int64_t rsqrt_residual(uint64_t D, uint32_t& Y, uint64_t& W) {
+    const uint32_t dh = (uint32_t)(D >> 32), dl = (uint32_t)D;
+    const float y0 = rsqrt_est((float)dh) * 35184372088832.0f;  // 2^45
+#if NB_FIX_DEV
+    Y = __float2uint_rz(y0);
+#else
+    Y = (uint32_t)y0;
+#endif
+    W = (uint64_t)Y * Y;
+    const uint32_t wh = (uint32_t)(W >> 32), wl = (uint32_t)W;
+    const uint64_t u = (((uint64_t)dl * wh) >> 32) + (((uint64_t)dh * wl) >> 32);
+    return (int64_t)((1ull << 58) - ((uint64_t)dh * wh + u));
+}
+
+// a (c / 2^58) for |c| < 2^38 and a < 2^61: the correction term of a (1 + c).
+NB_FIX_FN uint64_t scaled(uint64_t a, int64_t c) {
+    const int64_t c6 = (int64_t)((uint64_t)c << 6);
+    const int ch = (int)(c6 >> 32);
+    const uint32_t cl = (uint32_t)c6, ah = (uint32_t)(a >> 32), al = (uint32_t)a;
+    const uint64_t u = (uint64_t)ah * cl;
+    int64_t v = (int64_t)ch * (int)(al >> 1);
+    v = (v >> 31) + (int64_t)(u >> 32);
+    return (uint64_t)((int64_t)ch * (int)ah + v);
+}
+
+// D^(-3/2) 2^151 (64-bit, between 2^55 and 2^61)
+NB_FIX_FN uint64_t rinv3(uint64_t D) {
+    uint32_t Y;
+    uint64_t W;
+    const int64_t e = rsqrt_residual(D, Y, W);
+    // c = 3e/2 + 15e^2/8 in units 2^-58; e^2 from e's upper bits
+    const int eh = (int)(e >> 8);
+    const uint32_t q = (uint32_t)((uint64_t)((int64_t)eh * eh) >> 32);  // e^2 in units 2^-68
+    const int64_t c = e + (e >> 1) + (int64_t)((q * 15u) >> 13);
+    const uint64_t v = (uint64_t)(uint32_t)W * Y;
+    const uint64_t V = (uint64_t)(uint32_t)(W >> 32) * Y + (v >> 32);
+    return V + scaled(V, c);
+}
+
+// D^(-1/2) 2^90 (64-bit, between 2^58 and 2^60)
+NB_FIX_FN uint64_t rinv1(uint64_t D) {
+    uint32_t Y;
+    uint64_t W;
+    const int64_t e = rsqrt_residual(D, Y, W);
+    const int eh = (int)(e >> 8);
+    const uint32_t q = (uint32_t)((uint64_t)((int64_t)eh * eh) >> 32);
+    const int64_t c = (e >> 1) + (int64_t)((q * 3u) >> 13);
+    const uint64_t V = (uint64_t)Y << 29;
+    return V + scaled(V, c);
+}
+
+// A 64-bit integer v > 0 as a double scaled so that 2^64 would have the biased exponent `be`,
+// rounded to nearest.
+NB_FIX_FN double scaled_double(uint64_t v, int be) {
+    const uint32_t vh = (uint32_t)(v >> 32), vl = (uint32_t)v;
+    const int n = clz32(vh);
+    const uint32_t h = fsl(vl, vh, n), l = vl << n;
+    const uint32_t r = (l >> 10) & 1u;
+    uint64_t o = ((uint64_t)((((uint32_t)(be - n - 1)) << 20) + (h >> 11)) << 32) |
+                 ((h << 21) | (l >> 11));
+    o += r;
+    return double_of((uint32_t)(o >> 32), (uint32_t)o);
+}
+
+// m D^(-3/2) for a source's mass and exponent word: the double; `ok` false when its exponent
+// leaves the normal range.
+NB_FIX_FN double mass_rinv3(uint64_t S, uint32_t mh, uint32_t ml, int e, int sh, bool& ok) {
+    const uint32_t s_h = (uint32_t)(S >> 32), s_l = (uint32_t)S;
+    const uint64_t u = (((uint64_t)s_l * mh) >> 32) + (((uint64_t)s_h * ml) >> 32);
+    const uint64_t F = (uint64_t)s_h * mh + u;
+    const int be = e + 3 * sh;  // exponent of 2^64; F is below 2^61 and above 2^53
+    ok = (uint32_t)(be - 16) < 2016u;
+    return scaled_double(F, be);
+}
+
+// One axis of the separation as a double (its sign and top 53 bits). base = 1025 + K - sh. The
+// magnitude is the complement of a negative value, one unit of the last word short, which is below
+// 2^-64 of it as long as the first word is not 0; the rest (a component below 2^-30 of the
+// distance or of eps) is negated exactly.
+NB_FIX_FN double axis(uint32_t vh, uint32_t vl, uint32_t ve, int base) {
+    const uint32_t s = (uint32_t)((int)vh >> 31);
+    uint32_t h = vh ^ s, l = vl ^ s, x = ve ^ s;
+    if (h == 0) {
+        const uint64_t v = (((uint64_t)l << 32) | x) + (s & 1u);
+        if (v == 0) {
+            if (s == 0) return 0.0;
+            h = 1;  // -2^64 units
+            l = 0;
+        } else {
+            h = (uint32_t)(v >> 32);
+            l = (uint32_t)v;
+            base -= 32;
+            if (h == 0) {
+                h = l;
+                l = 0;
+                base -= 32;
+            }
+        }
+        x = 0;
+    }
+    const int n = clz32(h);
+    const uint32_t mh = fsl(l, h, n), ml = fsl(x, l, n);
+    const uint32_t hi = ((uint32_t)(base - n - 1) << 20) + (mh >> 11);
+    return double_of(hi | (s & 0x80000000u), (mh << 21) | (ml >> 11));
+}
+
+#ifdef __CUDACC__
+// eps^2 per shift, filled by one warp of a block (the caller's __syncthreads() follows).
+struct Eps2Table {
+    uint64_t units[32];
+    int sh_max;  // -1: the FP64 expressions for every pair
+};
+__device__ __forceinline__ void fill_eps2(Eps2Table& t, double eps2, int K) {
+    if (threadIdx.x >= 32) return;
+    const int sh = (int)threadIdx.x;
+    const double u = sh <= SH_MAX && k_usable(K) ? eps2_units(eps2, K, sh) : -1.0;
+    const bool fits = u >= 0.0 && u < EPS2_LIMIT;
+    t.units[sh] = fits ? __double2ull_rn(u) : 0;
+    const uint32_t b = __ballot_sync(0xffffffffu, fits);  // a run from bit 0
+    if (sh == 0) t.sh_max = __clz((int)~__brev(b)) - 1;
+}
+
+// Factor w = m (r^2 + eps^2)^(-3/2) and separation of a source seen from p: every sum is
+// fma(w, d, sum). False when the caller has to evaluate the pair in FP64.
+__device__ __forceinline__ bool term(const FixRec& f, const Fix3& p, int K, const Eps2Table& t,
+                                     int sh_max, double& w, double& dx, double& dy, double& dz) {
+    if (f.e == NO_EXP) return false;
+    const Fix3 c{f.x2, f.y2, f.z2, f.x1, f.y1, f.z1, f.x0, f.y0, f.z0};
+    Sep s;
+    if (!separation(c, p, sh_max, s)) return false;
+    const uint64_t D = norm2(s) + t.units[s.sh];
+    bool ok;
+    w = mass_rinv3(rinv3(D), f.mh, f.ml, f.e, s.sh, ok);
+    const int base = 1025 + K - s.sh;
+    dx = axis(s.xh, s.xl, s.xe, base);
+    dy = axis(s.yh, s.yl, s.ye, base);
+    dz = axis(s.zh, s.zl, s.ze, base);
+    return ok;
+}
+#endif
+
+}  // namespace nbfix

@@ -1,0 +1,108 @@
+"""NB_F64 Barnes-Hut with fixed-point monopoles (bh_theta_fix_kernel, bh_theta_team_kernel) against
+the FP64 IEEE traversal of the same tree, which accepts the same cells. Tolerance: the factor and
+the separation of each term are within 2^-52 of exact, a body's FP64 sum of A terms within
+A 2^-53 of their absolute sum; against the sum of the terms' magnitudes (bounded below by |a|) the
+IEEE traversal is within (A + 4) 2^-53 and NB_F64 within (A + 2) 2^-53, so bodies with no
+cancellation agree to 2 A 2^-52; 1e-12 per body covers A = 2,000 with cancellation by 2."""
+
+import numpy as np
+import pytest
+
+from helpers import bodies, dev, host, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from nbody.lib import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def both(ctx, d, theta, eps2, targets=None):
+    import torch
+    from nbody.lib import BHTree
+    n = len(d["m"])
+    t = {k: dev(d[k]) for k in ("m", "x", "y", "z")}
+    tree = BHTree(ctx, n, theta=theta)
+    tree.build(t["m"], t["x"], t["y"], t["z"], d["G"])
+    pos = targets or [t["x"], t["y"], t["z"]]
+    out = {}
+    for prec in ("f64_ieee", "f64", "f64"):  # the second NB_F64 call in the order of the first
+        a = [torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(3)]
+        tree.accel(*pos, *a, d["G"], eps2, "theta", prec)
+        ctx.sync()
+        a = [host(v) for v in a]
+        if prec in out:
+            for u, v in zip(a, out[prec]):
+                np.testing.assert_array_equal(u, v)
+        out[prec] = a
+    tree.close()
+    return out["f64"], out["f64_ieee"]
+
+
+# one, two and ragged bodies; either side of each lanes-per-body boundary of a 152-SM part
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 2280, 2281, 4560, 4561, 9120, 9121, 18240, 18241,
+                               36480, 36481, 72960, 72961])
+def test_sizes(ctx, n):
+    d = bodies("plummer", n, seed=n)
+    got, ref = both(ctx, d, 0.8, 1e-6)
+    if n > 1:
+        assert rel_err(*got, *ref).max() <= 1e-12
+    else:
+        assert all((g == 0).all() for g in got)
+
+
+@pytest.mark.parametrize("theta", [0.0, 0.4, 1.05])
+@pytest.mark.parametrize("eps2", [0.0, 1e-22, 1e-3, 1e6])
+def test_options(ctx, theta, eps2):
+    d = bodies("disc", 1500, seed=3)
+    got, ref = both(ctx, d, theta, eps2)
+    assert rel_err(*got, *ref).max() <= 1e-12
+
+
+@pytest.mark.parametrize("scale", [1e-120, 1e-30, 1e30, 1e120])
+def test_scales(ctx, scale):
+    """Boxes inside and outside the fixed point's exponent range."""
+    d = bodies("plummer", 600, seed=4)
+    for k in ("x", "y", "z"):
+        d[k] = d[k] * scale
+    d["m"] = d["m"] * (scale if scale > 1 else 1.0)
+    with np.errstate(all="ignore"):
+        got, ref = both(ctx, d, 0.7, 0.0)
+    fine = np.isfinite(ref[0])
+    assert np.array_equal(fine, np.isfinite(got[0]))
+    if fine.all() and np.abs(ref[0]).max() > 0:
+        assert rel_err(*got, *ref).max() <= 1e-12
+
+
+def test_close_pairs_and_masses(ctx):
+    """Pairs below the fixed point's resolution (but above the 42-level tree's), massless bodies, masses beyond its range, a thin
+    sheet (components far below the distance)."""
+    d = bodies("plummer", 3000, seed=5)
+    rng = np.random.default_rng(1)
+    for k in ("x", "y", "z"):
+        d[k][1::4] = d[k][0::4] + rng.choice((-1, 1), 750) * 10.0 ** rng.uniform(-10, -7, 750)
+    d["m"][5::50] = 0.0
+    d["m"][7::50] = 1e-310
+    d["z"][2::4] *= 1e-9
+    got, ref = both(ctx, d, 0.6, 0.0)
+    assert rel_err(*got, *ref).max() <= 1e-12
+
+
+def test_targets_outside_the_box(ctx):
+    d = bodies("plummer", 700, seed=6)
+    shifted = [dev(d["x"] + 100.0), dev(d["y"] * 3.0), dev(d["z"] - 1e5)]
+    got, ref = both(ctx, d, 0.6, 1e-6, shifted)
+    assert rel_err(*got, *ref).max() <= 1e-12
+
+
+def test_thin_disc_component(ctx):
+    """The small component of a sheet keeps its own relative accuracy."""
+    d = bodies("plummer", 2000, seed=7)
+    d["z"] = d["z"] * 1e-7
+    got, ref = both(ctx, d, 0.5, 0.0)
+    scale = np.sqrt((ref[2] ** 2).mean())
+    assert np.sqrt(((got[2] - ref[2]) ** 2).mean()) <= 1e-13 * scale
