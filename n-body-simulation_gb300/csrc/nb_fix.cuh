@@ -298,7 +298,7 @@ NB_FIX_FN uint64_t rinv1(uint64_t D) {
     return V + scaled(V, c);
 }
 
-// A 64-bit integer v > 0 as a double scaled so that 2^64 would have the biased exponent `be`,
+// A 64-bit integer v > 0 as a double scaled so that 2^63 has the biased exponent `be`,
 // rounded to nearest.
 NB_FIX_FN double scaled_double(uint64_t v, int be) {
     const uint32_t vh = (uint32_t)(v >> 32), vl = (uint32_t)v;
@@ -317,7 +317,7 @@ NB_FIX_FN double mass_rinv3(uint64_t S, uint32_t mh, uint32_t ml, int e, int sh,
     const uint32_t s_h = (uint32_t)(S >> 32), s_l = (uint32_t)S;
     const uint64_t u = (((uint64_t)s_l * mh) >> 32) + (((uint64_t)s_h * ml) >> 32);
     const uint64_t F = (uint64_t)s_h * mh + u;
-    const int be = e + 3 * sh;  // exponent of 2^64; F is below 2^61 and above 2^53
+    const int be = e + 3 * sh;  // exponent of 2^63; F is below 2^61 and above 2^53
     ok = (uint32_t)(be - 16) < 2016u;
     return scaled_double(F, be);
 }

@@ -106,3 +106,30 @@ def test_thin_disc_component(ctx):
     got, ref = both(ctx, d, 0.5, 0.0)
     scale = np.sqrt((ref[2] ** 2).mean())
     assert np.sqrt(((got[2] - ref[2]) ** 2).mean()) <= 1e-13 * scale
+
+
+# -- energy: 1/r in fixed point -------------------------------------------------------------------
+# Each term is within 2^-52 of exact and all potential terms have one sign, so the sum of P terms
+# added in rows is within (rows + 2) 2^-53 of the oracle's, itself within P 2^-53 in the worst order:
+# 1e-12 of the larger of |kinetic| and |potential|.
+@pytest.mark.parametrize("kind,n,scale", [
+    ("plummer", 1, 1.0), ("plummer", 2, 1.0), ("plummer", 127, 1.0), ("plummer", 128, 1.0),
+    ("plummer", 129, 1.0), ("disc", 1000, 1.0), ("plummer", 2048, 1.0), ("plummer", 2049, 1.0),
+    ("disc", 6000, 1.0), ("plummer", 500, 1e-120), ("plummer", 500, 1e120)])
+def test_energy(ctx, kind, n, scale):
+    import oracle
+    import torch
+    d = bodies(kind, n, seed=n)
+    for k in ("x", "y", "z"):
+        d[k] = d[k] * scale
+    if n >= 500:  # pairs closer than the fixed point's resolution
+        d["x"][21::100], d["y"][21::100] = d["x"][20::100] * (1 + 1e-14), d["y"][20::100]
+        d["z"][21::100] = d["z"][20::100]
+    keys = ("m", "x", "y", "z", "vx", "vy", "vz")
+    out = torch.zeros(4, dtype=torch.float64, device="cuda")
+    ctx.energy(*[dev(d[k]) for k in keys], d["G"], out)
+    ctx.sync()
+    got = out.cpu().numpy()
+    o = oracle.energy(*[d[k] for k in keys], d["G"])
+    want = np.array([o["kinetic"], o["potential"], o["total"]])
+    assert np.all(np.abs(got[:3] - want) <= 1e-12 * np.abs(want[:2]).max()), (got, want)
