@@ -8,13 +8,14 @@
 //  * Coordinates: 96-bit two's complement multiples of 2^(K - 93), K chosen so that every
 //    coordinate is below 2^K. A double above 2^(K - 40) is represented exactly, a smaller one to
 //    2^(K - 94).
-//  * A pair: the three exact differences are shifted left by a common `sh` until the largest has
-//    its top bit in place; r^2 + eps^2 as a 64-bit integer D in [2^60, 2^64) (relative error below
-//    2^-57); r^-3 from the MUFU estimate Y of D^(-1/2), the exact residual e = 1 - D Y^2 and
-//    Y^3 (1 + 3e/2 + 15e^2/8) (the binomial series; |e| < 2^-20, dropped terms below 2^-60),
-//    times the mass's 53 bits, rounded once to a double (relative error below 2^-53 + 2^-55).
+//  * A pair: the three exact differences as magnitudes, shifted left by a common `sh` until the
+//    largest is in [2^29, 2^30) by its first word; r^2 + eps^2 as a 64-bit integer D in [2^60, 2^64)
+//    (truncation errors below 2^-55 of it, centred); r^-3 from an estimate Y of D^(-1/2) good to
+//    2^-28 (MUFU and one Newton step), its residual e = 1 - D Y^2, of which 32 bits remain, and
+//    Y^3 (1 + 3e/2) (dropped terms below 2^-55), times the mass's 53 bits, rounded once to a double.
+//    In all within 2^-52.2 of exact, root mean square 2^-54.2 (the final rounding alone: 2^-54.4).
 //  * What the integers cannot hold is left to the caller's FP64 expressions: a pair closer than
-//    2^(K - 30), masses that are not positive normal numbers, coordinates outside 2^K, scales
+//    2^(K - 29), masses that are not positive normal numbers, coordinates outside 2^K, scales
 //    beyond the exponent range, eps^2 too large for the scale.
 //
 // Everything up to the device-only part also compiles as plain C++, for the CPU tests.
@@ -38,7 +39,7 @@ namespace nbfix {
 
 constexpr int NO_EXP = INT32_MIN;   // FixRec::e of a source the FP64 expressions must handle
 constexpr int K_MAX = 300;          // |K| beyond this: FP64 expressions for everything
-constexpr int SH_MAX = 30;          // largest common shift
+constexpr int SH_MAX = 29;          // largest common shift
 
 // A source: coordinate words (most significant first), the mass's mantissa (64 bits, top bit set)
 // and its biased exponent - 3 K.
@@ -101,6 +102,21 @@ NB_FIX_FN float rsqrt_est(float v) {
     return y;
 #else
     return 1.0f / sqrtf(v);
+#endif
+}
+// the high word of a * b
+NB_FIX_FN uint32_t mul_hi(uint32_t a, uint32_t b) {
+#if NB_FIX_DEV
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+NB_FIX_FN int mul_hi(int a, int b) {
+#if NB_FIX_DEV
+    return __mulhi(a, b);
+#else
+    return (int)(((int64_t)a * b) >> 32);
 #endif
 }
 // a - b over three words
@@ -194,108 +210,96 @@ NB_FIX_FN FixRec make_rec(double x, double y, double z, double m, int K) {
     return r;
 }
 
-// eps^2 in units of D at shift sh: D counts 4^(K - 29 - sh).
+// eps^2 in units of D at shift sh: D counts 4^(K - 30 - sh).
 NB_FIX_FN double eps2_units(double eps2, int K, int sh) {
 #if NB_FIX_DEV
-    return scalbn(eps2, 2 * (sh + 29 - K));
+    return scalbn(eps2, 2 * (sh + 30 - K));
 #else
-    return std::scalbn(eps2, 2 * (sh + 29 - K));
+    return std::scalbn(eps2, 2 * (sh + 30 - K));
 #endif
 }
 constexpr double EPS2_LIMIT = 4611686018427387904.0;  // 2^62: eps^2 in units of D stays below
 
-// A pair's separation, shifted: words (most significant first) of dx, dy, dz and the shift.
+// A pair's separation: per axis the sign (0 or all ones), the magnitude shifted by sh (two words;
+// complements of negative values, one unit of the exact difference's last word short) and the
+// difference's unshifted last word.
 struct Sep {
-    uint32_t xh, yh, zh, xl, yl, zl, xe, ye, ze;
+    uint32_t xs, ys, zs, xh, yh, zh, xl, yl, zl, x0, y0, z0;
     int sh;
 };
 
 // c - p, normalised; false when the pair is too close for the integers (the caller's FP64
 // expressions then).
 NB_FIX_FN bool separation(const Fix3& c, const Fix3& p, int sh_max, Sep& s) {
-    uint32_t x2, x1, x0, y2, y1, y0, z2, z1, z0;
-    sub96(c.x2, c.x1, c.x0, p.x2, p.x1, p.x0, x2, x1, x0);
-    sub96(c.y2, c.y1, c.y0, p.y2, p.y1, p.y0, y2, y1, y0);
-    sub96(c.z2, c.z1, c.z0, p.z2, p.z1, p.z0, z2, z1, z0);
-    const uint32_t t = (x2 ^ (uint32_t)((int)x2 >> 31)) | (y2 ^ (uint32_t)((int)y2 >> 31)) |
-                       (z2 ^ (uint32_t)((int)z2 >> 31));
-    const int n = clz32(t) - 1;
+    uint32_t x2, x1, y2, y1, z2, z1;
+    sub96(c.x2, c.x1, c.x0, p.x2, p.x1, p.x0, x2, x1, s.x0);
+    sub96(c.y2, c.y1, c.y0, p.y2, p.y1, p.y0, y2, y1, s.y0);
+    sub96(c.z2, c.z1, c.z0, p.z2, p.z1, p.z0, z2, z1, s.z0);
+    s.xs = (uint32_t)((int)x2 >> 31);
+    s.ys = (uint32_t)((int)y2 >> 31);
+    s.zs = (uint32_t)((int)z2 >> 31);
+    const uint32_t t = (x2 ^ s.xs) | (y2 ^ s.ys) | (z2 ^ s.zs);  // below 2^30
+    const int n = clz32(t) - 2;
     const int sh = n < sh_max ? n : sh_max;
     s.sh = sh;
-    s.xh = fsl(x1, x2, sh);
-    s.yh = fsl(y1, y2, sh);
-    s.zh = fsl(z1, z2, sh);
-    s.xl = fsl(x0, x1, sh);
-    s.yl = fsl(y0, y1, sh);
-    s.zl = fsl(z0, z1, sh);
-    s.xe = x0 << sh;
-    s.ye = y0 << sh;
-    s.ze = z0 << sh;
+    s.xh = fsl(x1, x2, sh) ^ s.xs;
+    s.yh = fsl(y1, y2, sh) ^ s.ys;
+    s.zh = fsl(z1, z2, sh) ^ s.zs;
+    s.xl = fsl(s.x0, x1, sh) ^ s.xs;
+    s.yl = fsl(s.y0, y1, sh) ^ s.ys;
+    s.zl = fsl(s.z0, z1, sh) ^ s.zs;
     return t != 0;
 }
 
-// r^2 in units 4^(K - 29 - sh): the high 64 bits of the squares' sum.
+// Truncation of norm2 in its own units, on average: 4/3 per axis (the squares of the low words) and
+// 4 per axis (the halves of the cross products).
+constexpr uint32_t NORM2_BIAS = 16;
+
+// r^2 in units 4^(K - 30 - sh), truncated by 0 to 36 units: 4 times the squares of the first words
+// and 8 times their products with the second words.
 NB_FIX_FN uint64_t norm2(const Sep& s) {
-    const int xh = (int)s.xh, yh = (int)s.yh, zh = (int)s.zh;
-    int64_t r = (int64_t)xh * xh;
-    int64_t q = (int64_t)xh * (int)(s.xl >> 2);
-    r = (int64_t)((uint64_t)r + (uint64_t)((int64_t)yh * yh));
-    q += (int64_t)yh * (int)(s.yl >> 2);
-    r = (int64_t)((uint64_t)r + (uint64_t)((int64_t)zh * zh));
-    q += (int64_t)zh * (int)(s.zl >> 2);
-    return (uint64_t)r + (uint64_t)(q >> 29);
+    const uint64_t r = (uint64_t)s.xh * s.xh + (uint64_t)s.yh * s.yh + (uint64_t)s.zh * s.zh;
+    const uint32_t h = mul_hi(s.xh, s.xl) + mul_hi(s.yh, s.yl) + mul_hi(s.zh, s.zl);
+    return (r << 2) + ((uint64_t)h << 3);
 }
 
-// Y ~ 2^61 D^(-1/2) and the residual e = 1 - D Y^2 / 2^122 in units 2^-58; W = Y^2.
-NB_FIX_FN int64_t rsqrt_residual(uint64_t D, uint32_t& Y, uint64_t& W) {
+// Y ~ 2^61 D^(-1/2) to 2^-28 and e = 1 - D Y^2 / 2^122 in units 2^-58 (|e| < 2^31); W = Y^2.
+// D Y^2 is so near 2^122 that of its upper half only the low 32 bits are formed.
+NB_FIX_FN int rsqrt_residual(uint64_t D, uint32_t& Y, uint64_t& W) {
     const uint32_t dh = (uint32_t)(D >> 32), dl = (uint32_t)D;
-    const float y0 = rsqrt_est((float)dh) * 35184372088832.0f;  // 2^45
+    const float f = rsqrt_est((float)dh) * 35184372088832.0f;  // 2^45: at most 2^31
 #if NB_FIX_DEV
-    Y = __float2uint_rz(y0);
+    const int y0 = __float2int_rz(f);  // saturates
 #else
-    Y = (uint32_t)y0;
+    const int y0 = f < 2147483648.0f ? (int)f : 2147483647;
 #endif
+    // the estimate's own residual to 2^-31: D y0^2 / 2^64 = 2^58 (1 - e0), |e0| < 2^-20
+    const uint64_t w0 = (uint64_t)(uint32_t)y0 * (uint32_t)y0;
+    const uint64_t p = (uint64_t)dh * (uint32_t)(w0 >> 32) + mul_hi(dh, (uint32_t)w0);
+    const int ne0 = (int)(fsl((uint32_t)p, (uint32_t)(p >> 32), 5) ^ 0x80000000u);  // -e0 2^31
+    Y = (uint32_t)(y0 - (int)(((int64_t)y0 * ne0 + 0x80000000ll) >> 32));  // rounded
     W = (uint64_t)Y * Y;
     const uint32_t wh = (uint32_t)(W >> 32), wl = (uint32_t)W;
-    const uint64_t u = (((uint64_t)dl * wh) >> 32) + (((uint64_t)dh * wl) >> 32);
-    return (int64_t)((1ull << 58) - ((uint64_t)dh * wh + u));
+    return -(int)(dh * wh + mul_hi(dh, wl) + mul_hi(dl, wh) + 1u);
 }
 
-// a (c / 2^58) for |c| < 2^38 and a < 2^61: the correction term of a (1 + c).
-NB_FIX_FN uint64_t scaled(uint64_t a, int64_t c) {
-    const int64_t c6 = (int64_t)((uint64_t)c << 6);
-    const int ch = (int)(c6 >> 32);
-    const uint32_t cl = (uint32_t)c6, ah = (uint32_t)(a >> 32), al = (uint32_t)a;
-    const uint64_t u = (uint64_t)ah * cl;
-    int64_t v = (int64_t)ch * (int)(al >> 1);
-    v = (v >> 31) + (int64_t)(u >> 32);
-    return (uint64_t)((int64_t)ch * (int)ah + v);
-}
-
-// D^(-3/2) 2^151 (64-bit, between 2^55 and 2^61)
+// D^(-3/2) 2^151 (between 2^55 and 2^61): Y^2 (Y + 3eY/2), the correction below Y's last bit
 NB_FIX_FN uint64_t rinv3(uint64_t D) {
     uint32_t Y;
     uint64_t W;
-    const int64_t e = rsqrt_residual(D, Y, W);
-    // c = 3e/2 + 15e^2/8 in units 2^-58; e^2 from e's upper bits
-    const int eh = (int)(e >> 8);
-    const uint32_t q = (uint32_t)((uint64_t)((int64_t)eh * eh) >> 32);  // e^2 in units 2^-68
-    const int64_t c = e + (e >> 1) + (int64_t)((q * 15u) >> 13);
-    const uint64_t v = (uint64_t)(uint32_t)W * Y;
-    const uint64_t V = (uint64_t)(uint32_t)(W >> 32) * Y + (v >> 32);
-    return V + scaled(V, c);
+    const int e = rsqrt_residual(D, Y, W);
+    const uint64_t c = (uint64_t)(((int64_t)(int)Y * (e + (e >> 1))) >> 26);  // in units 2^-32 of Y's
+    const uint32_t yh = Y + (uint32_t)(c >> 32), yl = (uint32_t)c;
+    const uint32_t wh = (uint32_t)(W >> 32), wl = (uint32_t)W;
+    return (uint64_t)wh * yh + mul_hi(wl, yh) + mul_hi(wh, yl);
 }
 
-// D^(-1/2) 2^90 (64-bit, between 2^58 and 2^60)
+// D^(-1/2) 2^93 (between 2^61 and 2^63): Y (1 + e/2)
 NB_FIX_FN uint64_t rinv1(uint64_t D) {
     uint32_t Y;
     uint64_t W;
-    const int64_t e = rsqrt_residual(D, Y, W);
-    const int eh = (int)(e >> 8);
-    const uint32_t q = (uint32_t)((uint64_t)((int64_t)eh * eh) >> 32);
-    const int64_t c = (e >> 1) + (int64_t)((q * 3u) >> 13);
-    const uint64_t V = (uint64_t)Y << 29;
-    return V + scaled(V, c);
+    const int e = rsqrt_residual(D, Y, W);
+    return ((uint64_t)Y << 32) + (uint64_t)(((int64_t)(int)Y * e) >> 27);
 }
 
 // A 64-bit integer v > 0 as a double scaled so that 2^63 has the biased exponent `be`,
@@ -315,20 +319,25 @@ NB_FIX_FN double scaled_double(uint64_t v, int be) {
 // leaves the normal range.
 NB_FIX_FN double mass_rinv3(uint64_t S, uint32_t mh, uint32_t ml, int e, int sh, bool& ok) {
     const uint32_t s_h = (uint32_t)(S >> 32), s_l = (uint32_t)S;
-    const uint64_t u = (((uint64_t)s_l * mh) >> 32) + (((uint64_t)s_h * ml) >> 32);
-    const uint64_t F = (uint64_t)s_h * mh + u;
-    const int be = e + 3 * sh;  // exponent of 2^63; F is below 2^61 and above 2^53
+    const uint64_t F = (uint64_t)s_h * mh + mul_hi(s_h, ml) + mul_hi(s_l, mh);
+    const int be = e + 3 * sh + 3;  // exponent of 2^63; F is below 2^61 and above 2^53
     ok = (uint32_t)(be - 16) < 2016u;
     return scaled_double(F, be);
 }
 
-// One axis of the separation as a double (its sign and top 53 bits). base = 1025 + K - sh. The
-// magnitude is the complement of a negative value, one unit of the last word short, which is below
-// 2^-64 of it as long as the first word is not 0; the rest (a component below 2^-30 of the
-// distance or of eps) is negated exactly.
-NB_FIX_FN double axis(uint32_t vh, uint32_t vl, uint32_t ve, int base) {
-    const uint32_t s = (uint32_t)((int)vh >> 31);
-    uint32_t h = vh ^ s, l = vl ^ s, x = ve ^ s;
+// One axis of the separation as a double (its sign and top 53 bits); base = 1025 + K - sh.
+// Components with 2^20 or more in the first word have their 53 bits in two words.
+constexpr uint32_t AXIS_TWO_WORDS = 1u << 20;
+NB_FIX_FN double axis(uint32_t s, uint32_t h, uint32_t l, int base) {
+    const int n = clz32(h);
+    const uint32_t mh = fsl(l, h, n), ml = l << n;
+    const uint32_t hi = ((uint32_t)(base - n - 1) << 20) + (mh >> 11);
+    return double_of(hi | (s & 0x80000000u), (mh << 21) | (ml >> 11));
+}
+
+// Any component, x = the third word: where the first word is 0 the complement's missing unit is
+// added back.
+NB_FIX_FN double axis_small(uint32_t s, uint32_t h, uint32_t l, uint32_t x, int base) {
     if (h == 0) {
         const uint64_t v = (((uint64_t)l << 32) | x) + (s & 1u);
         if (v == 0) {
@@ -353,6 +362,21 @@ NB_FIX_FN double axis(uint32_t vh, uint32_t vl, uint32_t ve, int base) {
     return double_of(hi | (s & 0x80000000u), (mh << 21) | (ml >> 11));
 }
 
+NB_FIX_FN void axes(const Sep& s, int K, double& dx, double& dy, double& dz) {
+    const int base = 1025 + K - s.sh;
+    uint32_t least = s.xh < s.yh ? s.xh : s.yh;
+    least = least < s.zh ? least : s.zh;
+    if (least >= AXIS_TWO_WORDS) {
+        dx = axis(s.xs, s.xh, s.xl, base);
+        dy = axis(s.ys, s.yh, s.yl, base);
+        dz = axis(s.zs, s.zh, s.zl, base);
+    } else {
+        dx = axis_small(s.xs, s.xh, s.xl, (s.x0 << s.sh) ^ s.xs, base);
+        dy = axis_small(s.ys, s.yh, s.yl, (s.y0 << s.sh) ^ s.ys, base);
+        dz = axis_small(s.zs, s.zh, s.zl, (s.z0 << s.sh) ^ s.zs, base);
+    }
+}
+
 #ifdef __CUDACC__
 // eps^2 per shift, filled by one warp of a block (the caller's __syncthreads() follows).
 struct Eps2Table {
@@ -364,7 +388,7 @@ __device__ __forceinline__ void fill_eps2(Eps2Table& t, double eps2, int K) {
     const int sh = (int)threadIdx.x;
     const double u = sh <= SH_MAX && k_usable(K) ? eps2_units(eps2, K, sh) : -1.0;
     const bool fits = u >= 0.0 && u < EPS2_LIMIT;
-    t.units[sh] = fits ? __double2ull_rn(u) : 0;
+    t.units[sh] = fits ? __double2ull_rn(u) + NORM2_BIAS : 0;
     const uint32_t b = __ballot_sync(0xffffffffu, fits);  // a run from bit 0
     if (sh == 0) t.sh_max = __clz((int)~__brev(b)) - 1;
 }
@@ -377,13 +401,10 @@ __device__ __forceinline__ bool term(const FixRec& f, const Fix3& p, int K, cons
     const Fix3 c{f.x2, f.y2, f.z2, f.x1, f.y1, f.z1, f.x0, f.y0, f.z0};
     Sep s;
     if (!separation(c, p, sh_max, s)) return false;
-    const uint64_t D = norm2(s) + t.units[s.sh];
+    const uint64_t D = norm2(s) + t.units[s.sh];  // with norm2's bias
     bool ok;
     w = mass_rinv3(rinv3(D), f.mh, f.ml, f.e, s.sh, ok);
-    const int base = 1025 + K - s.sh;
-    dx = axis(s.xh, s.xl, s.xe, base);
-    dy = axis(s.yh, s.yl, s.ye, base);
-    dz = axis(s.zh, s.zl, s.ze, base);
+    axes(s, K, dx, dy, dz);
     return ok;
 }
 #endif

@@ -194,7 +194,8 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
             nbfix::Sep s;
             double inv;
             if (usable && nbfix::separation(c, p, nbfix::SH_MAX, s)) {
-                inv = nbfix::scaled_double(nbfix::rinv1(nbfix::norm2(s)), 1025 - K + s.sh);
+                inv = nbfix::scaled_double(nbfix::rinv1(nbfix::norm2(s) + nbfix::NORM2_BIAS),
+                                           1023 - K + s.sh);
             } else {
                 const uint32_t i = i0 + ii;
                 const double rx = x[j] - x[i], ry = y[j] - y[i], rz = z[j] - z[i];

@@ -1,7 +1,7 @@
 """The fixed-point pair arithmetic of nb_fix.cuh, compiled as plain C++, against 60-digit decimal
 arithmetic. Tolerances: the factor m (r^2 + eps^2)^(-3/2) is one rounding (2^-53) after a chain
-whose truncations stay below 1.5 x 2^-57 (norm), 2^-56 (residual) and 2^-56 (products): 2^-52.4 in
-all; a separation component is exact up to its truncation to 53 bits (2^-52), where the fixed-point
+whose truncations stay below 1.5 x 20 / 2^60 (norm, centred), 1.5 x 2^-56.6 (residual) and 2^-54
+(products and dropped terms): 2^-52.4 in all; a separation component is exact up to its truncation to 53 bits (2^-52), where the fixed-point
 grid (2^(K - 94) per coordinate) holds the coordinates."""
 
 import ctypes as C
@@ -17,7 +17,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SOURCE = r"""
 #include "nb_fix.cuh"
 using namespace nbfix;
-// out: w, dx, dy, dz; returns 0 when the pair needs the FP64 expressions
+// out: w, dx, dy, dz, 1 / sqrt(r^2 + eps^2); returns 0 when the pair needs the FP64 expressions
 extern "C" int fix_pair(const double* c, const double* p, double m, double eps2, double v_max,
                         double* out) {
     const int K = k_of(v_max);
@@ -30,13 +30,11 @@ extern "C" int fix_pair(const double* c, const double* p, double m, double eps2,
     Sep s;
     const Fix3 q{r.x2, r.y2, r.z2, r.x1, r.y1, r.z1, r.x0, r.y0, r.z0};
     if (!separation(q, P, sh_max, s)) return 0;
-    const uint64_t D = norm2(s) + (uint64_t)(eps2_units(eps2, K, s.sh) + 0.5);
+    const uint64_t D = norm2(s) + (uint64_t)(eps2_units(eps2, K, s.sh) + 0.5) + NORM2_BIAS;
     bool ok;
     out[0] = mass_rinv3(rinv3(D), r.mh, r.ml, r.e, s.sh, ok);
-    const int base = 1025 + K - s.sh;
-    out[1] = axis(s.xh, s.xl, s.xe, base);
-    out[2] = axis(s.yh, s.yl, s.ye, base);
-    out[3] = axis(s.zh, s.zl, s.ze, base);
+    axes(s, K, out[1], out[2], out[3]);
+    out[4] = scaled_double(rinv1(D), 1023 - K + s.sh);
     return ok;
 }
 """
@@ -54,7 +52,7 @@ def fix(tmp_path_factory):
     lib.fix_pair.argtypes = [C.POINTER(C.c_double)] * 2 + [C.c_double] * 3 + [C.POINTER(C.c_double)]
 
     def pair(c, p, m, eps2, v_max):
-        out = (C.c_double * 4)()
+        out = (C.c_double * 5)()
         ok = lib.fix_pair((C.c_double * 3)(*c), (C.c_double * 3)(*p), m, eps2, v_max, out)
         return list(out) if ok else None
 
@@ -84,6 +82,7 @@ def test_pairs_against_decimal(fix, box, eps2, lo):
         r2 = sum(v * v for v in d) + Decimal(eps2)
         w = Decimal(m) / (r2 * r2.sqrt())
         assert abs(Decimal(got[0]) / w - 1) <= Decimal(2.0 ** -52.4)
+        assert abs(Decimal(got[4]) * r2.sqrt() - 1) <= Decimal(2.0 ** -52.4)
         for g, v in zip(got[1:], d):
             assert abs(Decimal(g) - v) <= abs(v) * Decimal(2.0 ** -52)
     assert used > 2000
