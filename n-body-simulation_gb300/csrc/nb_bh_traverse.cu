@@ -347,13 +347,12 @@ __device__ __forceinline__ Pretest pretest_of(const double* __restrict__ box, do
 // lists up to FIX_LIST accepted cells, then the warp evaluates its lanes' lists together, the next
 // cell's record loaded while the current one is computed.
 //  Bound: the load pipe (75% of its wavefronts: every lane reads its own 32-byte walk record per
-//  visited and 48-byte fixed-point record per accepted cell) and issue (61% of cycles, integer
-//  pipe 57%, FP64 pipe 41%). The monopole is ~190 instructions with 3 FP64 ones (nb_fix.cuh)
-//  against 16 FP64 operations before, whose pipe was 82% busy; 256-bit loads halve the load
-//  instructions (14.6 -> 13.45 ms), the lists (against one accepted cell at a time) keep 30.9 of
-//  32 lanes active (17.2 -> 14.6 ms with the record prefetch). 1,048,576-body disc, theta = 0.5:
-//  35.5 -> 13.5 ms per step. 24 warps per SM at 80 registers: 28 or 32 warps at 72 or 64 registers
-//  measured 1% and 6% slower.
+//  visited and 48-byte fixed-point record per accepted cell) and issue (61% of cycles). The
+//  monopole is ~130 instructions with 3 FP64 ones (nb_fix.cuh) against 16 FP64 operations before,
+//  whose pipe was 82% busy; 256-bit loads halve the load instructions (14.6 -> 13.45 ms), the
+//  lists (against one accepted cell at a time) keep 30.9 of 32 lanes active (17.2 -> 14.6 ms with
+//  the record prefetch). Step at 1,048,576 bodies (disc, theta = 0.5): 35.5 -> 13.1 ms. 24 warps
+//  per SM: 20 measured 4%, 28 2.5% and 32 4% slower; lists of 8 2% slower.
 constexpr int FIX_LIST = 16;
 constexpr int FIX_BLOCKS_PER_SM = 6;
 
@@ -433,8 +432,11 @@ bh_theta_fix_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __rest
 //  Bound: the latency of a walk of dependent windows and of ~accepted / T monopoles by one warp.
 //  Traversal at theta = 0.5 (disc), one lane per body -> T lanes: 777 bodies 135 -> 31 us (T = 32),
 //  4,000 273 -> 77 us (16), 16,411 471 -> 300 us (4), 32,768 625 -> 540 us (2).
+//  Registers for 20 warps per SM (24 warps: 3% slower at 16,411 bodies).
+constexpr int TEAM_BLOCKS_PER_SM = 5;
+
 template <int T>
-__global__ void __launch_bounds__(TR_THREADS, FIX_BLOCKS_PER_SM)
+__global__ void __launch_bounds__(TR_THREADS, TEAM_BLOCKS_PER_SM)
 bh_theta_team_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __restrict__ rec64,
                      const nbfix::FixHi* __restrict__ fix_hi, const uint4* __restrict__ fix_lo,
                      const uint32_t* __restrict__ info, const uint32_t* __restrict__ ids,

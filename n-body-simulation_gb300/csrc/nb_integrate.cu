@@ -83,11 +83,13 @@ __global__ void kick_kick_drift_kernel(double* __restrict__ vx, double* __restri
 // nb_fix.cuh (within one rounding of exact); of a pair's work only the sum, m_i * (1/r), is on the
 // FP64 pipe. Pairs the fixed point cannot hold (closer than 2^(K-30), or coordinates beyond its
 // exponent range) take the FP64 expression.
-//  Bound: integer pipe and issue (about 80 instructions per unordered pair against 14 FP64
-//  operations at 1/75 of the FP32 rate). 50,021 bodies: 49.3 ms before, EN_MS now.
+//  Bound: dispatch of 104 instructions per unordered pair, half of them 64-bit (issue 58%, integer
+//  pipe 54%, wide multiplies 57%, FP64 pipe 38% of cycles), against 14 FP64 operations at 1/75 of
+//  the FP32 rate before. 50,021 bodies: 49.2 -> 5.4 ms (25 -> 233 Gpairs/s). 48 warps per SM (24
+//  to 40: 1 to 7% slower).
 // ---------------------------------------------------------------------------------------------
 constexpr int EN_THREADS = 128;        // targets per row, sources per tile at most
-constexpr int EN_CTAS_PER_SM = 8;
+constexpr int EN_CTAS_PER_SM = 12;
 constexpr uint32_t EN_SCAN_N = 2048;   // up to here every CTA finds the largest coordinate itself
 constexpr uint32_t EN_K_BLOCKS = 128;  // else this many blocks do, into one word each
 
@@ -187,7 +189,7 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
         }
         __syncthreads();
         const uint32_t cnt = active && j > i0 ? min(tile, j - i0) : 0u;
-#pragma unroll 2
+#pragma unroll 1
         for (uint32_t ii = 0; ii < cnt; ++ii) {
             const nbfix::FixRec f = src[ii];
             const nbfix::Fix3 c{f.x2, f.y2, f.z2, f.x1, f.y1, f.z1, f.x0, f.y0, f.z0};
