@@ -69,8 +69,8 @@ nb_status nb_ctx_create(int device, nb_ctx** out) {
     cudaError_t e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->dev_error, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(ctx->dev_error, 0, sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->dev_counter, 64 * sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMemset(ctx->dev_counter, 0, 64 * sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->dev_counter, NB_COUNTER_WORDS * sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaMemset(ctx->dev_counter, 0, NB_COUNTER_WORDS * sizeof(unsigned int));
     if (e != cudaSuccess) {
         nb_ctx_destroy(ctx);
         return nb::cuda_error(e, "nb_ctx_create");

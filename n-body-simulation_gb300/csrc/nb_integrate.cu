@@ -90,40 +90,8 @@ __global__ void kick_kick_drift_kernel(double* __restrict__ vx, double* __restri
 // ---------------------------------------------------------------------------------------------
 constexpr int EN_THREADS = 128;        // targets per row, sources per tile at most
 constexpr int EN_CTAS_PER_SM = 12;
-constexpr uint32_t EN_SCAN_N = 2048;   // up to here every CTA finds the largest coordinate itself
-constexpr uint32_t EN_K_BLOCKS = 128;  // else this many blocks do, into one word each
 
-// Largest biased exponent of the coordinates of bodies b0, b0 + step, ...
-__device__ __forceinline__ uint32_t max_exponent(const double* __restrict__ x,
-                                                 const double* __restrict__ y,
-                                                 const double* __restrict__ z, uint32_t n,
-                                                 uint32_t b0, uint32_t step) {
-    uint32_t e = 0;
-    for (uint32_t b = b0; b < n; b += step) {
-        const uint32_t h = max((uint32_t)__double2hiint(x[b]) & 0x7fffffffu,
-                               max((uint32_t)__double2hiint(y[b]) & 0x7fffffffu,
-                                   (uint32_t)__double2hiint(z[b]) & 0x7fffffffu));
-        e = max(e, h >> 20);
-    }
-    return e;
-}
-
-__global__ void __launch_bounds__(256)
-energy_scale_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                    const double* __restrict__ z, uint32_t n, uint32_t* __restrict__ out) {
-    __shared__ uint32_t most;
-    if (threadIdx.x == 0) most = 0;
-    __syncthreads();
-    const uint32_t e = __reduce_max_sync(
-        0xffffffffu,
-        max_exponent(x, y, z, n, blockIdx.x * 256 + threadIdx.x, gridDim.x * 256));
-    if ((threadIdx.x & 31) == 0) atomicMax(&most, e);
-    __syncthreads();
-    if (threadIdx.x == 0) out[blockIdx.x] = most;
-}
-
-// tile: sources per unit (a divisor of EN_THREADS); k_words: results of energy_scale_kernel (0: the
-// CTA scans the bodies itself).
+// tile: sources per unit (a divisor of EN_THREADS); k_part, k_words: nbfix::block_scale.
 __global__ void __launch_bounds__(EN_THREADS, EN_CTAS_PER_SM)
 energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
               const double* __restrict__ y, const double* __restrict__ z,
@@ -132,22 +100,8 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
               const uint32_t* __restrict__ k_part, uint32_t k_words, double2* __restrict__ part) {
     __shared__ nbfix::FixRec src[EN_THREADS];  // positions; the mass as a double in (mh, ml)
     __shared__ double red_k[EN_THREADS / 32], red_p[EN_THREADS / 32];
-    __shared__ uint32_t most;
     const uint32_t tid = threadIdx.x;
-    if (tid == 0) most = 0;
-    __syncthreads();
-    {
-        uint32_t e = 0;
-        if (k_words == 0) {
-            e = max_exponent(x, y, z, n, tid, EN_THREADS);
-        } else if (tid < k_words) {
-            e = k_part[tid];
-        }
-        e = __reduce_max_sync(0xffffffffu, e);
-        if ((tid & 31) == 0) atomicMax(&most, e);
-    }
-    __syncthreads();
-    const int K = (int)most - 1022;
+    const int K = nbfix::block_scale(x, y, z, n, k_part, k_words);
     const bool usable = nbfix::k_usable(K);  // the same in all threads
     const uint32_t q = EN_THREADS / tile;    // tiles per row of sources
     const uint64_t u0 = units * blockIdx.x / gridDim.x, u1 = units * (blockIdx.x + 1) / gridDim.x;
@@ -281,11 +235,7 @@ nb_status energy_launch(const EnergyShape& e, const double* m, const double* x, 
                         uint32_t n, double G, uint32_t* k_part, double2* part, double* out,
                         cudaStream_t stream) {
     uint32_t k_words = 0;
-    if (n > EN_SCAN_N) {
-        k_words = std::min<uint32_t>(EN_K_BLOCKS, (uint32_t)nb::ceil_div(n, 1024));
-        energy_scale_kernel<<<k_words, 256, 0, stream>>>(x, y, z, n, k_part);
-        NB_TRY(nb::check_launch("energy_scale_kernel"));
-    }
+    NB_TRY(nb::launch_scale(x, y, z, n, k_part, &k_words, stream));
     energy_kernel<<<e.ctas, EN_THREADS, 0, stream>>>(m, x, y, z, vx, vy, vz, n, G, e.tile, e.units,
                                                      k_part, k_words, part);
     NB_TRY(nb::check_launch("energy_kernel"));
@@ -307,6 +257,21 @@ __device__ __forceinline__ long long ord_of(double v) {
 }
 __device__ __forceinline__ double val_of(long long o) {
     return __longlong_as_double(o >= 0 ? o : (o ^ 0x7fffffffffffffffLL));
+}
+
+// One word per block for nbfix::block_scale.
+__global__ void __launch_bounds__(256)
+scale_kernel(const double* __restrict__ x, const double* __restrict__ y,
+                    const double* __restrict__ z, uint32_t n, uint32_t* __restrict__ out) {
+    __shared__ uint32_t most;
+    if (threadIdx.x == 0) most = 0;
+    __syncthreads();
+    const uint32_t e = __reduce_max_sync(
+        0xffffffffu,
+        nbfix::max_exponent(x, y, z, n, blockIdx.x * 256 + threadIdx.x, gridDim.x * 256));
+    if ((threadIdx.x & 31) == 0) atomicMax(&most, e);
+    __syncthreads();
+    if (threadIdx.x == 0) out[blockIdx.x] = most;
 }
 
 struct MinMax6 {
@@ -435,6 +400,16 @@ aabb_kernel(const double* __restrict__ x, const double* __restrict__ y,
 
 namespace nb {
 
+// Words for nbfix::block_scale: none for systems that every CTA scans itself.
+nb_status launch_scale(const double* x, const double* y, const double* z, uint32_t n,
+                       uint32_t* k_part, uint32_t* k_words, cudaStream_t stream) {
+    *k_words = 0;
+    if (n <= nbfix::SCALE_SCAN_N) return NB_OK;
+    *k_words = std::min<uint32_t>(nbfix::SCALE_WORDS, (uint32_t)nb::ceil_div(n, 1024));
+    scale_kernel<<<*k_words, 256, 0, stream>>>(x, y, z, n, k_part);
+    return nb::check_launch("scale_kernel");
+}
+
 // Enqueues the AABB of (x, y, z) into out_dev[7]. Used by nb_aabb and the tree build.
 nb_status launch_aabb(nb_ctx* ctx, const double* x, const double* y, const double* z,
                       uint32_t n, double* out_dev, cudaStream_t stream) {
@@ -502,7 +477,7 @@ nb_status nb_energy(nb_ctx* ctx, const double* m, const double* x, const double*
     const EnergyShape e = energy_shape(n, ctx->sm_count, 0xffffffffu);
     const size_t part_bytes = (size_t)e.ctas * sizeof(double2);
     void* part = nullptr;
-    NB_TRY(nb::scratch(ctx, NB_SCRATCH_ENERGY, part_bytes + EN_K_BLOCKS * sizeof(uint32_t), &part));
+    NB_TRY(nb::scratch(ctx, NB_SCRATCH_ENERGY, part_bytes + nbfix::SCALE_WORDS * sizeof(uint32_t), &part));
     return energy_launch(e, m, x, y, z, vx, vy, vz, n, G, (uint32_t*)((char*)part + part_bytes),
                          (double2*)part, out_dev, (cudaStream_t)stream);
 }
@@ -536,7 +511,7 @@ constexpr uint32_t NOALLOC_MAX_BLOCKS = 8192;  // 8192 * 16 B = 128 KiB of scrat
 // until the process exits. Host code must not pass the symbol itself to a kernel: its host-side
 // name is only a stand-in, so the device address is looked up once per device below.
 static __device__ __align__(256) double2 g_energy_noalloc_partials[NOALLOC_MAX_BLOCKS];
-constexpr uint32_t NOALLOC_K_AT = NOALLOC_MAX_BLOCKS - EN_K_BLOCKS / 4;  // scale words at the end
+constexpr uint32_t NOALLOC_K_AT = NOALLOC_MAX_BLOCKS - nbfix::SCALE_WORDS / 4;  // scale words at the end
 
 constexpr int NOALLOC_MAX_DEVICES = 64;
 std::mutex g_noalloc_mutex;

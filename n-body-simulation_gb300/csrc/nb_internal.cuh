@@ -40,6 +40,10 @@ enum nb_scratch_slot : int {
     NB_SCRATCH_COUNT = 8,
 };
 
+// Words of nb_ctx::dev_counter: the AABB's last-block counter, then the words of
+// nbfix::block_scale (each launch writes the ones it reads).
+constexpr int NB_COUNTER_SCALE = 64, NB_COUNTER_WORDS = NB_COUNTER_SCALE + 128;
+
 // An instantiated CUDA graph of captured steps (nb_batch_graph_create, nb_bh_graph_create).
 struct nb_graph {
     cudaGraph_t graph = nullptr;
@@ -72,6 +76,11 @@ nb_status cuda_error(cudaError_t err, const char* what);
 // Grows scratch slot `slot` of the context to at least `bytes` (cudaMalloc; synchronous).
 nb_status scratch(nb_ctx* ctx, int slot, size_t bytes, void** out);
 nb_status check_launch(const char* what);
+
+// Enqueues the words of nbfix::block_scale for a system's coordinates: k_part has room for
+// nbfix::SCALE_WORDS, *k_words gets the number written (nb_integrate.cu).
+nb_status launch_scale(const double* x, const double* y, const double* z, uint32_t n,
+                       uint32_t* k_part, uint32_t* k_words, cudaStream_t stream);
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 

@@ -5,10 +5,10 @@
 //    operation separately rounded in the reference's order (r^2 summed left to right, den^3 as
 //    (den*den)*den, 1/sqrt for rsqrt, acc += m*(r*den), G last). Bit-identical to the host
 //    FP64 evaluation of NaiveAlgorithm.cpp:331-351.
-//  * NB_F64: over all bodies of a large system, the FP64 form of the symmetric pair kernel of
-//    nb_pair_sym.cu (each unordered pair once, 20 FP64 operations for both bodies); otherwise the
-//    same loop as the IEEE mode with FMAs and m (r^2 + eps^2)^(-3/2) from the hardware rsqrt
-//    estimate with one correction (nb_m_rinv3_f64; FP64-pipe bound on GB300).
+//  * NB_F64: the same sum with the pair's separation, r^2 + eps^2 and m r^-3 in the fixed point of
+//    nb_fix.cuh on the integer pipes and FP64 sums (3 FP64 operations per ordered pair): over all
+//    bodies of a large system the symmetric kernel of nb_pair_sym.cu (each unordered pair once),
+//    otherwise the one-sided naive_fix_kernel.
 //  * NB_F32C: over all bodies of a large system, the symmetric FP32 pair kernel of
 //    nb_pair_sym.cu (each unordered pair once, added to both bodies); otherwise (target ranges,
 //    small systems) the one-sided FP32-compensated pair kernel of nb_pair.cuh (scalar FP32 pair
@@ -16,6 +16,11 @@
 //    mbarrier waits), run as a batch of one system.
 //  * NB_DF64: double-float pair math on the FP32 pipe (FP64-accurate to ~1e-14); over all bodies
 //    of a large system the double-float form of the symmetric pair kernel.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+#include "nb_fix.cuh"
 #include "nb_internal.cuh"
 #include "nb_pair.cuh"
 #include "nb_pair_sym.cuh"
@@ -27,16 +32,11 @@ namespace {
 // ---------------------------------------------------------------------------------------------
 constexpr int F64_THREADS = 64;
 
-// blockIdx.y selects a chunk of `chunk` sources (NB_F64 at small n, for more warps per SM; the
-// IEEE mode always runs one chunk so that its sum order stays the reference's); with more than
-// one chunk the partial sums (times G) go to part[(chunk index * n_t + target) * 3 + axis].
-template <bool IEEE>
 __global__ void __launch_bounds__(F64_THREADS)
-naive_f64_kernel(const double* __restrict__ m, const double* __restrict__ x,
-                 const double* __restrict__ y, const double* __restrict__ z,
-                 double* __restrict__ ax, double* __restrict__ ay, double* __restrict__ az,
-                 uint32_t n, uint32_t i_begin, uint32_t i_end, double G, double eps2,
-                 uint32_t chunk, double* __restrict__ part) {
+naive_ieee_kernel(const double* __restrict__ m, const double* __restrict__ x,
+                  const double* __restrict__ y, const double* __restrict__ z,
+                  double* __restrict__ ax, double* __restrict__ ay, double* __restrict__ az,
+                  uint32_t n, uint32_t i_begin, uint32_t i_end, double G, double eps2) {
     __shared__ double sx[F64_THREADS], sy[F64_THREADS], sz[F64_THREADS], sm[F64_THREADS];
     const uint32_t i = i_begin + blockIdx.x * F64_THREADS + threadIdx.x;
     const bool active = i < i_end;
@@ -47,83 +47,222 @@ naive_f64_kernel(const double* __restrict__ m, const double* __restrict__ x,
         pz = z[i];
     }
     double acc_x = 0, acc_y = 0, acc_z = 0;
-    const uint32_t j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
-    for (uint32_t k = j0; k < j1; k += F64_THREADS) {
+    for (uint32_t k = 0; k < n; k += F64_THREADS) {
         const uint32_t j = k + threadIdx.x;
-        if (j < j1) {
+        if (j < n) {
             sx[threadIdx.x] = x[j];
             sy[threadIdx.x] = y[j];
             sz[threadIdx.x] = z[j];
             sm[threadIdx.x] = m[j];
         }
         __syncthreads();
-        const uint32_t cnt = min((uint32_t)F64_THREADS, j1 - k);
+        const uint32_t cnt = min((uint32_t)F64_THREADS, n - k);
         if (active) {
-            if (IEEE) {
-                for (uint32_t jj = 0; jj < cnt; ++jj) {
-                    const double r_x = __dsub_rn(sx[jj], px);
-                    const double r_y = __dsub_rn(sy[jj], py);
-                    const double r_z = __dsub_rn(sz[jj], pz);
-                    double den = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(r_x, r_x), __dmul_rn(r_y, r_y)),
-                                                     __dmul_rn(r_z, r_z)),
-                                           eps2);
-                    den = __dmul_rn(__dmul_rn(den, den), den);
-                    den = __ddiv_rn(1.0, __dsqrt_rn(den));
-                    acc_x = __dadd_rn(acc_x, __dmul_rn(sm[jj], __dmul_rn(r_x, den)));
-                    acc_y = __dadd_rn(acc_y, __dmul_rn(sm[jj], __dmul_rn(r_y, den)));
-                    acc_z = __dadd_rn(acc_z, __dmul_rn(sm[jj], __dmul_rn(r_z, den)));
-                }
-            } else {
-#pragma unroll 4
-                for (uint32_t jj = 0; jj < cnt; ++jj) {
-                    const double r_x = sx[jj] - px;
-                    const double r_y = sy[jj] - py;
-                    const double r_z = sz[jj] - pz;
-                    const double den = fma(r_x, r_x, fma(r_y, r_y, fma(r_z, r_z, eps2)));
-                    const double s = nb_m_rinv3_f64(sm[jj], den);
-                    acc_x = fma(s, r_x, acc_x);
-                    acc_y = fma(s, r_y, acc_y);
-                    acc_z = fma(s, r_z, acc_z);
-                }
+            for (uint32_t jj = 0; jj < cnt; ++jj) {
+                const double r_x = __dsub_rn(sx[jj], px);
+                const double r_y = __dsub_rn(sy[jj], py);
+                const double r_z = __dsub_rn(sz[jj], pz);
+                double den = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(r_x, r_x), __dmul_rn(r_y, r_y)),
+                                                 __dmul_rn(r_z, r_z)),
+                                       eps2);
+                den = __dmul_rn(__dmul_rn(den, den), den);
+                den = __ddiv_rn(1.0, __dsqrt_rn(den));
+                acc_x = __dadd_rn(acc_x, __dmul_rn(sm[jj], __dmul_rn(r_x, den)));
+                acc_y = __dadd_rn(acc_y, __dmul_rn(sm[jj], __dmul_rn(r_y, den)));
+                acc_z = __dadd_rn(acc_z, __dmul_rn(sm[jj], __dmul_rn(r_z, den)));
             }
         }
         __syncthreads();
     }
     if (active) {
-        if (IEEE) {
-            ax[i] = __dmul_rn(acc_x, G);
-            ay[i] = __dmul_rn(acc_y, G);
-            az[i] = __dmul_rn(acc_z, G);
-        } else if (gridDim.y == 1) {
-            ax[i] = acc_x * G;
-            ay[i] = acc_y * G;
-            az[i] = acc_z * G;
-        } else {
-            double* o = part + ((size_t)blockIdx.y * (i_end - i_begin) + (i - i_begin)) * 3;
-            o[0] = acc_x * G;
-            o[1] = acc_y * G;
-            o[2] = acc_z * G;
-        }
+        ax[i] = __dmul_rn(acc_x, G);
+        ay[i] = __dmul_rn(acc_y, G);
+        az[i] = __dmul_rn(acc_z, G);
     }
 }
 
-// Adds the chunks' partial sums of each target in chunk order.
-__global__ void chunk_combine_kernel(const double* __restrict__ part, uint32_t chunks,
-                                  uint32_t i_begin, uint32_t i_end, double* __restrict__ ax,
-                                  double* __restrict__ ay, double* __restrict__ az) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n_t = i_end - i_begin;
-    if (t >= n_t) return;
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    for (uint32_t c = 0; c < chunks; ++c) {
-        const double* o = part + ((size_t)c * n_t + t) * 3;
-        sx += o[0];
-        sy += o[1];
-        sz += o[2];
+// Adds the pair (source record f, body q) seen from body i at p to the sums: NB_F64's arithmetic. The
+// pairs the fixed point cannot hold take the FP64 expressions; the self pair (its separation is 0)
+// and massless sources mostly add nothing.
+struct FixSums {
+    double x, y, z;
+};
+__device__ __forceinline__ void fix_pair(const nbfix::FixRec& f, uint32_t q, uint32_t i,
+                                         const nbfix::Fix3& p, int K, const nbfix::Eps2Table& e2,
+                                         int sh_max, double eps2, const double* __restrict__ m,
+                                         const double* __restrict__ x,
+                                         const double* __restrict__ y,
+                                         const double* __restrict__ z, FixSums& a) {
+    double w, dx, dy, dz;
+    if (sh_max < 0 || !nbfix::term(f, p, K, e2, sh_max, w, dx, dy, dz)) {
+        w = dx = dy = dz = 0.0;
+        if (!nbfix::adds_nothing(f, q == i, K, sh_max, eps2)) {
+            dx = x[q] - x[i];
+            dy = y[q] - y[i];
+            dz = z[q] - z[i];
+            w = nb_m_rinv3_f64(m[q], fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+        }
     }
-    ax[i_begin + t] = sx;
-    ay[i_begin + t] = sy;
-    az[i_begin + t] = sz;
+    a.x = fma(w, dx, a.x);
+    a.y = fma(w, dy, a.y);
+    a.z = fma(w, dz, a.z);
+}
+
+// NB_F64, one-sided: target ranges, listed targets, systems below the symmetric kernel's sizes. One thread per target; the
+// sources of a tile are converted to the fixed point of nb_fix.cuh by the block as it loads them,
+// and a pair costs ~115 integer instructions and 3 FP64 ones instead of 16 FP64 ones. blockIdx.y selects a chunk of `chunk` sources; with more than one chunk the partial sums (times
+// G) go to part[(chunk index * targets + target) * 3 + axis].
+//  Bound: the FP64 pipe (81% busy at 3 FMAs per pair) and dispatch. 8,192 bodies 2.16 -> 0.50 ms
+//  (31 -> 133 Gpairs/s), 4,096 0.53 -> 0.15. 32 warps per SM in blocks of 256 (blocks of 128: 3% slower, of 64: 16%).
+constexpr int FX_THREADS = 256;
+constexpr int FX_BLOCKS_PER_SM = 4;
+// Source chunks: 32 blocks per SM in all (fewer leave a longer last wave: 16 are 4% slower at 16,384
+// bodies, 8 8%), but at most 128 chunks and at least 4 sources each, since every pair of a lone
+// block's chain of tiles is ~0.5 us while its start and the combine pass are ~2 us each.
+constexpr long long FX_GRID_PER_SM = 32;
+constexpr uint32_t FX_CHUNKS_MAX = 128, FX_CHUNK_MIN = 4;
+static_assert(NB_COUNTER_WORDS - NB_COUNTER_SCALE >= (int)nbfix::SCALE_WORDS, "scale words");
+
+__global__ void __launch_bounds__(FX_THREADS, FX_BLOCKS_PER_SM)
+naive_fix_kernel(const double* __restrict__ m, const double* __restrict__ x,
+                 const double* __restrict__ y, const double* __restrict__ z,
+                 double* __restrict__ ax, double* __restrict__ ay, double* __restrict__ az,
+                 uint32_t n, const uint32_t* __restrict__ targets, uint32_t i_begin, uint32_t n_t,
+                 double G, double eps2, uint32_t chunk, double* __restrict__ part,
+                 const uint32_t* __restrict__ k_part, uint32_t k_words) {
+    __shared__ nbfix::FixRec src[FX_THREADS];
+    __shared__ nbfix::Eps2Table e2;
+    const int K = nbfix::block_scale(x, y, z, n, k_part, k_words);
+    nbfix::fill_eps2(e2, eps2, K);
+    __syncthreads();
+    const uint32_t t = blockIdx.x * FX_THREADS + threadIdx.x;
+    const bool active = t < n_t;
+    const uint32_t i = active ? (targets != nullptr ? targets[t] : i_begin + t) : 0u;
+    nbfix::Fix3 p;
+    const int sh_max = nbfix::split3(x[i], y[i], z[i], K, p) ? e2.sh_max : -1;
+    FixSums acc{0.0, 0.0, 0.0};
+    const uint32_t j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
+    for (uint32_t k = j0; k < j1; k += FX_THREADS) {
+        const uint32_t j = k + threadIdx.x;
+        __syncthreads();
+        if (j < j1) src[threadIdx.x] = nbfix::make_rec(x[j], y[j], z[j], m[j], K);
+        __syncthreads();
+        const uint32_t cnt = active ? min((uint32_t)FX_THREADS, j1 - k) : 0u;
+#pragma unroll 1
+        for (uint32_t jj = 0; jj < cnt; ++jj)
+            fix_pair(src[jj], k + jj, i, p, K, e2, sh_max, eps2, m, x, y, z, acc);
+    }
+    if (!active) return;
+    if (gridDim.y == 1) {
+        const uint32_t o = targets != nullptr ? t : i;
+        ax[o] = acc.x * G;
+        ay[o] = acc.y * G;
+        az[o] = acc.z * G;
+    } else {
+        double* o = part + ((size_t)blockIdx.y * n_t + t) * 3;
+        o[0] = acc.x * G;
+        o[1] = acc.y * G;
+        o[2] = acc.z * G;
+    }
+}
+
+// The same for systems of up to FXC_MAX_N bodies, where one launch without global partials counts:
+// a cluster of 8 CTAs per 32 targets, the sources split over the CTAs and each CTA's share over its 8
+// warps. The warps' sums are added in warp order in shared memory, the CTAs' sums in rank order by
+// rank 0 through distributed shared memory.
+//  Bound: the ~0.5 us latency of each of the n / 64 pairs a warp evaluates one after the other, and
+//  ~4 us of start and reductions. 1,009 bodies: 48 us (FP64, chunks and a combine pass) -> 19 us;
+//  2,048: 144 -> 50. At 3,000 bodies the chunked kernel above is 8% faster.
+constexpr int FXC_CTAS = 8, FXC_WARPS = 8, FXC_THREADS = 32 * FXC_WARPS;
+constexpr uint32_t FXC_MAX_N = 2048;
+static_assert(FXC_MAX_N <= nbfix::SCALE_SCAN_N, "one launch");
+
+__global__ void __cluster_dims__(FXC_CTAS, 1, 1) __launch_bounds__(FXC_THREADS)
+naive_fix_cluster_kernel(const double* __restrict__ m, const double* __restrict__ x,
+                         const double* __restrict__ y, const double* __restrict__ z,
+                         double* __restrict__ ax, double* __restrict__ ay,
+                         double* __restrict__ az, uint32_t n,
+                         const uint32_t* __restrict__ targets, uint32_t i_begin, uint32_t n_t,
+                         double G, double eps2, const uint32_t* __restrict__ k_part,
+                         uint32_t k_words) {
+    namespace cg = cooperative_groups;
+    __shared__ nbfix::FixRec src[FXC_THREADS];
+    __shared__ nbfix::Eps2Table e2;
+    __shared__ double sums[FXC_WARPS][3][32], total[3][32];
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank();
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int K = nbfix::block_scale(x, y, z, n, k_part, k_words);
+    nbfix::fill_eps2(e2, eps2, K);
+    __syncthreads();
+    const uint32_t t = (blockIdx.x / FXC_CTAS) * 32 + lane;
+    const bool active = t < n_t;
+    const uint32_t i = active ? (targets != nullptr ? targets[t] : i_begin + t) : 0u;
+    nbfix::Fix3 p;
+    const int sh_max = nbfix::split3(x[i], y[i], z[i], K, p) ? e2.sh_max : -1;
+    FixSums acc{0.0, 0.0, 0.0};
+    const uint32_t share = (n + FXC_CTAS - 1) / FXC_CTAS;
+    const uint32_t j0 = min(n, rank * share), j1 = min(n, j0 + share);
+    for (uint32_t k = j0; k < j1; k += FXC_THREADS) {
+        const uint32_t j = k + threadIdx.x;
+        __syncthreads();
+        if (j < j1) src[threadIdx.x] = nbfix::make_rec(x[j], y[j], z[j], m[j], K);
+        __syncthreads();
+        const uint32_t cnt = min((uint32_t)FXC_THREADS, j1 - k);
+#pragma unroll 1
+        for (uint32_t jj = w; jj < cnt; jj += FXC_WARPS)
+            fix_pair(src[jj], k + jj, i, p, K, e2, sh_max, eps2, m, x, y, z, acc);
+    }
+    sums[w][0][lane] = acc.x;
+    sums[w][1][lane] = acc.y;
+    sums[w][2][lane] = acc.z;
+    __syncthreads();
+    if (w < 3) {
+        double s = sums[0][w][lane];
+#pragma unroll
+        for (int v = 1; v < FXC_WARPS; ++v) s += sums[v][w][lane];
+        total[w][lane] = s;
+    }
+    cluster.sync();
+    if (rank == 0 && w < 3) {
+        double s = total[w][lane];
+#pragma unroll
+        for (int r = 1; r < FXC_CTAS; ++r) s += *cluster.map_shared_rank(&total[w][lane], r);
+        if (active) (w == 0 ? ax : (w == 1 ? ay : az))[targets != nullptr ? t : i] = s * G;
+    }
+    cluster.sync();  // no CTA leaves while rank 0 reads its shared memory
+}
+
+// Adds the chunks' partial sums of each target in a fixed order: 32 targets per block, warp w takes
+// chunks w, w + 8, ..., then the warps' sums in warp order (a chain of one thread per target over
+// 64 chunks took 24 us: one load and one FP64 latency after the other).
+constexpr int CC_WARPS = 8;
+
+__global__ void __launch_bounds__(32 * CC_WARPS)
+chunk_combine_kernel(const double* __restrict__ part, uint32_t chunks, uint32_t i_begin,
+                     uint32_t i_end, double* __restrict__ ax, double* __restrict__ ay,
+                     double* __restrict__ az) {
+    __shared__ double sum[CC_WARPS][3][32];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, n_t = i_end - i_begin;
+    const uint32_t t = blockIdx.x * 32 + lane;
+    double s[3] = {0.0, 0.0, 0.0};
+    if (t < n_t) {
+#pragma unroll 4
+        for (uint32_t c = w; c < chunks; c += CC_WARPS) {
+            const double* o = part + ((size_t)c * n_t + t) * 3;
+            s[0] += o[0];
+            s[1] += o[1];
+            s[2] += o[2];
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) sum[w][a][lane] = s[a];
+    __syncthreads();
+    if (w >= 3 || t >= n_t) return;
+    double r = sum[0][w][lane];
+    for (uint32_t v = 1; v < min((uint32_t)CC_WARPS, chunks); ++v) r += sum[v][w][lane];
+    double* out = w == 0 ? ax : (w == 1 ? ay : az);
+    out[i_begin + t] = r;
 }
 
 // Number and size (a multiple of `tile`) of the source chunks that give at least ~8 warps per SM
@@ -138,49 +277,6 @@ void choose_chunks(const nb_ctx* ctx, int blocks_per_chunk, uint32_t n, uint32_t
     *chunks = (uint32_t)nb::ceil_div(n, *chunk);
 }
 
-// FP64 accelerations of listed target bodies (ax[t] for targets[t]); FMAs + refined rsqrt.
-__global__ void __launch_bounds__(F64_THREADS)
-naive_f64_targets_kernel(const double* __restrict__ m, const double* __restrict__ x,
-                         const double* __restrict__ y, const double* __restrict__ z, uint32_t n,
-                         const uint32_t* __restrict__ targets, uint32_t n_t,
-                         double* __restrict__ ax, double* __restrict__ ay,
-                         double* __restrict__ az, double G, double eps2) {
-    __shared__ double sx[F64_THREADS], sy[F64_THREADS], sz[F64_THREADS], sm[F64_THREADS];
-    const uint32_t t = blockIdx.x * F64_THREADS + threadIdx.x;
-    const bool active = t < n_t;
-    const uint32_t i = active ? targets[t] : 0;
-    const double px = active ? x[i] : 0, py = active ? y[i] : 0, pz = active ? z[i] : 0;
-    double acc_x = 0, acc_y = 0, acc_z = 0;
-    for (uint32_t k = 0; k < n; k += F64_THREADS) {
-        const uint32_t j = k + threadIdx.x;
-        if (j < n) {
-            sx[threadIdx.x] = x[j];
-            sy[threadIdx.x] = y[j];
-            sz[threadIdx.x] = z[j];
-            sm[threadIdx.x] = m[j];
-        }
-        __syncthreads();
-        const uint32_t cnt = min((uint32_t)F64_THREADS, n - k);
-        if (active) {
-#pragma unroll 4
-            for (uint32_t jj = 0; jj < cnt; ++jj) {
-                const double r_x = sx[jj] - px, r_y = sy[jj] - py, r_z = sz[jj] - pz;
-                const double den = fma(r_x, r_x, fma(r_y, r_y, fma(r_z, r_z, eps2)));
-                const double s = nb_m_rinv3_f64(sm[jj], den);
-                acc_x = fma(s, r_x, acc_x);
-                acc_y = fma(s, r_y, acc_y);
-                acc_z = fma(s, r_z, acc_z);
-            }
-        }
-        __syncthreads();
-    }
-    if (active) {
-        ax[t] = acc_x * G;
-        ay[t] = acc_y * G;
-        az[t] = acc_z * G;
-    }
-}
-
 // ---------------------------------------------------------------------------------------------
 // FP32, compensated: the batched pair kernel (nb_pair.cuh) with a batch of one system whose
 // targets are [i_begin, i_end).
@@ -192,9 +288,11 @@ int g_naive_sym_mode = 1;
 int g_naive_sym_cfg[3] = {0, 0, 0};
 // Automatic selection wants at least this many units per persistent CTA (the one-sided kernels
 // spread small systems better) and j-side partials (3 values per unit and tile body) below the
-// cap. With 7, a 16,384-body system takes the FP64 shape (4,2,64) at its 7 resident CTAs per SM
-// (8,320 units over 1,064 CTAs) and the larger (4,4,64) I-block from ~18,000 bodies on.
+// cap.
 constexpr uint64_t SYM_MIN_UNITS_PER_CTA = 7;
+// FP64: from 4 units per CTA on (~9,900 bodies). 12,000 bodies (5.8 units): 0.95 ms against 1.04
+// one-sided, 8,192 (2.8 units): 0.50 either way, 4,096: 0.23 against 0.15.
+constexpr uint64_t SYM_MIN_UNITS_F64 = 4;
 constexpr size_t SYM_PART_CAP_BYTES = (size_t)4 << 30;
 
 // Runs the symmetric kernel of arithmetic form `form` (nb::SymForm) for the whole system when
@@ -205,17 +303,15 @@ nb_status naive_sym(nb_ctx* ctx, int form, const double* m, const double* x, con
     *done = false;
     if (g_naive_sym_mode == 0) return NB_OK;
     // candidate shapes: the configured one, except in the automatic mode of the FP64 and
-    // double-float forms, where shape 1 is (4,4,64) with 512-body I-blocks and shape 0 (4,2,64)
-    // with 256: FP64 prefers the larger I-block (same speed, half the partials: 24 bytes per
-    // unit and tile body), double-float the smaller one (faster: fewer registers per thread)
+    // double-float forms, which take shape 0 (4,2,64) with 256-body I-blocks (fewer registers per
+    // thread); where its partials do not fit, double-float takes shape 1 (4,4,64) with 512, FP64 the
+    // one-sided kernel (as fast as its shape 1)
     int cand[2] = {g_naive_sym_cfg[form], -1};
-    if (g_naive_sym_mode == 1 && form == nb::SYM_F64) {
-        cand[0] = 1;
-        cand[1] = 0;
-    } else if (g_naive_sym_mode == 1 && form == nb::SYM_DF) {
+    if (g_naive_sym_mode == 1 && form != nb::SYM_F32) {
         cand[0] = 0;
-        cand[1] = 1;
+        cand[1] = form == nb::SYM_DF ? 1 : -1;
     }
+    const uint64_t min_units = form == nb::SYM_F64 ? SYM_MIN_UNITS_F64 : SYM_MIN_UNITS_PER_CTA;
     int cfg = -1;
     nb::SymHostPlan hp;
     size_t pj_bytes = 0;
@@ -223,7 +319,7 @@ nb_status naive_sym(nb_ctx* ctx, int form, const double* m, const double* x, con
         if (c < 0) break;
         NB_TRY(nb::sym_host_plan(form, c, &n, 1, ctx->sm_count, &hp));
         pj_bytes = nb::sym_part_j_bytes(form, c, hp.units);
-        if (g_naive_sym_mode == 2 || (hp.units >= SYM_MIN_UNITS_PER_CTA * hp.ctas &&
+        if (g_naive_sym_mode == 2 || (hp.units >= min_units * hp.ctas &&
                                       pj_bytes <= SYM_PART_CAP_BYTES)) {
             cfg = c;
             break;
@@ -248,6 +344,11 @@ nb_status naive_sym(nb_ctx* ctx, int form, const double* m, const double* x, con
     S.n_records = hp.n_records;
     S.units = hp.units;
     S.wait_limit = ctx->wait_limit;
+    S.k_part = ctx->dev_counter + NB_COUNTER_SCALE;
+    S.k_words = 0;
+    if (form == nb::SYM_F64)
+        NB_TRY(nb::launch_scale(x, y, z, n, ctx->dev_counter + NB_COUNTER_SCALE, &S.k_words,
+                                stream));
     b += table_bytes;
     *done = true;
     return nb::sym_launch(form, cfg, S, m, x, y, z, G, eps2, b, b + src_bytes,
@@ -436,8 +537,54 @@ nb_status naive_df64(nb_ctx* ctx, const double* m, const double* x, const double
         src, n, i_begin, i_end, chunk, e2h, e2l, ax, ay, az, part);
     NB_TRY(nb::check_launch("naive_df_kernel"));
     if (chunks == 1) return NB_OK;
-    chunk_combine_kernel<<<nb::ceil_div(n_t, 256), 256, 0, stream>>>(part, chunks, i_begin,
+    chunk_combine_kernel<<<nb::ceil_div(n_t, 32), 32 * CC_WARPS, 0, stream>>>(part, chunks, i_begin,
                                                                      i_end, ax, ay, az);
+    return nb::check_launch("chunk_combine_kernel");
+}
+
+// One-sided NB_F64 for the n_t targets i_begin .. or the listed ones (whose results are packed).
+nb_status naive_fix(nb_ctx* ctx, const double* m, const double* x, const double* y,
+                    const double* z, double* ax, double* ay, double* az, uint32_t n,
+                    const uint32_t* targets, uint32_t i_begin, uint32_t n_t, double G, double eps2,
+                    cudaStream_t stream) {
+    uint32_t* k_part = ctx->dev_counter + NB_COUNTER_SCALE;
+    uint32_t k_words = 0;
+    NB_TRY(nb::launch_scale(x, y, z, n, k_part, &k_words, stream));
+    if (n <= FXC_MAX_N) {
+        naive_fix_cluster_kernel<<<nb::ceil_div(n_t, 32) * FXC_CTAS, FXC_THREADS, 0, stream>>>(
+            m, x, y, z, ax, ay, az, n, targets, i_begin, n_t, G, eps2, k_part, k_words);
+        return nb::check_launch("naive_fix_cluster_kernel");
+    }
+    const int blocks = nb::ceil_div(n_t, FX_THREADS);
+    uint32_t chunks = (uint32_t)std::min<long long>(
+        nb::ceil_div(FX_GRID_PER_SM * ctx->sm_count, blocks), FX_CHUNKS_MAX);
+    uint32_t chunk = std::max<uint32_t>((uint32_t)nb::ceil_div(n, chunks), FX_CHUNK_MIN);
+    if (chunk > FX_THREADS) chunk = (uint32_t)nb::ceil_div(chunk, FX_THREADS) * FX_THREADS;
+    chunks = (uint32_t)nb::ceil_div(n, chunk);
+    size_t part_bytes = chunks > 1 ? (size_t)chunks * n_t * 3 * sizeof(double) : 0;
+    if (part_bytes > ctx->scratch[NB_SCRATCH_NAIVE_DF].bytes) {
+        // a stream being captured cannot wait for an allocation: one chunk needs none
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        NB_CUDA_TRY(cudaStreamIsCapturing(stream, &capture));
+        if (capture != cudaStreamCaptureStatusNone) {
+            chunk = (uint32_t)nb::ceil_div(n, FX_THREADS) * FX_THREADS;
+            chunks = 1;
+            part_bytes = 0;
+        }
+    }
+    double* part = nullptr;
+    if (chunks > 1) {
+        void* base = nullptr;
+        NB_TRY(nb::scratch(ctx, NB_SCRATCH_NAIVE_DF, part_bytes, &base));
+        part = (double*)base;
+    }
+    naive_fix_kernel<<<dim3(blocks, chunks), FX_THREADS, 0, stream>>>(
+        m, x, y, z, ax, ay, az, n, targets, i_begin, n_t, G, eps2, chunk, part, k_part, k_words);
+    NB_TRY(nb::check_launch("naive_fix_kernel"));
+    if (chunks == 1) return NB_OK;
+    const uint32_t first = targets != nullptr ? 0 : i_begin;
+    chunk_combine_kernel<<<nb::ceil_div(n_t, 32), 32 * CC_WARPS, 0, stream>>>(part, chunks, first,
+                                                                     first + n_t, ax, ay, az);
     return nb::check_launch("chunk_combine_kernel");
 }
 
@@ -453,9 +600,9 @@ nb_status naive_dispatch(nb_ctx* ctx, const double* m, const double* x, const do
     const uint32_t n_t = i_end - i_begin;
     switch (prec) {
         case NB_F64_IEEE:
-            naive_f64_kernel<true><<<nb::ceil_div(n_t, F64_THREADS), F64_THREADS, 0, stream>>>(
-                m, x, y, z, ax, ay, az, n, i_begin, i_end, G, eps2, n, nullptr);
-            return nb::check_launch("naive_f64_kernel<ieee>");
+            naive_ieee_kernel<<<nb::ceil_div(n_t, F64_THREADS), F64_THREADS, 0, stream>>>(
+                m, x, y, z, ax, ay, az, n, i_begin, i_end, G, eps2);
+            return nb::check_launch("naive_ieee_kernel");
         case NB_F64: {
             if (i_begin == 0 && i_end == n) {
                 bool done = false;
@@ -463,22 +610,8 @@ nb_status naive_dispatch(nb_ctx* ctx, const double* m, const double* x, const do
                                  &done));
                 if (done) return NB_OK;
             }
-            const int blocks = nb::ceil_div(n_t, F64_THREADS);
-            uint32_t chunks = 1, chunk = n;
-            choose_chunks(ctx, blocks, n, F64_THREADS, &chunks, &chunk);
-            double* part = nullptr;
-            if (chunks > 1) {
-                void* base = nullptr;
-                NB_TRY(nb::scratch(ctx, NB_SCRATCH_NAIVE_DF, (size_t)chunks * n_t * 3 * 8, &base));
-                part = (double*)base;
-            }
-            naive_f64_kernel<false><<<dim3(blocks, chunks), F64_THREADS, 0, stream>>>(
-                m, x, y, z, ax, ay, az, n, i_begin, i_end, G, eps2, chunk, part);
-            NB_TRY(nb::check_launch("naive_f64_kernel"));
-            if (chunks == 1) return NB_OK;
-            chunk_combine_kernel<<<nb::ceil_div(n_t, 256), 256, 0, stream>>>(part, chunks, i_begin,
-                                                                             i_end, ax, ay, az);
-            return nb::check_launch("chunk_combine_kernel");
+            return naive_fix(ctx, m, x, y, z, ax, ay, az, n, nullptr, i_begin, n_t, G, eps2,
+                             stream);
         }
         case NB_F32C:
             return naive_f32c(ctx, m, x, y, z, ax, ay, az, n, i_begin, i_end, G, eps2, stream);
@@ -519,10 +652,8 @@ nb_status nb_naive_accel_targets(nb_ctx* ctx, const double* m, const double* x, 
     if (!m || !x || !y || !z || !targets || !ax || !ay || !az)
         return nb::set_error(NB_ERR_INVALID_ARG, "nb_naive_accel_targets: null pointer");
     if (n == 0 || n_targets == 0) return NB_OK;
-    naive_f64_targets_kernel<<<nb::ceil_div(n_targets, F64_THREADS), F64_THREADS, 0,
-                               (cudaStream_t)stream>>>(m, x, y, z, n, targets, n_targets, ax, ay,
-                                                       az, G, eps2);
-    return nb::check_launch("naive_f64_targets_kernel");
+    return naive_fix(ctx, m, x, y, z, ax, ay, az, n, targets, 0, n_targets, G, eps2,
+                     (cudaStream_t)stream);
 }
 
 nb_status nb_naive_set_pair_config(int config) {

@@ -6,10 +6,9 @@
 //    3 FMA for r^2 + eps^2, one MUFU rsqrt, 2 multiplies for r^-3, 2 for the two mass factors and
 //    3 FMAs into each body's sums: 16 FP32 instructions and one rsqrt, against 24 and two for the
 //    two ordered pairs one at a time (nb_pair.cuh).
-//  * FP64 (nb_naive_accel NB_F64 over whole systems): the positions and masses as given; r^-3 from
-//    the hardware rsqrt estimate with one correction of its cube (6 FP64 operations), 20 FP64
-//    operations per unordered pair against 32 for the two ordered pairs; G applied once at the end
-//    as in NaiveAlgorithm.cpp:348-351.
+//  * FP64 (nb_naive_accel NB_F64 over whole systems): separation, r^2 + eps^2 and the two m r^-3 in
+//    the fixed point of nb_fix.cuh on the integer pipes, 6 FP64 operations (the sums) per unordered
+//    pair (pair_sym_fix_kernel); G applied once at the end as in NaiveAlgorithm.cpp:348-351.
 //  * Double-float (nb_naive_accel NB_DF64 over whole systems): positions relative to the system's
 //    first body as exact triple-floats and G*m as a double-float; the separation, r^2 + eps^2,
 //    1/r and r^-3 in double-float arithmetic are shared by the two bodies, only the mass products,
@@ -37,6 +36,7 @@
 // sets the timeout bit, drains its copies in flight with bounded waits and returns).
 #include <type_traits>
 
+#include "nb_fix.cuh"
 #include "nb_internal.cuh"
 #include "nb_pair.cuh"
 #include "nb_pair_sym.cuh"
@@ -47,20 +47,6 @@ using nbpair::bulk_g2s;
 using nbpair::mbar_expect_tx;
 using nbpair::mbar_init;
 using nbpair::mbar_wait;
-
-// FP64 source record {x, y, z, m}.
-struct __align__(32) Rec64 {
-    double x, y, z, m;
-};
-
-template <typename R>
-struct RecOf {
-    using type = float4;
-};
-template <>
-struct RecOf<double> {
-    using type = Rec64;
-};
 
 // Largest s in [0, count) with key(s) <= v (key non-decreasing in s, key(0) <= v).
 template <typename F, typename T>
@@ -108,28 +94,42 @@ __device__ __forceinline__ Loc locate(const SymPlan& P, uint64_t u) {
 }
 
 // Source records of all systems, each padded to whole I-blocks. FP32: positions relative to the
-// system's first body (FP64 subtraction, then rounded) and G*m; FP64: positions and m as given.
-// Pad records are massless and far away (they add exactly 0 to every real body).
-template <typename R>
+// system's first body (FP64 subtraction, then rounded) and G*m. Pad records are massless and far
+// away (they add exactly 0 to every real body).
 __global__ void sym_prepare_kernel(SymPlan P, const double* __restrict__ m,
                                    const double* __restrict__ x, const double* __restrict__ y,
                                    const double* __restrict__ z, double G,
-                                   typename RecOf<R>::type* __restrict__ out) {
+                                   float4* __restrict__ out) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= P.n_records) return;
     const uint32_t s = last_le(P.n_systems, r, [&](uint32_t k) { return P.sys[k].poff; });
     const SymSys A = P.sys[s], B = P.sys[s + 1];
     const uint32_t t = r - A.poff;
-    const bool real = t < B.off - A.off;
-    const uint32_t b = A.off + t;
-    if constexpr (std::is_same<R, double>::value) {
-        out[r] = real ? Rec64{x[b], y[b], z[b], m[b]} : Rec64{1e150, 1e150, 1e150, 0.0};
-    } else {
-        const uint32_t a0 = A.off;
-        out[r] = real ? make_float4((float)(x[b] - x[a0]), (float)(y[b] - y[a0]),
-                                    (float)(z[b] - z[a0]), (float)(G * m[b]))
-                      : make_float4(1e18f, 1e18f, 1e18f, 0.f);
+    const uint32_t b = A.off + t, a0 = A.off;
+    out[r] = t < B.off - A.off
+                 ? make_float4((float)(x[b] - x[a0]), (float)(y[b] - y[a0]),
+                               (float)(z[b] - z[a0]), (float)(G * m[b]))
+                 : make_float4(1e18f, 1e18f, 1e18f, 0.f);
+}
+
+// FP64 form: the bodies in fixed point; pad records are refused by the pair arithmetic (NO_EXP).
+__global__ void sym_prepare_fix_kernel(SymPlan P, const double* __restrict__ m,
+                                       const double* __restrict__ x, const double* __restrict__ y,
+                                       const double* __restrict__ z,
+                                       nbfix::FixRec* __restrict__ out) {
+    const int K = nbfix::block_scale(x, y, z, P.n_total, P.k_part, P.k_words);
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= P.n_records) return;
+    const uint32_t s = last_le(P.n_systems, r, [&](uint32_t k) { return P.sys[k].poff; });
+    const SymSys A = P.sys[s], B = P.sys[s + 1];
+    const uint32_t t = r - A.poff;
+    nbfix::FixRec o{};
+    o.e = nbfix::NO_EXP;
+    if (t < B.off - A.off) {
+        const uint32_t b = A.off + t;
+        o = nbfix::make_rec(x[b], y[b], z[b], m[b], K);
     }
+    out[r] = o;
 }
 
 // The table of a single system of n bodies (nb I-blocks, `records` padded records, `units`
@@ -168,49 +168,29 @@ __global__ void sym_prepare_tf_kernel(SymPlan P, const double* __restrict__ m,
     out[r] = o;
 }
 
-template <typename R>
-__device__ __forceinline__ R fma_r(R a, R b, R c) {
-    if constexpr (std::is_same<R, float>::value) return fmaf(a, b, c); else return fma(a, b, c);
-}
-
-// den^(-3/2) in FP64: hardware estimate y0 of den^(-1/2) and one correction of its cube,
-// (1 - e)^(-3/2) = 1 + 3e/2 + 15e^2/8 + O(e^3) with e = 1 - den y0^2 (|e| < 2^-21, dropped terms
-// below 2^-62): 6 FP64 operations.
-__device__ __forceinline__ double nb_rinv3_f64(double den) {
-    double y0;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(den));
-    const double y2 = y0 * y0;
-    const double e = fma(-den, y2, 1.0);
-    const double p = fma(1.875, e, 1.5);
-    const double w0 = y2 * y0;
-    return fma(w0 * e, p, w0);
-}
-
-// Shared memory of a shape: two j-tiles, two buffers of per-warp j sums and, for FP32, the
-// compensated i sums.
-template <typename R, int W, int P, int JT>
+// Shared memory of a shape: two j-tiles, two buffers of per-warp j sums and the compensated i sums.
+template <int W, int P, int JT>
 constexpr size_t sym_smem_bytes() {
-    return 2 * JT * sizeof(typename RecOf<R>::type) + (size_t)2 * W * 3 * JT * sizeof(R) +
-           (std::is_same<R, float>::value ? (size_t)6 * P * 32 * W * sizeof(float) : 0);
+    return 2 * JT * sizeof(float4) + (size_t)2 * W * 3 * JT * sizeof(float) +
+           (size_t)6 * P * 32 * W * sizeof(float);
 }
 
-template <typename R, int W, int P, int JT>
+template <int W, int P, int JT>
 __global__ void __launch_bounds__(32 * W)
-pair_sym_kernel(SymPlan S, const typename RecOf<R>::type* __restrict__ src, R eps2,
-                R* __restrict__ part_i, R* __restrict__ part_j, uint32_t* __restrict__ err_word) {
-    using Rec = typename RecOf<R>::type;
-    constexpr bool F64 = std::is_same<R, double>::value;
+pair_sym_kernel(SymPlan S, const float4* __restrict__ src, float eps2,
+                float* __restrict__ part_i, float* __restrict__ part_j, uint32_t* __restrict__ err_word) {
     constexpr int THREADS = 32 * W;
     constexpr int IB = THREADS * P;
     constexpr uint32_t TPB = IB / JT;
     static_assert(IB % JT == 0 && JT % 32 == 0, "tile shape");
     extern __shared__ __align__(128) unsigned char sym_smem[];
-    Rec (*tile)[JT] = reinterpret_cast<Rec (*)[JT]>(sym_smem);
+    float4 (*tile)[JT] = reinterpret_cast<float4 (*)[JT]>(sym_smem);
     // per-warp j sums of the current unit, two buffers (alternating units)
-    R (*jacc)[W][3][JT] = reinterpret_cast<R (*)[W][3][JT]>(sym_smem + 2 * JT * sizeof(Rec));
-    // FP32: compensated i sums hl[c][k][thread], c = hx, hy, hz, lx, ly, lz
+    float (*jacc)[W][3][JT] =
+        reinterpret_cast<float (*)[W][3][JT]>(sym_smem + 2 * JT * sizeof(float4));
+    // compensated i sums hl[c][k][thread], c = hx, hy, hz, lx, ly, lz
     float (*hl)[P][THREADS] = reinterpret_cast<float (*)[P][THREADS]>(
-        sym_smem + 2 * JT * sizeof(Rec) + (size_t)2 * W * 3 * JT * sizeof(R));
+        sym_smem + 2 * JT * sizeof(float4) + (size_t)2 * W * 3 * JT * sizeof(float));
     __shared__ __align__(8) uint64_t full[2];
 
     const uint32_t cta = blockIdx.x;
@@ -226,8 +206,8 @@ pair_sym_kernel(SymPlan S, const typename RecOf<R>::type* __restrict__ src, R ep
     uint64_t c_u = u0;
     auto issue = [&](int buf) {
         const Loc L = locate<TPB, JT>(S, c_u);
-        mbar_expect_tx(&full[buf], JT * (uint32_t)sizeof(Rec));
-        bulk_g2s(&tile[buf][0], src + L.poff + (size_t)L.jt * JT, JT * (uint32_t)sizeof(Rec),
+        mbar_expect_tx(&full[buf], JT * (uint32_t)sizeof(float4));
+        bulk_g2s(&tile[buf][0], src + L.poff + (size_t)L.jt * JT, JT * (uint32_t)sizeof(float4),
                  &full[buf]);
         ++c_u;
     };
@@ -237,7 +217,7 @@ pair_sym_kernel(SymPlan S, const typename RecOf<R>::type* __restrict__ src, R ep
     }
 
     const int th = threadIdx.x, lane = th & 31, w = th >> 5;
-    R xi[P], yi[P], zi[P], mi[P], fx[P], fy[P], fz[P];
+    float xi[P], yi[P], zi[P], mi[P], fx[P], fy[P], fz[P];
     uint64_t u = u0;
     uint32_t iter = 0;
     bool failed = false;
@@ -246,21 +226,16 @@ pair_sym_kernel(SymPlan S, const typename RecOf<R>::type* __restrict__ src, R ep
         const uint32_t a = L.a;
         const uint64_t seg_end = min(u1, L.ubase + row_off(L.n_jt, TPB, a + 1));
         uint32_t jt = L.jt;
-        const Rec* isrc = src + L.poff + (size_t)a * IB + w * 32 * P + lane;
+        const float4* isrc = src + L.poff + (size_t)a * IB + w * 32 * P + lane;
 #pragma unroll
         for (int k = 0; k < P; ++k) {
-            const Rec b = isrc[k * 32];
+            const float4 b = isrc[k * 32];
             xi[k] = b.x;
             yi[k] = b.y;
             zi[k] = b.z;
-            if constexpr (F64) {
-                mi[k] = b.m;
-                fx[k] = fy[k] = fz[k] = 0.0;
-            } else {
-                mi[k] = b.w;
+            mi[k] = b.w;
 #pragma unroll
-                for (int c = 0; c < 6; ++c) hl[c][k][th] = 0.f;
-            }
+            for (int c = 0; c < 6; ++c) hl[c][k][th] = 0.f;
         }
         for (; u < seg_end; ++u, ++iter, ++jt) {
             const int buf = iter & 1;
@@ -269,37 +244,28 @@ pair_sym_kernel(SymPlan S, const typename RecOf<R>::type* __restrict__ src, R ep
                 failed = true;
                 break;
             }
-            if constexpr (!F64) {
 #pragma unroll
-                for (int k = 0; k < P; ++k) fx[k] = fy[k] = fz[k] = 0.f;
-            }
+            for (int k = 0; k < P; ++k) fx[k] = fy[k] = fz[k] = 0.f;
 #pragma unroll 1
             for (int g = 0; g < JT / 32; ++g) {
-                const Rec* G4 = &tile[buf][g * 32];
-                R jx = 0, jy = 0, jz = 0;  // sums of body (lane + s) mod 32 of the group
+                const float4* G4 = &tile[buf][g * 32];
+                float jx = 0, jy = 0, jz = 0;  // sums of body (lane + s) mod 32 of the group
 #pragma unroll 8
                 for (int s = 0; s < 32; ++s) {
-                    const Rec J = G4[(lane + s) & 31];
-                    R jm;
-                    if constexpr (F64) jm = J.m; else jm = J.w;
+                    const float4 J = G4[(lane + s) & 31];
 #pragma unroll
                     for (int k = 0; k < P; ++k) {
-                        const R dx = J.x - xi[k], dy = J.y - yi[k], dz = J.z - zi[k];
-                        R inv3;
-                        if constexpr (F64) {
-                            inv3 = nb_rinv3_f64(fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
-                        } else {
-                            const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-                            const float inv = nb_rsqrt_f32(r2);
-                            inv3 = (inv * inv) * inv;
-                        }
-                        const R sj = jm * inv3, si = mi[k] * inv3;
-                        fx[k] = fma_r(dx, sj, fx[k]);
-                        fy[k] = fma_r(dy, sj, fy[k]);
-                        fz[k] = fma_r(dz, sj, fz[k]);
-                        jx = fma_r(-dx, si, jx);
-                        jy = fma_r(-dy, si, jy);
-                        jz = fma_r(-dz, si, jz);
+                        const float dx = J.x - xi[k], dy = J.y - yi[k], dz = J.z - zi[k];
+                        const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
+                        const float inv = nb_rsqrt_f32(r2);
+                        const float inv3 = (inv * inv) * inv;
+                        const float sj = J.w * inv3, si = mi[k] * inv3;
+                        fx[k] = fmaf(dx, sj, fx[k]);
+                        fy[k] = fmaf(dy, sj, fy[k]);
+                        fz[k] = fmaf(dz, sj, fz[k]);
+                        jx = fmaf(-dx, si, jx);
+                        jy = fmaf(-dy, si, jy);
+                        jz = fmaf(-dz, si, jz);
                     }
                     // the sum of body (l + s + 1) mod 32 comes from lane l + 1
                     jx = __shfl_sync(0xffffffffu, jx, (lane + 1) & 31);
@@ -311,29 +277,27 @@ pair_sym_kernel(SymPlan S, const typename RecOf<R>::type* __restrict__ src, R ep
                 jacc[buf][w][1][g * 32 + lane] = jy;
                 jacc[buf][w][2][g * 32 + lane] = jz;
             }
-            if constexpr (!F64) {
 #pragma unroll
-                for (int k = 0; k < P; ++k) {
-                    float h0 = hl[0][k][th], h1 = hl[1][k][th], h2 = hl[2][k][th];
-                    float l0 = hl[3][k][th], l1 = hl[4][k][th], l2 = hl[5][k][th];
-                    NB_TWOSUM(h0, l0, fx[k]);
-                    NB_TWOSUM(h1, l1, fy[k]);
-                    NB_TWOSUM(h2, l2, fz[k]);
-                    hl[0][k][th] = h0;
-                    hl[1][k][th] = h1;
-                    hl[2][k][th] = h2;
-                    hl[3][k][th] = l0;
-                    hl[4][k][th] = l1;
-                    hl[5][k][th] = l2;
-                }
+            for (int k = 0; k < P; ++k) {
+                float h0 = hl[0][k][th], h1 = hl[1][k][th], h2 = hl[2][k][th];
+                float l0 = hl[3][k][th], l1 = hl[4][k][th], l2 = hl[5][k][th];
+                NB_TWOSUM(h0, l0, fx[k]);
+                NB_TWOSUM(h1, l1, fy[k]);
+                NB_TWOSUM(h2, l2, fz[k]);
+                hl[0][k][th] = h0;
+                hl[1][k][th] = h1;
+                hl[2][k][th] = h2;
+                hl[3][k][th] = l0;
+                hl[4][k][th] = l1;
+                hl[5][k][th] = l2;
             }
             __syncthreads();
             if (jt >= (a + 1) * TPB) {  // above the diagonal: the j sums of this unit
-                R* out = part_j + u * 3 * JT;
+                float* out = part_j + u * 3 * JT;
                 for (int jl = th; jl < JT; jl += THREADS) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        R s = jacc[buf][0][c][jl];
+                        float s = jacc[buf][0][c][jl];
 #pragma unroll
                         for (int v = 1; v < W; ++v) s += jacc[buf][v][c][jl];
                         out[c * JT + jl] = s;
@@ -343,20 +307,195 @@ pair_sym_kernel(SymPlan S, const typename RecOf<R>::type* __restrict__ src, R ep
             if (threadIdx.x == 0 && u + 2 < u1) issue(buf);  // the cursor is at u + 2
         }
         if (failed) break;
-        if constexpr (F64) {
-            R* out = part_i + (size_t)(cta + L.bbase + a) * 3 * IB + w * 32 * P + lane;
+        float* out = part_i + (size_t)(cta + L.bbase + a) * 6 * IB + w * 32 * P + lane;
 #pragma unroll
-            for (int k = 0; k < P; ++k) {
-                out[0 * IB + k * 32] = fx[k];
-                out[1 * IB + k * 32] = fy[k];
-                out[2 * IB + k * 32] = fz[k];
+        for (int k = 0; k < P; ++k)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) out[c * IB + k * 32] = hl[c][k][th];
+    }
+    if (failed) {  // drain the copies of units iter, iter + 1 before leaving (default limit)
+        bool drained = true;
+        for (uint32_t k = iter; k < iter + 2 && u0 + k < u1; ++k)
+            drained &= mbar_wait(&full[k & 1], (k >> 1) & 1, NB_WAIT_LIMIT_DEFAULT);
+        if (threadIdx.x == 0)
+            atomicOr(err_word, NB_DEVERR_TIMEOUT | (drained ? 0u : NB_DEVERR_DRAIN));
+    }
+}
+
+// FP64 form: the pair's separation, r^2 + eps^2 and r^-3 in fixed point (nb_fix.cuh), shared by the
+// two bodies, and a mass product each; FP64 sums, kept in registers for a whole row segment (i) or
+// rotated through the lanes (j). Pairs the fixed point cannot hold are added one side at a time.
+//  Bound: the FP64 pipe, 92% busy with 3 FMAs per ordered pair (10 FP64 operations before).
+//  65,536 bodies 76.8 -> 26.7 ms (56 -> 161 Gpairs/s), 16,384 4.96 -> 1.72 ms. Registers for 20 warps
+//  per SM: 12, 16 and 24 warps measured 15%, 3% and 2% slower.
+constexpr int FIX_WARPS_PER_SM = 20;
+
+template <int W, int P, int JT>
+constexpr size_t sym_fix_smem_bytes() {
+    return 2 * JT * sizeof(nbfix::FixRec) + (size_t)2 * W * 3 * JT * sizeof(double);
+}
+
+template <int W, int P, int JT>
+__global__ void __launch_bounds__(32 * W, FIX_WARPS_PER_SM / W)
+pair_sym_fix_kernel(SymPlan S, const nbfix::FixRec* __restrict__ src,
+                    const double* __restrict__ m, const double* __restrict__ x,
+                    const double* __restrict__ y, const double* __restrict__ z, double eps2,
+                    double* __restrict__ part_i, double* __restrict__ part_j,
+                    uint32_t* __restrict__ err_word) {
+    constexpr int THREADS = 32 * W;
+    constexpr int IB = THREADS * P;
+    constexpr uint32_t TPB = IB / JT;
+    static_assert(IB % JT == 0 && JT % 32 == 0, "tile shape");
+    extern __shared__ __align__(128) unsigned char sym_smem[];
+    nbfix::FixRec (*tile)[JT] = reinterpret_cast<nbfix::FixRec (*)[JT]>(sym_smem);
+    double (*jacc)[W][3][JT] =
+        reinterpret_cast<double (*)[W][3][JT]>(sym_smem + 2 * JT * sizeof(nbfix::FixRec));
+    __shared__ __align__(8) uint64_t full[2];
+    __shared__ nbfix::Eps2Table e2;
+    const int K = nbfix::block_scale(x, y, z, S.n_total, S.k_part, S.k_words);
+    nbfix::fill_eps2(e2, eps2, K);
+
+    const uint32_t cta = blockIdx.x;
+    const uint64_t u0 = unit_begin(S, cta), u1 = unit_begin(S, cta + 1);
+    if (u0 >= u1) return;
+    if (threadIdx.x == 0) {
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    uint64_t c_u = u0;
+    auto issue = [&](int buf) {
+        const Loc L = locate<TPB, JT>(S, c_u);
+        mbar_expect_tx(&full[buf], JT * (uint32_t)sizeof(nbfix::FixRec));
+        bulk_g2s(&tile[buf][0], src + L.poff + (size_t)L.jt * JT, JT * (uint32_t)sizeof(nbfix::FixRec),
+                 &full[buf]);
+        ++c_u;
+    };
+    if (threadIdx.x == 0) {
+        issue(0);
+        if (u0 + 1 < u1) issue(1);
+    }
+
+    const int th = threadIdx.x, lane = th & 31, w = th >> 5;
+    const int sh_max = e2.sh_max;
+    nbfix::FixRec I[P];
+    double tx[P], ty[P], tz[P];
+    // Adds the pair (source at record f, body b) seen from the body `at` (record t) in FP64 or by
+    // the one-sided arithmetic: the pairs the loop below leaves.
+    auto one_side = [&](const nbfix::FixRec& f, uint32_t b, const nbfix::FixRec& t, uint32_t at,
+                        double& sx, double& sy, double& sz) {
+        const nbfix::Fix3 p{t.x2, t.y2, t.z2, t.x1, t.y1, t.z1, t.x0, t.y0, t.z0};
+        const int lim = t.e == nbfix::NO_EXP ? -1 : sh_max;
+        double w, dx, dy, dz;
+        if (lim < 0 || !nbfix::term(f, p, K, e2, lim, w, dx, dy, dz)) {
+            if (nbfix::adds_nothing(f, b == at, K, lim, eps2)) return;
+            dx = x[b] - x[at];
+            dy = y[b] - y[at];
+            dz = z[b] - z[at];
+            w = nb_m_rinv3_f64(m[b], fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
+        }
+        sx = fma(w, dx, sx);
+        sy = fma(w, dy, sy);
+        sz = fma(w, dz, sz);
+    };
+    uint64_t u = u0;
+    uint32_t iter = 0;
+    bool failed = false;
+    while (u < u1 && !failed) {
+        const Loc L = locate<TPB, JT>(S, u);
+        const uint32_t a = L.a;
+        const uint64_t seg_end = min(u1, L.ubase + row_off(L.n_jt, TPB, a + 1));
+        uint32_t jt = L.jt;
+        const uint32_t off = S.sys[L.s].off, count = S.sys[L.s + 1].off - off;
+        const nbfix::FixRec* isrc = src + L.poff + (size_t)a * IB + w * 32 * P + lane;
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            I[k] = isrc[k * 32];
+            tx[k] = ty[k] = tz[k] = 0.0;
+        }
+        for (; u < seg_end; ++u, ++iter, ++jt) {
+            const int buf = iter & 1;
+            const bool ok = mbar_wait(&full[buf], (iter >> 1) & 1, S.wait_limit);
+            if (__syncthreads_or(!ok)) {
+                failed = true;
+                break;
             }
-        } else {
-            R* out = part_i + (size_t)(cta + L.bbase + a) * 6 * IB + w * 32 * P + lane;
+#pragma unroll 1
+            for (int g = 0; g < JT / 32; ++g) {
+                const nbfix::FixRec* G4 = &tile[buf][g * 32];
+                double jx = 0.0, jy = 0.0, jz = 0.0;  // sums of body (lane + s) mod 32 of the group
+#pragma unroll 1
+                for (int s = 0; s < 32; ++s) {
+                    const nbfix::FixRec J = G4[(lane + s) & 31];
+                    const nbfix::Fix3 jp{J.x2, J.y2, J.z2, J.x1, J.y1, J.z1, J.x0, J.y0, J.z0};
 #pragma unroll
-            for (int k = 0; k < P; ++k)
+                    for (int k = 0; k < P; ++k) {
+                        const nbfix::Fix3 ip{I[k].x2, I[k].y2, I[k].z2, I[k].x1, I[k].y1,
+                                             I[k].z1, I[k].x0, I[k].y0, I[k].z0};
+                        nbfix::Sep sep;
+                        bool ok = min(J.e, I[k].e) > nbfix::ZERO_MASS && sh_max >= 0;
+                        if (ok) ok = nbfix::separation(jp, ip, sh_max, sep);
+                        if (ok) {
+                            const uint64_t inv3 =
+                                nbfix::rinv3(nbfix::norm2(sep) + e2.units[sep.sh]);
+                            bool oj, oi;
+                            const double sj = nbfix::mass_rinv3(inv3, J.mh, J.ml, J.e, sep.sh, oj);
+                            const double si = nbfix::mass_rinv3(inv3, I[k].mh, I[k].ml, I[k].e,
+                                                                sep.sh, oi);
+                            double dx, dy, dz;
+                            nbfix::axes(sep, K, dx, dy, dz);
+                            ok = oj && oi;
+                            if (ok) {
+                                tx[k] = fma(dx, sj, tx[k]);
+                                ty[k] = fma(dy, sj, ty[k]);
+                                tz[k] = fma(dz, sj, tz[k]);
+                                jx = fma(-dx, si, jx);
+                                jy = fma(-dy, si, jy);
+                                jz = fma(-dz, si, jz);
+                            }
+                        }
+                        if (!ok) {  // pads, and what the fixed point cannot hold
+                            const uint32_t li = a * IB + (w * P + k) * 32 + lane,
+                                           lj = jt * JT + g * 32 + ((lane + s) & 31);
+                            if (li < count && lj < count) {
+                                one_side(J, off + lj, I[k], off + li, tx[k], ty[k], tz[k]);
+                                one_side(I[k], off + li, J, off + lj, jx, jy, jz);
+                            }
+                        }
+                    }
+                    // the sum of body (l + s + 1) mod 32 comes from lane l + 1
+                    jx = __shfl_sync(0xffffffffu, jx, (lane + 1) & 31);
+                    jy = __shfl_sync(0xffffffffu, jy, (lane + 1) & 31);
+                    jz = __shfl_sync(0xffffffffu, jz, (lane + 1) & 31);
+                }
+                // after 32 rotations lane l holds the sum of body l of the group
+                jacc[buf][w][0][g * 32 + lane] = jx;
+                jacc[buf][w][1][g * 32 + lane] = jy;
+                jacc[buf][w][2][g * 32 + lane] = jz;
+            }
+            __syncthreads();
+            if (jt >= (a + 1) * TPB) {  // above the diagonal: the j sums of this unit
+                double* out = part_j + u * 3 * JT;
+                for (int jl = th; jl < JT; jl += THREADS) {
 #pragma unroll
-                for (int c = 0; c < 6; ++c) out[c * IB + k * 32] = hl[c][k][th];
+                    for (int c = 0; c < 3; ++c) {
+                        double s = jacc[buf][0][c][jl];
+#pragma unroll
+                        for (int v = 1; v < W; ++v) s += jacc[buf][v][c][jl];
+                        out[c * JT + jl] = s;
+                    }
+                }
+            }
+            if (threadIdx.x == 0 && u + 2 < u1) issue(buf);  // the cursor is at u + 2
+        }
+        if (failed) break;
+        double* out = part_i + (size_t)(cta + L.bbase + a) * 3 * IB + w * 32 * P + lane;
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            out[0 * IB + k * 32] = tx[k];
+            out[1 * IB + k * 32] = ty[k];
+            out[2 * IB + k * 32] = tz[k];
         }
     }
     if (failed) {  // drain the copies of units iter, iter + 1 before leaving (default limit)
@@ -635,10 +774,16 @@ nb_status occupancy(K kernel, int threads, size_t smem, int* out) {
     return NB_OK;
 }
 
-template <typename R, int W, int P, int JT>
+template <int W, int P, int JT>
 nb_status sym_prepare(int* out) {
-    return occupancy(nbsym::pair_sym_kernel<R, W, P, JT>, 32 * W,
-                     nbsym::sym_smem_bytes<R, W, P, JT>(), out);
+    return occupancy(nbsym::pair_sym_kernel<W, P, JT>, 32 * W, nbsym::sym_smem_bytes<W, P, JT>(),
+                     out);
+}
+
+template <int W, int P, int JT>
+nb_status sym_fix_prepare(int* out) {
+    return occupancy(nbsym::pair_sym_fix_kernel<W, P, JT>, 32 * W,
+                     nbsym::sym_fix_smem_bytes<W, P, JT>(), out);
 }
 
 template <int W, int P, int JT>
@@ -647,17 +792,32 @@ nb_status sym_df_prepare(int* out) {
                      nbsym::sym_df_smem_bytes<W, P, JT>(), out);
 }
 
-template <typename R, int W, int P, int JT>
+template <int W, int P, int JT>
 nb_status sym_launch_cfg(const nbsym::SymPlan& S, const void* src, double eps2, void* part_i,
                          void* part_j, double G, double* ax, double* ay, double* az,
                          uint32_t* err_word, cudaStream_t stream) {
-    using Rec = typename nbsym::RecOf<R>::type;
-    nbsym::pair_sym_kernel<R, W, P, JT>
-        <<<S.ctas, 32 * W, nbsym::sym_smem_bytes<R, W, P, JT>(), stream>>>(
-            S, (const Rec*)src, (R)eps2, (R*)part_i, (R*)part_j, err_word);
+    nbsym::pair_sym_kernel<W, P, JT>
+        <<<S.ctas, 32 * W, nbsym::sym_smem_bytes<W, P, JT>(), stream>>>(
+            S, (const float4*)src, (float)eps2, (float*)part_i, (float*)part_j, err_word);
     NB_TRY(check_launch("pair_sym_kernel"));
-    nbsym::sym_combine_kernel<R, 32 * W * P, JT><<<ceil_div(S.n_total, 256), 256, 0, stream>>>(
-        S, (const R*)part_i, (const R*)part_j, G, ax, ay, az);
+    nbsym::sym_combine_kernel<float, 32 * W * P, JT><<<ceil_div(S.n_total, 256), 256, 0, stream>>>(
+        S, (const float*)part_i, (const float*)part_j, G, ax, ay, az);
+    return check_launch("sym_combine_kernel");
+}
+
+template <int W, int P, int JT>
+nb_status sym_fix_launch_cfg(const nbsym::SymPlan& S, const void* src, const double* m,
+                             const double* x, const double* y, const double* z, double eps2,
+                             void* part_i, void* part_j, double G, double* ax, double* ay,
+                             double* az, uint32_t* err_word, cudaStream_t stream) {
+    nbsym::pair_sym_fix_kernel<W, P, JT>
+        <<<S.ctas, 32 * W, nbsym::sym_fix_smem_bytes<W, P, JT>(), stream>>>(
+            S, (const nbfix::FixRec*)src, m, x, y, z, eps2, (double*)part_i, (double*)part_j,
+            err_word);
+    NB_TRY(check_launch("pair_sym_fix_kernel"));
+    nbsym::sym_combine_kernel<double, 32 * W * P, JT>
+        <<<ceil_div(S.n_total, 256), 256, 0, stream>>>(S, (const double*)part_i,
+                                                       (const double*)part_j, G, ax, ay, az);
     return check_launch("sym_combine_kernel");
 }
 
@@ -695,7 +855,7 @@ uint32_t sym_ib(int form, int cfg) {
 }
 
 size_t sym_record_bytes(int form) {
-    return form == SYM_F64 ? sizeof(nbsym::Rec64)
+    return form == SYM_F64 ? sizeof(nbfix::FixRec)
                            : (form == SYM_DF ? sizeof(nbsym::RecTF) : sizeof(float4));
 }
 
@@ -708,7 +868,7 @@ nb_status sym_ctas_per_sm(int form, int cfg, int* out) {
         if (form == SYM_F64) {
             switch (cfg) {
 #define NB_SYM_PREP(i, W, P, JT) \
-    case i: NB_TRY((sym_prepare<double, W, P, JT>(&v))); break;
+    case i: NB_TRY((sym_fix_prepare<W, P, JT>(&v))); break;
                 NB_SYM64_CONFIG_LIST(NB_SYM_PREP)
 #undef NB_SYM_PREP
             }
@@ -722,7 +882,7 @@ nb_status sym_ctas_per_sm(int form, int cfg, int* out) {
         } else {
             switch (cfg) {
 #define NB_SYM_PREP(i, W, P, JT) \
-    case i: NB_TRY((sym_prepare<float, W, P, JT>(&v))); break;
+    case i: NB_TRY((sym_prepare<W, P, JT>(&v))); break;
                 NB_SYM_CONFIG_LIST(NB_SYM_PREP)
 #undef NB_SYM_PREP
             }
@@ -784,22 +944,21 @@ nb_status sym_launch(int form, int cfg, const nbsym::SymPlan& S, const double* m
     if (S.units == 0) return NB_OK;
     const int blocks = ceil_div(S.n_records, 256);
     if (form == SYM_F64) {
-        nbsym::sym_prepare_kernel<double><<<blocks, 256, 0, stream>>>(S, m, x, y, z, G,
-                                                                      (nbsym::Rec64*)src);
+        nbsym::sym_prepare_fix_kernel<<<blocks, 256, 0, stream>>>(S, m, x, y, z,
+                                                                  (nbfix::FixRec*)src);
     } else if (form == SYM_DF) {
         nbsym::sym_prepare_tf_kernel<<<blocks, 256, 0, stream>>>(S, m, x, y, z, G,
                                                                  (nbsym::RecTF*)src);
     } else {
-        nbsym::sym_prepare_kernel<float><<<blocks, 256, 0, stream>>>(S, m, x, y, z, G,
-                                                                     (float4*)src);
+        nbsym::sym_prepare_kernel<<<blocks, 256, 0, stream>>>(S, m, x, y, z, G, (float4*)src);
     }
     NB_TRY(check_launch("sym_prepare_kernel"));
     if (form == SYM_F64) {
         switch (cfg) {
 #define NB_SYM_LAUNCH(i, W, P, JT)                                                          \
     case i:                                                                                 \
-        return sym_launch_cfg<double, W, P, JT>(S, src, eps2, part_i, part_j, G, ax, ay, az, \
-                                                err_word, stream);
+        return sym_fix_launch_cfg<W, P, JT>(S, src, m, x, y, z, eps2, part_i, part_j, G, ax, ay,    \
+                                            az, err_word, stream);
             NB_SYM64_CONFIG_LIST(NB_SYM_LAUNCH)
 #undef NB_SYM_LAUNCH
         }
@@ -816,8 +975,8 @@ nb_status sym_launch(int form, int cfg, const nbsym::SymPlan& S, const double* m
         switch (cfg) {
 #define NB_SYM_LAUNCH(i, W, P, JT)                                                          \
     case i:                                                                                 \
-        return sym_launch_cfg<float, W, P, JT>(S, src, eps2, part_i, part_j, G, ax, ay, az, \
-                                               err_word, stream);
+        return sym_launch_cfg<W, P, JT>(S, src, eps2, part_i, part_j, G, ax, ay, az, err_word,      \
+                                        stream);
             NB_SYM_CONFIG_LIST(NB_SYM_LAUNCH)
 #undef NB_SYM_LAUNCH
         }

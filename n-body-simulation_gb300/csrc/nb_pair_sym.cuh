@@ -21,6 +21,8 @@ struct SymPlan {
     uint32_t n_systems, ctas, n_total, n_records;
     uint64_t units;
     unsigned long long wait_limit;  // polls of a tile wait before it gives up (context's limit)
+    const uint32_t* k_part;         // FP64 form: words of nbfix::block_scale and their number
+    uint32_t k_words;
 };
 
 // First unit of I-block a of a system with n_jt j-tiles (row a holds the j-tiles a * tpb ..
@@ -50,7 +52,7 @@ extern const SymConfig kSym64Configs[NB_SYM64_CONFIGS];
 extern const SymConfig kSymDfConfigs[NB_SYMDF_CONFIGS];
 int sym_config_count(int form);
 
-// Bodies per I-block of a shape, and bytes per source record (16 FP32, 32 FP64, 48 double-float).
+// Bodies per I-block of a shape, and bytes per source record (16 FP32, 48 FP64 and double-float).
 uint32_t sym_ib(int form, int cfg);
 size_t sym_record_bytes(int form);
 

@@ -23,7 +23,7 @@ extern "C" int fix_pair(const double* c, const double* p, double m, double eps2,
     const int K = k_of(v_max);
     Fix3 P;
     const FixRec r = make_rec(c[0], c[1], c[2], m, K);
-    if (!split3(p[0], p[1], p[2], K, P) || r.e == NO_EXP) return 0;
+    if (!split3(p[0], p[1], p[2], K, P) || r.e <= ZERO_MASS) return 0;
     int sh_max = -1;
     while (sh_max < SH_MAX && eps2 >= 0 && eps2_units(eps2, K, sh_max + 1) < EPS2_LIMIT) ++sh_max;
     if (sh_max < 0) return 0;

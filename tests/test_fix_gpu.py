@@ -133,3 +133,83 @@ def test_energy(ctx, kind, n, scale):
     o = oracle.energy(*[d[k] for k in keys], d["G"])
     want = np.array([o["kinetic"], o["potential"], o["total"]])
     assert np.all(np.abs(got[:3] - want) <= 1e-12 * np.abs(want[:2]).max()), (got, want)
+
+
+# -- all pairs: naive_fix_kernel against the IEEE kernel (tolerance as for the tree: A = n terms) ---
+def naive(ctx, d, eps2, precision, rng=None, targets=None):
+    import torch
+    n = len(d["m"])
+    a = [torch.full((n,), 7.0, dtype=torch.float64, device="cuda") for _ in range(3)]
+    t = [dev(d[k]) for k in ("m", "x", "y", "z")]
+    if targets is not None:
+        tg = torch.as_tensor(targets.astype(np.int32), device="cuda")
+        a = [v[:len(targets)].clone() for v in a]
+        ctx.naive_accel_targets(*t, tg, *a, d["G"], eps2)
+    elif rng is None:
+        ctx.naive_accel(*t, *a, d["G"], eps2, precision)
+    else:
+        ctx.naive_accel_range(*t, *a, *rng, d["G"], eps2, precision)
+    ctx.sync()
+    return [host(v) for v in a]
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 255, 256, 257, 512, 513, 2048, 2049, 5000])
+@pytest.mark.parametrize("eps2", [1e-22, 1e-4, 1e9])
+def test_naive_sizes(ctx, n, eps2):
+    d = bodies("plummer", n, seed=n)
+    got, ref = naive(ctx, d, eps2, "f64"), naive(ctx, d, eps2, "f64_ieee")
+    if n > 1:
+        assert rel_err(*got, *ref).max() <= 1e-12
+    else:
+        assert all((g == 0).all() for g in got)
+
+
+def test_naive_ranges_targets_and_special_bodies(ctx):
+    d = bodies("plummer", 3001, seed=2)
+    rng = np.random.default_rng(1)
+    for k in ("x", "y", "z"):  # pairs down to the last bits of the coordinates
+        d[k][1:3001:4] = d[k][0:3000:4] * (1 + rng.choice((-1, 1), 750) * 10.0 ** rng.uniform(-15, -7, 750))
+    d["m"][5::50] = 0.0
+    d["m"][7::50] = -d["m"][7::50]
+    d["m"][9::50] = 1e-310
+    d["z"][2::4] *= 1e-9
+    ref = naive(ctx, d, 1e-20, "f64_ieee")
+    got = naive(ctx, d, 1e-20, "f64")
+    assert rel_err(*got, *ref).max() <= 1e-12
+    part = naive(ctx, d, 1e-20, "f64", rng=(1000, 1777))
+    for g, p, r in zip(got, part, ref):
+        assert (p[:1000] == 7.0).all() and (p[1777:] == 7.0).all()
+    assert rel_err(*[p[1000:1777] for p in part], *[r[1000:1777] for r in ref]).max() <= 1e-12
+    tg = rng.choice(3001, size=300, replace=False)
+    some = naive(ctx, d, 1e-20, "f64", targets=tg)
+    assert rel_err(*some, *[r[tg] for r in ref]).max() <= 1e-12
+
+
+def test_naive_without_softening_and_without_mass(ctx):
+    """The self pair without softening is 0 * inf, in NB_F64 as in the IEEE arithmetic; a system
+    without mass has no acceleration."""
+    d = bodies("plummer", 300, seed=3)
+    assert all(np.isnan(v).all() for v in naive(ctx, d, 0.0, "f64_ieee"))
+    assert all(np.isnan(v).all() for v in naive(ctx, d, 0.0, "f64"))
+    d["m"][:] = 0.0
+    assert all((v == 0).all() for v in naive(ctx, d, 1e-6, "f64"))
+
+
+def test_naive_in_a_capture_without_scratch():
+    """The first NB_F64 call of a context may be captured: it then needs no allocation."""
+    import torch
+    from nbody.lib import Context
+    c = Context(0)
+    d = bodies("plummer", 3000, seed=4)
+    t = [dev(d[k]) for k in ("m", "x", "y", "z")]
+    a = [torch.zeros(3000, dtype=torch.float64, device="cuda") for _ in range(3)]
+    tg = torch.arange(3000, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        c.naive_accel_targets(*t, tg, *a, 1.0, 1e-6)
+    g.replay()
+    torch.cuda.synchronize()
+    ref = naive(c, d, 1e-6, "f64_ieee")
+    assert rel_err(*[host(v) for v in a], *ref).max() <= 1e-12
+    c.close()
