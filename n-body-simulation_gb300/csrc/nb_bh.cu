@@ -15,9 +15,9 @@
 //     leftmost split of each cell ("first split") stands for the cell.
 //  6. DFS numbering: each sorted position p starts popc(mask[p]) internal cells plus its leaf;
 //     an exclusive scan gives every node its DFS pre-order index and skip link.
-//  7. bottom-up centre of mass: leaves one thread each, cells by blocks over chunks of 4,096
-//     sorted positions (deepest level first), the cells reaching past their chunk (at most one
-//     per level) by tiers of blocks over 64 chunks each; children summed in octant order 0..7
+//  7. bottom-up centre of mass: leaves and cells by blocks over chunks of 1,024 sorted positions
+//     (deepest level first), the cells reaching past their chunk (at most one per level) by tiers
+//     of blocks over 64 chunks each; children summed in octant order 0..7
 //     (bit-identical to BarnesHutOctree.cpp:304-311), node records written with the sums.
 #include <algorithm>
 
@@ -627,7 +627,12 @@ __device__ void cell_records(const ComArgs& A, uint32_t idx) {
 // its body: the FP64 records keep the reference's quotient (c / m, mostly decided without a
 // division by leaf_quotient), the FP32 records take the body position itself (within their own
 // rounding of that quotient), and the spread of a single body is 0.
-__device__ void leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32_t b) {
+struct NodeSums {
+    double x, y, z, m, q;
+    uint32_t count;
+};
+
+__device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32_t b) {
     const double mb = A.m[b];
     const double bx = A.x[b], by = A.y[b], bz = A.z[b];
     const double cx = __dmul_rn(bx, mb), cy = __dmul_rn(by, mb), cz = __dmul_rn(bz, mb);
@@ -682,9 +687,11 @@ __device__ void leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32_t b
         A.rec32lo[idx] = lo;
         A.rec32lo2[idx] = lo2;
     }
+    NodeSums sums{cx, cy, cz, mb, 0.0, 1};
     if (A.records & NB_REC_LEARNED) {  // spread sums and the FP32 body copies of the policy
         const double rx = bx - ox, ry = by - oy, rz = bz - oz;
-        A.q[idx] = mb * (rx * rx + ry * ry + rz * rz);
+        sums.q = mb * (rx * rx + ry * ry + rz * rz);
+        A.q[idx] = sums.q;
         const float hx = (float)rx, hy = (float)ry, hz = (float)rz;
         A.sorted4[p] = make_float4(hx, hy, hz, q.gm);
         A.sorted4lo[p] = make_float4((float)(rx - (double)hx), (float)(ry - (double)hy),
@@ -696,6 +703,7 @@ __device__ void leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32_t b
         x.lg_gm = __log2f(fmaxf(q.gm, 1e-37f));
         A.aux[idx] = x;
     }
+    return sums;
 }
 
 // Centre of mass and records, bottom-up, in chunks of CW consecutive sorted positions. The nodes
@@ -707,26 +715,25 @@ __device__ void leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32_t b
 // the rest up again, until one block spans all bodies. Every sum has its children's sums final
 // before it starts (kernel order, then levels deepest first within a block), so no thread waits
 // on another, and the FP64 work is spread over all SMs at every tier.
-//  * com_leaf_kernel: one thread per sorted position sums its leaf and writes its records;
-//  * com_cells_kernel: one block per chunk sums the chunk's local cells level by level, then
-//    writes their records in one sweep over the compacted cell list (FP64 work with full warps:
-//    on this part an FP64 warp instruction costs the FP64 pipe the same time however few of its
-//    lanes are active);
+//  * com_chunk_kernel: one block per chunk. Its leaves' sums go to shared memory (and, like all sums
+//    and records, to global memory), the local cells are sorted by level, each thread keeps its
+//    cells' children as slots of the shared sums, and the levels are summed from there; the cells'
+//    records follow in one sweep (FP64 work with full warps: on this part an FP64 warp instruction
+//    costs the FP64 pipe the same time however few of its lanes are active).
+//    Bound: per level a barrier and a chain of FP64 additions (68 cycles each) in the reference's
+//    order. Against a leaf kernel and level sums through L2 by blocks of 4,096 positions
+//    (~1,200 cycles per level): COM_NOTE
 //  * com_tier_kernel: one block per span of CM_FAN lower-tier chunks, same scheme on the listed
 //    cells.
-constexpr int CW = 4096;                          // sorted positions per chunk
+constexpr int CW = 1024;                          // sorted positions per chunk
 constexpr int CM_LEVELS = 2 * NB_KEY_LEVELS + 1;  // node levels 0..42
 constexpr int CM_FAN = 64;                        // lower-tier chunks per upper-tier chunk
 constexpr int CM_TIER_MAX = CM_LEVELS * CM_FAN;   // listed cells one upper-tier block reads
-constexpr int CM_TIERS = 5;                       // 2048 * 64^4 > 2^27 bodies
-constexpr int CC_THREADS = 256;                   // threads per block of the cell kernels
-constexpr int CC_BATCH = 4;  // node-table entries each thread loads together in the scan
-
-__global__ void __launch_bounds__(256, 5) com_leaf_kernel(ComArgs A) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= A.n) return;
-    leaf_sums(A, A.base[p] + __popcll(A.mask[p]), p, A.ids[p]);
-}
+constexpr int CM_TIERS = 5;                       // 1024 * 64^4 > 2^27 bodies
+constexpr int CC_THREADS = 256;                   // threads per block of the tier kernel
+constexpr int CH_THREADS = 512;                   // threads per block of the chunk kernel
+constexpr int CH_NODES = 2 * CW + CM_LEVELS;      // nodes starting in a chunk, at most
+constexpr int CH_CELLS = CW / CH_THREADS;         // local cells per thread, at most
 
 // Sums the `nf` cells found[k] (level flev[k]) level by level, deepest first, then writes their
 // records. Block-wide; smem arrays given by the caller.
@@ -776,60 +783,177 @@ __device__ void sum_by_level(const ComArgs& A, const uint32_t* found, const uint
     for (uint32_t k = threadIdx.x; k < nf; k += blockDim.x) cell_records(A, nodes[k]);
 }
 
-__global__ void __launch_bounds__(CC_THREADS) com_cells_kernel(ComArgs A, uint2* up,
+// Shared memory of com_chunk_kernel: the sums of the chunk's nodes (the spread sums only when the
+// learned records are built) and their body counts.
+constexpr size_t chunk_smem_bytes(bool learned) {
+    return (size_t)CH_NODES * ((learned ? 5 : 4) * sizeof(double) + sizeof(uint32_t));
+}
+
+__global__ void __launch_bounds__(CH_THREADS, 2) com_chunk_kernel(ComArgs A, uint2* up,
                                                                uint32_t* up_count) {
-    __shared__ uint32_t found[CW];  // the chunk's local cells as found
-    __shared__ uint8_t flev[CW];    // and their levels
-    __shared__ uint32_t nodes[CW];  // the same cells, grouped by level
+    extern __shared__ __align__(16) unsigned char com_smem[];
+    const bool learned = (A.records & NB_REC_LEARNED) != 0;
+    double* sx = reinterpret_cast<double*>(com_smem);
+    double* sy = sx + CH_NODES;
+    double* sz = sy + CH_NODES;
+    double* sm = sz + CH_NODES;
+    double* sq = sm + CH_NODES;  // learned only
+    uint32_t* sc = reinterpret_cast<uint32_t*>(sm + (learned ? 2 : 1) * CH_NODES);
+    __shared__ uint16_t found[CW], order[CW];  // local cells as slots: as found, by level
+    __shared__ uint8_t flev[CW];
     __shared__ uint32_t cnt[CM_LEVELS], off[CM_LEVELS], fill[CM_LEVELS];
     __shared__ uint32_t n_found, n_up;
-    const uint32_t P = blockIdx.x * CW;
-    if (P >= A.n) return;
+    const uint32_t tid = threadIdx.x, P = blockIdx.x * CW;
     const uint32_t Pend = min(P + (uint32_t)CW, A.n);
     const uint32_t d0 = A.base[P], d1 = A.base[Pend];
-    for (int l = threadIdx.x; l < CM_LEVELS; l += CC_THREADS) cnt[l] = fill[l] = 0;
-    if (threadIdx.x == 0) n_found = n_up = 0;
-    __syncthreads();
-    // one scan of the chunk's node range, CC_BATCH entries per thread in flight together
-    for (uint32_t i0 = d0 + threadIdx.x; i0 < d1; i0 += CC_THREADS * CC_BATCH) {
-        uint32_t body[CC_BATCH], last[CC_BATCH];
-        uint8_t lvl[CC_BATCH];
-#pragma unroll
-        for (int k = 0; k < CC_BATCH; ++k) {
-            const uint32_t idx = i0 + k * CC_THREADS;
-            body[k] = idx < d1 ? A.node_body[idx] : 0u;
-            last[k] = idx < d1 ? A.node_last[idx] : 0u;
-            lvl[k] = idx < d1 ? A.node_level[idx] : 0;
+    if (tid < CM_LEVELS) cnt[tid] = fill[tid] = 0;
+    if (tid == 0) n_found = n_up = 0;
+    if (d1 - d0 > (uint32_t)CH_NODES) {  // a consistent tree never gets here
+        if (tid == 0) {
+            atomicOr(A.err, NB_DEVERR_DEPTH);
+            up_count[blockIdx.x] = 0;
         }
-#pragma unroll
-        for (int k = 0; k < CC_BATCH; ++k) {
-            const uint32_t idx = i0 + k * CC_THREADS;
-            if (idx >= d1 || body[k] != NB_NONE) continue;  // past the range, or a leaf
-            const int l = min((int)lvl[k], CM_LEVELS - 1);
-            if (last[k] >= Pend) {  // reaches past the chunk: for the next tier
-                const uint32_t g = atomicAdd(&n_up, 1u);
-                if (g < (uint32_t)CM_LEVELS)
-                    up[(size_t)blockIdx.x * CM_LEVELS + g] = make_uint2(idx, (uint32_t)l);
-                else
-                    atomicOr(A.err, NB_DEVERR_DEPTH);  // more than one per level: inconsistent
-                continue;
-            }
+        return;
+    }
+    __syncthreads();
+    for (uint32_t p = P + tid; p < Pend; p += CH_THREADS) {
+        const uint32_t idx = A.base[p] + __popcll(A.mask[p]), k = idx - d0;
+        const NodeSums s = leaf_sums(A, idx, p, A.ids[p]);
+        sx[k] = s.x;
+        sy[k] = s.y;
+        sz[k] = s.z;
+        sm[k] = s.m;
+        if (learned) sq[k] = s.q;
+        sc[k] = 1;
+    }
+    for (uint32_t idx = d0 + tid; idx < d1; idx += CH_THREADS) {
+        if (A.node_body[idx] != NB_NONE) continue;  // a leaf
+        const int l = min((int)A.node_level[idx], CM_LEVELS - 1);
+        if (A.node_last[idx] >= Pend) {  // reaches past the chunk: for the next tier
+            const uint32_t g = atomicAdd(&n_up, 1u);
+            if (g < (uint32_t)CM_LEVELS)
+                up[(size_t)blockIdx.x * CM_LEVELS + g] = make_uint2(idx, (uint32_t)l);
+            else
+                atomicOr(A.err, NB_DEVERR_DEPTH);  // more than one per level: inconsistent
+            continue;
+        }
+        const uint32_t slot = atomicAdd(&n_found, 1u);
+        if (slot < (uint32_t)CW) {
+            found[slot] = (uint16_t)(idx - d0);
+            flev[slot] = (uint8_t)l;
             atomicAdd(&cnt[l], 1u);
-            const uint32_t slot = atomicAdd(&n_found, 1u);
-            if (slot < (uint32_t)CW) {
-                found[slot] = idx;
-                flev[slot] = (uint8_t)l;
-            } else {
-                atomicOr(A.err, NB_DEVERR_DEPTH);  // a consistent tree never gets here
-            }
+        } else {
+            atomicOr(A.err, NB_DEVERR_DEPTH);  // a consistent tree never gets here
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) up_count[blockIdx.x] = min(n_up, (uint32_t)CM_LEVELS);
-    // more local cells than a chunk's bodies allow: only an inconsistent tree (error bit set);
-    // stop here, before any index beyond what the scan recorded is used
-    if (n_found > (uint32_t)CW) return;
-    sum_by_level(A, found, flev, n_found, nodes, cnt, off, fill);
+    const uint32_t nf = min(n_found, (uint32_t)CW);
+    if (tid == 0) up_count[blockIdx.x] = min(n_up, (uint32_t)CM_LEVELS);
+    if (tid < 32) {  // exclusive prefix of the level counts, deepest level last
+        uint32_t run = 0;
+        for (int l0 = 0; l0 < CM_LEVELS; l0 += 32) {
+            const int l = l0 + (int)tid;
+            const uint32_t c = l < CM_LEVELS ? cnt[l] : 0u;
+            uint32_t incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)tid >= o) incl += v;
+            }
+            if (l < CM_LEVELS) off[l] = run + incl - c;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    __syncthreads();
+    for (uint32_t k = tid; k < nf; k += CH_THREADS) {
+        const uint32_t l = flev[k];
+        order[off[l] + atomicAdd(&fill[l], 1u)] = found[k];
+    }
+    __syncthreads();
+    // this thread's cells: the children in octant order as slots (two per word), and the compacted
+    // visit-order child list the learned traversal reads
+    uint32_t kids[CH_CELLS][4], nkids[CH_CELLS];
+#pragma unroll
+    for (int j = 0; j < CH_CELLS; ++j) {
+        const uint32_t pos = tid + j * CH_THREADS;
+        nkids[j] = 0;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) kids[j][w] = 0;
+        if (pos >= nf) continue;
+        uint4* cl = reinterpret_cast<uint4*>(A.children + (size_t)(d0 + order[pos]) * 8);
+        const uint4 c0 = cl[0], c1 = cl[1];
+        const uint32_t vs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        uint32_t list[8];
+        int nch = 0;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            list[t] = NB_NONE;
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            if (vs[t] == NB_NONE) continue;
+#pragma unroll
+            for (int q = 0; q <= t; ++q)
+                if (q == nch) list[q] = vs[t];
+            ++nch;
+        }
+        cl[0] = make_uint4(list[0], list[1], list[2], list[3]);
+        cl[1] = make_uint4(list[4], list[5], list[6], list[7]);
+        uint32_t m = 0;
+#pragma unroll
+        for (int o = 0; o < 8; ++o) {  // the reference's octant order 0..7
+            const uint32_t ch = vs[nb_visit_of_octant(o)];
+            if (ch == NB_NONE) continue;
+            const uint32_t k = min(ch - d0, (uint32_t)CH_NODES - 1);
+#pragma unroll
+            for (int w = 0; w < 4; ++w)
+                if (w == (int)(m >> 1)) kids[j][w] |= k << (16 * (m & 1));
+            ++m;
+        }
+        nkids[j] = m;
+    }
+    // deepest level first
+    for (int l = CM_LEVELS - 1; l >= 0; --l) {
+        const uint32_t c = cnt[l];
+        if (c == 0) continue;  // uniform across the block
+        const uint32_t o0 = off[l];
+#pragma unroll
+        for (int j = 0; j < CH_CELLS; ++j) {
+            const uint32_t pos = tid + j * CH_THREADS;
+            if (pos < o0 || pos >= o0 + c) continue;
+            NodeSums s{0.0, 0.0, 0.0, 0.0, 0.0, 0};
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                if (i >= nkids[j]) break;
+                const uint32_t k = (kids[j][i >> 1] >> (16 * (i & 1))) & 0xffffu;
+                s.x = __dadd_rn(s.x, sx[k]);
+                s.y = __dadd_rn(s.y, sy[k]);
+                s.z = __dadd_rn(s.z, sz[k]);
+                s.m = __dadd_rn(s.m, sm[k]);
+                if (learned) s.q += sq[k];
+                s.count += sc[k];
+            }
+            const uint32_t k = order[pos];
+            sx[k] = s.x;
+            sy[k] = s.y;
+            sz[k] = s.z;
+            sm[k] = s.m;
+            if (learned) sq[k] = s.q;
+            sc[k] = s.count;
+        }
+        __syncthreads();
+    }
+    for (uint32_t pos = tid; pos < nf; pos += CH_THREADS) {
+        const uint32_t k = order[pos], idx = d0 + k;
+        A.comx[idx] = sx[k];
+        A.comy[idx] = sy[k];
+        A.comz[idx] = sz[k];
+        A.mass[idx] = sm[k];
+        if (learned) A.q[idx] = sq[k];
+        A.node_count[idx] = sc[k];
+        write_records(A, idx, sx[k], sy[k], sz[k], sm[k], learned ? sq[k] : 0.0, sc[k],
+                      A.node_level[idx], A.node_skip[idx], NB_NONE);
+    }
 }
 
 // Tier of `span` sorted positions per block (span = CW * CM_FAN^t): the cells listed by the
@@ -974,6 +1098,8 @@ nb_status nb_bh_tree_create(nb_ctx* ctx, uint32_t n_max, const nb_bh_params* par
         nb_bh_params_default(&t->params);
     }
     NB_TRY(nb::radix_prepare());  // before any capture of a build
+    NB_CUDA_TRY(cudaFuncSetAttribute(com_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)chunk_smem_bytes(true)));
     Carver sizing;
     carve(t, sizing);
     void* mem = nullptr;
@@ -1134,15 +1260,15 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     A.children = t->children;
     A.sorted4 = t->sorted4;
     A.sorted4lo = t->sorted4lo;
-    com_leaf_kernel<<<grid, BH_THREADS, 0, s>>>(A);
-    NB_TRY(nb::check_launch("com_leaf_kernel"));
     {
         uint32_t chunks = (uint32_t)nb::ceil_div(n, CW);
-        com_cells_kernel<<<chunks, CC_THREADS, 0, s>>>(A, t->tier_cells[0], t->tier_count[0]);
-        NB_TRY(nb::check_launch("com_cells_kernel"));
+        com_chunk_kernel<<<chunks, CH_THREADS,
+                           chunk_smem_bytes((t->records & NB_REC_LEARNED) != 0), s>>>(
+            A, t->tier_cells[0], t->tier_count[0]);
+        NB_TRY(nb::check_launch("com_chunk_kernel"));
         uint64_t span = CW;
         int in = 0;
-        for (int tier = 1; tier <= CM_TIERS; ++tier) {
+        for (int tier = 1; tier <= CM_TIERS && chunks > 1; ++tier) {
             span *= CM_FAN;
             const uint32_t blocks = (uint32_t)((n + span - 1) / span);
             const bool last = blocks == 1;
