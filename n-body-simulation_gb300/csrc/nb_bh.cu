@@ -21,6 +21,7 @@
 //     (bit-identical to BarnesHutOctree.cpp:304-311), node records written with the sums.
 #include <algorithm>
 
+#include "nb_aabb.cuh"
 #include "nb_bh.cuh"
 #include "nb_sort.cuh"
 
@@ -140,10 +141,12 @@ __device__ uint64_t key_word_quantized(const double* __restrict__ box, double px
 __device__ __forceinline__ void box_extras(double* __restrict__ box, uint32_t i) {
     if (i < 3) box[7 + i] = box[i] + box[6] / 2;
     if (i == 3) {
-        double v = 0.0;
-        for (int k = 0; k < 6; ++k) v = fmax(v, fabs(box[k]));
-        box[10] = (double)nbfix::k_of(v);
+        long long v = 0;
+        for (int k = 0; k < 6; ++k)
+            v = max(v, __double_as_longlong(box[k]) & 0x7fffffffffffffffll);
+        box[10] = (double)nbfix::k_of(__longlong_as_double(v));
     }
+    if (i == 4) box[11] = box[6] * box[6];
 }
 
 __global__ void keys_quantized_kernel(const double* __restrict__ x, const double* __restrict__ y,
@@ -192,10 +195,28 @@ __device__ FixedGrid fixed_grid(const double* __restrict__ box) {
 // coordinate is outside the box or NaN).
 __device__ __forceinline__ long long fixed_digits(double v, double mn, double scale, long long m) {
     const double u = __dmul_rn(__dsub_rn(v, mn), scale);
-    if (!(u >= 0.0 && u <= 4503599627370496.0)) return -1;
-    const long long U = (long long)u;
+    // 0 <= u <= 2^52, by its bits; the integer part by a shift
+    const long long b = __double_as_longlong(u);
+    if ((uint64_t)b > 0x4330000000000000ull && (b << 1) != 0) return -1;
+    const int e = (int)(b >> 52);
+    const long long U = e < 1023 ? 0 : ((b & 0xfffffffffffffll) | (1ll << 52)) >> (1075 - e);
     const long long hi = (U + m) >> 31, lo = (U - m - 1) >> 31;
     return hi == lo ? hi : -1;
+}
+
+// First key word of a body by the rule above.
+__device__ __forceinline__ uint64_t exact_key(const double* __restrict__ box, const FixedGrid& g,
+                                              double px, double py, double pz) {
+    long long hx = -1, hy = -1, hz = -1;
+    if (g.ok) {
+        hx = fixed_digits(px, box[0], g.scale, g.margin[0]);
+        hy = fixed_digits(py, box[1], g.scale, g.margin[1]);
+        hz = fixed_digits(pz, box[2], g.scale, g.margin[2]);
+    }
+    if ((hx | hy | hz) < 0) return key_word(box, px, py, pz, 0);
+    const uint64_t m = 0x1fffffull;  // visit rank = 4 (y upper) + 2 (z lower) + (x lower)
+    return (spread3((uint64_t)hy) << 2) | (spread3(~(uint64_t)hz & m) << 1) |
+           spread3(~(uint64_t)hx & m);
 }
 
 __global__ void __launch_bounds__(BH_THREADS)
@@ -208,33 +229,17 @@ keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
     if (threadIdx.x == 0) grid_s = fixed_grid(box);
     __syncthreads();
     if (i >= n) return;
-    const FixedGrid g = grid_s;
-    const double px = x[i], py = y[i], pz = z[i];
-    long long hx = -1, hy = -1, hz = -1;
-    if (g.ok) {
-        hx = fixed_digits(px, box[0], g.scale, g.margin[0]);
-        hy = fixed_digits(py, box[1], g.scale, g.margin[1]);
-        hz = fixed_digits(pz, box[2], g.scale, g.margin[2]);
-    }
-    uint64_t key;
-    if ((hx | hy | hz) >= 0) {  // visit rank = 4 (y upper) + 2 (z lower) + (x lower)
-        const uint64_t m = 0x1fffffull;
-        key = (spread3((uint64_t)hy) << 2) | (spread3(~(uint64_t)hz & m) << 1) |
-              spread3(~(uint64_t)hx & m);
-    } else {
-        key = key_word(box, px, py, pz, 0);
-    }
-    key0[i] = key;
+    key0[i] = exact_key(box, grid_s, x[i], y[i], z[i]);
     ids[i] = i;
 }
 
 // Runs of equal first words: compute the second word and insertion-sort the run (stable).
-__global__ void runs_fixup_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                                  const double* __restrict__ z, uint32_t n,
-                                  const double* __restrict__ box, const uint64_t* __restrict__ key0,
-                                  uint64_t* __restrict__ key1, uint32_t* __restrict__ ids,
-                                  uint32_t* __restrict__ err, int quantized) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void fix_run(uint32_t p, const double* __restrict__ x,
+                                        const double* __restrict__ y,
+                                        const double* __restrict__ z, uint32_t n,
+                                        const double* __restrict__ box, const uint64_t* key0,
+                                        uint64_t* key1, uint32_t* ids, uint32_t* err,
+                                        int quantized) {
     if (p + 1 >= n) return;
     const uint64_t k = key0[p];
     if (key0[p + 1] != k) return;
@@ -264,6 +269,15 @@ __global__ void runs_fixup_kernel(const double* __restrict__ x, const double* __
     }
 }
 
+__global__ void runs_fixup_kernel(const double* __restrict__ x, const double* __restrict__ y,
+                                  const double* __restrict__ z, uint32_t n,
+                                  const double* __restrict__ box, const uint64_t* __restrict__ key0,
+                                  uint64_t* __restrict__ key1, uint32_t* __restrict__ ids,
+                                  uint32_t* __restrict__ err, int quantized) {
+    fix_run(blockIdx.x * blockDim.x + threadIdx.x, x, y, z, n, box, key0, key1, ids, err,
+            quantized);
+}
+
 // Number of leading octal digits two sorted positions share (0 .. 42).
 __device__ __forceinline__ int shared_digits(const uint64_t* __restrict__ key0,
                                              const uint64_t* __restrict__ key1, uint32_t p,
@@ -275,11 +289,11 @@ __device__ __forceinline__ int shared_digits(const uint64_t* __restrict__ key0,
     return 2 * NB_KEY_LEVELS;
 }
 
-__global__ void splits_kernel(const uint64_t* __restrict__ key0, const uint64_t* __restrict__ key1,
-                              uint32_t n, uint8_t* __restrict__ split_level,
-                              uint32_t* __restrict__ split_start, uint32_t* __restrict__ split_end,
-                              unsigned long long* __restrict__ mask, uint32_t* __restrict__ err) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void split_at(uint32_t j, const uint64_t* __restrict__ key0,
+                                         const uint64_t* __restrict__ key1, uint32_t n,
+                                         uint8_t* split_level, uint32_t* split_start,
+                                         uint32_t* split_end, unsigned long long* mask,
+                                         uint32_t* err) {
     if (j + 1 >= n) return;
     int L = shared_digits(key0, key1, j, j + 1);
     if (L >= 2 * NB_KEY_LEVELS) {
@@ -330,6 +344,14 @@ __global__ void splits_kernel(const uint64_t* __restrict__ key0, const uint64_t*
     atomicOr(&mask[a], 1ull << L);
 }
 
+__global__ void splits_kernel(const uint64_t* __restrict__ key0, const uint64_t* __restrict__ key1,
+                              uint32_t n, uint8_t* __restrict__ split_level,
+                              uint32_t* __restrict__ split_start, uint32_t* __restrict__ split_end,
+                              unsigned long long* __restrict__ mask, uint32_t* __restrict__ err) {
+    split_at(blockIdx.x * blockDim.x + threadIdx.x, key0, key1, n, split_level, split_start,
+             split_end, mask, err);
+}
+
 __global__ void count_kernel(const unsigned long long* __restrict__ mask, uint32_t n,
                              uint32_t* __restrict__ cnt) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -360,53 +382,245 @@ __device__ __forceinline__ uint32_t digit_at(const uint64_t* __restrict__ key0,
     return (uint32_t)(key1[q] >> (60 - 3 * (L - NB_KEY_LEVELS))) & 7u;
 }
 
-__global__ void emit_kernel(uint32_t n, const uint32_t* __restrict__ ids,
-                            const uint8_t* __restrict__ split_level,
-                            const uint32_t* __restrict__ split_start,
-                            const uint32_t* __restrict__ split_end,
-                            const unsigned long long* __restrict__ mask,
-                            const uint32_t* __restrict__ base, uint8_t* __restrict__ node_level,
-                            uint32_t* __restrict__ node_first, uint32_t* __restrict__ node_last,
-                            uint32_t* __restrict__ node_skip, uint32_t* __restrict__ node_parent,
-                            uint32_t* __restrict__ node_body,
-                            uint32_t* __restrict__ info, const uint64_t* __restrict__ key0,
-                            const uint64_t* __restrict__ key1, uint32_t* __restrict__ children) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+// The node tables emit_at writes (global memory).
+struct NodeTable {
+    uint8_t* level;
+    uint32_t *first, *last, *skip, *parent, *body, *info, *children;
+};
+
+// The leaf of sorted position p and the internal cell whose first split it is.
+__device__ __forceinline__ void emit_at(uint32_t p, uint32_t n, const uint32_t* ids,
+                                        const uint8_t* split_level, const uint32_t* split_start,
+                                        const uint32_t* split_end, const unsigned long long* mask,
+                                        const uint32_t* base, const uint64_t* key0,
+                                        const uint64_t* key1, const NodeTable& T) {
     if (p >= n) return;
-    if (p == 0) info[0] = base[n];
+    if (p == 0) T.info[0] = base[n];
     {  // leaf of the body at sorted position p
         const int dl = p > 0 ? (int)split_level[p - 1] : -1;
         const int dr = p + 1 < n ? (int)split_level[p] : -1;
         const uint32_t idx = base[p] + __popcll(mask[p]);
-        node_level[idx] = (uint8_t)(max(dl, dr) + 1);
-        node_first[idx] = p;
-        node_last[idx] = p;
-        node_skip[idx] = base[p + 1];
-        node_body[idx] = ids[p];
+        T.level[idx] = (uint8_t)(max(dl, dr) + 1);
+        T.first[idx] = p;
+        T.last[idx] = p;
+        T.skip[idx] = base[p + 1];
+        T.body[idx] = ids[p];
         const uint32_t par = parent_of(p, p, dl, dr, split_level, split_start, base, mask);
-        node_parent[idx] = par;
+        T.parent[idx] = par;
         if (par != NB_NONE) {
             // the parent's level is the deeper boundary split; slot = visit rank there
-            children[(size_t)par * 8 + digit_at(key0, key1, p, max(dl, dr))] = idx;
+            T.children[(size_t)par * 8 + digit_at(key0, key1, p, max(dl, dr))] = idx;
         }
     }
     if (p + 1 < n && split_end[p] != NB_NONE) {  // internal cell whose first split is p
         const uint32_t a = split_start[p], b = split_end[p];
         const int L = split_level[p];
         const uint32_t idx = node_index(base, mask, a, L);
-        node_level[idx] = (uint8_t)L;
-        node_first[idx] = a;
-        node_last[idx] = b;
-        node_skip[idx] = base[b + 1];
-        node_body[idx] = NB_NONE;
+        T.level[idx] = (uint8_t)L;
+        T.first[idx] = a;
+        T.last[idx] = b;
+        T.skip[idx] = base[b + 1];
+        T.body[idx] = NB_NONE;
         const int dl = a > 0 ? (int)split_level[a - 1] : -1;
         const int dr = b + 1 < n ? (int)split_level[b] : -1;
         const uint32_t par = parent_of(a, b, dl, dr, split_level, split_start, base, mask);
-        node_parent[idx] = par;
+        T.parent[idx] = par;
         if (par != NB_NONE) {
-            children[(size_t)par * 8 + digit_at(key0, key1, a, max(dl, dr))] = idx;
+            T.children[(size_t)par * 8 + digit_at(key0, key1, a, max(dl, dr))] = idx;
         }
     }
+}
+
+__global__ void emit_kernel(uint32_t n, const uint32_t* __restrict__ ids,
+                            const uint8_t* __restrict__ split_level,
+                            const uint32_t* __restrict__ split_start,
+                            const uint32_t* __restrict__ split_end,
+                            const unsigned long long* __restrict__ mask,
+                            const uint32_t* __restrict__ base, const uint64_t* __restrict__ key0,
+                            const uint64_t* __restrict__ key1, NodeTable T) {
+    emit_at(blockIdx.x * blockDim.x + threadIdx.x, n, ids, split_level, split_start, split_end,
+            mask, base, key0, key1, T);
+}
+
+// Steps 1 to 6 for small systems in one block, sharing the device functions above: the chain of 18
+// launches cost 135 us at 777 bodies and 167 at 4,096, this one 40 and 115. (Key, body) pairs by a bitonic sort in shared memory
+// (ties by body id: the stable order), the DFS numbering by a block scan.
+constexpr uint32_t SB_MAX_N = 4096;
+
+template <uint32_t CAP>
+constexpr size_t small_smem_bytes() {
+    return CAP * (8 + 8 + 8 + 4 + 4 + 4 + 4 + 1) + 64;
+}
+
+__device__ __forceinline__ uint32_t small_block_scan(uint32_t v, uint32_t* warp_sums,
+                                                     uint32_t* total) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += t;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    uint32_t ws = lane < blockDim.x / 32 ? warp_sums[lane] : 0u, wi = ws;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
+        if (lane >= (uint32_t)o) wi += t;
+    }
+    *total = __shfl_sync(0xffffffffu, wi, 31);
+    return __shfl_sync(0xffffffffu, wi - ws, warp) + incl - v;
+}
+
+template <uint32_t CAP, uint32_t THREADS>
+__global__ void __launch_bounds__(THREADS)
+build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
+                   const double* __restrict__ z, uint32_t n, double* __restrict__ box,
+                   uint64_t* __restrict__ key0_out, uint64_t* __restrict__ key1_out,
+                   uint32_t* __restrict__ ids_out, unsigned long long* __restrict__ mask_out,
+                   uint32_t* __restrict__ base_out, NodeTable T, uint32_t* __restrict__ err,
+                   int quantized) {
+    constexpr int PER = CAP / THREADS;  // positions per thread
+    static_assert(PER == 2 || PER == 4, "positions per thread");
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    uint64_t* key0 = reinterpret_cast<uint64_t*>(small_smem);
+    uint64_t* key1 = key0 + CAP;
+    unsigned long long* mask = reinterpret_cast<unsigned long long*>(key1 + CAP);
+    uint32_t* ids = reinterpret_cast<uint32_t*>(mask + CAP);
+    uint32_t* split_start = ids + CAP;
+    uint32_t* split_end = split_start + CAP;
+    uint32_t* base = split_end + CAP;  // CAP + 1 entries
+    uint8_t* split_level = reinterpret_cast<uint8_t*>(base + CAP + 1);
+    __shared__ long long wmin[3][32], wmax[3][32];
+    __shared__ uint32_t warp_sums[32];
+    __shared__ double sbox[12];
+    __shared__ FixedGrid grid_s;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // children lists start empty; written before the barriers below, filled after them
+    for (uint32_t k = tid; k < 4 * n; k += THREADS)
+        reinterpret_cast<uint4*>(T.children)[k] = make_uint4(NB_NONE, NB_NONE, NB_NONE, NB_NONE);
+    // box, with the reference's zero-initialised bounds
+    double px[PER], py[PER], pz[PER];
+    const long long zero = nbaabb::ord_of(0.0);
+    long long mn[3] = {zero, zero, zero}, mx[3] = {zero, zero, zero};
+#pragma unroll
+    for (int h = 0; h < PER; ++h) {
+        const uint32_t i = tid + h * THREADS;
+        const bool in = i < n;
+        px[h] = in ? x[i] : 0.0;
+        py[h] = in ? y[i] : 0.0;
+        pz[h] = in ? z[i] : 0.0;
+        const long long o[3] = {nbaabb::ord_of(px[h]), nbaabb::ord_of(py[h]),
+                                nbaabb::ord_of(pz[h])};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (!in) continue;
+            mn[a] = min(mn[a], o[a]);
+            mx[a] = max(mx[a], o[a]);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
+            mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
+        }
+        if (lane == 0) {
+            wmin[a][warp] = mn[a];
+            wmax[a][warp] = mx[a];
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            mn[a] = lane < THREADS / 32 ? wmin[a][lane] : zero;
+            mx[a] = lane < THREADS / 32 ? wmax[a][lane] : zero;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
+                mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
+            }
+        }
+        if (lane == 0)
+            nbaabb::cube_rule(nbaabb::val_of(mn[0]), nbaabb::val_of(mn[1]), nbaabb::val_of(mn[2]),
+                              nbaabb::val_of(mx[0]), nbaabb::val_of(mx[1]), nbaabb::val_of(mx[2]),
+                              sbox);
+        __syncwarp();
+        box_extras(sbox, lane);
+        __syncwarp();
+        if (lane < 12) box[lane] = sbox[lane];
+        if (lane == 0 && !quantized) grid_s = fixed_grid(sbox);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < PER; ++h) {
+        const uint32_t i = tid + h * THREADS;
+        uint64_t k = ~0ull;  // above every key (63 bits)
+        if (i < n)
+            k = quantized ? key_word_quantized(sbox, px[h], py[h], pz[h], 0)
+                          : exact_key(sbox, grid_s, px[h], py[h], pz[h]);
+        key0[i] = k;
+        ids[i] = i;
+        key1[i] = 0;
+        mask[i] = 0;
+    }
+    __syncthreads();
+    uint32_t m = 2;  // positions to sort: a power of two
+    while (m < n) m <<= 1;
+    for (uint32_t k = 2; k <= m; k <<= 1) {
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            for (uint32_t q = tid; q < m / 2; q += THREADS) {  // compare-exchange number q
+                const uint32_t lo = ((q & ~(j - 1)) << 1) | (q & (j - 1)), hi = lo | j;
+                const uint64_t a = key0[lo], b = key0[hi];
+                const uint32_t ia = ids[lo], ib = ids[hi];
+                const bool gt = a > b || (a == b && ia > ib);
+                if (gt == ((lo & k) == 0)) {
+                    key0[lo] = b;
+                    key0[hi] = a;
+                    ids[lo] = ib;
+                    ids[hi] = ia;
+                }
+            }
+            // exchanges at a distance of up to 32 stay within a warp's blocks of 64 positions
+            if (j > 32) __syncthreads(); else __syncwarp();
+        }
+        __syncthreads();
+    }
+    for (uint32_t p = tid; p < n; p += THREADS)
+        fix_run(p, x, y, z, n, sbox, key0, key1, ids, err, quantized);
+    __syncthreads();
+    for (uint32_t p = tid; p < n; p += THREADS)
+        split_at(p, key0, key1, n, split_level, split_start, split_end, mask, err);
+    __syncthreads();
+    {
+        const uint32_t p = PER * tid;
+        uint32_t c[PER], sum = 0, total;
+#pragma unroll
+        for (int h = 0; h < PER; ++h) {
+            c[h] = p + h < n ? __popcll(mask[p + h]) + 1 : 0u;
+            sum += c[h];
+        }
+        uint32_t before = small_block_scan(sum, warp_sums, &total);
+#pragma unroll
+        for (int h = 0; h < PER; ++h) {
+            if (p + h < n) base[p + h] = before;
+            before += c[h];
+        }
+        if (tid == 0) base[n] = total;
+    }
+    __syncthreads();
+    for (uint32_t p = tid; p < n; p += THREADS) {
+        key0_out[p] = key0[p];
+        key1_out[p] = key1[p];
+        ids_out[p] = ids[p];
+        mask_out[p] = mask[p];
+        base_out[p] = base[p];
+        emit_at(p, n, ids, split_level, split_start, split_end, mask, base, key0, key1, T);
+    }
+    if (tid == 0) base_out[n] = base[n];
 }
 
 struct ComArgs {
@@ -448,22 +662,76 @@ __device__ __forceinline__ double cell_edge64(double box_edge, int level) {
     return ldexp(box_edge, -level);
 }
 
+__device__ __forceinline__ int biased_exp(double v) {
+    return (int)(((uint64_t)__double_as_longlong(v) >> 52) & 0x7ff);
+}
+
 // RN(c / m) for the rounded product c = RN(x * m) of a leaf (its centre-of-mass numerator over its
-// mass): that quotient is x itself whenever |c / m - x| < ulp(x) / 2, and the difference is known
-// exactly, since the rounding error x * m - c of a product is exact in one FMA. So
-// |x * m - c| * 2^(53 - e(x)) < m (a power-of-two scaling, exact) decides it without a division;
-// the IEEE division remains for the rest (x a power of two, zero, subnormal or extreme, or the
-// quotient rounding to a neighbour of x).
+// mass), without a division: c / m = x - err / m with err = x * m - c, the rounding error of the
+// product, exact in one FMA and at most half a unit in c's last place, so c / m lies within one unit
+// of x and rounds to x or to its neighbour on err's side. Which of them is decided by comparing
+// |err| 2^(53 - e(x)) with m (beyond half a unit; a tie goes to the even one), both positive normal
+// numbers, as integers. The IEEE division remains for x a power of two (whose units differ on its
+// two sides), subnormal or extreme values, and masses that are not positive.
 __device__ __forceinline__ double leaf_quotient(double x, double m, double c) {
     const long long xb = __double_as_longlong(x);
-    const int biased = (int)((xb >> 52) & 0x7ff);
-    const int s = 1023 + 53 - (biased - 1023);  // biased exponent of 2^(53 - e(x))
-    const bool pow2 = (xb & 0xfffffffffffffll) == 0;
-    if (biased == 0 || biased == 0x7ff || pow2 || s < 1 || s > 2046 || !(m > 0.0))
+    const int ex = biased_exp(x), em = biased_exp(m), ec = biased_exp(c);
+    const bool m_ok = m > 0.0 && em >= 64 && em <= 2040;
+    if (m_ok && (xb << 1) == 0) return c;  // 0 / m
+    if (!m_ok || ex == 0 || ex == 0x7ff || (xb & 0xfffffffffffffll) == 0 || ec < 128 || ec > 2040)
         return __ddiv_rn(c, m);
-    const double err = fma(x, m, -c);
-    if (fabs(err) * __longlong_as_double((long long)s << 52) < m) return x;
-    return __ddiv_rn(c, m);
+    const long long err = __double_as_longlong(fma(x, m, -c));
+    if ((err << 1) == 0) return x;
+    const long long t = (err & 0x7fffffffffffffffll) + ((long long)(1023 + 53 - ex) << 52);
+    const long long mb = __double_as_longlong(m);
+    if (t < mb || (t == mb && (xb & 1) == 0)) return x;
+    return __longlong_as_double((err ^ xb) < 0 ? xb + 1 : xb - 1);
+}
+
+// RN(cx / m), RN(cy / m), RN(cz / m) from one reciprocal (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990): y = RN(1 / m) by Newton steps from the
+// hardware estimate (m's mantissa not all ones); q1 = q0 + r0 y is within one unit of the quotient
+// and q1 + r1 y with the exact remainder r1 = c - m q1 rounds to it. The IEEE division remains
+// outside a range in which every intermediate is normal.
+__device__ __forceinline__ void exact_quotients(double cx, double cy, double cz, double m,
+                                                double& qx, double& qy, double& qz) {
+    const int em = biased_exp(m);
+    const uint64_t mant = (uint64_t)__double_as_longlong(m) & 0xfffffffffffffull;
+    auto fits = [&](double c) {
+        const int e = biased_exp(c);
+        return (e >= 300 && e <= 1700) || ((__double_as_longlong(c) << 1) == 0);
+    };
+    if (em < 300 || em > 1700 || mant == 0xfffffffffffffull || !fits(cx) || !fits(cy) ||
+        !fits(cz)) {
+        qx = __ddiv_rn(cx, m);
+        qy = __ddiv_rn(cy, m);
+        qz = __ddiv_rn(cz, m);
+        return;
+    }
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(m));
+    y = fma(y, fma(-m, y, 1.0), y);
+    y = fma(y, fma(-m, y, 1.0), y);
+    y = fma(y, fma(-m, y, 1.0), y);
+    auto quotient = [&](double c) {
+        double q = c * y;
+        q = fma(fma(-m, q, c), y, q);
+        const double r = fma(fma(-m, q, c), y, q);
+        return (__double_as_longlong(c) << 1) == 0 ? (m > 0.0 ? c : -c) : r;
+    };
+    qx = quotient(cx);
+    qy = quotient(cy);
+    qz = quotient(cz);
+}
+
+// The FP32 edge^2 of a cell of the given level: (float)(edge * edge), both scaled exactly from the
+// box's while they stay normal.
+__device__ __forceinline__ float cell_edge2(double box_edge, double edge, float box_edge2,
+                                            int level) {
+    const int e = (int)((__float_as_uint(box_edge2) >> 23) & 0xff);
+    if (e > 2 * level + 1 && e < 0xff && biased_exp(box_edge) > 600)
+        return __uint_as_float(__float_as_uint(box_edge2) - ((uint32_t)(2 * level) << 23));
+    return (float)(edge * edge);
 }
 
 // Fixed-point record of a node with centre (cx, cy, cz) and mass m.
@@ -484,15 +752,14 @@ __device__ void write_records(const ComArgs& A, uint32_t idx, double cx, double 
     // records round it); massless cells get a finite centre (never used)
     double rcx = 0.0, rcy = 0.0, rcz = 0.0, inv = 0.0;
     if (sm != 0) {
+        if (A.records & NB_REC_FP64) exact_quotients(cx, cy, cz, sm, rcx, rcy, rcz);
         // 1/M from the hardware estimate and one Newton step (~2^-44: ample for the FP32
         // centres and the spread)
-        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(inv) : "d"(sm));
-        inv = inv * fma(-sm, inv, 2.0);
-        if (A.records & NB_REC_FP64) {
-            rcx = __ddiv_rn(cx, sm);
-            rcy = __ddiv_rn(cy, sm);
-            rcz = __ddiv_rn(cz, sm);
-        } else {
+        if (!(A.records & NB_REC_FP64) || (A.records & NB_REC_LEARNED)) {
+            asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(inv) : "d"(sm));
+            inv = inv * fma(-sm, inv, 2.0);
+        }
+        if (!(A.records & NB_REC_FP64)) {
             rcx = cx * inv;
             rcy = cy * inv;
             rcz = cz * inv;
@@ -520,7 +787,7 @@ __device__ void write_records(const ComArgs& A, uint32_t idx, double cx, double 
         q.cx = q.cy = q.cz = 1e30f;
     }
     q.gm = (float)(A.G * sm);
-    q.edge2 = (float)(edge * edge);
+    q.edge2 = cell_edge2(A.box[6], edge, (float)A.box[11], level);
     q.skip = skip;
     q.body = body;
     q.level = (uint32_t)level;
@@ -670,7 +937,7 @@ __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32
     q.cy = mb != 0 ? (float)gy : 1e30f;
     q.cz = mb != 0 ? (float)gz : 1e30f;
     q.gm = (float)(A.G * mb);
-    q.edge2 = (float)(edge * edge);
+    q.edge2 = cell_edge2(A.box[6], edge, (float)A.box[11], level);
     q.skip = skip;
     q.body = b;
     q.level = (uint32_t)level;
@@ -722,18 +989,16 @@ __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32
 //    costs the FP64 pipe the same time however few of its lanes are active).
 //    Bound: per level a barrier and a chain of FP64 additions (68 cycles each) in the reference's
 //    order. Against a leaf kernel and level sums through L2 by blocks of 4,096 positions
-//    (~1,200 cycles per level): COM_NOTE
+//    (~1,200 cycles per level): 777 bodies 53 -> 35 us, 16,411 127 -> 63, 131,101 145 -> 104,
+//    1,048,576 332 -> 309.
 //  * com_tier_kernel: one block per span of CM_FAN lower-tier chunks, same scheme on the listed
 //    cells.
-constexpr int CW = 1024;                          // sorted positions per chunk
+constexpr int CW_MIN = 256;                       // sorted positions per chunk, at least
 constexpr int CM_LEVELS = 2 * NB_KEY_LEVELS + 1;  // node levels 0..42
-constexpr int CM_FAN = 64;                        // lower-tier chunks per upper-tier chunk
+constexpr int CM_FAN = 96;                        // lower-tier chunks per upper-tier chunk
 constexpr int CM_TIER_MAX = CM_LEVELS * CM_FAN;   // listed cells one upper-tier block reads
-constexpr int CM_TIERS = 5;                       // 1024 * 64^4 > 2^27 bodies
+constexpr int CM_TIERS = 5;                       // 256 * 96^4 > 2^27 bodies
 constexpr int CC_THREADS = 256;                   // threads per block of the tier kernel
-constexpr int CH_THREADS = 512;                   // threads per block of the chunk kernel
-constexpr int CH_NODES = 2 * CW + CM_LEVELS;      // nodes starting in a chunk, at most
-constexpr int CH_CELLS = CW / CH_THREADS;         // local cells per thread, at most
 
 // Sums the `nf` cells found[k] (level flev[k]) level by level, deepest first, then writes their
 // records. Block-wide; smem arrays given by the caller.
@@ -783,14 +1048,24 @@ __device__ void sum_by_level(const ComArgs& A, const uint32_t* found, const uint
     for (uint32_t k = threadIdx.x; k < nf; k += blockDim.x) cell_records(A, nodes[k]);
 }
 
-// Shared memory of com_chunk_kernel: the sums of the chunk's nodes (the spread sums only when the
-// learned records are built) and their body counts.
-constexpr size_t chunk_smem_bytes(bool learned) {
-    return (size_t)CH_NODES * ((learned ? 5 : 4) * sizeof(double) + sizeof(uint32_t));
+// 0.0 + v
+__device__ __forceinline__ double plus_zero(double v) {
+    const long long b = __double_as_longlong(v);
+    return __longlong_as_double((b << 1) == 0 ? 0ll : b);
 }
 
-__global__ void __launch_bounds__(CH_THREADS, 2) com_chunk_kernel(ComArgs A, uint2* up,
-                                                               uint32_t* up_count) {
+// Shared memory of com_chunk_kernel: the sums of the chunk's nodes (the spread sums only when the
+// learned records are built) and their body counts.
+template <int CW>
+constexpr size_t chunk_smem_bytes(bool learned) {
+    return (size_t)(2 * CW + CM_LEVELS) * ((learned ? 5 : 4) * sizeof(double) + sizeof(uint32_t));
+}
+
+template <int CW, int CH_THREADS>
+__global__ void __launch_bounds__(CH_THREADS, 1024 / CH_THREADS)
+com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
+    static_assert(CW == CH_THREADS, "one leaf and at most one local cell per thread");
+    constexpr int CH_NODES = 2 * CW + CM_LEVELS;  // nodes starting in a chunk, at most
     extern __shared__ __align__(16) unsigned char com_smem[];
     const bool learned = (A.records & NB_REC_LEARNED) != 0;
     double* sx = reinterpret_cast<double*>(com_smem);
@@ -800,7 +1075,9 @@ __global__ void __launch_bounds__(CH_THREADS, 2) com_chunk_kernel(ComArgs A, uin
     double* sq = sm + CH_NODES;  // learned only
     uint32_t* sc = reinterpret_cast<uint32_t*>(sm + (learned ? 2 : 1) * CH_NODES);
     __shared__ uint16_t found[CW], order[CW];  // local cells as slots: as found, by level
+    __shared__ __align__(16) uint16_t kids[CW][8];  // a cell's children as slots, octant order
     __shared__ uint8_t flev[CW];
+    __shared__ int deepest;
     __shared__ uint32_t cnt[CM_LEVELS], off[CM_LEVELS], fill[CM_LEVELS];
     __shared__ uint32_t n_found, n_up;
     const uint32_t tid = threadIdx.x, P = blockIdx.x * CW;
@@ -816,7 +1093,7 @@ __global__ void __launch_bounds__(CH_THREADS, 2) com_chunk_kernel(ComArgs A, uin
         return;
     }
     __syncthreads();
-    for (uint32_t p = P + tid; p < Pend; p += CH_THREADS) {
+    if (const uint32_t p = P + tid; p < Pend) {
         const uint32_t idx = A.base[p] + __popcll(A.mask[p]), k = idx - d0;
         const NodeSums s = leaf_sums(A, idx, p, A.ids[p]);
         sx[k] = s.x;
@@ -851,6 +1128,7 @@ __global__ void __launch_bounds__(CH_THREADS, 2) com_chunk_kernel(ComArgs A, uin
     if (tid == 0) up_count[blockIdx.x] = min(n_up, (uint32_t)CM_LEVELS);
     if (tid < 32) {  // exclusive prefix of the level counts, deepest level last
         uint32_t run = 0;
+        int top = -1;
         for (int l0 = 0; l0 < CM_LEVELS; l0 += 32) {
             const int l = l0 + (int)tid;
             const uint32_t c = l < CM_LEVELS ? cnt[l] : 0u;
@@ -862,7 +1140,10 @@ __global__ void __launch_bounds__(CH_THREADS, 2) com_chunk_kernel(ComArgs A, uin
             }
             if (l < CM_LEVELS) off[l] = run + incl - c;
             run += __shfl_sync(0xffffffffu, incl, 31);
+            const uint32_t some = __ballot_sync(0xffffffffu, c != 0);
+            if (some) top = l0 + 31 - __clz((int)some);
         }
+        if (tid == 0) deepest = top;
     }
     __syncthreads();
     for (uint32_t k = tid; k < nf; k += CH_THREADS) {
@@ -870,62 +1151,39 @@ __global__ void __launch_bounds__(CH_THREADS, 2) com_chunk_kernel(ComArgs A, uin
         order[off[l] + atomicAdd(&fill[l], 1u)] = found[k];
     }
     __syncthreads();
-    // this thread's cells: the children in octant order as slots (two per word), and the compacted
-    // visit-order child list the learned traversal reads
-    uint32_t kids[CH_CELLS][4], nkids[CH_CELLS];
-#pragma unroll
-    for (int j = 0; j < CH_CELLS; ++j) {
-        const uint32_t pos = tid + j * CH_THREADS;
-        nkids[j] = 0;
-#pragma unroll
-        for (int w = 0; w < 4; ++w) kids[j][w] = 0;
-        if (pos >= nf) continue;
-        uint4* cl = reinterpret_cast<uint4*>(A.children + (size_t)(d0 + order[pos]) * 8);
-        const uint4 c0 = cl[0], c1 = cl[1];
+    // this thread's cell: its children in octant order as slots, and the compacted visit-order child
+    // list the learned traversal reads
+    const bool cell = tid < nf;
+    const uint32_t my = cell ? order[tid] : 0u;
+    uint32_t nkids = 0;
+    if (cell) {
+        uint32_t* cl = A.children + (size_t)(d0 + my) * 8;
+        const uint4 c0 = reinterpret_cast<const uint4*>(cl)[0],
+                    c1 = reinterpret_cast<const uint4*>(cl)[1];
         const uint32_t vs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-        uint32_t list[8];
-        int nch = 0;
+        uint32_t nch = 0;
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            list[t] = NB_NONE;
-        }
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            if (vs[t] == NB_NONE) continue;
-#pragma unroll
-            for (int q = 0; q <= t; ++q)
-                if (q == nch) list[q] = vs[t];
-            ++nch;
-        }
-        cl[0] = make_uint4(list[0], list[1], list[2], list[3]);
-        cl[1] = make_uint4(list[4], list[5], list[6], list[7]);
-        uint32_t m = 0;
+        for (int t = 0; t < 8; ++t)
+            if (vs[t] != NB_NONE) cl[nch++] = vs[t];
+        for (uint32_t t = nch; t < 8; ++t) cl[t] = NB_NONE;
 #pragma unroll
         for (int o = 0; o < 8; ++o) {  // the reference's octant order 0..7
             const uint32_t ch = vs[nb_visit_of_octant(o)];
-            if (ch == NB_NONE) continue;
-            const uint32_t k = min(ch - d0, (uint32_t)CH_NODES - 1);
-#pragma unroll
-            for (int w = 0; w < 4; ++w)
-                if (w == (int)(m >> 1)) kids[j][w] |= k << (16 * (m & 1));
-            ++m;
+            if (ch != NB_NONE)
+                kids[tid][nkids++] = (uint16_t)min(ch - d0, (uint32_t)CH_NODES - 1);
         }
-        nkids[j] = m;
     }
     // deepest level first
-    for (int l = CM_LEVELS - 1; l >= 0; --l) {
-        const uint32_t c = cnt[l];
+    for (int l = deepest; l >= 0; --l) {
+        const uint32_t c = cnt[l], o0 = off[l];
         if (c == 0) continue;  // uniform across the block
-        const uint32_t o0 = off[l];
-#pragma unroll
-        for (int j = 0; j < CH_CELLS; ++j) {
-            const uint32_t pos = tid + j * CH_THREADS;
-            if (pos < o0 || pos >= o0 + c) continue;
-            NodeSums s{0.0, 0.0, 0.0, 0.0, 0.0, 0};
-#pragma unroll
-            for (uint32_t i = 0; i < 8; ++i) {
-                if (i >= nkids[j]) break;
-                const uint32_t k = (kids[j][i >> 1] >> (16 * (i & 1))) & 0xffffu;
+        if (tid >= o0 && tid < o0 + c) {
+            // the reference's sums start at 0.0: 0.0 + c is c, with -0.0 as +0.0
+            const uint32_t k0 = kids[tid][0];
+            NodeSums s{plus_zero(sx[k0]), plus_zero(sy[k0]), plus_zero(sz[k0]), plus_zero(sm[k0]),
+                       learned ? 0.0 + sq[k0] : 0.0, sc[k0]};
+            for (uint32_t i = 1; i < nkids; ++i) {
+                const uint32_t k = kids[tid][i];
                 s.x = __dadd_rn(s.x, sx[k]);
                 s.y = __dadd_rn(s.y, sy[k]);
                 s.z = __dadd_rn(s.z, sz[k]);
@@ -933,25 +1191,24 @@ __global__ void __launch_bounds__(CH_THREADS, 2) com_chunk_kernel(ComArgs A, uin
                 if (learned) s.q += sq[k];
                 s.count += sc[k];
             }
-            const uint32_t k = order[pos];
-            sx[k] = s.x;
-            sy[k] = s.y;
-            sz[k] = s.z;
-            sm[k] = s.m;
-            if (learned) sq[k] = s.q;
-            sc[k] = s.count;
+            sx[my] = s.x;
+            sy[my] = s.y;
+            sz[my] = s.z;
+            sm[my] = s.m;
+            if (learned) sq[my] = s.q;
+            sc[my] = s.count;
         }
         __syncthreads();
     }
-    for (uint32_t pos = tid; pos < nf; pos += CH_THREADS) {
-        const uint32_t k = order[pos], idx = d0 + k;
-        A.comx[idx] = sx[k];
-        A.comy[idx] = sy[k];
-        A.comz[idx] = sz[k];
-        A.mass[idx] = sm[k];
-        if (learned) A.q[idx] = sq[k];
-        A.node_count[idx] = sc[k];
-        write_records(A, idx, sx[k], sy[k], sz[k], sm[k], learned ? sq[k] : 0.0, sc[k],
+    if (cell) {
+        const uint32_t idx = d0 + my;
+        A.comx[idx] = sx[my];
+        A.comy[idx] = sy[my];
+        A.comz[idx] = sz[my];
+        A.mass[idx] = sm[my];
+        if (learned) A.q[idx] = sq[my];
+        A.node_count[idx] = sc[my];
+        write_records(A, idx, sx[my], sy[my], sz[my], sm[my], learned ? sq[my] : 0.0, sc[my],
                       A.node_level[idx], A.node_skip[idx], NB_NONE);
     }
 }
@@ -997,6 +1254,19 @@ com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
     if (threadIdx.x == 0 && up_count != nullptr) up_count[blockIdx.x] = min(n_up, (uint32_t)CM_LEVELS);
     if (n_found > (uint32_t)CM_TIER_MAX) return;  // cannot happen: <= CM_LEVELS per chunk
     sum_by_level(A, found, flev, n_found, nodes, cnt, off, fill);
+}
+
+// The kernels whose dynamic shared memory is above the default limit (before any capture of a build).
+template <typename K>
+nb_status allow_smem(K kernel, size_t bytes) {
+    NB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)bytes));
+    return NB_OK;
+}
+nb_status build_prepare() {
+    NB_TRY(allow_smem(build_small_kernel<2048, 1024>, small_smem_bytes<2048>()));
+    NB_TRY(allow_smem(build_small_kernel<SB_MAX_N, 1024>, small_smem_bytes<SB_MAX_N>()));
+    return allow_smem(com_chunk_kernel<1024, 1024>, chunk_smem_bytes<1024>(true));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1061,7 +1331,7 @@ void carve(nb_bh_tree* t, Carver& c) {
     t->sorted4 = c.take<float4>(n);
     t->sorted4lo = c.take<float4>(n);
     // per tier, CM_LEVELS listed cells and a count per chunk (two lists, used in turn)
-    const size_t chunks = (n + CW - 1) / CW;
+    const size_t chunks = (n + CW_MIN - 1) / CW_MIN;
     for (int k = 0; k < 2; ++k) {
         t->tier_cells[k] = c.take<uint2>(chunks * CM_LEVELS);
         t->tier_count[k] = c.take<uint32_t>(chunks);
@@ -1098,8 +1368,7 @@ nb_status nb_bh_tree_create(nb_ctx* ctx, uint32_t n_max, const nb_bh_params* par
         nb_bh_params_default(&t->params);
     }
     NB_TRY(nb::radix_prepare());  // before any capture of a build
-    NB_CUDA_TRY(cudaFuncSetAttribute(com_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)chunk_smem_bytes(true)));
+    NB_TRY(build_prepare());
     Carver sizing;
     carve(t, sizing);
     void* mem = nullptr;
@@ -1182,44 +1451,57 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
         return NB_OK;
     };
     NB_TRY(mark(0));
-    NB_TRY(nb::launch_aabb(ctx, x, y, z, n, t->box, s));
-    NB_TRY(mark(1));
     const bool quantized = (t->records & NB_BUILD_QUANTIZED_KEYS) != 0;
-    if (quantized) {
-        keys_quantized_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids);
+    const NodeTable T{t->node_level,  t->node_first, t->node_last, t->node_skip,
+                      t->node_parent, t->node_body,  t->info,      t->children};
+    if (n <= SB_MAX_N) {  // one block; its whole time counts as the cells phase
+        for (int phase = 1; phase <= 3; ++phase) NB_TRY(mark(phase));
+        auto go = [&](auto kernel, uint32_t threads, size_t smem) {
+            kernel<<<1, threads, smem, s>>>(x, y, z, n, t->box, t->key0, t->key1, t->ids,
+                                            (unsigned long long*)t->mask, t->base, T,
+                                            ctx->dev_error, quantized ? 1 : 0);
+        };
+        if (n <= 512) go(build_small_kernel<512, 256>, 256, small_smem_bytes<512>());
+        else if (n <= 2048) go(build_small_kernel<2048, 1024>, 1024, small_smem_bytes<2048>());
+        else go(build_small_kernel<SB_MAX_N, 1024>, 1024, small_smem_bytes<SB_MAX_N>());
+        NB_TRY(nb::check_launch("build_small_kernel"));
     } else {
-        keys_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids);
+        NB_TRY(nb::launch_aabb(ctx, x, y, z, n, t->box, s));
+        NB_TRY(mark(1));
+        if (quantized) {
+            keys_quantized_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids);
+        } else {
+            keys_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids);
+        }
+        NB_TRY(nb::check_launch("keys_kernel"));
+        NB_TRY(mark(2));
+        int in_alt = 0;
+        NB_TRY(nb::radix_sort_pairs(t->key0, t->ids, t->key_alt, t->ids_alt, n, 0, 3 * NB_KEY_LEVELS,
+                                    t->sort_temp, ctx->dev_error, s, &in_alt));
+        if (in_alt) {  // an odd number of passes leaves the result in the alternate buffers
+            NB_CUDA_TRY(cudaMemcpyAsync(t->key0, t->key_alt, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
+            NB_CUDA_TRY(cudaMemcpyAsync(t->ids, t->ids_alt, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
+        }
+        NB_TRY(mark(3));
+        NB_CUDA_TRY(cudaMemsetAsync(t->key1, 0, (size_t)n * 8, s));
+        runs_fixup_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->key1, t->ids,
+                                                      ctx->dev_error, quantized ? 1 : 0);
+        NB_TRY(nb::check_launch("runs_fixup_kernel"));
+        NB_CUDA_TRY(cudaMemsetAsync(t->mask, 0, (size_t)n * 8, s));
+        splits_kernel<<<grid, BH_THREADS, 0, s>>>(t->key0, t->key1, n, t->split_level, t->split_start,
+                                                  t->split_end, (unsigned long long*)t->mask,
+                                                  ctx->dev_error);
+        NB_TRY(nb::check_launch("splits_kernel"));
+        count_kernel<<<grid, BH_THREADS, 0, s>>>((const unsigned long long*)t->mask, n, t->cnt);
+        NB_TRY(nb::check_launch("count_kernel"));
+        NB_TRY(nb::exclusive_scan_u32(t->cnt, t->base, n, 1, t->scan_temp, s));
+        const size_t nodes_max = 2 * (size_t)n;
+        NB_CUDA_TRY(cudaMemsetAsync(t->children, 0xff, nodes_max * 8 * 4, s));  // NB_NONE
+        emit_kernel<<<grid, BH_THREADS, 0, s>>>(n, t->ids, t->split_level, t->split_start, t->split_end,
+                                                (const unsigned long long*)t->mask, t->base, t->key0,
+                                                t->key1, T);
+        NB_TRY(nb::check_launch("emit_kernel"));
     }
-    NB_TRY(nb::check_launch("keys_kernel"));
-    NB_TRY(mark(2));
-    int in_alt = 0;
-    NB_TRY(nb::radix_sort_pairs(t->key0, t->ids, t->key_alt, t->ids_alt, n, 0, 3 * NB_KEY_LEVELS,
-                                t->sort_temp, ctx->dev_error, s, &in_alt));
-    if (in_alt) {  // an odd number of passes leaves the result in the alternate buffers
-        NB_CUDA_TRY(cudaMemcpyAsync(t->key0, t->key_alt, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
-        NB_CUDA_TRY(cudaMemcpyAsync(t->ids, t->ids_alt, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
-    }
-    NB_TRY(mark(3));
-    NB_CUDA_TRY(cudaMemsetAsync(t->key1, 0, (size_t)n * 8, s));
-    runs_fixup_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->key1, t->ids,
-                                                  ctx->dev_error, quantized ? 1 : 0);
-    NB_TRY(nb::check_launch("runs_fixup_kernel"));
-    NB_CUDA_TRY(cudaMemsetAsync(t->mask, 0, (size_t)n * 8, s));
-    splits_kernel<<<grid, BH_THREADS, 0, s>>>(t->key0, t->key1, n, t->split_level, t->split_start,
-                                              t->split_end, (unsigned long long*)t->mask,
-                                              ctx->dev_error);
-    NB_TRY(nb::check_launch("splits_kernel"));
-    count_kernel<<<grid, BH_THREADS, 0, s>>>((const unsigned long long*)t->mask, n, t->cnt);
-    NB_TRY(nb::check_launch("count_kernel"));
-    NB_TRY(nb::exclusive_scan_u32(t->cnt, t->base, n, 1, t->scan_temp, s));
-    const size_t nodes_max = 2 * (size_t)n;
-    NB_CUDA_TRY(cudaMemsetAsync(t->children, 0xff, nodes_max * 8 * 4, s));  // NB_NONE
-    emit_kernel<<<grid, BH_THREADS, 0, s>>>(n, t->ids, t->split_level, t->split_start, t->split_end,
-                                            (const unsigned long long*)t->mask, t->base,
-                                            t->node_level, t->node_first, t->node_last, t->node_skip,
-                                            t->node_parent, t->node_body, t->info,
-                                            t->key0, t->key1, t->children);
-    NB_TRY(nb::check_launch("emit_kernel"));
     NB_TRY(mark(4));
     ComArgs A;
     A.n = n;
@@ -1261,12 +1543,17 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     A.sorted4 = t->sorted4;
     A.sorted4lo = t->sorted4lo;
     {
-        uint32_t chunks = (uint32_t)nb::ceil_div(n, CW);
-        com_chunk_kernel<<<chunks, CH_THREADS,
-                           chunk_smem_bytes((t->records & NB_REC_LEARNED) != 0), s>>>(
-            A, t->tier_cells[0], t->tier_count[0]);
+        const bool learned = (t->records & NB_REC_LEARNED) != 0;
+        // one chunk for the smallest systems (no tier pass), else 256 positions per chunk
+        const uint32_t cw = n <= 1024 ? 1024 : 256;
+        uint32_t chunks = (uint32_t)nb::ceil_div(n, cw);
+        auto go = [&](auto kernel, size_t smem) {
+            kernel<<<chunks, cw, smem, s>>>(A, t->tier_cells[0], t->tier_count[0]);
+        };
+        if (cw == 1024) go(com_chunk_kernel<1024, 1024>, chunk_smem_bytes<1024>(learned));
+        else go(com_chunk_kernel<256, 256>, chunk_smem_bytes<256>(learned));
         NB_TRY(nb::check_launch("com_chunk_kernel"));
-        uint64_t span = CW;
+        uint64_t span = cw;
         int in = 0;
         for (int tier = 1; tier <= CM_TIERS && chunks > 1; ++tier) {
             span *= CM_FAN;

@@ -49,7 +49,7 @@ struct nb_bh_tree {
     int device = 0;
 
     double* box = nullptr;  // [0..6] AABB (min xyz, max xyz, edge), [7..9] box centre, [10] the
-                            // scale exponent K of the fixed-point records (nb_fix.cuh)
+                            // scale exponent K of the fixed-point records (nb_fix.cuh), [11] edge^2
     uint32_t* info = nullptr;  // [0] node count (copy of base[n])
     uint2* tier_cells[2] = {};      // centre-of-mass tiers: cells passed up, (node, level)
     uint32_t* tier_count[2] = {};   // their count per chunk

@@ -1,0 +1,97 @@
+"""Octree build at the edges of its kernels -- the one-block build (up to 4,096 bodies, two sizes of
+it), the centre-of-mass chunks (1,024 positions, or 256 and tiers of 96 chunks) -- and of its
+division-free quotients: every cell equal to the oracle's, bit for bit, and the accelerations of the
+IEEE traversal (which read the quotients) too."""
+
+import numpy as np
+import pytest
+
+import oracle
+from helpers import bodies, canonical_compare, dev, host
+from test_bh_gpu import _clustered, _midpoints
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from nbody.lib import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def check(ctx, d, storage=16, accelerations=True):
+    import torch
+    from nbody.lib import BHTree
+    n = len(d["m"])
+    t = {k: dev(d[k]) for k in ("m", "x", "y", "z")}
+    tree = BHTree(ctx, n, theta=0.7)
+    tree.build(t["m"], t["x"], t["y"], t["z"], d["G"])
+    ctx.sync()
+    ot = oracle.build_subtrees(d["m"], d["x"], d["y"], d["z"], max_level=7, threads=4,
+                               storage_param=storage)
+    assert tree.stats()["ref_node_count"] == ot.node_count
+    np.testing.assert_array_equal(np.array(tree.stats()["aabb"]), ot.aabb)
+    assert canonical_compare(ot, tree.export_ref_layout(n), n) == ot.node_count
+    if accelerations:
+        a = [torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(3)]
+        tree.accel(t["x"], t["y"], t["z"], *a, d["G"], 1e-6, "theta", "f64_ieee")
+        ctx.sync()
+        ref = oracle.bh_accel(ot, d["x"], d["y"], d["z"], d["G"], 1e-6, 0.7, threads=4)
+        for g, r in zip(a, ref):
+            np.testing.assert_array_equal(host(g), r)
+    tree.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 33, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 2048,
+                               2049, 4095, 4096, 4097, 24576, 24577])
+def test_sizes(ctx, n):
+    check(ctx, bodies("plummer", n, seed=n))
+
+
+@pytest.mark.parametrize("n", [1000, 2400, 6000])
+def test_deep_clumps_and_midpoints(ctx, n):
+    check(ctx, _clustered(n, 3), storage=256)
+    check(ctx, _midpoints(n, 4), storage=256)
+
+
+@pytest.mark.parametrize("n", [900, 5000])
+def test_quotients_of_special_values(ctx, n):
+    """Coordinates and masses on powers of two, zeros, mantissas of ones, wide exponent ranges."""
+    rng = np.random.default_rng(n)
+    d = bodies("plummer", n, seed=2)
+    d["m"] = d["m"] * 2.0 ** rng.integers(-60, 60, n)
+    d["m"][1::7] = 2.0 ** rng.integers(-20, 20, len(d["m"][1::7]))
+    d["m"][2::7] = np.nextafter(2.0, 0.0)
+    d["m"][3::50] = 1e-300
+    for k, o in (("x", 0), ("y", 1), ("z", 2)):
+        v = d[k]
+        v[o::11] = np.sign(v[o::11]) * 2.0 ** rng.integers(-12, 2, len(v[o::11]))
+        v[o + 3::13] = 0.0
+        v[o + 5::17] = np.nextafter(1.0, 0.0) * rng.uniform(0.5, 2.0, len(v[o + 5::17]))
+    p = np.stack([d["x"], d["y"], d["z"]], axis=1)
+    keep = np.unique(p, axis=0, return_index=True)[1]
+    for k in ("m", "x", "y", "z"):
+        d[k] = np.ascontiguousarray(d[k][np.sort(keep)])
+    check(ctx, d, storage=64)
+
+
+@pytest.mark.parametrize("n", [700, 5000])
+def test_massless_bodies(ctx, n):
+    d = bodies("plummer", n, seed=9)
+    d["m"][::3] = 0.0
+    check(ctx, d)
+
+
+@pytest.mark.parametrize("n", [2000, 4500])
+def test_coincident_bodies_are_reported(ctx, n):
+    from nbody.lib import BHTree, NBodyError
+    d = bodies("plummer", n, seed=1)
+    for k in ("x", "y", "z"):
+        d[k][7] = d[k][1003]
+    tree = BHTree(ctx, n)
+    tree.build(*[dev(d[k]) for k in ("m", "x", "y", "z")], 1.0)
+    with pytest.raises(NBodyError, match="DEPTH"):
+        ctx.sync()
+    tree.close()
