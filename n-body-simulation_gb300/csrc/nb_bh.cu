@@ -643,8 +643,7 @@ struct ComArgs {
     nbfix::FixHi* fix_hi;
     uint4* fix_lo;
     NodeRec32* rec32;
-    float4* rec32lo;
-    float4* rec32lo2;
+    DfTerms* df_terms;
     NodeAux* aux;
     const uint32_t* node_first_pos;
     uint32_t* children;
@@ -734,6 +733,22 @@ __device__ __forceinline__ float cell_edge2(double box_edge, double edge, float 
     return (float)(edge * edge);
 }
 
+// Terms beyond rec32's: the centre minus the box centre, exactly, as a triple-float and G*mass as a
+// double-float (their first terms are rec32's: both round the same FP64 values).
+__device__ __forceinline__ DfTerms df_terms_of(double cx, double cy, double cz, double ox,
+                                               double oy, double oz, double gm, float gmf,
+                                               bool massive) {
+    DfTerms t{};
+    if (massive) {
+        float hx, hy, hz;
+        tf_split_diff(cx, ox, hx, t.mx, t.lx);
+        tf_split_diff(cy, oy, hy, t.my, t.ly);
+        tf_split_diff(cz, oz, hz, t.mz, t.lz);
+        t.gl = (float)(gm - (double)gmf);
+    }
+    return t;
+}
+
 // Fixed-point record of a node with centre (cx, cy, cz) and mass m.
 __device__ __forceinline__ void write_fix(const ComArgs& A, uint32_t idx, double cx, double cy,
                                           double cz, double m) {
@@ -793,18 +808,7 @@ __device__ void write_records(const ComArgs& A, uint32_t idx, double cx, double 
     q.level = (uint32_t)level;
     A.rec32[idx] = q;
     if (A.records & NB_REC_DF) {
-        // further FP32 terms: the centre minus the box centre, exactly, as a triple-float (rec32,
-        // rec32lo, rec32lo2 .xyz) and G*mass as a double-float (rec32.gm, rec32lo.w)
-        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), lo2 = lo;
-        if (sm != 0) {
-            float hx, hy, hz;  // equal to q.cx, q.cy, q.cz (both round the same FP64 difference)
-            tf_split_diff(rcx, ox, hx, lo.x, lo2.x);
-            tf_split_diff(rcy, oy, hy, lo.y, lo2.y);
-            tf_split_diff(rcz, oz, hz, lo.z, lo2.z);
-            lo.w = (float)(A.G * sm - (double)q.gm);
-        }
-        A.rec32lo[idx] = lo;
-        A.rec32lo2[idx] = lo2;
+        A.df_terms[idx] = df_terms_of(rcx, rcy, rcz, ox, oy, oz, A.G * sm, q.gm, sm != 0);
     }
     if (A.records & NB_REC_LEARNED) {
         // spread^2 = sum m |x-o|^2 / M - |c-o|^2 (o = box centre, which keeps both terms small);
@@ -943,16 +947,7 @@ __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32
     q.level = (uint32_t)level;
     A.rec32[idx] = q;
     if (A.records & NB_REC_DF) {
-        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), lo2 = lo;
-        if (mb != 0) {
-            float hx, hy, hz;
-            tf_split_diff(rcx, ox, hx, lo.x, lo2.x);
-            tf_split_diff(rcy, oy, hy, lo.y, lo2.y);
-            tf_split_diff(rcz, oz, hz, lo.z, lo2.z);
-            lo.w = (float)(A.G * mb - (double)q.gm);
-        }
-        A.rec32lo[idx] = lo;
-        A.rec32lo2[idx] = lo2;
+        A.df_terms[idx] = df_terms_of(rcx, rcy, rcz, ox, oy, oz, A.G * mb, q.gm, mb != 0);
     }
     NodeSums sums{cx, cy, cz, mb, 0.0, 1};
     if (A.records & NB_REC_LEARNED) {  // spread sums and the FP32 body copies of the policy
@@ -1323,8 +1318,7 @@ void carve(nb_bh_tree* t, Carver& c) {
     t->fix_hi = c.take<nbfix::FixHi>(cap);
     t->fix_lo = c.take<uint4>(cap);
     t->rec32 = c.take<NodeRec32>(cap);
-    t->rec32lo = c.take<float4>(cap);
-    t->rec32lo2 = c.take<float4>(cap);
+    t->df_terms = c.take<DfTerms>(cap);
     t->node_q = c.take<double>(cap);
     t->aux = c.take<NodeAux>(cap);
     t->children = c.take<uint32_t>(cap * 8);
@@ -1534,8 +1528,7 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     A.fix_hi = t->fix_hi;
     A.fix_lo = t->fix_lo;
     A.rec32 = t->rec32;
-    A.rec32lo = t->rec32lo;
-    A.rec32lo2 = t->rec32lo2;
+    A.df_terms = t->df_terms;
     A.q = t->node_q;
     A.aux = t->aux;
     A.node_first_pos = t->node_first;

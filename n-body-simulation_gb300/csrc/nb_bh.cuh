@@ -30,6 +30,12 @@ struct __align__(16) NodeRec32 {
     uint32_t skip, body, level;
 };
 
+// Further FP32 terms of rec32's centre (with them a triple-float: exact) and G*mass (a double-float).
+struct __align__(32) DfTerms {
+    float mx, my, mz, gl;  // second terms of the centre and of G * mass
+    float lx, ly, lz, pad;  // third terms of the centre
+};
+
 // Extra per-node data of the learned opening policy.
 struct __align__(16) NodeAux {
     float spread_rel;  // mass-weighted rms distance of the cell's bodies from its centre of
@@ -90,8 +96,7 @@ struct nb_bh_tree {
     nbfix::FixHi* fix_hi = nullptr;
     uint4* fix_lo = nullptr;
     NodeRec32* rec32 = nullptr;
-    float4* rec32lo = nullptr;   // second FP32 terms of rec32's centre and G*mass
-    float4* rec32lo2 = nullptr;  // third FP32 terms of the centre (triple-float: exact FP64)
+    DfTerms* df_terms = nullptr;  // further FP32 terms of rec32's centre and G*mass
     double* node_q = nullptr;  // sum of m |x - box centre|^2 (for the spread)
     NodeAux* aux = nullptr;
     uint32_t* children = nullptr;  // 8 per node: children in visit order, NB_NONE padded

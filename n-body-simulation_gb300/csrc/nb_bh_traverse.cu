@@ -556,119 +556,140 @@ regroup_kernel(const uint32_t* __restrict__ ids, const uint32_t* __restrict__ wa
     if (p < n) order[p] = ids[blockIdx.x * RG_WINDOW + (uint32_t)(key[i] & 0xffffffffu)];
 }
 
-// Per-body reference rule with FP64-accurate double-float monopoles (NB_DF64). The walk and the
-// opening decisions are those of bh_theta_lane_kernel (FP32 pre-test with a proven margin, the
-// reference's FP64 expression for undecided cells), so each body accepts exactly the reference's
-// cells; the accepted monopoles are evaluated in double-float arithmetic on the FP32 pipe
-// (~2^-48 relative per operation) instead of on the FP64 pipe, which this part runs at 1/64 of
-// the FP32 rate. Centres and the body are exact triple-floats relative to the box centre (rec32,
-// rec32lo, rec32lo2), so the separation is accurate to ~2^-48 of itself; G*mass is rec32.gm +
-// rec32lo.w. rsqrt: hardware estimate y0 plus the third-order step
+// Per-body reference rule with FP64-accurate double-float monopoles (NB_DF64, systems of one lane per
+// body; smaller ones take bh_theta_team_kernel's fixed point, which is faster there and more
+// accurate). The walk, the decisions and the lists are those of bh_theta_fix_kernel, so each body
+// accepts exactly the reference's cells; the accepted monopoles are evaluated in double-float
+// arithmetic on the FP32 pipe (~2^-48 relative per operation). Centres and the body are exact
+// triple-floats relative to the box centre (rec32 and df_terms), so the separation is accurate to
+// ~2^-48 of itself. rsqrt: hardware estimate y0 plus the third-order step
 // y = y0 (1 + e/2 + 3e^2/8), e = 1 - r^2 y0^2 evaluated with error-free products. The sums are
 // Neumaier-compensated (hi + running lo), converted to FP64 at the end and scaled by G / G_build.
-__global__ void __launch_bounds__(TR_THREADS)
-bh_theta_df_kernel(const NodeRec32* __restrict__ rec32, const float4* __restrict__ rec32lo,
-                   const float4* __restrict__ rec32lo2, const NodeRec64* __restrict__ rec64,
-                   const uint32_t* __restrict__ info,
+//  Bound: the load pipe and issue, as bh_theta_fix_kernel. Lists, record prefetch and 256-bit loads
+//  against one cell at a time inside the divergent walk: 262,144 bodies 3.18 -> 2.63 ms, 1,048,576
+//  11.9 -> 11.0 ms (disc, theta = 0.5); 20 warps per SM (32: 3 to 12% slower). Same bits as before.
+struct DfBody {
+    float hx, hy, hz, mx, my, mz, lx, ly, lz;  // minus the box centre, exactly
+    float e2h, e2l;                            // eps^2
+    float ahx, ahy, ahz, alx, aly, alz;        // compensated sums
+};
+
+__device__ __forceinline__ void df_monopole(const float4 c, const DfTerms& t, DfBody& b) {
+    if (c.w == 0.f && t.gl == 0.f) return;
+    const nb_df dx = tf_diff(c.x, t.mx, t.lx, b.hx, b.mx, b.lx);
+    const nb_df dy = tf_diff(c.y, t.my, t.ly, b.hy, b.my, b.ly);
+    const nb_df dz = tf_diff(c.z, t.mz, t.lz, b.hz, b.mz, b.lz);
+    // r^2 + eps^2
+    const nb_df sx = df_sqr(dx), sy = df_sqr(dy), sz = df_sqr(dz);
+    nb_df u = df_two_sum(sx.h, sy.h);
+    u.l += sx.l + sy.l;
+    nb_df v = df_two_sum(u.h, sz.h);
+    v.l += u.l + sz.l;
+    nb_df w2 = df_two_sum(v.h, b.e2h);  // eps^2 may be as large as r^2
+    w2.l += v.l + b.e2l;
+    const nb_df r2 = df_two_sum(w2.h, w2.l);
+    // 1/r
+    const float y0 = nb_rsqrt_f32(r2.h);
+    const float q = y0 * y0, qe = fmaf(y0, y0, -q);  // y0^2 = q + qe exactly
+    const float th = r2.h * q;
+    float te = fmaf(r2.h, q, -th);
+    te = fmaf(r2.h, qe, te);
+    te = fmaf(r2.l, q, te);
+    const float e = (1.0f - th) - te;  // 1 - th is exact (th is within 2^-21 of 1)
+    const nb_df inv = df_fast_two_sum(y0, y0 * (e * fmaf(0.375f, e, 0.5f)));
+    // G m / r^3
+    const nb_df w = df_mul(nb_df{c.w, t.gl}, df_mul(df_sqr(inv), inv));
+    // compensated sums
+    const nb_df tx = df_mul(dx, w), ty = df_mul(dy, w), tz = df_mul(dz, w);
+    nb_df s = df_two_sum(b.ahx, tx.h);
+    b.ahx = s.h;
+    b.alx += s.l + tx.l;
+    s = df_two_sum(b.ahy, ty.h);
+    b.ahy = s.h;
+    b.aly += s.l + ty.l;
+    s = df_two_sum(b.ahz, tz.h);
+    b.ahz = s.h;
+    b.alz += s.l + tz.l;
+}
+
+__device__ __forceinline__ DfTerms load_df(const DfTerms* __restrict__ p) {
+    DfTerms t;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(t.mx), "=f"(t.my), "=f"(t.mz), "=f"(t.gl), "=f"(t.lx), "=f"(t.ly), "=f"(t.lz),
+          "=f"(t.pad)
+        : "l"(p));
+    return t;
+}
+
+constexpr int DF_BLOCKS_PER_SM = 5;
+
+__global__ void __launch_bounds__(TR_THREADS, DF_BLOCKS_PER_SM)
+bh_theta_df_kernel(const NodeRec32* __restrict__ rec32, const DfTerms* __restrict__ df_terms,
+                   const NodeRec64* __restrict__ rec64, const uint32_t* __restrict__ info,
                    const uint32_t* __restrict__ ids, const double* __restrict__ x,
                    const double* __restrict__ y, const double* __restrict__ z,
                    const double* __restrict__ box, uint32_t n, double theta, double eps2,
                    double gscale, double* __restrict__ ax, double* __restrict__ ay,
-                   double* __restrict__ az, const uint32_t* __restrict__ order,
-                   uint32_t* __restrict__ walk_len) {
-    using A = Arith<FAST64>;
-    const uint32_t p = blockIdx.x * TR_THREADS + threadIdx.x;
-    if (p >= n) return;
-    const uint32_t nn = info[0];
-    const uint32_t me = order != nullptr ? order[p] : ids[p];  // as bh_theta_lane_kernel
-    uint32_t accepted = 0;
-    const double px = x[me], py = y[me], pz = z[me];
-    const double E = box[6];
-    const double ox = box[0] + E / 2, oy = box[1] + E / 2, oz = box[2] + E / 2;
-    const float pxf = (float)(px - ox), pyf = (float)(py - oy), pzf = (float)(pz - oz);
-    // the body minus the box centre, exactly, as triple-floats (pxf etc. are their leading terms)
-    float hx, hy, hz, pxm, pym, pzm, pxl, pyl, pzl;
-    tf_split_diff(px, ox, hx, pxm, pxl);
-    tf_split_diff(py, oy, hy, pym, pyl);
-    tf_split_diff(pz, oz, hz, pzm, pzl);
-    const float e2h = (float)eps2, e2l = (float)(eps2 - (double)e2h);
-    const float th2 = (float)(theta * theta);
-    const float u4 = 4.0f * 5.9604645e-8f;  // 4 * 2^-24
-    const float Ef = (float)E;
-    float ahx = 0.f, ahy = 0.f, ahz = 0.f, alx = 0.f, aly = 0.f, alz = 0.f;
-    uint32_t k = 0;
-    while (k < nn) {
-        const NodeRec32 r = rec32[k];
-        if (r.body == me) {
-            k = r.skip;
-            continue;
+                   double* __restrict__ az, uint32_t* __restrict__ next_group,
+                   const uint32_t* __restrict__ order, uint32_t* __restrict__ walk_len) {
+    __shared__ uint32_t list[FIX_LIST][TR_THREADS];
+    const uint32_t n_groups = (n + 31) / 32, nn = info[0];
+    const int lane = threadIdx.x & 31, tid = threadIdx.x;
+    for (;;) {  // persistent warps, as bh_theta_lane_kernel
+        uint32_t grp = 0;
+        if (lane == 0) grp = atomicAdd(next_group, 1u);
+        grp = __shfl_sync(0xffffffffu, grp, 0);
+        if (grp >= n_groups) break;
+        const uint32_t p = grp * 32 + lane;
+        const bool valid = p < n;
+        const uint32_t me = valid ? (order != nullptr ? order[p] : ids[p]) : 0u;
+        Pretest pre;
+        DfBody b{};
+        {
+            const double px = x[me], py = y[me], pz = z[me], E = box[6];
+            pre = pretest_of(box, px, py, pz, theta);
+            tf_split_diff(px, box[0] + E / 2, b.hx, b.mx, b.lx);
+            tf_split_diff(py, box[1] + E / 2, b.hy, b.my, b.ly);
+            tf_split_diff(pz, box[2] + E / 2, b.hz, b.mz, b.lz);
+            b.e2h = (float)eps2;
+            b.e2l = (float)(eps2 - (double)b.e2h);
         }
-        bool accept = r.body != NB_NONE;
-        if (!accept) {
-            const float dxf = r.cx - pxf, dyf = r.cy - pyf, dzf = r.cz - pzf;
-            const float d2f = fmaf(dxf, dxf, fmaf(dyf, dyf, dzf * dzf));
-            const float t = th2 * d2f;
-            const float rel = u4 * (3.5f * Ef * nb_rsqrt_f32(d2f) + 8.0f);
-            const float margin = t * rel + u4 * r.edge2;
-            if (r.edge2 > t + margin) {
-                accept = false;
-            } else if (r.edge2 < t - margin) {
-                accept = true;
-            } else {
-                const NodeRec64 q = rec64[k];
-                const double dx = A::sub(q.cx, px), dy = A::sub(q.cy, py), dz = A::sub(q.cz, pz);
-                accept = A::mul(q.edge, A::rsqrt(A::norm2(dx, dy, dz))) < theta;
+        uint32_t accepted = 0, k = valid ? 0u : nn;
+        for (;;) {
+            int cnt = 0;
+            while (cnt < FIX_LIST && k < nn) {
+                const NodeRec32 r = load_rec32(rec32 + k);
+                const bool accept = accepts(r, pre, rec64, k, x, y, z, me, theta);
+                if (accept && r.body != me) {
+                    list[cnt][tid] = k;
+                    ++cnt;
+                }
+                k = accept ? r.skip : k + 1;
+            }
+            accepted += cnt;
+            const int most = __reduce_max_sync(0xffffffffu, cnt);
+            if (most == 0) break;
+            uint32_t at = cnt > 0 ? list[0][tid] : 0u;
+            float4 next_c = *reinterpret_cast<const float4*>(rec32 + at);
+            DfTerms next_t = load_df(df_terms + at);
+            for (int i = 0; i < most; ++i) {
+                const float4 c = next_c;
+                const DfTerms t = next_t;
+                if (i + 1 < cnt) {
+                    at = list[i + 1][tid];
+                    next_c = *reinterpret_cast<const float4*>(rec32 + at);
+                    next_t = load_df(df_terms + at);
+                }
+                if (i < cnt) df_monopole(c, t, b);
             }
         }
-        if (accept) {
-            ++accepted;
-            const float4 lo = rec32lo[k];
-            if (r.gm != 0.f || lo.w != 0.f) {
-                const float4 lo2 = rec32lo2[k];
-                const nb_df dx = tf_diff(r.cx, lo.x, lo2.x, pxf, pxm, pxl);
-                const nb_df dy = tf_diff(r.cy, lo.y, lo2.y, pyf, pym, pyl);
-                const nb_df dz = tf_diff(r.cz, lo.z, lo2.z, pzf, pzm, pzl);
-                // r^2 + eps^2
-                const nb_df sx = df_sqr(dx), sy = df_sqr(dy), sz = df_sqr(dz);
-                nb_df a = df_two_sum(sx.h, sy.h);
-                a.l += sx.l + sy.l;
-                nb_df b = df_two_sum(a.h, sz.h);
-                b.l += a.l + sz.l;
-                nb_df c = df_two_sum(b.h, e2h);  // eps^2 may be as large as r^2
-                c.l += b.l + e2l;
-                const nb_df r2 = df_two_sum(c.h, c.l);
-                // 1/r
-                const float y0 = nb_rsqrt_f32(r2.h);
-                const float q = y0 * y0, qe = fmaf(y0, y0, -q);  // y0^2 = q + qe exactly
-                const float th = r2.h * q;
-                float te = fmaf(r2.h, q, -th);
-                te = fmaf(r2.h, qe, te);
-                te = fmaf(r2.l, q, te);
-                const float e = (1.0f - th) - te;  // 1 - th is exact (th is within 2^-21 of 1)
-                const nb_df inv = df_fast_two_sum(y0, y0 * (e * fmaf(0.375f, e, 0.5f)));
-                // G m / r^3
-                const nb_df w = df_mul(nb_df{r.gm, lo.w}, df_mul(df_sqr(inv), inv));
-                // compensated sums
-                const nb_df tx = df_mul(dx, w), ty = df_mul(dy, w), tz = df_mul(dz, w);
-                nb_df s = df_two_sum(ahx, tx.h);
-                ahx = s.h;
-                alx += s.l + tx.l;
-                s = df_two_sum(ahy, ty.h);
-                ahy = s.h;
-                aly += s.l + ty.l;
-                s = df_two_sum(ahz, tz.h);
-                ahz = s.h;
-                alz += s.l + tz.l;
-            }
-            k = r.skip;
-        } else {
-            k = k + 1;
+        if (valid) {
+            walk_len[me] = accepted;
+            ax[me] = ((double)b.ahx + (double)b.alx) * gscale;
+            ay[me] = ((double)b.ahy + (double)b.aly) * gscale;
+            az[me] = ((double)b.ahz + (double)b.alz) * gscale;
         }
     }
-    walk_len[me] = accepted;
-    ax[me] = ((double)ahx + (double)alx) * gscale;
-    ay[me] = ((double)ahy + (double)aly) * gscale;
-    az[me] = ((double)ahz + (double)alz) * gscale;
 }
 
 // Per-body reference rule with FP32 pair math and compensated accumulation.
@@ -901,16 +922,19 @@ bh_count_kernel(const NodeRec64* __restrict__ rec, const uint32_t* __restrict__ 
 int g_lockstep = 0;
 
 // Resident blocks per SM of the persistent kernels (queried once, before any stream capture uses
-// them): the IEEE lane kernel, the fixed-point kernel.
-int g_lane_per_sm[2] = {0, 0};
+// them): the IEEE lane kernel, the fixed-point and the double-float kernel.
+int g_lane_per_sm[3] = {0, 0, 0};
 
-nb_status lane_per_sm(bool ieee, int* out) {
-    int& ps = g_lane_per_sm[ieee ? 0 : 1];
+nb_status lane_per_sm(nb_precision prec, int* out) {
+    const int which = prec == NB_F64_IEEE ? 0 : (prec == NB_F64 ? 1 : 2);
+    int& ps = g_lane_per_sm[which];
     if (ps == 0) {
-        NB_CUDA_TRY(ieee ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, bh_theta_lane_kernel,
-                                                                         TR_THREADS, 0)
-                         : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, bh_theta_fix_kernel,
-                                                                         TR_THREADS, 0));
+        auto query = [&](auto kernel) {
+            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, kernel, TR_THREADS, 0);
+        };
+        NB_CUDA_TRY(which == 0 ? query(bh_theta_lane_kernel)
+                               : (which == 1 ? query(bh_theta_fix_kernel)
+                                             : query(bh_theta_df_kernel)));
         if (ps < 1) ps = 1;
     }
     *out = ps;
@@ -950,37 +974,41 @@ nb_status walk_order(const nb_bh_tree* t, cudaStream_t s, const uint32_t** order
 // 1,048,576 bodies than 40, 0.2% faster than 24 or 16).
 constexpr int LANE_BLOCKS_PER_SM = 5;
 
-nb_status launch_lane(nb_ctx* ctx, const nb_bh_tree* t, bool ieee, const double* x,
+nb_status launch_lane(nb_ctx* ctx, const nb_bh_tree* t, nb_precision prec, const double* x,
                       const double* y, const double* z, double* ax, double* ay, double* az,
                       double G, double eps2, cudaStream_t s) {
     int ps = 0;
-    NB_TRY(lane_per_sm(ieee, &ps));
-    if (ieee) ps = std::min(ps, LANE_BLOCKS_PER_SM);
+    NB_TRY(lane_per_sm(prec, &ps));
+    if (prec == NB_F64_IEEE) ps = std::min(ps, LANE_BLOCKS_PER_SM);
     int grid = nb::ceil_div(t->n, TR_THREADS);
     if (grid > ctx->sm_count * ps) grid = ctx->sm_count * ps;
     NB_CUDA_TRY(cudaMemsetAsync(t->work + 1, 0, sizeof(uint32_t), s));
     const uint32_t* order = nullptr;
     NB_TRY(walk_order(t, s, &order));
-    if (ieee)
+    if (prec == NB_F64_IEEE)
         bh_theta_lane_kernel<<<grid, TR_THREADS, 0, s>>>(
             t->rec32, t->rec64, t->info, t->ids, x, y, z, t->box, t->n, t->params.theta, eps2, G,
             ax, ay, az, t->work + 1, order, t->walk_len);
-    else
+    else if (prec == NB_F64)
         bh_theta_fix_kernel<<<grid, TR_THREADS, 0, s>>>(
             t->rec32, t->rec64, t->fix_hi, t->fix_lo, t->info, t->ids, x, y, z, t->box, t->n,
             t->params.theta, eps2, G, ax, ay, az, t->work + 1, order, t->walk_len);
-    NB_TRY(nb::check_launch(ieee ? "bh_theta_lane_kernel" : "bh_theta_fix_kernel"));
+    else
+        bh_theta_df_kernel<<<grid, TR_THREADS, 0, s>>>(
+            t->rec32, t->df_terms, t->rec64, t->info, t->ids, x, y, z, t->box, t->n,
+            t->params.theta, eps2, G / t->G, ax, ay, az, t->work + 1, order, t->walk_len);
+    NB_TRY(nb::check_launch("Barnes-Hut lane kernel"));
     t->walk_n = t->n;
     return NB_OK;
 }
 
-// NB_F64 under the per-body rule: teams of lanes for small systems (in tree order: neighbouring
-// bodies share their windows' loads), one lane per body otherwise.
-nb_status launch_f64(nb_ctx* ctx, const nb_bh_tree* t, const double* x, const double* y,
-                     const double* z, double* ax, double* ay, double* az, double G, double eps2,
-                     cudaStream_t s) {
+// NB_F64 and NB_DF64 under the per-body rule: teams of lanes for small systems (in tree order:
+// neighbouring bodies share their windows' loads), one lane per body otherwise.
+nb_status launch_f64(nb_ctx* ctx, const nb_bh_tree* t, nb_precision prec, const double* x,
+                     const double* y, const double* z, double* ax, double* ay, double* az,
+                     double G, double eps2, cudaStream_t s) {
     const int team = team_lanes(ctx, t->n);
-    if (team == 1) return launch_lane(ctx, t, false, x, y, z, ax, ay, az, G, eps2, s);
+    if (team == 1) return launch_lane(ctx, t, prec, x, y, z, ax, ay, az, G, eps2, s);
     const int grid = nb::ceil_div((long long)t->n * team, TR_THREADS);
     auto go = [&](auto kernel) {
         kernel<<<grid, TR_THREADS, 0, s>>>(t->rec32, t->rec64, t->fix_hi, t->fix_lo, t->info,
@@ -1038,7 +1066,7 @@ nb_status nb_bh_accel(nb_ctx* ctx, const nb_bh_tree* t, const double* x, const d
                         eps2, G, team, ax, ay, az);
                     return nb::check_launch("bh_theta_f64_kernel<ieee>");
                 }
-                return launch_lane(ctx, t, true, x, y, z, ax, ay, az, G, eps2, s);
+                return launch_lane(ctx, t, prec, x, y, z, ax, ay, az, G, eps2, s);
             case NB_F64:
                 NB_TRY(nb_need_records(t, NB_REC_FP64, "nb_bh_accel"));
                 if (g_lockstep) {
@@ -1047,22 +1075,13 @@ nb_status nb_bh_accel(nb_ctx* ctx, const nb_bh_tree* t, const double* x, const d
                         eps2, G, team, ax, ay, az);
                     return nb::check_launch("bh_theta_f64_kernel");
                 }
-                return launch_f64(ctx, t, x, y, z, ax, ay, az, G, eps2, s);
+                return launch_f64(ctx, t, prec, x, y, z, ax, ay, az, G, eps2, s);
             case NB_DF64:
                 NB_TRY(nb_need_records(t, NB_REC_FP64 | NB_REC_DF, "nb_bh_accel"));
                 if (t->G == 0)
                     return nb::set_error(NB_ERR_INVALID_ARG,
                                          "nb_bh_accel: NB_DF64 needs a build with G != 0");
-            {
-                const uint32_t* order = nullptr;
-                NB_TRY(walk_order(t, s, &order));
-                bh_theta_df_kernel<<<grid, TR_THREADS, 0, s>>>(
-                    t->rec32, t->rec32lo, t->rec32lo2, t->rec64, t->info, t->ids, x, y, z, t->box,
-                    n, theta, eps2, G / t->G, ax, ay, az, order, t->walk_len);
-                NB_TRY(nb::check_launch("bh_theta_df_kernel"));
-                t->walk_n = t->n;
-                return NB_OK;
-            }
+                return launch_f64(ctx, t, prec, x, y, z, ax, ay, az, G, eps2, s);
             case NB_F32C:
                 if (G != t->G)
                     return nb::set_error(NB_ERR_INVALID_ARG, "nb_bh_accel: G differs from the build's");
@@ -1144,8 +1163,7 @@ nb_status nb_bh_graph_create(nb_ctx* ctx, nb_bh_tree* t, const double* m, double
         return nb::set_error(NB_ERR_INVALID_ARG, "nb_bh_graph_create: phase timing is on");
     *out = nullptr;
     int ps = 0;  // one-time queries happen here, outside the capture
-    NB_TRY(lane_per_sm(true, &ps));
-    NB_TRY(lane_per_sm(false, &ps));
+    for (nb_precision p : {NB_F64_IEEE, NB_F64, NB_DF64}) NB_TRY(lane_per_sm(p, &ps));
     NB_TRY(nb::learned_per_sm(&ps));
     cudaStream_t s;
     NB_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
