@@ -144,9 +144,11 @@ __device__ __forceinline__ void box_extras(double* __restrict__ box, uint32_t i)
         long long v = 0;
         for (int k = 0; k < 6; ++k)
             v = max(v, __double_as_longlong(box[k]) & 0x7fffffffffffffffll);
-        box[10] = (double)nbfix::k_of(__longlong_as_double(v));
+        const int K = nbfix::k_of(__longlong_as_double(v));
+        box[10] = (double)K;
+        // K and (float)(edge^2) as bits, for the record writers
+        box[11] = __hiloint2double(K, __float_as_int((float)(box[6] * box[6])));
     }
-    if (i == 4) box[11] = box[6] * box[6];
 }
 
 __global__ void keys_quantized_kernel(const double* __restrict__ x, const double* __restrict__ y,
@@ -200,7 +202,7 @@ __device__ __forceinline__ long long fixed_digits(double v, double mn, double sc
     if ((uint64_t)b > 0x4330000000000000ull && (b << 1) != 0) return -1;
     const int e = (int)(b >> 52);
     const long long U = e < 1023 ? 0 : ((b & 0xfffffffffffffll) | (1ll << 52)) >> (1075 - e);
-    const long long hi = (U + m) >> 31, lo = (U - m - 1) >> 31;
+    const long long hi = min((U + m) >> 31, 0x1fffffll), lo = max((U - m - 1) >> 31, 0ll);
     return hi == lo ? hi : -1;
 }
 
@@ -385,7 +387,7 @@ __device__ __forceinline__ uint32_t digit_at(const uint64_t* __restrict__ key0,
 // The node tables emit_at writes (global memory).
 struct NodeTable {
     uint8_t* level;
-    uint32_t *first, *last, *skip, *parent, *body, *info, *children;
+    uint32_t *first, *last, *skip, *body, *info, *children;
 };
 
 // The leaf of sorted position p and the internal cell whose first split it is.
@@ -406,7 +408,6 @@ __device__ __forceinline__ void emit_at(uint32_t p, uint32_t n, const uint32_t* 
         T.skip[idx] = base[p + 1];
         T.body[idx] = ids[p];
         const uint32_t par = parent_of(p, p, dl, dr, split_level, split_start, base, mask);
-        T.parent[idx] = par;
         if (par != NB_NONE) {
             // the parent's level is the deeper boundary split; slot = visit rank there
             T.children[(size_t)par * 8 + digit_at(key0, key1, p, max(dl, dr))] = idx;
@@ -424,7 +425,6 @@ __device__ __forceinline__ void emit_at(uint32_t p, uint32_t n, const uint32_t* 
         const int dl = a > 0 ? (int)split_level[a - 1] : -1;
         const int dr = b + 1 < n ? (int)split_level[b] : -1;
         const uint32_t par = parent_of(a, b, dl, dr, split_level, split_start, base, mask);
-        T.parent[idx] = par;
         if (par != NB_NONE) {
             T.children[(size_t)par * 8 + digit_at(key0, key1, a, max(dl, dr))] = idx;
         }
@@ -442,14 +442,19 @@ __global__ void emit_kernel(uint32_t n, const uint32_t* __restrict__ ids,
             mask, base, key0, key1, T);
 }
 
-// Steps 1 to 6 for small systems in one block, sharing the device functions above: the chain of 18
-// launches cost 135 us at 777 bodies and 167 at 4,096, this one 40 and 115. (Key, body) pairs by a bitonic sort in shared memory
-// (ties by body id: the stable order), the DFS numbering by a block scan.
+// Steps 1 to 6 for small systems in one block, sharing the device functions above: the chain of
+// launches costs 135 us at 777 bodies and 167 at 4,096, this one 28 and 98. Bound by latency: one
+// block's barriers and dependent instructions. (Key, body) pairs sort bitonically (ties by body id:
+// the stable order) in registers, with exchanges by shuffle within a warp; the cells' ranges come
+// from the splits' levels and their minima over powers of two, a halving walk over bytes in shared
+// memory; with all exchanges through shared memory and searches over the keys 41 and 115 us. The
+// DFS numbering is a block scan.
 constexpr uint32_t SB_MAX_N = 4096;
 
+constexpr int small_log2(uint32_t v) { return v <= 1 ? 0 : 1 + small_log2(v / 2); }
 template <uint32_t CAP>
-constexpr size_t small_smem_bytes() {
-    return CAP * (8 + 8 + 8 + 4 + 4 + 4 + 4 + 1) + 64;
+constexpr size_t small_smem_bytes() {  // keys, masks, ids, cell ranges, indices, split levels' minima
+    return CAP * (8 + 8 + 8 + 4 + 4 + 4 + 4 + small_log2(CAP)) + 64;
 }
 
 __device__ __forceinline__ uint32_t small_block_scan(uint32_t v, uint32_t* warp_sums,
@@ -482,7 +487,6 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
                    uint32_t* __restrict__ base_out, NodeTable T, uint32_t* __restrict__ err,
                    int quantized) {
     constexpr int PER = CAP / THREADS;  // positions per thread
-    static_assert(PER == 2 || PER == 4, "positions per thread");
     extern __shared__ __align__(16) unsigned char small_smem[];
     uint64_t* key0 = reinterpret_cast<uint64_t*>(small_smem);
     uint64_t* key1 = key0 + CAP;
@@ -491,10 +495,12 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
     uint32_t* split_start = ids + CAP;
     uint32_t* split_end = split_start + CAP;
     uint32_t* base = split_end + CAP;  // CAP + 1 entries
-    uint8_t* split_level = reinterpret_cast<uint8_t*>(base + CAP + 1);
+    // level_min[d][p]: the least split level of positions p .. p + 2^d - 1; d = 0: the levels
+    uint8_t (*level_min)[CAP] = reinterpret_cast<uint8_t (*)[CAP]>(base + CAP + 1);
+    uint8_t* split_level = level_min[0];
     __shared__ long long wmin[3][32], wmax[3][32];
     __shared__ uint32_t warp_sums[32];
-    __shared__ double sbox[12];
+    __shared__ double sbox[11];
     __shared__ FixedGrid grid_s;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // children lists start empty; written before the barriers below, filled after them
@@ -506,7 +512,7 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
     long long mn[3] = {zero, zero, zero}, mx[3] = {zero, zero, zero};
 #pragma unroll
     for (int h = 0; h < PER; ++h) {
-        const uint32_t i = tid + h * THREADS;
+        const uint32_t i = tid * PER + h;
         const bool in = i < n;
         px[h] = in ? x[i] : 0.0;
         py[h] = in ? y[i] : 0.0;
@@ -555,45 +561,132 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
         if (lane == 0 && !quantized) grid_s = fixed_grid(sbox);
     }
     __syncthreads();
+    // (key, body) number e = tid * PER + h in registers; exchanges within a thread, by shuffles within
+    // a warp, and through shared memory beyond
+    uint64_t key[PER];
+    uint32_t id[PER];
 #pragma unroll
     for (int h = 0; h < PER; ++h) {
-        const uint32_t i = tid + h * THREADS;
-        uint64_t k = ~0ull;  // above every key (63 bits)
+        const uint32_t i = tid * PER + h;
+        key[h] = ~0ull;  // above every key (63 bits)
+        id[h] = i;
         if (i < n)
-            k = quantized ? key_word_quantized(sbox, px[h], py[h], pz[h], 0)
-                          : exact_key(sbox, grid_s, px[h], py[h], pz[h]);
-        key0[i] = k;
-        ids[i] = i;
+            key[h] = quantized ? key_word_quantized(sbox, px[h], py[h], pz[h], 0)
+                               : exact_key(sbox, grid_s, px[h], py[h], pz[h]);
         key1[i] = 0;
         mask[i] = 0;
     }
-    __syncthreads();
     uint32_t m = 2;  // positions to sort: a power of two
     while (m < n) m <<= 1;
     for (uint32_t k = 2; k <= m; k <<= 1) {
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t q = tid; q < m / 2; q += THREADS) {  // compare-exchange number q
-                const uint32_t lo = ((q & ~(j - 1)) << 1) | (q & (j - 1)), hi = lo | j;
-                const uint64_t a = key0[lo], b = key0[hi];
-                const uint32_t ia = ids[lo], ib = ids[hi];
-                const bool gt = a > b || (a == b && ia > ib);
-                if (gt == ((lo & k) == 0)) {
-                    key0[lo] = b;
-                    key0[hi] = a;
-                    ids[lo] = ib;
-                    ids[hi] = ia;
+            if (j < (uint32_t)PER) {
+#pragma unroll
+                for (int h = 0; h < PER; ++h) {
+#pragma unroll
+                    for (int g = h + 1; g < PER; ++g) {
+                        if ((uint32_t)(h ^ g) != j) continue;
+                        const bool up = ((tid * PER + h) & k) == 0;
+                        const bool gt = key[h] > key[g] || (key[h] == key[g] && id[h] > id[g]);
+                        if (gt == up) {
+                            const uint64_t tk = key[h];
+                            key[h] = key[g];
+                            key[g] = tk;
+                            const uint32_t ti = id[h];
+                            id[h] = id[g];
+                            id[g] = ti;
+                        }
+                    }
+                }
+                continue;
+            }
+            const bool far = j >= 32u * PER;
+            if (far) {
+#pragma unroll
+                for (int h = 0; h < PER; ++h) {
+                    key0[tid * PER + h] = key[h];
+                    ids[tid * PER + h] = id[h];
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int h = 0; h < PER; ++h) {
+                const uint32_t e = tid * PER + h;
+                uint64_t ok;
+                uint32_t oi;
+                if (far) {
+                    ok = key0[e ^ j];
+                    oi = ids[e ^ j];
+                } else {
+                    ok = __shfl_xor_sync(0xffffffffu, key[h], j / PER);
+                    oi = __shfl_xor_sync(0xffffffffu, id[h], j / PER);
+                }
+                const bool low = (e & j) == 0, up = (e & k) == 0;
+                const bool gt = key[h] > ok || (key[h] == ok && id[h] > oi);
+                if (gt == (low == up)) {  // the other one belongs here
+                    key[h] = ok;
+                    id[h] = oi;
                 }
             }
-            // exchanges at a distance of up to 32 stay within a warp's blocks of 64 positions
-            if (j > 32) __syncthreads(); else __syncwarp();
+            if (far) __syncthreads();
         }
-        __syncthreads();
     }
+#pragma unroll
+    for (int h = 0; h < PER; ++h) {
+        key0[tid * PER + h] = key[h];
+        ids[tid * PER + h] = id[h];
+    }
+    __syncthreads();
     for (uint32_t p = tid; p < n; p += THREADS)
         fix_run(p, x, y, z, n, sbox, key0, key1, ids, err, quantized);
     __syncthreads();
-    for (uint32_t p = tid; p < n; p += THREADS)
-        split_at(p, key0, key1, n, split_level, split_start, split_end, mask, err);
+    // the splits' levels and their minima over powers of two, then the cells' ranges: a cell of level
+    // L reaches from its split as far as no split is below L, and the split whose left side has none
+    // at L stands for the cell (split_at's rules)
+    const int log = __ffs((int)m) - 1;
+    for (uint32_t p = tid; p < m; p += THREADS) {
+        int L = 0;  // past the last split: below or at every level, never crossed
+        if (p + 1 < n) {
+            L = shared_digits(key0, key1, p, p + 1);
+            if (L >= 2 * NB_KEY_LEVELS) {
+                atomicOr(err, NB_DEVERR_DEPTH);
+                L = 2 * NB_KEY_LEVELS - 1;
+            }
+        }
+        split_level[p] = (uint8_t)L;
+    }
+    __syncthreads();
+    for (int d = 1; d < log; ++d) {
+        const uint32_t half = 1u << (d - 1);
+        for (uint32_t p = tid; p < m; p += THREADS)
+            level_min[d][p] = p + half < m ? min(level_min[d - 1][p], level_min[d - 1][p + half])
+                                             : level_min[d - 1][p];
+        __syncthreads();
+    }
+    for (uint32_t p = tid; p + 1 < n; p += THREADS) {
+        const uint32_t L = split_level[p];
+        uint32_t a = p, least = 255;
+        for (int d = log - 1; d >= 0; --d) {
+            const uint32_t w = 1u << d;
+            if (a < w) continue;
+            const uint32_t v = level_min[d][a - w];
+            if (v >= L) {
+                a -= w;
+                least = min(least, v);
+            }
+        }
+        split_start[p] = a;
+        split_end[p] = NB_NONE;
+        if (least > L) {  // the leftmost split of its cell
+            uint32_t b = p;
+            for (int d = log - 1; d >= 0; --d) {
+                const uint32_t w = 1u << d;
+                if (b + w < n && level_min[d][b] >= L) b += w;
+            }
+            split_end[p] = b;
+            atomicOr(&mask[a], 1ull << L);
+        }
+    }
     __syncthreads();
     {
         const uint32_t p = PER * tid;
@@ -636,7 +729,7 @@ struct ComArgs {
     const unsigned long long* mask;
     const uint32_t* base;
     const uint8_t* node_level;
-    const uint32_t *node_first, *node_last, *node_skip, *node_parent, *node_body;
+    const uint32_t *node_first, *node_last, *node_skip, *node_body;
     uint32_t* node_count;
     double *comx, *comy, *comz, *mass, *q;
     NodeRec64* rec64;
@@ -675,7 +768,7 @@ __device__ __forceinline__ int biased_exp(double v) {
 __device__ __forceinline__ double leaf_quotient(double x, double m, double c) {
     const long long xb = __double_as_longlong(x);
     const int ex = biased_exp(x), em = biased_exp(m), ec = biased_exp(c);
-    const bool m_ok = m > 0.0 && em >= 64 && em <= 2040;
+    const bool m_ok = __double_as_longlong(m) > 0 && em >= 64 && em <= 2040;
     if (m_ok && (xb << 1) == 0) return c;  // 0 / m
     if (!m_ok || ex == 0 || ex == 0x7ff || (xb & 0xfffffffffffffll) == 0 || ec < 128 || ec > 2040)
         return __ddiv_rn(c, m);
@@ -752,7 +845,7 @@ __device__ __forceinline__ DfTerms df_terms_of(double cx, double cy, double cz, 
 // Fixed-point record of a node with centre (cx, cy, cz) and mass m.
 __device__ __forceinline__ void write_fix(const ComArgs& A, uint32_t idx, double cx, double cy,
                                           double cz, double m) {
-    const nbfix::FixRec r = nbfix::make_rec(cx, cy, cz, m, (int)A.box[10]);
+    const nbfix::FixRec r = nbfix::make_rec(cx, cy, cz, m, __double2hiint(A.box[11]));
     A.fix_hi[idx] = nbfix::FixHi{r.x2, r.y2, r.z2, r.mh, r.x1, r.y1, r.z1, r.e};
     A.fix_lo[idx] = make_uint4(r.x0, r.y0, r.z0, r.ml);
 }
@@ -760,13 +853,14 @@ __device__ __forceinline__ void write_fix(const ComArgs& A, uint32_t idx, double
 __device__ void write_records(const ComArgs& A, uint32_t idx, double cx, double cy, double cz,
                               double sm, double qsum, uint32_t count, int level, uint32_t skip,
                               uint32_t body) {
+    const bool massive = (__double_as_longlong(sm) << 1) != 0;  // sm != 0
     const double edge = cell_edge64(A.box[6], level);
     const double ox = A.box[7], oy = A.box[8], oz = A.box[9];  // box centre
     // centre = sums / mass: the IEEE quotients when the FP64 records are built (the reference's
     // values, also behind the FP32 pre-test's proven margin), else from one reciprocal (the FP32
     // records round it); massless cells get a finite centre (never used)
     double rcx = 0.0, rcy = 0.0, rcz = 0.0, inv = 0.0;
-    if (sm != 0) {
+    if (massive) {
         if (A.records & NB_REC_FP64) exact_quotients(cx, cy, cz, sm, rcx, rcy, rcz);
         // 1/M from the hardware estimate and one Newton step (~2^-44: ample for the FP32
         // centres and the spread)
@@ -794,7 +888,7 @@ __device__ void write_records(const ComArgs& A, uint32_t idx, double cx, double 
     }
     NodeRec32 q;
     const double gx = rcx - ox, gy = rcy - oy, gz = rcz - oz;
-    if (sm != 0) {
+    if (massive) {
         q.cx = (float)gx;
         q.cy = (float)gy;
         q.cz = (float)gz;
@@ -802,13 +896,13 @@ __device__ void write_records(const ComArgs& A, uint32_t idx, double cx, double 
         q.cx = q.cy = q.cz = 1e30f;
     }
     q.gm = (float)(A.G * sm);
-    q.edge2 = cell_edge2(A.box[6], edge, (float)A.box[11], level);
+    q.edge2 = cell_edge2(A.box[6], edge, __int_as_float(__double2loint(A.box[11])), level);
     q.skip = skip;
     q.body = body;
     q.level = (uint32_t)level;
     A.rec32[idx] = q;
     if (A.records & NB_REC_DF) {
-        A.df_terms[idx] = df_terms_of(rcx, rcy, rcz, ox, oy, oz, A.G * sm, q.gm, sm != 0);
+        A.df_terms[idx] = df_terms_of(rcx, rcy, rcz, ox, oy, oz, A.G * sm, q.gm, massive);
     }
     if (A.records & NB_REC_LEARNED) {
         // spread^2 = sum m |x-o|^2 / M - |c-o|^2 (o = box centre, which keeps both terms small);
@@ -817,7 +911,7 @@ __device__ void write_records(const ComArgs& A, uint32_t idx, double cx, double 
         NodeAux x;
         x.spread_rel = 0.f;
         x.lg_gm = __log2f(fmaxf(q.gm, 1e-37f));
-        if (sm != 0) {
+        if (massive) {
             const double s2 = qsum * inv - (gx * gx + gy * gy + gz * gz);
             const float e = (float)edge;
             if (e > 0.f) x.spread_rel = sqrtf((float)(s2 > 0 ? s2 : 0.0)) / e;
@@ -905,6 +999,7 @@ struct NodeSums {
 
 __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32_t b) {
     const double mb = A.m[b];
+    const bool massive = (__double_as_longlong(mb) << 1) != 0;  // mb != 0
     const double bx = A.x[b], by = A.y[b], bz = A.z[b];
     const double cx = __dmul_rn(bx, mb), cy = __dmul_rn(by, mb), cz = __dmul_rn(bz, mb);
     A.comx[idx] = cx;
@@ -918,16 +1013,16 @@ __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32
     const double ox = A.box[7], oy = A.box[8], oz = A.box[9];
     const bool fp64 = (A.records & NB_REC_FP64) != 0;
     double rcx = bx, rcy = by, rcz = bz;
-    if (fp64 && mb != 0) {
+    if (fp64 && massive) {
         rcx = leaf_quotient(bx, mb, cx);
         rcy = leaf_quotient(by, mb, cy);
         rcz = leaf_quotient(bz, mb, cz);
     }
     if (fp64) {
         NodeRec64 r;
-        r.cx = mb != 0 ? rcx : 0.0;
-        r.cy = mb != 0 ? rcy : 0.0;
-        r.cz = mb != 0 ? rcz : 0.0;
+        r.cx = massive ? rcx : 0.0;
+        r.cy = massive ? rcy : 0.0;
+        r.cz = massive ? rcz : 0.0;
         r.mass = mb;
         r.edge = edge;
         r.skip = skip;
@@ -937,17 +1032,17 @@ __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32
     }
     const double gx = rcx - ox, gy = rcy - oy, gz = rcz - oz;
     NodeRec32 q;
-    q.cx = mb != 0 ? (float)gx : 1e30f;  // a massless body: far away, contributes exactly 0
-    q.cy = mb != 0 ? (float)gy : 1e30f;
-    q.cz = mb != 0 ? (float)gz : 1e30f;
+    q.cx = massive ? (float)gx : 1e30f;  // a massless body: far away, contributes exactly 0
+    q.cy = massive ? (float)gy : 1e30f;
+    q.cz = massive ? (float)gz : 1e30f;
     q.gm = (float)(A.G * mb);
-    q.edge2 = cell_edge2(A.box[6], edge, (float)A.box[11], level);
+    q.edge2 = cell_edge2(A.box[6], edge, __int_as_float(__double2loint(A.box[11])), level);
     q.skip = skip;
     q.body = b;
     q.level = (uint32_t)level;
     A.rec32[idx] = q;
     if (A.records & NB_REC_DF) {
-        A.df_terms[idx] = df_terms_of(rcx, rcy, rcz, ox, oy, oz, A.G * mb, q.gm, mb != 0);
+        A.df_terms[idx] = df_terms_of(rcx, rcy, rcz, ox, oy, oz, A.G * mb, q.gm, massive);
     }
     NodeSums sums{cx, cy, cz, mb, 0.0, 1};
     if (A.records & NB_REC_LEARNED) {  // spread sums and the FP32 body copies of the policy
@@ -1050,10 +1145,10 @@ __device__ __forceinline__ double plus_zero(double v) {
 }
 
 // Shared memory of com_chunk_kernel: the sums of the chunk's nodes (the spread sums only when the
-// learned records are built) and their body counts.
+// learned records are built).
 template <int CW>
 constexpr size_t chunk_smem_bytes(bool learned) {
-    return (size_t)(2 * CW + CM_LEVELS) * ((learned ? 5 : 4) * sizeof(double) + sizeof(uint32_t));
+    return (size_t)(2 * CW + CM_LEVELS) * ((learned ? 5 : 4) * sizeof(double));
 }
 
 template <int CW, int CH_THREADS>
@@ -1068,7 +1163,6 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
     double* sz = sy + CH_NODES;
     double* sm = sz + CH_NODES;
     double* sq = sm + CH_NODES;  // learned only
-    uint32_t* sc = reinterpret_cast<uint32_t*>(sm + (learned ? 2 : 1) * CH_NODES);
     __shared__ uint16_t found[CW], order[CW];  // local cells as slots: as found, by level
     __shared__ __align__(16) uint16_t kids[CW][8];  // a cell's children as slots, octant order
     __shared__ uint8_t flev[CW];
@@ -1096,7 +1190,6 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
         sz[k] = s.z;
         sm[k] = s.m;
         if (learned) sq[k] = s.q;
-        sc[k] = 1;
     }
     for (uint32_t idx = d0 + tid; idx < d1; idx += CH_THREADS) {
         if (A.node_body[idx] != NB_NONE) continue;  // a leaf
@@ -1176,7 +1269,7 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
             // the reference's sums start at 0.0: 0.0 + c is c, with -0.0 as +0.0
             const uint32_t k0 = kids[tid][0];
             NodeSums s{plus_zero(sx[k0]), plus_zero(sy[k0]), plus_zero(sz[k0]), plus_zero(sm[k0]),
-                       learned ? 0.0 + sq[k0] : 0.0, sc[k0]};
+                       learned ? 0.0 + sq[k0] : 0.0, 0};
             for (uint32_t i = 1; i < nkids; ++i) {
                 const uint32_t k = kids[tid][i];
                 s.x = __dadd_rn(s.x, sx[k]);
@@ -1184,14 +1277,12 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
                 s.z = __dadd_rn(s.z, sz[k]);
                 s.m = __dadd_rn(s.m, sm[k]);
                 if (learned) s.q += sq[k];
-                s.count += sc[k];
             }
             sx[my] = s.x;
             sy[my] = s.y;
             sz[my] = s.z;
             sm[my] = s.m;
             if (learned) sq[my] = s.q;
-            sc[my] = s.count;
         }
         __syncthreads();
     }
@@ -1202,8 +1293,9 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
         A.comz[idx] = sz[my];
         A.mass[idx] = sm[my];
         if (learned) A.q[idx] = sq[my];
-        A.node_count[idx] = sc[my];
-        write_records(A, idx, sx[my], sy[my], sz[my], sm[my], learned ? sq[my] : 0.0, sc[my],
+        const uint32_t count = A.node_last[idx] - A.node_first[idx] + 1;
+        A.node_count[idx] = count;
+        write_records(A, idx, sx[my], sy[my], sz[my], sm[my], learned ? sq[my] : 0.0, count,
                       A.node_level[idx], A.node_skip[idx], NB_NONE);
     }
 }
@@ -1259,6 +1351,7 @@ nb_status allow_smem(K kernel, size_t bytes) {
     return NB_OK;
 }
 nb_status build_prepare() {
+    NB_TRY(allow_smem(build_small_kernel<1024, 1024>, small_smem_bytes<1024>()));
     NB_TRY(allow_smem(build_small_kernel<2048, 1024>, small_smem_bytes<2048>()));
     NB_TRY(allow_smem(build_small_kernel<SB_MAX_N, 1024>, small_smem_bytes<SB_MAX_N>()));
     return allow_smem(com_chunk_kernel<1024, 1024>, chunk_smem_bytes<1024>(true));
@@ -1307,7 +1400,6 @@ void carve(nb_bh_tree* t, Carver& c) {
     t->node_first = c.take<uint32_t>(cap);
     t->node_last = c.take<uint32_t>(cap);
     t->node_skip = c.take<uint32_t>(cap);
-    t->node_parent = c.take<uint32_t>(cap);
     t->node_body = c.take<uint32_t>(cap);
     t->node_count = c.take<uint32_t>(cap);
     t->node_comx = c.take<double>(cap);
@@ -1446,8 +1538,8 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     };
     NB_TRY(mark(0));
     const bool quantized = (t->records & NB_BUILD_QUANTIZED_KEYS) != 0;
-    const NodeTable T{t->node_level,  t->node_first, t->node_last, t->node_skip,
-                      t->node_parent, t->node_body,  t->info,      t->children};
+    const NodeTable T{t->node_level, t->node_first, t->node_last, t->node_skip,
+                      t->node_body,  t->info,       t->children};
     if (n <= SB_MAX_N) {  // one block; its whole time counts as the cells phase
         for (int phase = 1; phase <= 3; ++phase) NB_TRY(mark(phase));
         auto go = [&](auto kernel, uint32_t threads, size_t smem) {
@@ -1455,7 +1547,8 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
                                             (unsigned long long*)t->mask, t->base, T,
                                             ctx->dev_error, quantized ? 1 : 0);
         };
-        if (n <= 512) go(build_small_kernel<512, 256>, 256, small_smem_bytes<512>());
+        if (n <= 512) go(build_small_kernel<512, 512>, 512, small_smem_bytes<512>());
+        else if (n <= 1024) go(build_small_kernel<1024, 1024>, 1024, small_smem_bytes<1024>());
         else if (n <= 2048) go(build_small_kernel<2048, 1024>, 1024, small_smem_bytes<2048>());
         else go(build_small_kernel<SB_MAX_N, 1024>, 1024, small_smem_bytes<SB_MAX_N>());
         NB_TRY(nb::check_launch("build_small_kernel"));
@@ -1517,7 +1610,6 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     A.node_skip = t->node_skip;
     A.err = ctx->dev_error;
 
-    A.node_parent = t->node_parent;
     A.node_body = t->node_body;
     A.node_count = t->node_count;
     A.comx = t->node_comx;

@@ -55,7 +55,8 @@ struct nb_bh_tree {
     int device = 0;
 
     double* box = nullptr;  // [0..6] AABB (min xyz, max xyz, edge), [7..9] box centre, [10] the
-                            // scale exponent K of the fixed-point records (nb_fix.cuh), [11] edge^2
+                            // scale exponent K of the fixed-point records (nb_fix.cuh), [11] K and
+                            // (float) edge^2 as bits
     uint32_t* info = nullptr;  // [0] node count (copy of base[n])
     uint2* tier_cells[2] = {};      // centre-of-mass tiers: cells passed up, (node, level)
     uint32_t* tier_count[2] = {};   // their count per chunk
@@ -88,7 +89,7 @@ struct nb_bh_tree {
 
     uint8_t* node_level = nullptr;
     uint32_t *node_first = nullptr, *node_last = nullptr, *node_skip = nullptr;
-    uint32_t *node_parent = nullptr, *node_body = nullptr;
+    uint32_t* node_body = nullptr;
     uint32_t* node_count = nullptr;
     double *node_comx = nullptr, *node_comy = nullptr, *node_comz = nullptr, *node_mass = nullptr;
     NodeRec64* rec64 = nullptr;
