@@ -15,9 +15,13 @@
 //     leftmost split of each cell ("first split") stands for the cell.
 //  6. DFS numbering: each sorted position p starts popc(mask[p]) internal cells plus its leaf;
 //     an exclusive scan gives every node its DFS pre-order index and skip link.
-//  7. bottom-up centre of mass: leaves and cells by blocks over chunks of 1,024 sorted positions
+// What later launches want zeroed or filled is written by earlier ones (keys: the sort's counters,
+// second key words and level masks; splits: the child lists), the digit offsets are summed by the
+// sort's passes and the node counts by the scan: 18 launches, where separate ones took 26 and 22 us
+// more at 16,411 bodies.
+//  7. bottom-up centre of mass: leaves and cells by blocks over chunks of 256 sorted positions
 //     (deepest level first), the cells reaching past their chunk (at most one per level) by tiers
-//     of blocks over 64 chunks each; children summed in octant order 0..7
+//     of blocks over 96 chunks each; children summed in octant order 0..7
 //     (bit-identical to BarnesHutOctree.cpp:304-311), node records written with the sums.
 #include <algorithm>
 
@@ -151,12 +155,30 @@ __device__ __forceinline__ void box_extras(double* __restrict__ box, uint32_t i)
     }
 }
 
+// Zeroes what the launches after the keys count on: the sort's counters, the second key words and
+// the level masks, by all threads of the grid.
+struct BuildZero {
+    uint4* sort;
+    uint32_t sort_n;  // in 16-byte words
+    uint64_t* key1;
+    unsigned long long* mask;
+};
+__device__ __forceinline__ void build_zero(const BuildZero& Z, uint32_t i, uint32_t n) {
+    for (uint32_t k = i; k < Z.sort_n; k += gridDim.x * blockDim.x)
+        Z.sort[k] = make_uint4(0, 0, 0, 0);
+    if (i < n) {
+        Z.key1[i] = 0;
+        Z.mask[i] = 0;
+    }
+}
+
 __global__ void keys_quantized_kernel(const double* __restrict__ x, const double* __restrict__ y,
                                       const double* __restrict__ z, uint32_t n,
                                       double* __restrict__ box, uint64_t* __restrict__ key0,
-                                      uint32_t* __restrict__ ids) {
+                                      uint32_t* __restrict__ ids, BuildZero Z) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     box_extras(box, i);
+    build_zero(Z, i, n);
     if (i >= n) return;
     key0[i] = key_word_quantized(box, x[i], y[i], z[i], 0);
     ids[i] = i;
@@ -224,10 +246,11 @@ __device__ __forceinline__ uint64_t exact_key(const double* __restrict__ box, co
 __global__ void __launch_bounds__(BH_THREADS)
 keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
             const double* __restrict__ z, uint32_t n, double* __restrict__ box,
-            uint64_t* __restrict__ key0, uint32_t* __restrict__ ids) {
+            uint64_t* __restrict__ key0, uint32_t* __restrict__ ids, BuildZero Z) {
     __shared__ FixedGrid grid_s;  // once per block: it takes an FP64 division
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     box_extras(box, i);
+    build_zero(Z, i, n);
     if (threadIdx.x == 0) grid_s = fixed_grid(box);
     __syncthreads();
     if (i >= n) return;
@@ -349,15 +372,16 @@ __device__ __forceinline__ void split_at(uint32_t j, const uint64_t* __restrict_
 __global__ void splits_kernel(const uint64_t* __restrict__ key0, const uint64_t* __restrict__ key1,
                               uint32_t n, uint8_t* __restrict__ split_level,
                               uint32_t* __restrict__ split_start, uint32_t* __restrict__ split_end,
-                              unsigned long long* __restrict__ mask, uint32_t* __restrict__ err) {
+                              unsigned long long* __restrict__ mask, uint32_t* __restrict__ children,
+                              uint32_t* __restrict__ err) {
+    // the child lists start empty (two nodes per position at most): stores that the searches' round
+    // trips leave room for
+    const uint32_t blk = min(blockDim.x, n - blockIdx.x * blockDim.x);
+    uint4* cl = reinterpret_cast<uint4*>(children) + (size_t)blockIdx.x * blockDim.x * 4;
+    for (uint32_t k = threadIdx.x; k < blk * 4; k += blockDim.x)
+        cl[k] = make_uint4(NB_NONE, NB_NONE, NB_NONE, NB_NONE);
     split_at(blockIdx.x * blockDim.x + threadIdx.x, key0, key1, n, split_level, split_start,
              split_end, mask, err);
-}
-
-__global__ void count_kernel(const unsigned long long* __restrict__ mask, uint32_t n,
-                             uint32_t* __restrict__ cnt) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) cnt[p] = __popcll(mask[p]) + 1;
 }
 
 __device__ __forceinline__ uint32_t node_index(const uint32_t* __restrict__ base,
@@ -1392,7 +1416,6 @@ void carve(nb_bh_tree* t, Carver& c) {
     t->split_start = c.take<uint32_t>(n);
     t->split_end = c.take<uint32_t>(n);
     t->mask = c.take<uint64_t>(n);
-    t->cnt = c.take<uint32_t>(n + 1);
     t->base = c.take<uint32_t>(n + 1);
     t->sort_temp = c.take<char>(nb::radix_temp_bytes((uint32_t)n));
     t->scan_temp = c.take<uint32_t>(nb::scan_temp_bytes((uint32_t)n + 1) / 4 + 16);
@@ -1555,35 +1578,32 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     } else {
         NB_TRY(nb::launch_aabb(ctx, x, y, z, n, t->box, s));
         NB_TRY(mark(1));
+        const BuildZero Z{(uint4*)t->sort_temp, (uint32_t)(nb::radix_zero_bytes(n) / 16), t->key1,
+                          (unsigned long long*)t->mask};
         if (quantized) {
-            keys_quantized_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids);
+            keys_quantized_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids, Z);
         } else {
-            keys_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids);
+            keys_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids, Z);
         }
         NB_TRY(nb::check_launch("keys_kernel"));
         NB_TRY(mark(2));
         int in_alt = 0;
         NB_TRY(nb::radix_sort_pairs(t->key0, t->ids, t->key_alt, t->ids_alt, n, 0, 3 * NB_KEY_LEVELS,
-                                    t->sort_temp, ctx->dev_error, s, &in_alt));
+                                    t->sort_temp, ctx->dev_error, s, &in_alt, NB_WAIT_LIMIT_DEFAULT, 0,
+                                    true));
         if (in_alt) {  // an odd number of passes leaves the result in the alternate buffers
             NB_CUDA_TRY(cudaMemcpyAsync(t->key0, t->key_alt, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
             NB_CUDA_TRY(cudaMemcpyAsync(t->ids, t->ids_alt, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
         }
         NB_TRY(mark(3));
-        NB_CUDA_TRY(cudaMemsetAsync(t->key1, 0, (size_t)n * 8, s));
         runs_fixup_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->key1, t->ids,
                                                       ctx->dev_error, quantized ? 1 : 0);
         NB_TRY(nb::check_launch("runs_fixup_kernel"));
-        NB_CUDA_TRY(cudaMemsetAsync(t->mask, 0, (size_t)n * 8, s));
         splits_kernel<<<grid, BH_THREADS, 0, s>>>(t->key0, t->key1, n, t->split_level, t->split_start,
                                                   t->split_end, (unsigned long long*)t->mask,
-                                                  ctx->dev_error);
+                                                  t->children, ctx->dev_error);
         NB_TRY(nb::check_launch("splits_kernel"));
-        count_kernel<<<grid, BH_THREADS, 0, s>>>((const unsigned long long*)t->mask, n, t->cnt);
-        NB_TRY(nb::check_launch("count_kernel"));
-        NB_TRY(nb::exclusive_scan_u32(t->cnt, t->base, n, 1, t->scan_temp, s));
-        const size_t nodes_max = 2 * (size_t)n;
-        NB_CUDA_TRY(cudaMemsetAsync(t->children, 0xff, nodes_max * 8 * 4, s));  // NB_NONE
+        NB_TRY(nb::node_offsets((const unsigned long long*)t->mask, t->base, n, t->scan_temp, s));
         emit_kernel<<<grid, BH_THREADS, 0, s>>>(n, t->ids, t->split_level, t->split_start, t->split_end,
                                                 (const unsigned long long*)t->mask, t->base, t->key0,
                                                 t->key1, T);

@@ -83,7 +83,7 @@ struct nb_bh_tree {
     uint8_t* split_level = nullptr;
     uint32_t *split_start = nullptr, *split_end = nullptr;
     uint64_t* mask = nullptr;
-    uint32_t *cnt = nullptr, *base = nullptr;
+    uint32_t* base = nullptr;
     void* sort_temp = nullptr;
     uint32_t* scan_temp = nullptr;
 

@@ -375,7 +375,7 @@ nb_status launch_scale(const double* x, const double* y, const double* z, uint32
 // Enqueues the AABB of (x, y, z) into out_dev[7]. Used by nb_aabb and the tree build.
 nb_status launch_aabb(nb_ctx* ctx, const double* x, const double* y, const double* z,
                       uint32_t n, double* out_dev, cudaStream_t stream) {
-    int blocks = nb::ceil_div(n, AABB_THREADS * 8);
+    int blocks = nb::ceil_div(n, AABB_THREADS * 4);
     if (blocks > ctx->sm_count * 4) blocks = ctx->sm_count * 4;
     if (blocks < 1) blocks = 1;
     void* part = nullptr;

@@ -9,6 +9,9 @@ namespace {
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+// Up to this many tiles (2M items) a tile adds the totals before it itself, two loads per thread at
+// most, instead of waiting for one more launch.
+constexpr uint32_t SCAN_SELF_TILES = 2 * SCAN_THREADS;
 
 // Block-wide exclusive scan of one value per thread; returns the block total in *total.
 __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total) {
@@ -41,14 +44,28 @@ __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total) {
     return res;
 }
 
+// The scanned values: in[i] itself, or the number of nodes that start at position i, one more than
+// the bits of its level mask.
+struct PlainItems {
+    const uint32_t* in;
+    __device__ __forceinline__ uint32_t operator()(uint32_t i) const { return in[i]; }
+};
+struct MaskItems {
+    const unsigned long long* mask;
+    __device__ __forceinline__ uint32_t operator()(uint32_t i) const {
+        return (uint32_t)__popcll(mask[i]) + 1u;
+    }
+};
+
+template <class Items>
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_reduce_kernel(const uint32_t* __restrict__ in, uint32_t n, uint32_t* __restrict__ sums) {
+scan_reduce_kernel(Items in, uint32_t n, uint32_t* __restrict__ sums) {
     const uint32_t base = blockIdx.x * SCAN_TILE;
     uint32_t s = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
         const uint32_t i = base + k * SCAN_THREADS + threadIdx.x;
-        if (i < n) s += in[i];
+        if (i < n) s += in(i);
     }
     uint32_t total;
     block_exclusive_scan(s, &total);
@@ -70,32 +87,43 @@ scan_sums_kernel(uint32_t* __restrict__ sums, uint32_t nb) {
     if (threadIdx.x == 0) sums[nb] = carry;
 }
 
+// `summed`: sums[] holds the tiles' own totals and each block adds those before its own (up to
+// SCAN_SELF_TILES of them); else scan_sums_kernel has made them the prefixes.
+template <class Items>
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_apply_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t n,
-                  const uint32_t* __restrict__ sums, int write_total) {
+scan_apply_kernel(Items in, uint32_t* __restrict__ out, uint32_t n,
+                  const uint32_t* __restrict__ sums, int write_total, int summed) {
     const uint32_t base = blockIdx.x * SCAN_TILE;
+    uint32_t before = 0;
+    if (summed) {
+        uint32_t mine = 0;
+        for (uint32_t t = threadIdx.x; t < blockIdx.x; t += SCAN_THREADS) mine += sums[t];
+        block_exclusive_scan(mine, &before);
+    } else {
+        before = sums[blockIdx.x];
+    }
     // blocked arrangement: thread t owns items base + t*ITEMS .. +ITEMS-1
     uint32_t v[SCAN_ITEMS];
     uint32_t s = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
         const uint32_t i = base + threadIdx.x * SCAN_ITEMS + k;
-        v[k] = i < n ? in[i] : 0;
+        v[k] = i < n ? in(i) : 0;
         s += v[k];
     }
     uint32_t total;
-    uint32_t run = block_exclusive_scan(s, &total) + sums[blockIdx.x];
+    uint32_t run = block_exclusive_scan(s, &total) + before;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
         const uint32_t i = base + threadIdx.x * SCAN_ITEMS + k;
         if (i < n) out[i] = run;
         run += v[k];
     }
-    if (write_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = sums[gridDim.x];
+    if (write_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = before + total;
 }
 
 // ---------------------------------------------------------------------------------------------
-// Radix sort: 8-bit digits, tiles of 2048 keys (256 threads x 8 items), one launch per digit
+// Radix sort: 8-bit digits, tiles of 256 threads x RS_ITEMS keys, one launch per digit
 // pass. The digit histograms of all passes come from one read of the keys up front; within a
 // pass each tile finds the keys of its digit in earlier tiles by decoupled look-back (Merrill and
 // Garland, "Single-pass parallel prefix scan with decoupled look-back", NVIDIA TR 2016; the
@@ -107,16 +135,15 @@ scan_apply_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, u
 // depend on the counts only.
 // ---------------------------------------------------------------------------------------------
 constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_BINS = 256;
 constexpr int RS_MAX_PASSES = 8;
+constexpr int LB_WINDOW = 8;  // predecessor words read per look-back round trip (16, 32: slower)
+constexpr uint32_t RS_HIST_KEYS = 1024;  // keys per block of the histogram, up to 1,024 blocks
 // look-back words: 2 flag bits over a 30-bit count (tile counts <= 4096, totals <= n < 2^30)
 constexpr uint32_t LB_AGGREGATE = 1u << 30;
 constexpr uint32_t LB_TOTAL = 2u << 30;
 constexpr uint32_t LB_VALUE = (1u << 30) - 1u;
-constexpr int LB_WINDOW = 8;  // predecessor words read per look-back round trip
 static_assert(RS_THREADS == RS_BINS, "the look-back and the digit scan run one thread per digit");
 
 // hist[p][d]: keys whose digit of pass p is d, for all passes in one read.
@@ -137,13 +164,6 @@ radix_hist_all_kernel(const uint64_t* __restrict__ keys, uint32_t n, int begin_b
     }
 }
 
-// hist[p][d] -> exclusive prefix over d (block p, thread d).
-__global__ void __launch_bounds__(RS_BINS) radix_offsets_kernel(uint32_t* __restrict__ hist) {
-    uint32_t total;
-    uint32_t* h = hist + blockIdx.x * RS_BINS;
-    h[threadIdx.x] = block_exclusive_scan(h[threadIdx.x], &total);
-}
-
 __device__ __forceinline__ void lb_store(uint32_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -154,16 +174,19 @@ __device__ __forceinline__ uint32_t lb_load(const uint32_t* p) {
 }
 
 // The tile's keys and values reordered by digit (dynamic shared memory: above the static limit).
-constexpr int RS_REORDER_BYTES = RS_TILE * (int)(sizeof(uint64_t) + sizeof(uint32_t));
+template <int RS_ITEMS>
+constexpr int RS_REORDER_BYTES = RS_THREADS * RS_ITEMS * (int)(sizeof(uint64_t) + sizeof(uint32_t));
 
 // One digit pass: keys of tile `ticket` in, ranked within the tile (warp-striped, stable),
 // placed at digit offset + keys of the digit in earlier tiles + rank.
+template <int RS_ITEMS>
 __global__ void __launch_bounds__(RS_THREADS)
 radix_pass_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                   uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
-                  int shift, const uint32_t* __restrict__ digit_off, uint32_t* __restrict__ lb,
+                  int shift, const uint32_t* __restrict__ hist, uint32_t* __restrict__ lb,
                   uint32_t* __restrict__ ticket, uint32_t* __restrict__ err,
                   unsigned long long wait_limit, int drop_first) {
+    constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
     __shared__ uint32_t wcnt[RS_WARPS][RS_BINS];
     __shared__ uint32_t tile_base[RS_BINS];   // first output position of the tile's digit d
     __shared__ uint32_t digit_local[RS_BINS];  // first tile position of digit d after the reorder
@@ -174,19 +197,25 @@ radix_pass_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restri
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) tile_s = atomicAdd(ticket, 1u);
     for (int b = threadIdx.x; b < RS_WARPS * RS_BINS; b += RS_THREADS) (&wcnt[0][0])[b] = 0;
+    const uint32_t hist_d = hist[threadIdx.x];
     __syncthreads();
     const uint32_t tile = tile_s;
-    // warp-striped: warp w owns tile positions [w*512, w*512+512); item k, lane l -> w*512+k*32+l
+    // warp-striped: warp w owns RS_ITEMS * 32 positions of the tile, item k of lane l the
+    // (k * 32 + l)-th of them
     const uint32_t base = tile * RS_TILE + warp * (RS_ITEMS * 32);
     uint64_t key[RS_ITEMS];
     uint32_t val[RS_ITEMS], digit[RS_ITEMS], rank[RS_ITEMS];
     const uint32_t lt_mask = (1u << lane) - 1u;
 #pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k) {
+    for (int k = 0; k < RS_ITEMS; ++k) {  // every load before the first is ranked
         const uint32_t i = base + k * 32 + lane;
         const bool valid = i < n;
         key[k] = valid ? keys_in[i] : 0;
         val[k] = valid ? vals_in[i] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < RS_ITEMS; ++k) {
+        const bool valid = base + k * 32 + lane < n;
         digit[k] = valid ? ((uint32_t)(key[k] >> shift) & 0xffu) : RS_BINS;
         const uint32_t peers = __match_any_sync(0xffffffffu, digit[k]);
         const int leader = __ffs(peers) - 1;
@@ -246,8 +275,9 @@ radix_pass_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restri
             if (timed_out) atomicOr(err, NB_DEVERR_TIMEOUT);
             lb_store(mine, LB_TOTAL | (before + run));
         }
-        tile_base[d] = digit_off[d] + before;
+        // digit d's first output position: the keys of smaller digits in the whole input
         uint32_t tile_total;
+        tile_base[d] = block_exclusive_scan(hist_d, &tile_total) + before;
         digit_local[d] = block_exclusive_scan(run, &tile_total);  // one digit per thread
     }
     __syncthreads();
@@ -281,8 +311,10 @@ size_t scan_temp_bytes(uint32_t n) {
     return ((size_t)nb + 1) * sizeof(uint32_t);
 }
 
-nb_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, int write_total,
-                             uint32_t* temp, cudaStream_t stream) {
+namespace {
+template <class Items>
+nb_status scan_items(Items in, uint32_t* out, uint32_t n, int write_total, uint32_t* temp,
+                     cudaStream_t stream) {
     if (n == 0) {
         if (write_total) NB_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(uint32_t), stream));
         return NB_OK;
@@ -290,12 +322,37 @@ nb_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, int 
     const uint32_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (nb > 64u * SCAN_THREADS)
         return set_error(NB_ERR_INVALID_ARG, "exclusive_scan_u32: n = %u too large", n);
+    const bool summed = nb <= SCAN_SELF_TILES;
     scan_reduce_kernel<<<nb, SCAN_THREADS, 0, stream>>>(in, n, temp);
     NB_TRY(check_launch("scan_reduce_kernel"));
-    scan_sums_kernel<<<1, SCAN_THREADS, 0, stream>>>(temp, nb);
-    NB_TRY(check_launch("scan_sums_kernel"));
-    scan_apply_kernel<<<nb, SCAN_THREADS, 0, stream>>>(in, out, n, temp, write_total);
+    if (!summed) {
+        scan_sums_kernel<<<1, SCAN_THREADS, 0, stream>>>(temp, nb);
+        NB_TRY(check_launch("scan_sums_kernel"));
+    }
+    scan_apply_kernel<<<nb, SCAN_THREADS, 0, stream>>>(in, out, n, temp, write_total,
+                                                       summed ? 1 : 0);
     return check_launch("scan_apply_kernel");
+}
+}  // namespace
+
+nb_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, int write_total,
+                             uint32_t* temp, cudaStream_t stream) {
+    return scan_items(PlainItems{in}, out, n, write_total, temp, stream);
+}
+
+nb_status node_offsets(const unsigned long long* mask, uint32_t* out, uint32_t n, uint32_t* temp,
+                       cudaStream_t stream) {
+    return scan_items(MaskItems{mask}, out, n, 1, temp, stream);
+}
+
+// Keys per thread of a pass: as few as give the small sorts enough blocks, as many as the large ones
+// need for short look-backs. All eight passes with their histogram at 4 / 8 / 16 keys per thread:
+// 16,411 keys 68 / 70 / 101 us, 65,536 72 / 80 / 105, 131,101 85 / 85 / 113, 262,144 103 / 89 / 119,
+// 524,288 146 / 119 / 126, 1,048,576 222 / 185 / 171.
+constexpr uint32_t RS_N4 = 1u << 17, RS_N8 = 1u << 19;
+static uint32_t radix_tiles(uint32_t n) {
+    const uint32_t tile = RS_THREADS * (n <= RS_N4 ? 4 : (n <= RS_N8 ? 8 : 16));
+    return (uint32_t)(((uint64_t)n + tile - 1) / tile);
 }
 
 nb_status radix_prepare() {
@@ -303,25 +360,28 @@ nb_status radix_prepare() {
     int dev = 0;
     NB_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || done[dev]) return NB_OK;
-    NB_CUDA_TRY(cudaFuncSetAttribute(radix_pass_kernel,
+    NB_CUDA_TRY(cudaFuncSetAttribute(radix_pass_kernel<16>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     RS_REORDER_BYTES));
+                                     RS_REORDER_BYTES<16>));
     done[dev] = true;
     return NB_OK;
 }
 
-// Temporary storage of radix_sort_pairs: digit offsets and tickets of all passes, then one
+// Temporary storage of radix_sort_pairs: the digit counts and tickets of all passes, then one
 // look-back word per (pass, tile, digit).
-size_t radix_temp_bytes(uint32_t n) {
-    const size_t tiles = (n + RS_TILE - 1) / RS_TILE;
-    return ((size_t)RS_MAX_PASSES * RS_BINS + 64 + (size_t)RS_MAX_PASSES * tiles * RS_BINS) *
-           sizeof(uint32_t);
+size_t radix_zero_bytes(uint32_t n) {
+    return ((size_t)RS_MAX_PASSES * RS_BINS + 64 +
+            (size_t)RS_MAX_PASSES * radix_tiles(n) * RS_BINS) * sizeof(uint32_t);
+}
+size_t radix_temp_bytes(uint32_t n) {  // enough for any count up to n
+    return std::max({radix_zero_bytes(n), radix_zero_bytes(std::min(n, RS_N4)),
+                     radix_zero_bytes(std::min(n, RS_N8))});
 }
 
 nb_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt,
                            uint32_t* vals_alt, uint32_t n, int begin_bit, int end_bit,
                            void* temp, uint32_t* err, cudaStream_t stream, int* result_in_alt,
-                           unsigned long long wait_limit, int drop_first) {
+                           unsigned long long wait_limit, int drop_first, bool zeroed) {
     *result_in_alt = 0;
     if (n <= 1) return NB_OK;
     if (n > LB_VALUE)  // look-back words count keys in 30 bits
@@ -331,25 +391,28 @@ nb_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt,
         return set_error(NB_ERR_INVALID_ARG, "radix_sort_pairs: bit range [%d, %d)", begin_bit,
                          end_bit);
     NB_TRY(radix_prepare());
-    const uint32_t tiles = (n + RS_TILE - 1) / RS_TILE;
-    uint32_t* offs = (uint32_t*)temp;                   // [passes][256]
-    uint32_t* tickets = offs + RS_MAX_PASSES * RS_BINS;  // [passes]
+    const uint32_t tiles = radix_tiles(n);
+    uint32_t* hist = (uint32_t*)temp;                   // [passes][256]
+    uint32_t* tickets = hist + RS_MAX_PASSES * RS_BINS;  // [passes]
     uint32_t* lb = tickets + 64;                         // [passes][tiles][256]
-    NB_CUDA_TRY(cudaMemsetAsync(temp, 0, radix_temp_bytes(n), stream));
-    const int hist_blocks = (int)std::min<uint32_t>(tiles, 1024u);
-    radix_hist_all_kernel<<<hist_blocks, RS_THREADS, 0, stream>>>(keys, n, begin_bit, passes, offs);
+    if (!zeroed) NB_CUDA_TRY(cudaMemsetAsync(temp, 0, radix_zero_bytes(n), stream));
+    const int hist_blocks = (int)std::min<uint32_t>((n + RS_HIST_KEYS - 1) / RS_HIST_KEYS, 1024u);
+    radix_hist_all_kernel<<<hist_blocks, RS_THREADS, 0, stream>>>(keys, n, begin_bit, passes, hist);
     NB_TRY(check_launch("radix_hist_all_kernel"));
-    radix_offsets_kernel<<<passes, RS_BINS, 0, stream>>>(offs);
-    NB_TRY(check_launch("radix_offsets_kernel"));
     uint64_t* kin = keys;
     uint32_t* vin = vals;
     uint64_t* kout = keys_alt;
     uint32_t* vout = vals_alt;
     int flips = 0;
     for (int p = 0; p < passes; ++p) {
-        radix_pass_kernel<<<tiles, RS_THREADS, RS_REORDER_BYTES, stream>>>(
-            kin, vin, kout, vout, n, begin_bit + 8 * p, offs + p * RS_BINS,
-            lb + (size_t)p * tiles * RS_BINS, tickets + p, err, wait_limit, drop_first);
+        auto go = [&](auto kernel, int smem) {
+            kernel<<<tiles, RS_THREADS, smem, stream>>>(
+                kin, vin, kout, vout, n, begin_bit + 8 * p, hist + p * RS_BINS,
+                lb + (size_t)p * tiles * RS_BINS, tickets + p, err, wait_limit, drop_first);
+        };
+        if (n <= RS_N4) go(radix_pass_kernel<4>, RS_REORDER_BYTES<4>);
+        else if (n <= RS_N8) go(radix_pass_kernel<8>, RS_REORDER_BYTES<8>);
+        else go(radix_pass_kernel<16>, RS_REORDER_BYTES<16>);
         NB_TRY(check_launch("radix_pass_kernel"));
         uint64_t* tk = kin;
         kin = kout;

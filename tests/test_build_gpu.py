@@ -95,3 +95,31 @@ def test_coincident_bodies_are_reported(ctx, n):
     with pytest.raises(NBodyError, match="DEPTH"):
         ctx.sync()
     tree.close()
+
+
+@pytest.mark.parametrize("n", [1023, 1025, 131072, 131073, 524288, 524289])
+def test_sort_at_tile_edges(ctx, n):
+    """The three tile sizes of the sort's passes: stable, with many equal keys."""
+    import torch
+    from nbody.lib import util_radix_sort_pairs
+    rng = np.random.default_rng(n)
+    k = (rng.integers(0, 997, n).astype(np.int64) << 40) | rng.integers(0, 3, n)
+    keys, vals = torch.from_numpy(k).cuda(), torch.arange(n, dtype=torch.int32, device="cuda")
+    util_radix_sort_pairs(ctx, keys, vals, 0, 63)
+    ctx.sync()
+    order = np.argsort(k, kind="stable")
+    np.testing.assert_array_equal(host(vals), order)
+    np.testing.assert_array_equal(host(keys), k[order])
+
+
+@pytest.mark.parametrize("n", [4096, 4097, 2048 * 4096, 2048 * 4096 + 1])
+def test_scan_at_tile_edges(ctx, n):
+    """Tiles that add the totals before them themselves (up to 2,048) and the launch that does it."""
+    import torch
+    from nbody.lib import util_exclusive_scan_u32
+    v = np.random.default_rng(n).integers(0, 5, n).astype(np.int32)
+    t = torch.from_numpy(v).cuda()
+    out = torch.empty(n + 1, dtype=torch.int32, device="cuda")
+    util_exclusive_scan_u32(ctx, t, out)
+    ctx.sync()
+    np.testing.assert_array_equal(host(out), np.concatenate([[0], np.cumsum(v)]))
