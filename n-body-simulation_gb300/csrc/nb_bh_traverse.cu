@@ -211,12 +211,19 @@ bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const nbfix::FixHi* __res
     }
 }
 
+// The part of the opening test's margin that no distance reduces: theta^2 * 4 (2^-24 E)^2.
+__device__ __forceinline__ float margin_floor(float th2, float edge) {
+    const float u = 2.0f * 5.9604645e-8f * edge;
+    return th2 * (u * u);
+}
+
 // Per-body reference rule, FP64, each lane walking its own DFS sequence (no union walk).
 // The opening test is decided in FP32 on the anchored FP32 records whenever the FP32 error
 // bound proves the answer; only undecided cells evaluate the reference's FP64 expression.
 // FP32 error bound of d^2 with positions rounded relative to the box centre (|c-a|, |p-a| <=
-// E/2 per axis, u = 2^-24): |d2f - d2| <= u d^2 (2*sqrt(3) E/d + 5); the test below widens it
-// by 4x and adds the roundings of edge^2 and theta^2*d2f. Accumulation order per body is the
+// E/2 per axis, u = 2^-24): |d2f - d2| <= u d^2 (2*sqrt(3) E/d + 5) + 3 u^2 E^2; the test below
+// widens it by 4x (the last term to 4 u^2 E^2: it decides only where d2f is far below u^2 E^2, when
+// one axis resolves less than the others) and adds the roundings of edge^2 and theta^2*d2f. Accumulation order per body is the
 // reference's DFS order, so MODE IEEE64 stays bit-identical. Warps take groups of 32 sorted
 // positions; with `order` != nullptr the bodies of the positions come from it (the previous
 // walk's lengths regrouped within windows, regroup_kernel) instead of from ids. Each body's
@@ -251,7 +258,7 @@ bh_theta_lane_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
         const float pxf = (float)(px - ox), pyf = (float)(py - oy), pzf = (float)(pz - oz);
         const float th2 = (float)(theta * theta);
         const float u4 = 4.0f * 5.9604645e-8f;  // 4 * 2^-24
-        const float Ef = (float)E;
+        const float Ef = (float)E, floor2 = margin_floor(th2, Ef);
         double acx = 0, acy = 0, acz = 0;
         uint32_t k = valid ? 0u : nn;
         // Find, then compute: every lane walks (FP32 tests, divergent but off the FP64 pipe) to its
@@ -272,7 +279,7 @@ bh_theta_lane_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
                     const float d2f = fmaf(dxf, dxf, fmaf(dyf, dyf, dzf * dzf));
                     const float t = th2 * d2f;
                     const float rel = u4 * (3.5f * Ef * nb_rsqrt_f32(d2f) + 8.0f);
-                    const float margin = t * rel + u4 * r.edge2;
+                    const float margin = fmaf(t, rel, fmaf(u4, r.edge2, floor2));
                     if (r.edge2 > t + margin) {
                         accept = false;  // certainly opened
                     } else if (r.edge2 < t - margin) {
@@ -314,33 +321,39 @@ bh_theta_lane_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
 // Decision of the reference's opening rule for node `idx` seen from a body: true = accepted (a
 // leaf, or certainly below theta), by the FP32 test where its margin allows (see
 // bh_theta_lane_kernel), else by the FP64 expression.
+// Opening parameter as a kernel argument: its FP32 square stays in the constant bank.
+struct Theta {
+    double value;
+    float sq;
+    explicit Theta(double theta) : value(theta), sq((float)(theta * theta)) {}
+};
 struct Pretest {
-    float px, py, pz, th2, edge;  // body relative to the box centre, theta^2, box edge
+    float px, py, pz, edge, floor2;  // body relative to the box centre, box edge, margin_floor
 };
 __device__ __forceinline__ bool accepts(const NodeRec32& r, const Pretest& b,
                                         const NodeRec64* __restrict__ rec64, uint32_t idx,
                                         const double* __restrict__ x,
                                         const double* __restrict__ y,
-                                        const double* __restrict__ z, uint32_t me, double theta) {
+                                        const double* __restrict__ z, uint32_t me, Theta theta) {
     using A = Arith<FAST64>;
     const float u4 = 4.0f * 5.9604645e-8f;  // 4 * 2^-24
     const float dx = r.cx - b.px, dy = r.cy - b.py, dz = r.cz - b.pz;
     const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    const float t = b.th2 * d2;
+    const float t = theta.sq * d2;
     const float rel = u4 * (3.5f * b.edge * nb_rsqrt_f32(d2) + 8.0f);
-    const float margin = t * rel + u4 * r.edge2;
+    const float margin = fmaf(t, rel, fmaf(u4, r.edge2, b.floor2));
     if (r.body != NB_NONE || r.edge2 < t - margin) return true;
     if (r.edge2 > t + margin) return false;
     const NodeRec64 q = rec64[idx];
     const double ex = A::sub(q.cx, x[me]), ey = A::sub(q.cy, y[me]), ez = A::sub(q.cz, z[me]);
-    return A::mul(q.edge, A::rsqrt(A::norm2(ex, ey, ez))) < theta;
+    return A::mul(q.edge, A::rsqrt(A::norm2(ex, ey, ez))) < theta.value;
 }
 
 __device__ __forceinline__ Pretest pretest_of(const double* __restrict__ box, double px, double py,
-                                              double pz, double theta) {
+                                              double pz, Theta theta) {
     const double E = box[6];
     return Pretest{(float)(px - (box[0] + E / 2)), (float)(py - (box[1] + E / 2)),
-                   (float)(pz - (box[2] + E / 2)), (float)(theta * theta), (float)E};
+                   (float)(pz - (box[2] + E / 2)), (float)E, margin_floor(theta.sq, (float)E)};
 }
 
 // Per-body reference rule, NB_F64: one lane per body. Each lane walks its body's DFS sequence and
@@ -362,7 +375,7 @@ bh_theta_fix_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __rest
                     const uint32_t* __restrict__ info, const uint32_t* __restrict__ ids,
                     const double* __restrict__ x, const double* __restrict__ y,
                     const double* __restrict__ z, const double* __restrict__ box, uint32_t n,
-                    double theta, double eps2, double G, double* __restrict__ ax,
+                    Theta theta, double eps2, double G, double* __restrict__ ax,
                     double* __restrict__ ay, double* __restrict__ az,
                     uint32_t* __restrict__ next_group, const uint32_t* __restrict__ order,
                     uint32_t* __restrict__ walk_len) {
@@ -442,7 +455,7 @@ bh_theta_team_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
                      const uint32_t* __restrict__ info, const uint32_t* __restrict__ ids,
                      const double* __restrict__ x, const double* __restrict__ y,
                      const double* __restrict__ z, const double* __restrict__ box, uint32_t n,
-                     double theta, double eps2, double G, double* __restrict__ ax,
+                     Theta theta, double eps2, double G, double* __restrict__ ax,
                      double* __restrict__ ay, double* __restrict__ az,
                      uint32_t* __restrict__ walk_len) {
     constexpr int B = 32 / T;                     // bodies per warp
@@ -628,7 +641,7 @@ bh_theta_df_kernel(const NodeRec32* __restrict__ rec32, const DfTerms* __restric
                    const NodeRec64* __restrict__ rec64, const uint32_t* __restrict__ info,
                    const uint32_t* __restrict__ ids, const double* __restrict__ x,
                    const double* __restrict__ y, const double* __restrict__ z,
-                   const double* __restrict__ box, uint32_t n, double theta, double eps2,
+                   const double* __restrict__ box, uint32_t n, Theta theta, double eps2,
                    double gscale, double* __restrict__ ax, double* __restrict__ ay,
                    double* __restrict__ az, uint32_t* __restrict__ next_group,
                    const uint32_t* __restrict__ order, uint32_t* __restrict__ walk_len) {
@@ -992,11 +1005,11 @@ nb_status launch_lane(nb_ctx* ctx, const nb_bh_tree* t, nb_precision prec, const
     else if (prec == NB_F64)
         bh_theta_fix_kernel<<<grid, TR_THREADS, 0, s>>>(
             t->rec32, t->rec64, t->fix_hi, t->fix_lo, t->info, t->ids, x, y, z, t->box, t->n,
-            t->params.theta, eps2, G, ax, ay, az, t->work + 1, order, t->walk_len);
+            Theta(t->params.theta), eps2, G, ax, ay, az, t->work + 1, order, t->walk_len);
     else
         bh_theta_df_kernel<<<grid, TR_THREADS, 0, s>>>(
             t->rec32, t->df_terms, t->rec64, t->info, t->ids, x, y, z, t->box, t->n,
-            t->params.theta, eps2, G / t->G, ax, ay, az, t->work + 1, order, t->walk_len);
+            Theta(t->params.theta), eps2, G / t->G, ax, ay, az, t->work + 1, order, t->walk_len);
     NB_TRY(nb::check_launch("Barnes-Hut lane kernel"));
     t->walk_n = t->n;
     return NB_OK;
@@ -1012,7 +1025,7 @@ nb_status launch_f64(nb_ctx* ctx, const nb_bh_tree* t, nb_precision prec, const 
     const int grid = nb::ceil_div((long long)t->n * team, TR_THREADS);
     auto go = [&](auto kernel) {
         kernel<<<grid, TR_THREADS, 0, s>>>(t->rec32, t->rec64, t->fix_hi, t->fix_lo, t->info,
-                                           t->ids, x, y, z, t->box, t->n, t->params.theta, eps2, G,
+                                           t->ids, x, y, z, t->box, t->n, Theta(t->params.theta), eps2, G,
                                            ax, ay, az, t->walk_len);
     };
     switch (team) {

@@ -123,3 +123,24 @@ def test_scan_at_tile_edges(ctx, n):
     util_exclusive_scan_u32(ctx, t, out)
     ctx.sync()
     np.testing.assert_array_equal(host(out), np.concatenate([[0], np.cumsum(v)]))
+
+
+def _nested(clumps, levels, per_level, seed):
+    """Clumps whose bodies halve their distance to the centre every `per_level` bodies."""
+    rng = np.random.default_rng(seed)
+    k = np.repeat(np.arange(levels), per_level)
+    c = np.repeat(rng.uniform(-1, 1, (clumps, 3)), len(k), axis=0)
+    r = 2.0 ** -(7.0 + np.tile(k, clumps))[:, None] * rng.uniform(0.5, 1.0, (len(c), 3))
+    p = c + r * rng.choice([-1.0, 1.0], (len(c), 3))
+    d = {key: np.ascontiguousarray(p[:, i]) for i, key in enumerate("xyz")}
+    d["m"] = rng.uniform(0.5, 1.5, len(c))
+    d["G"] = 1.0
+    return d
+
+
+@pytest.mark.parametrize("clumps", [20, 100, 130])
+def test_many_cells_across_chunks(ctx, clumps):
+    """Deep clumps: a tier with more cells than it keeps in shared memory (from about 50 clumps on),
+    and one below; one and two tiers. The clumps' cores are smaller than the FP32 records resolve, so
+    the walk's opening tests there have to be left to FP64."""
+    check(ctx, _nested(clumps, 28, 9, clumps), storage=512)
