@@ -754,6 +754,7 @@ struct ComArgs {
     const uint32_t* base;
     const uint8_t* node_level;
     const uint32_t *node_first, *node_last, *node_skip, *node_body;
+    uint32_t* tier_slot;
     uint32_t* node_count;
     double *comx, *comy, *comz, *mass, *q;
     NodeRec64* rec64;
@@ -1112,26 +1113,47 @@ constexpr int CM_LEVELS = 2 * NB_KEY_LEVELS + 1;  // node levels 0..42
 constexpr int CM_FAN = 96;                        // lower-tier chunks per upper-tier chunk
 constexpr int CM_TIER_MAX = CM_LEVELS * CM_FAN;   // listed cells one upper-tier block reads
 constexpr int CM_TIERS = 5;                       // 256 * 96^4 > 2^27 bodies
-constexpr int CC_THREADS = 256;                   // threads per block of the tier kernel
+constexpr int CC_THREADS = 512;                   // threads per block of the tier kernel
 
-// Sums the `nf` cells found[k] (level flev[k]) level by level, deepest first, then writes their
-// records. Block-wide; smem arrays given by the caller.
-__device__ void sum_by_level(const ComArgs& A, const uint32_t* found, const uint8_t* flev,
-                             uint32_t nf, uint32_t* nodes, uint32_t* cnt, uint32_t* off,
-                             uint32_t* fill) {
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int l = 0; l < CM_LEVELS; ++l) {
-            off[l] = run;
-            run += cnt[l];
+// Exclusive prefix of the level counts and the deepest level with a cell (-1: none), by warp 0.
+__device__ __forceinline__ void level_offsets(const uint32_t* cnt, uint32_t* off, int* deepest) {
+    const uint32_t lane = threadIdx.x;
+    if (lane >= 32) return;
+    uint32_t run = 0;
+    int top = -1;
+    for (int l0 = 0; l0 < CM_LEVELS; l0 += 32) {
+        const int l = l0 + (int)lane;
+        const uint32_t c = l < CM_LEVELS ? cnt[l] : 0u;
+        uint32_t incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((int)lane >= o) incl += v;
         }
+        if (l < CM_LEVELS) off[l] = run + incl - c;
+        run += __shfl_sync(0xffffffffu, incl, 31);
+        const uint32_t some = __ballot_sync(0xffffffffu, c != 0);
+        if (some) top = l0 + 31 - __clz((int)some);
     }
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < nf; k += blockDim.x) {
-        const uint32_t l = flev[k];
-        nodes[off[l] + atomicAdd(&fill[l], 1u)] = found[k];
-    }
-    __syncthreads();
+    if (lane == 0) *deepest = top;
+}
+
+// The visit-order child list of a cell, compacted: as the learned traversal reads it.
+__device__ __forceinline__ void compact_children(const ComArgs& A, uint32_t idx) {
+    uint32_t* cl = A.children + (size_t)idx * 8;
+    const uint4 c0 = reinterpret_cast<const uint4*>(cl)[0], c1 = reinterpret_cast<const uint4*>(cl)[1];
+    const uint32_t vs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+    uint32_t nch = 0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+        if (vs[t] != NB_NONE) cl[nch++] = vs[t];
+    for (uint32_t t = nch; t < 8; ++t) cl[t] = NB_NONE;
+}
+
+// Sums the `nf` cells nodes[off[l] .. off[l] + cnt[l]) of each level l, deepest first, in global
+// memory, then writes their records. Block-wide; smem arrays given by the caller.
+__device__ void sum_by_level(const ComArgs& A, uint32_t nf, const uint32_t* nodes,
+                             const uint32_t* cnt, const uint32_t* off) {
     // deepest level first; each thread's first cell of the next level has its child list loaded
     // before the barrier (a list only changes when its own cell is summed), so a level costs one
     // round trip to the children's sums instead of two
@@ -1238,25 +1260,7 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
     __syncthreads();
     const uint32_t nf = min(n_found, (uint32_t)CW);
     if (tid == 0) up_count[blockIdx.x] = min(n_up, (uint32_t)CM_LEVELS);
-    if (tid < 32) {  // exclusive prefix of the level counts, deepest level last
-        uint32_t run = 0;
-        int top = -1;
-        for (int l0 = 0; l0 < CM_LEVELS; l0 += 32) {
-            const int l = l0 + (int)tid;
-            const uint32_t c = l < CM_LEVELS ? cnt[l] : 0u;
-            uint32_t incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)tid >= o) incl += v;
-            }
-            if (l < CM_LEVELS) off[l] = run + incl - c;
-            run += __shfl_sync(0xffffffffu, incl, 31);
-            const uint32_t some = __ballot_sync(0xffffffffu, c != 0);
-            if (some) top = l0 + 31 - __clz((int)some);
-        }
-        if (tid == 0) deepest = top;
-    }
+    level_offsets(cnt, off, &deepest);
     __syncthreads();
     for (uint32_t k = tid; k < nf; k += CH_THREADS) {
         const uint32_t l = flev[k];
@@ -1324,30 +1328,70 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
     }
 }
 
-// Tier of `span` sorted positions per block (span = CW * CM_FAN^t): the cells listed by the
-// CM_FAN lower-tier chunks of the span (in[c * CM_LEVELS + k], k < in_count[c]) that end inside
-// it are summed here; the others go to up[] for the next tier (up == nullptr: the last tier,
-// whose single block spans all bodies).
+// Tier of `span` sorted positions per block: the cells listed by the CM_FAN lower-tier chunks of the
+// span (in[c * CM_LEVELS + k], k < in_count[c]) that end inside it are summed here; the others go to
+// up[] for the next tier (up == nullptr: the last tier, whose single block spans all bodies).
+// Bound by latency: a block has a few hundred cells over 8 to 12 levels and a level waits for the one
+// below. Up to CM_KEPT cells therefore sum from shared memory: all children outside the tier, which
+// are final, are read ahead of the first level, the sums of the tier's own cells stay in shared memory
+// (tier_slot finds a child's place in the block's list; what it names is checked, so that whatever an
+// earlier launch left there does not matter), and four lanes take a cell's four components. With the
+// children's sums read from global memory level by level, as for more cells than that, a level took
+// 5,300 cycles; this way the whole centre-of-mass phase takes 49 us instead of 64 at 16,411 bodies (one
+// tier), 80 instead of 106 at 131,101 (two).
+constexpr int CM_KEPT = 512;
+constexpr size_t tier_smem_bytes(bool learned) {
+    return (size_t)CM_TIER_MAX * sizeof(uint32_t) +
+           (size_t)CM_KEPT * ((learned ? 5 : 4) * 9 * sizeof(double) + 8 * sizeof(uint16_t));
+}
+constexpr uint32_t KID_NONE = 0xffff, KID_OUTSIDE = 0xfffe;  // else a place in the tier's list
+
 __global__ void __launch_bounds__(CC_THREADS)
 com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
                 const uint32_t* __restrict__ in_count, uint32_t in_chunks, uint2* up,
                 uint32_t* up_count) {
-    __shared__ uint32_t found[CM_TIER_MAX];
-    __shared__ uint8_t flev[CM_TIER_MAX];
-    __shared__ uint32_t nodes[CM_TIER_MAX];
-    __shared__ uint32_t cnt[CM_LEVELS], off[CM_LEVELS], fill[CM_LEVELS];
+    extern __shared__ __align__(16) unsigned char com_smem[];
+    const bool learned = (A.records & NB_REC_LEARNED) != 0;
+    const int comps = learned ? 5 : 4;
+    uint16_t* kid = reinterpret_cast<uint16_t*>(com_smem);             // [CM_KEPT][8], octant order
+    double* kept = reinterpret_cast<double*>(kid + 8 * CM_KEPT);       // [comps][CM_KEPT]
+    double* val = kept + comps * CM_KEPT;                              // [comps][CM_KEPT][8]
+    uint32_t* nodes = reinterpret_cast<uint32_t*>(val + comps * CM_KEPT * 8);  // [CM_TIER_MAX]
+    // the cells as found, only until they are in nodes[] by level
+    uint32_t* found = reinterpret_cast<uint32_t*>(val);
+    uint8_t* flev = reinterpret_cast<uint8_t*>(found + CM_TIER_MAX);
+    static_assert((size_t)CM_TIER_MAX * 5 <= (size_t)CM_KEPT * 4 * 8 * sizeof(double), "found, flev");
+    __shared__ uint32_t cnt[CM_LEVELS], off[CM_LEVELS], fill[CM_LEVELS], first[CM_FAN + 1];
     __shared__ uint32_t n_found, n_up;
-    const uint32_t P = blockIdx.x * span;
+    const uint32_t tid = threadIdx.x, P = blockIdx.x * span;
     if (P >= A.n) return;
     const uint32_t Pend = (uint32_t)min((uint64_t)P + span, (uint64_t)A.n);
-    for (int l = threadIdx.x; l < CM_LEVELS; l += CC_THREADS) cnt[l] = fill[l] = 0;
-    if (threadIdx.x == 0) n_found = n_up = 0;
+    if (tid < CM_LEVELS) cnt[tid] = fill[tid] = 0;
+    if (tid == 0) n_found = n_up = 0;
+    const uint32_t c0 = blockIdx.x * CM_FAN, chunks = min((uint32_t)CM_FAN, in_chunks - c0);
+    if (tid < 32) {  // the chunks' entries, one after the other
+        uint32_t run = 0;
+        for (uint32_t b = 0; b < CM_FAN; b += 32) {
+            const uint32_t c = b + tid < chunks ? in_count[c0 + b + tid] : 0u;
+            uint32_t incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)tid >= o) incl += v;
+            }
+            first[b + tid] = run + incl - c;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (tid == 0) first[CM_FAN] = run;
+    }
     __syncthreads();
-    const uint32_t c0 = blockIdx.x * CM_FAN, c1 = min(c0 + (uint32_t)CM_FAN, in_chunks);
-    for (uint32_t e = threadIdx.x; e < (c1 - c0) * CM_LEVELS; e += CC_THREADS) {
-        const uint32_t c = c0 + e / CM_LEVELS, k = e % CM_LEVELS;
-        if (k >= in_count[c]) continue;
-        const uint2 g = in[(size_t)c * CM_LEVELS + k];
+    for (uint32_t e = tid; e < min(first[CM_FAN], (uint32_t)CM_TIER_MAX); e += CC_THREADS) {
+        uint32_t lo = 0, hi = CM_FAN;  // first[lo] <= e < first[hi]
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (first[mid] <= e) lo = mid; else hi = mid;
+        }
+        const uint2 g = in[(size_t)(c0 + lo) * CM_LEVELS + (e - first[lo])];
         if (up != nullptr && A.node_last[g.x] >= Pend) {
             const uint32_t u = atomicAdd(&n_up, 1u);
             if (u < (uint32_t)CM_LEVELS) up[(size_t)blockIdx.x * CM_LEVELS + u] = g;
@@ -1355,16 +1399,105 @@ com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
             continue;
         }
         atomicAdd(&cnt[g.y], 1u);
-        const uint32_t slot = atomicAdd(&n_found, 1u);
-        if (slot < (uint32_t)CM_TIER_MAX) {
-            found[slot] = g.x;
-            flev[slot] = (uint8_t)g.y;
+        const uint32_t slot = atomicAdd(&n_found, 1u);  // < CM_TIER_MAX: one per entry
+        found[slot] = g.x;
+        flev[slot] = (uint8_t)g.y;
+    }
+    __syncthreads();
+    const uint32_t nf = n_found;
+    if (tid == 0 && up_count != nullptr) up_count[blockIdx.x] = min(n_up, (uint32_t)CM_LEVELS);
+    __shared__ int deepest;
+    level_offsets(cnt, off, &deepest);
+    __syncthreads();
+    for (uint32_t k = tid; k < nf; k += CC_THREADS) {
+        const uint32_t l = flev[k], idx = found[k], at = off[l] + atomicAdd(&fill[l], 1u);
+        nodes[at] = idx;
+        A.tier_slot[idx] = at;
+    }
+    __syncthreads();
+    if (nf > (uint32_t)CM_KEPT) {
+        sum_by_level(A, nf, nodes, cnt, off);
+        return;
+    }
+    // the children: their places in the list, or their sums
+    constexpr int AHEAD = 4;
+    double* const sums[5] = {A.comx, A.comy, A.comz, A.mass, A.q};
+    for (uint32_t e0 = tid; e0 < nf * 8; e0 += CC_THREADS * AHEAD) {
+        uint32_t ch[AHEAD], at[AHEAD];
+        double v[AHEAD][5];
+#pragma unroll
+        for (int r = 0; r < AHEAD; ++r) {
+            const uint32_t e = e0 + r * CC_THREADS;
+            ch[r] = NB_NONE;
+            if (e < nf * 8) ch[r] = A.children[(size_t)nodes[e >> 3] * 8 + nb_visit_of_octant(e & 7)];
+        }
+#pragma unroll
+        for (int r = 0; r < AHEAD; ++r) {
+            if (ch[r] == NB_NONE) continue;
+            at[r] = A.tier_slot[ch[r]];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v[r][c] = __ldcg(sums[c] + ch[r]);
+            if (learned) v[r][4] = __ldcg(sums[4] + ch[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < AHEAD; ++r) {
+            const uint32_t e = e0 + r * CC_THREADS;
+            if (e >= nf * 8) continue;
+            if (ch[r] == NB_NONE) {
+                kid[e] = (uint16_t)KID_NONE;
+            } else if (at[r] < nf && nodes[at[r]] == ch[r]) {
+                kid[e] = (uint16_t)at[r];
+            } else {
+                kid[e] = (uint16_t)KID_OUTSIDE;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) val[c * (CM_KEPT * 8) + e] = v[r][c];
+                if (learned) val[4 * (CM_KEPT * 8) + e] = v[r][4];
+            }
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && up_count != nullptr) up_count[blockIdx.x] = min(n_up, (uint32_t)CM_LEVELS);
-    if (n_found > (uint32_t)CM_TIER_MAX) return;  // cannot happen: <= CM_LEVELS per chunk
-    sum_by_level(A, found, flev, n_found, nodes, cnt, off, fill);
+    auto add_up = [&](uint32_t pos, int comp) {
+        const uint4 kk = *reinterpret_cast<const uint4*>(kid + 8 * pos);
+        const uint32_t kw[4] = {kk.x, kk.y, kk.z, kk.w};
+        const double* const kc = kept + comp * CM_KEPT;
+        const double* const vc = val + comp * (CM_KEPT * 8) + 8 * pos;
+        uint32_t k[8];
+        double v[8];
+#pragma unroll
+        for (int o = 0; o < 8; ++o) {
+            k[o] = (kw[o >> 1] >> (16 * (o & 1))) & 0xffffu;
+            v[o] = k[o] < (uint32_t)CM_KEPT ? kc[k[o]] : (k[o] == KID_OUTSIDE ? vc[o] : 0.0);
+        }
+        double sum = 0.0;
+#pragma unroll
+        for (int o = 0; o < 8; ++o)
+            if (k[o] != KID_NONE) sum = __dadd_rn(sum, v[o]);  // absent children add nothing
+        kept[comp * CM_KEPT + pos] = sum;
+    };
+    for (int l = deepest; l >= 0; --l) {
+        const uint32_t c = cnt[l], o0 = off[l];
+        if (c == 0) continue;  // uniform across the block
+        for (uint32_t k = tid >> 2; k < c; k += CC_THREADS / 4) {
+            add_up(o0 + k, (int)(tid & 3));
+            if (learned && (tid & 3) == 0) add_up(o0 + k, 4);
+        }
+        __syncthreads();
+    }
+    for (uint32_t k = tid; k < nf; k += CC_THREADS) {
+        const uint32_t idx = nodes[k];
+        const double sx = kept[k], sy = kept[CM_KEPT + k], sz = kept[2 * CM_KEPT + k],
+                     sm = kept[3 * CM_KEPT + k], sq = learned ? kept[4 * CM_KEPT + k] : 0.0;
+        A.comx[idx] = sx;
+        A.comy[idx] = sy;
+        A.comz[idx] = sz;
+        A.mass[idx] = sm;
+        if (learned) A.q[idx] = sq;
+        const uint32_t count = A.node_last[idx] - A.node_first[idx] + 1;
+        A.node_count[idx] = count;
+        compact_children(A, idx);
+        write_records(A, idx, sx, sy, sz, sm, sq, count, A.node_level[idx], A.node_skip[idx],
+                      NB_NONE);
+    }
 }
 
 // The kernels whose dynamic shared memory is above the default limit (before any capture of a build).
@@ -1378,6 +1511,7 @@ nb_status build_prepare() {
     NB_TRY(allow_smem(build_small_kernel<1024, 1024>, small_smem_bytes<1024>()));
     NB_TRY(allow_smem(build_small_kernel<2048, 1024>, small_smem_bytes<2048>()));
     NB_TRY(allow_smem(build_small_kernel<SB_MAX_N, 1024>, small_smem_bytes<SB_MAX_N>()));
+    NB_TRY(allow_smem(com_tier_kernel, tier_smem_bytes(true)));
     return allow_smem(com_chunk_kernel<1024, 1024>, chunk_smem_bytes<1024>(true));
 }
 
@@ -1424,6 +1558,7 @@ void carve(nb_bh_tree* t, Carver& c) {
     t->node_last = c.take<uint32_t>(cap);
     t->node_skip = c.take<uint32_t>(cap);
     t->node_body = c.take<uint32_t>(cap);
+    t->tier_slot = c.take<uint32_t>(cap);
     t->node_count = c.take<uint32_t>(cap);
     t->node_comx = c.take<double>(cap);
     t->node_comy = c.take<double>(cap);
@@ -1631,6 +1766,7 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     A.err = ctx->dev_error;
 
     A.node_body = t->node_body;
+    A.tier_slot = t->tier_slot;
     A.node_count = t->node_count;
     A.comx = t->node_comx;
     A.comy = t->node_comy;
@@ -1664,7 +1800,7 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
             span *= CM_FAN;
             const uint32_t blocks = (uint32_t)((n + span - 1) / span);
             const bool last = blocks == 1;
-            com_tier_kernel<<<blocks, CC_THREADS, 0, s>>>(
+            com_tier_kernel<<<blocks, CC_THREADS, tier_smem_bytes(learned), s>>>(
                 A, (uint32_t)std::min<uint64_t>(span, 0xffffffffu), t->tier_cells[in],
                 t->tier_count[in], chunks, last ? nullptr : t->tier_cells[1 - in],
                 last ? nullptr : t->tier_count[1 - in]);

@@ -89,7 +89,7 @@ struct nb_bh_tree {
 
     uint8_t* node_level = nullptr;
     uint32_t *node_first = nullptr, *node_last = nullptr, *node_skip = nullptr;
-    uint32_t* node_body = nullptr;
+    uint32_t *node_body = nullptr, *tier_slot = nullptr;  // tier_slot: see com_tier_kernel
     uint32_t* node_count = nullptr;
     double *node_comx = nullptr, *node_comy = nullptr, *node_comz = nullptr, *node_mass = nullptr;
     NodeRec64* rec64 = nullptr;
