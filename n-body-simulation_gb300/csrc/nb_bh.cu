@@ -18,7 +18,8 @@
 // What later launches want zeroed or filled is written by earlier ones (keys: the sort's counters,
 // second key words and level masks; splits: the child lists), the digit offsets are summed by the
 // sort's passes and the node counts by the scan: 18 launches, where separate ones took 26 and 22 us
-// more at 16,411 bodies.
+// more at 16,411 bodies. Each launch of the chain may start while the one before it ends (nb_grid_wait):
+// 122 us for that build instead of 162.
 //  7. bottom-up centre of mass: leaves and cells by blocks over chunks of 256 sorted positions
 //     (deepest level first), the cells reaching past their chunk (at most one per level) by tiers
 //     of blocks over 96 chunks each; children summed in octant order 0..7
@@ -176,6 +177,7 @@ __global__ void keys_quantized_kernel(const double* __restrict__ x, const double
                                       const double* __restrict__ z, uint32_t n,
                                       double* __restrict__ box, uint64_t* __restrict__ key0,
                                       uint32_t* __restrict__ ids, BuildZero Z) {
+    nb_grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     box_extras(box, i);
     build_zero(Z, i, n);
@@ -248,6 +250,7 @@ keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
             const double* __restrict__ z, uint32_t n, double* __restrict__ box,
             uint64_t* __restrict__ key0, uint32_t* __restrict__ ids, BuildZero Z) {
     __shared__ FixedGrid grid_s;  // once per block: it takes an FP64 division
+    nb_grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     box_extras(box, i);
     build_zero(Z, i, n);
@@ -299,6 +302,7 @@ __global__ void runs_fixup_kernel(const double* __restrict__ x, const double* __
                                   const double* __restrict__ box, const uint64_t* __restrict__ key0,
                                   uint64_t* __restrict__ key1, uint32_t* __restrict__ ids,
                                   uint32_t* __restrict__ err, int quantized) {
+    nb_grid_wait();
     fix_run(blockIdx.x * blockDim.x + threadIdx.x, x, y, z, n, box, key0, key1, ids, err,
             quantized);
 }
@@ -374,6 +378,7 @@ __global__ void splits_kernel(const uint64_t* __restrict__ key0, const uint64_t*
                               uint32_t* __restrict__ split_start, uint32_t* __restrict__ split_end,
                               unsigned long long* __restrict__ mask, uint32_t* __restrict__ children,
                               uint32_t* __restrict__ err) {
+    nb_grid_wait();
     // the child lists start empty (two nodes per position at most): stores that the searches' round
     // trips leave room for
     const uint32_t blk = min(blockDim.x, n - blockIdx.x * blockDim.x);
@@ -462,6 +467,7 @@ __global__ void emit_kernel(uint32_t n, const uint32_t* __restrict__ ids,
                             const unsigned long long* __restrict__ mask,
                             const uint32_t* __restrict__ base, const uint64_t* __restrict__ key0,
                             const uint64_t* __restrict__ key1, NodeTable T) {
+    nb_grid_wait();
     emit_at(blockIdx.x * blockDim.x + threadIdx.x, n, ids, split_level, split_start, split_end,
             mask, base, key0, key1, T);
 }
@@ -510,6 +516,7 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
                    uint32_t* __restrict__ ids_out, unsigned long long* __restrict__ mask_out,
                    uint32_t* __restrict__ base_out, NodeTable T, uint32_t* __restrict__ err,
                    int quantized) {
+    nb_grid_wait();  // an ordinary launch: only lets the dependent one start
     constexpr int PER = CAP / THREADS;  // positions per thread
     extern __shared__ __align__(16) unsigned char small_smem[];
     uint64_t* key0 = reinterpret_cast<uint64_t*>(small_smem);
@@ -1216,6 +1223,7 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
     __shared__ uint32_t cnt[CM_LEVELS], off[CM_LEVELS], fill[CM_LEVELS];
     __shared__ uint32_t n_found, n_up;
     const uint32_t tid = threadIdx.x, P = blockIdx.x * CW;
+    nb_grid_wait();
     const uint32_t Pend = min(P + (uint32_t)CW, A.n);
     const uint32_t d0 = A.base[P], d1 = A.base[Pend];
     if (tid < CM_LEVELS) cnt[tid] = fill[tid] = 0;
@@ -1363,6 +1371,7 @@ com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
     static_assert((size_t)CM_TIER_MAX * 5 <= (size_t)CM_KEPT * 4 * 8 * sizeof(double), "found, flev");
     __shared__ uint32_t cnt[CM_LEVELS], off[CM_LEVELS], fill[CM_LEVELS], first[CM_FAN + 1];
     __shared__ uint32_t n_found, n_up;
+    nb_grid_wait();
     const uint32_t tid = threadIdx.x, P = blockIdx.x * span;
     if (P >= A.n) return;
     const uint32_t Pend = (uint32_t)min((uint64_t)P + span, (uint64_t)A.n);
@@ -1716,11 +1725,12 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
         const BuildZero Z{(uint4*)t->sort_temp, (uint32_t)(nb::radix_zero_bytes(n) / 16), t->key1,
                           (unsigned long long*)t->mask};
         if (quantized) {
-            keys_quantized_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids, Z);
+            NB_CUDA_TRY(nb::launch_after(keys_quantized_kernel, grid, BH_THREADS, 0, s, x, y, z, n,
+                                         t->box, t->key0, t->ids, Z));
         } else {
-            keys_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->ids, Z);
+            NB_CUDA_TRY(nb::launch_after(keys_kernel, grid, BH_THREADS, 0, s, x, y, z, n, t->box,
+                                         t->key0, t->ids, Z));
         }
-        NB_TRY(nb::check_launch("keys_kernel"));
         NB_TRY(mark(2));
         int in_alt = 0;
         NB_TRY(nb::radix_sort_pairs(t->key0, t->ids, t->key_alt, t->ids_alt, n, 0, 3 * NB_KEY_LEVELS,
@@ -1731,18 +1741,16 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
             NB_CUDA_TRY(cudaMemcpyAsync(t->ids, t->ids_alt, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
         }
         NB_TRY(mark(3));
-        runs_fixup_kernel<<<grid, BH_THREADS, 0, s>>>(x, y, z, n, t->box, t->key0, t->key1, t->ids,
-                                                      ctx->dev_error, quantized ? 1 : 0);
-        NB_TRY(nb::check_launch("runs_fixup_kernel"));
-        splits_kernel<<<grid, BH_THREADS, 0, s>>>(t->key0, t->key1, n, t->split_level, t->split_start,
-                                                  t->split_end, (unsigned long long*)t->mask,
-                                                  t->children, ctx->dev_error);
-        NB_TRY(nb::check_launch("splits_kernel"));
+        NB_CUDA_TRY(nb::launch_after(runs_fixup_kernel, grid, BH_THREADS, 0, s, x, y, z, n, t->box,
+                                     t->key0, t->key1, t->ids, ctx->dev_error, quantized ? 1 : 0));
+        NB_CUDA_TRY(nb::launch_after(splits_kernel, grid, BH_THREADS, 0, s, t->key0, t->key1, n,
+                                     t->split_level, t->split_start, t->split_end,
+                                     (unsigned long long*)t->mask, t->children, ctx->dev_error));
         NB_TRY(nb::node_offsets((const unsigned long long*)t->mask, t->base, n, t->scan_temp, s));
-        emit_kernel<<<grid, BH_THREADS, 0, s>>>(n, t->ids, t->split_level, t->split_start, t->split_end,
-                                                (const unsigned long long*)t->mask, t->base, t->key0,
-                                                t->key1, T);
-        NB_TRY(nb::check_launch("emit_kernel"));
+        NB_CUDA_TRY(nb::launch_after(emit_kernel, grid, BH_THREADS, 0, s, n, t->ids, t->split_level,
+                                     t->split_start, t->split_end,
+                                     (const unsigned long long*)t->mask, t->base, t->key0, t->key1,
+                                     T));
     }
     NB_TRY(mark(4));
     ComArgs A;
@@ -1789,22 +1797,22 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
         const uint32_t cw = n <= 1024 ? 1024 : 256;
         uint32_t chunks = (uint32_t)nb::ceil_div(n, cw);
         auto go = [&](auto kernel, size_t smem) {
-            kernel<<<chunks, cw, smem, s>>>(A, t->tier_cells[0], t->tier_count[0]);
+            return nb::launch_after(kernel, chunks, cw, smem, s, A, t->tier_cells[0],
+                                    t->tier_count[0]);
         };
-        if (cw == 1024) go(com_chunk_kernel<1024, 1024>, chunk_smem_bytes<1024>(learned));
-        else go(com_chunk_kernel<256, 256>, chunk_smem_bytes<256>(learned));
-        NB_TRY(nb::check_launch("com_chunk_kernel"));
+        NB_CUDA_TRY(cw == 1024 ? go(com_chunk_kernel<1024, 1024>, chunk_smem_bytes<1024>(learned))
+                               : go(com_chunk_kernel<256, 256>, chunk_smem_bytes<256>(learned)));
         uint64_t span = cw;
         int in = 0;
         for (int tier = 1; tier <= CM_TIERS && chunks > 1; ++tier) {
             span *= CM_FAN;
             const uint32_t blocks = (uint32_t)((n + span - 1) / span);
             const bool last = blocks == 1;
-            com_tier_kernel<<<blocks, CC_THREADS, tier_smem_bytes(learned), s>>>(
-                A, (uint32_t)std::min<uint64_t>(span, 0xffffffffu), t->tier_cells[in],
+            NB_CUDA_TRY(nb::launch_after(
+                com_tier_kernel, blocks, CC_THREADS, tier_smem_bytes(learned), s, A,
+                (uint32_t)std::min<uint64_t>(span, 0xffffffffu), t->tier_cells[in],
                 t->tier_count[in], chunks, last ? nullptr : t->tier_cells[1 - in],
-                last ? nullptr : t->tier_count[1 - in]);
-            NB_TRY(nb::check_launch("com_tier_kernel"));
+                last ? nullptr : t->tier_count[1 - in]));
             if (last) break;
             chunks = blocks;
             in = 1 - in;

@@ -458,6 +458,7 @@ bh_theta_team_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
                      Theta theta, double eps2, double G, double* __restrict__ ax,
                      double* __restrict__ ay, double* __restrict__ az,
                      uint32_t* __restrict__ walk_len) {
+    nb_grid_wait();
     constexpr int B = 32 / T;                     // bodies per warp
     constexpr int CAP = T * 8 > 64 ? T * 8 : 64;  // listed cells per body and round
     constexpr int WARPS = TR_THREADS / 32;
@@ -1024,18 +1025,17 @@ nb_status launch_f64(nb_ctx* ctx, const nb_bh_tree* t, nb_precision prec, const 
     if (team == 1) return launch_lane(ctx, t, prec, x, y, z, ax, ay, az, G, eps2, s);
     const int grid = nb::ceil_div((long long)t->n * team, TR_THREADS);
     auto go = [&](auto kernel) {
-        kernel<<<grid, TR_THREADS, 0, s>>>(t->rec32, t->rec64, t->fix_hi, t->fix_lo, t->info,
-                                           t->ids, x, y, z, t->box, t->n, Theta(t->params.theta), eps2, G,
-                                           ax, ay, az, t->walk_len);
+        return nb::launch_after(kernel, grid, TR_THREADS, 0, s, t->rec32, t->rec64, t->fix_hi,
+                                t->fix_lo, t->info, t->ids, x, y, z, t->box, t->n,
+                                Theta(t->params.theta), eps2, G, ax, ay, az, t->walk_len);
     };
     switch (team) {
-        case 2: go(bh_theta_team_kernel<2>); break;
-        case 4: go(bh_theta_team_kernel<4>); break;
-        case 8: go(bh_theta_team_kernel<8>); break;
-        case 16: go(bh_theta_team_kernel<16>); break;
-        default: go(bh_theta_team_kernel<32>); break;
+        case 2: NB_CUDA_TRY(go(bh_theta_team_kernel<2>)); break;
+        case 4: NB_CUDA_TRY(go(bh_theta_team_kernel<4>)); break;
+        case 8: NB_CUDA_TRY(go(bh_theta_team_kernel<8>)); break;
+        case 16: NB_CUDA_TRY(go(bh_theta_team_kernel<16>)); break;
+        default: NB_CUDA_TRY(go(bh_theta_team_kernel<32>)); break;
     }
-    NB_TRY(nb::check_launch("bh_theta_team_kernel"));
     t->walk_n = t->n;
     return NB_OK;
 }

@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(AABB_THREADS)
 aabb_kernel(const double* __restrict__ x, const double* __restrict__ y,
             const double* __restrict__ z, uint32_t n, MinMax6* __restrict__ part,
             unsigned int* __restrict__ counter, double* __restrict__ out) {
+    nb_grid_wait();  // an ordinary launch: only lets a dependent one start
     const long long zero = ord_of(0.0);
     long long mn[3] = {zero, zero, zero}, mx[3] = {zero, zero, zero};
     const double* p[3] = {x, y, z};

@@ -147,6 +147,33 @@ __device__ __forceinline__ float nb_rsqrt_f32(float x) {
 }
 
 // Packed FP32x2 arithmetic (sm_100+ f32x2 instructions): one instruction, two lanes.
+// Dependent launches. A kernel launched with nb::launch_after may start while the kernel before it in
+// the stream still runs; nb_grid_wait, which such a kernel calls before it touches memory that earlier
+// launches write, returns when that kernel has finished and its writes are visible, and lets the next
+// dependent launch start in turn. (So everything before the preceding kernel has finished already
+// when a dependent one starts.) Saves the gap between the short launches of a chain, 1 to 1.5 us each.
+__device__ __forceinline__ void nb_grid_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+namespace nb {
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                         A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+}  // namespace nb
+
 typedef unsigned long long nb_f2;
 __device__ __forceinline__ nb_f2 f2_pack(float lo, float hi) {
     nb_f2 r;

@@ -60,6 +60,7 @@ struct MaskItems {
 template <class Items>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_reduce_kernel(Items in, uint32_t n, uint32_t* __restrict__ sums) {
+    nb_grid_wait();
     const uint32_t base = blockIdx.x * SCAN_TILE;
     uint32_t s = 0;
 #pragma unroll
@@ -75,6 +76,7 @@ scan_reduce_kernel(Items in, uint32_t n, uint32_t* __restrict__ sums) {
 // Exclusive scan of sums[0..nb) in place by one block; sums[nb] = grand total.
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_sums_kernel(uint32_t* __restrict__ sums, uint32_t nb) {
+    nb_grid_wait();
     uint32_t carry = 0;
     for (uint32_t base = 0; base < nb; base += SCAN_THREADS) {
         const uint32_t i = base + threadIdx.x;
@@ -93,6 +95,7 @@ template <class Items>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_apply_kernel(Items in, uint32_t* __restrict__ out, uint32_t n,
                   const uint32_t* __restrict__ sums, int write_total, int summed) {
+    nb_grid_wait();
     const uint32_t base = blockIdx.x * SCAN_TILE;
     uint32_t before = 0;
     if (summed) {
@@ -152,6 +155,7 @@ radix_hist_all_kernel(const uint64_t* __restrict__ keys, uint32_t n, int begin_b
                       uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[RS_MAX_PASSES][RS_BINS];
     for (int e = threadIdx.x; e < RS_MAX_PASSES * RS_BINS; e += RS_THREADS) (&h[0][0])[e] = 0;
+    nb_grid_wait();
     __syncthreads();
     for (uint32_t i = blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += gridDim.x * RS_THREADS) {
         const uint64_t k = keys[i] >> begin_bit;
@@ -195,8 +199,10 @@ radix_pass_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restri
     uint32_t* svals = reinterpret_cast<uint32_t*>(rs_reorder + RS_TILE * sizeof(uint64_t));
     __shared__ uint32_t tile_s;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the tickets were zeroed before the kernel that precedes this one started
     if (threadIdx.x == 0) tile_s = atomicAdd(ticket, 1u);
     for (int b = threadIdx.x; b < RS_WARPS * RS_BINS; b += RS_THREADS) (&wcnt[0][0])[b] = 0;
+    nb_grid_wait();
     const uint32_t hist_d = hist[threadIdx.x];
     __syncthreads();
     const uint32_t tile = tile_s;
@@ -323,15 +329,13 @@ nb_status scan_items(Items in, uint32_t* out, uint32_t n, int write_total, uint3
     if (nb > 64u * SCAN_THREADS)
         return set_error(NB_ERR_INVALID_ARG, "exclusive_scan_u32: n = %u too large", n);
     const bool summed = nb <= SCAN_SELF_TILES;
-    scan_reduce_kernel<<<nb, SCAN_THREADS, 0, stream>>>(in, n, temp);
-    NB_TRY(check_launch("scan_reduce_kernel"));
+    NB_CUDA_TRY(launch_after(scan_reduce_kernel<Items>, nb, SCAN_THREADS, 0, stream, in, n, temp));
     if (!summed) {
-        scan_sums_kernel<<<1, SCAN_THREADS, 0, stream>>>(temp, nb);
-        NB_TRY(check_launch("scan_sums_kernel"));
+        NB_CUDA_TRY(launch_after(scan_sums_kernel, 1, SCAN_THREADS, 0, stream, temp, nb));
     }
-    scan_apply_kernel<<<nb, SCAN_THREADS, 0, stream>>>(in, out, n, temp, write_total,
-                                                       summed ? 1 : 0);
-    return check_launch("scan_apply_kernel");
+    NB_CUDA_TRY(launch_after(scan_apply_kernel<Items>, nb, SCAN_THREADS, 0, stream, in, out, n, temp,
+                             write_total, summed ? 1 : 0));
+    return NB_OK;
 }
 }  // namespace
 
@@ -345,13 +349,13 @@ nb_status node_offsets(const unsigned long long* mask, uint32_t* out, uint32_t n
     return scan_items(MaskItems{mask}, out, n, 1, temp, stream);
 }
 
-// Keys per thread of a pass: as few as give the small sorts enough blocks, as many as the large ones
-// need for short look-backs. All eight passes with their histogram at 4 / 8 / 16 keys per thread:
-// 16,411 keys 68 / 70 / 101 us, 65,536 72 / 80 / 105, 131,101 85 / 85 / 113, 262,144 103 / 89 / 119,
-// 524,288 146 / 119 / 126, 1,048,576 222 / 185 / 171.
-constexpr uint32_t RS_N4 = 1u << 17, RS_N8 = 1u << 19;
+// Keys per thread of a pass: few give the small sorts enough blocks, many give the large ones short
+// look-backs. All eight passes with their histogram at 4 / 8 / 16 keys per thread: 16,411 keys 47 /
+// 55 / 81 us, 65,536 52 / 58 / 89, 131,101 63 / 71 / 93, 262,144 83 / 87 / 97, 524,288 119 / 130 /
+// 107, 1,048,576 185 / 162 / 150.
+constexpr uint32_t RS_N4 = 1u << 18;
 static uint32_t radix_tiles(uint32_t n) {
-    const uint32_t tile = RS_THREADS * (n <= RS_N4 ? 4 : (n <= RS_N8 ? 8 : 16));
+    const uint32_t tile = RS_THREADS * (n <= RS_N4 ? 4 : 16);
     return (uint32_t)(((uint64_t)n + tile - 1) / tile);
 }
 
@@ -374,8 +378,7 @@ size_t radix_zero_bytes(uint32_t n) {
             (size_t)RS_MAX_PASSES * radix_tiles(n) * RS_BINS) * sizeof(uint32_t);
 }
 size_t radix_temp_bytes(uint32_t n) {  // enough for any count up to n
-    return std::max({radix_zero_bytes(n), radix_zero_bytes(std::min(n, RS_N4)),
-                     radix_zero_bytes(std::min(n, RS_N8))});
+    return std::max(radix_zero_bytes(n), radix_zero_bytes(std::min(n, RS_N4)));
 }
 
 nb_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt,
@@ -397,8 +400,8 @@ nb_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt,
     uint32_t* lb = tickets + 64;                         // [passes][tiles][256]
     if (!zeroed) NB_CUDA_TRY(cudaMemsetAsync(temp, 0, radix_zero_bytes(n), stream));
     const int hist_blocks = (int)std::min<uint32_t>((n + RS_HIST_KEYS - 1) / RS_HIST_KEYS, 1024u);
-    radix_hist_all_kernel<<<hist_blocks, RS_THREADS, 0, stream>>>(keys, n, begin_bit, passes, hist);
-    NB_TRY(check_launch("radix_hist_all_kernel"));
+    NB_CUDA_TRY(launch_after(radix_hist_all_kernel, hist_blocks, RS_THREADS, 0, stream, keys, n,
+                             begin_bit, passes, hist));
     uint64_t* kin = keys;
     uint32_t* vin = vals;
     uint64_t* kout = keys_alt;
@@ -406,14 +409,13 @@ nb_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt,
     int flips = 0;
     for (int p = 0; p < passes; ++p) {
         auto go = [&](auto kernel, int smem) {
-            kernel<<<tiles, RS_THREADS, smem, stream>>>(
-                kin, vin, kout, vout, n, begin_bit + 8 * p, hist + p * RS_BINS,
-                lb + (size_t)p * tiles * RS_BINS, tickets + p, err, wait_limit, drop_first);
+            return launch_after(kernel, tiles, RS_THREADS, smem, stream, kin, vin, kout, vout, n,
+                                begin_bit + 8 * p, hist + p * RS_BINS,
+                                lb + (size_t)p * tiles * RS_BINS, tickets + p, err, wait_limit,
+                                drop_first);
         };
-        if (n <= RS_N4) go(radix_pass_kernel<4>, RS_REORDER_BYTES<4>);
-        else if (n <= RS_N8) go(radix_pass_kernel<8>, RS_REORDER_BYTES<8>);
-        else go(radix_pass_kernel<16>, RS_REORDER_BYTES<16>);
-        NB_TRY(check_launch("radix_pass_kernel"));
+        NB_CUDA_TRY(n <= RS_N4 ? go(radix_pass_kernel<4>, RS_REORDER_BYTES<4>)
+                              : go(radix_pass_kernel<16>, RS_REORDER_BYTES<16>));
         uint64_t* tk = kin;
         kin = kout;
         kout = tk;

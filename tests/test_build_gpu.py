@@ -97,9 +97,9 @@ def test_coincident_bodies_are_reported(ctx, n):
     tree.close()
 
 
-@pytest.mark.parametrize("n", [1023, 1025, 131072, 131073, 524288, 524289])
+@pytest.mark.parametrize("n", [1023, 1025, 131072, 131073, 262144, 262145, 524289])
 def test_sort_at_tile_edges(ctx, n):
-    """The three tile sizes of the sort's passes: stable, with many equal keys."""
+    """The tile sizes of the sort's passes: stable, with many equal keys."""
     import torch
     from nbody.lib import util_radix_sort_pairs
     rng = np.random.default_rng(n)
