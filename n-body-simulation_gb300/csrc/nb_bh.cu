@@ -516,7 +516,7 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
                    uint32_t* __restrict__ ids_out, unsigned long long* __restrict__ mask_out,
                    uint32_t* __restrict__ base_out, NodeTable T, uint32_t* __restrict__ err,
                    int quantized) {
-    nb_grid_wait();  // an ordinary launch: only lets the dependent one start
+    nb_grid_wait();
     constexpr int PER = CAP / THREADS;  // positions per thread
     extern __shared__ __align__(16) unsigned char small_smem[];
     uint64_t* key0 = reinterpret_cast<uint64_t*>(small_smem);
@@ -1710,15 +1710,18 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     if (n <= SB_MAX_N) {  // one block; its whole time counts as the cells phase
         for (int phase = 1; phase <= 3; ++phase) NB_TRY(mark(phase));
         auto go = [&](auto kernel, uint32_t threads, size_t smem) {
-            kernel<<<1, threads, smem, s>>>(x, y, z, n, t->box, t->key0, t->key1, t->ids,
-                                            (unsigned long long*)t->mask, t->base, T,
-                                            ctx->dev_error, quantized ? 1 : 0);
+            return nb::launch_after(kernel, 1, threads, smem, s, x, y, z, n, t->box, t->key0,
+                                    t->key1, t->ids, (unsigned long long*)t->mask, t->base, T,
+                                    ctx->dev_error, quantized ? 1 : 0);
         };
-        if (n <= 512) go(build_small_kernel<512, 512>, 512, small_smem_bytes<512>());
-        else if (n <= 1024) go(build_small_kernel<1024, 1024>, 1024, small_smem_bytes<1024>());
-        else if (n <= 2048) go(build_small_kernel<2048, 1024>, 1024, small_smem_bytes<2048>());
-        else go(build_small_kernel<SB_MAX_N, 1024>, 1024, small_smem_bytes<SB_MAX_N>());
-        NB_TRY(nb::check_launch("build_small_kernel"));
+        if (n <= 512)
+            NB_CUDA_TRY(go(build_small_kernel<512, 512>, 512, small_smem_bytes<512>()));
+        else if (n <= 1024)
+            NB_CUDA_TRY(go(build_small_kernel<1024, 1024>, 1024, small_smem_bytes<1024>()));
+        else if (n <= 2048)
+            NB_CUDA_TRY(go(build_small_kernel<2048, 1024>, 1024, small_smem_bytes<2048>()));
+        else
+            NB_CUDA_TRY(go(build_small_kernel<SB_MAX_N, 1024>, 1024, small_smem_bytes<SB_MAX_N>()));
     } else {
         NB_TRY(nb::launch_aabb(ctx, x, y, z, n, t->box, s));
         NB_TRY(mark(1));

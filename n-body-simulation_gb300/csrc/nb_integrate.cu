@@ -19,6 +19,7 @@ __global__ void kick_drift_kernel(double* __restrict__ vhx, double* __restrict__
                                   double* __restrict__ z, const double* __restrict__ ax,
                                   const double* __restrict__ ay, const double* __restrict__ az,
                                   uint32_t n, double dt) {
+    nb_grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double h = dt / 2.0;
@@ -39,6 +40,7 @@ __global__ void kick_kernel(double* __restrict__ vx, double* __restrict__ vy,
                             const double* __restrict__ vhy, const double* __restrict__ vhz,
                             const double* __restrict__ ax, const double* __restrict__ ay,
                             const double* __restrict__ az, uint32_t n, double dt) {
+    nb_grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double h = dt / 2.0;
@@ -56,6 +58,7 @@ __global__ void kick_kick_drift_kernel(double* __restrict__ vx, double* __restri
                                        double* __restrict__ z, const double* __restrict__ ax,
                                        const double* __restrict__ ay,
                                        const double* __restrict__ az, uint32_t n, double dt) {
+    nb_grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double h = dt / 2.0;
@@ -275,7 +278,7 @@ __global__ void __launch_bounds__(AABB_THREADS)
 aabb_kernel(const double* __restrict__ x, const double* __restrict__ y,
             const double* __restrict__ z, uint32_t n, MinMax6* __restrict__ part,
             unsigned int* __restrict__ counter, double* __restrict__ out) {
-    nb_grid_wait();  // an ordinary launch: only lets a dependent one start
+    nb_grid_wait();
     const long long zero = ord_of(0.0);
     long long mn[3] = {zero, zero, zero}, mx[3] = {zero, zero, zero};
     const double* p[3] = {x, y, z};
@@ -381,9 +384,9 @@ nb_status launch_aabb(nb_ctx* ctx, const double* x, const double* y, const doubl
     if (blocks < 1) blocks = 1;
     void* part = nullptr;
     NB_TRY(nb::scratch(ctx, NB_SCRATCH_AABB, (size_t)blocks * sizeof(MinMax6), &part));
-    aabb_kernel<<<blocks, AABB_THREADS, 0, stream>>>(x, y, z, n, (MinMax6*)part,
-                                                     ctx->dev_counter + 0, out_dev);
-    return nb::check_launch("aabb_kernel");
+    NB_CUDA_TRY(nb::launch_after(aabb_kernel, blocks, AABB_THREADS, 0, stream, x, y, z, n,
+                                 (MinMax6*)part, ctx->dev_counter + 0, out_dev));
+    return NB_OK;
 }
 
 }  // namespace nb
@@ -398,9 +401,9 @@ nb_status nb_leapfrog_kick_drift(nb_ctx* ctx, double* vhx, double* vhy, double* 
     if (n == 0) return NB_OK;
     if (!vhx || !vhy || !vhz || !vx || !vy || !vz || !x || !y || !z || !ax || !ay || !az)
         return nb::set_error(NB_ERR_INVALID_ARG, "nb_leapfrog_kick_drift: null array pointer");
-    kick_drift_kernel<<<nb::ceil_div(n, EW_THREADS), EW_THREADS, 0, (cudaStream_t)stream>>>(
-        vhx, vhy, vhz, vx, vy, vz, x, y, z, ax, ay, az, n, dt);
-    return nb::check_launch("kick_drift_kernel");
+    NB_CUDA_TRY(nb::launch_after(kick_drift_kernel, nb::ceil_div(n, EW_THREADS), EW_THREADS, 0,
+                                 (cudaStream_t)stream, vhx, vhy, vhz, vx, vy, vz, x, y, z, ax, ay, az, n, dt));
+    return NB_OK;
 }
 
 nb_status nb_leapfrog_kick(nb_ctx* ctx, double* vx, double* vy, double* vz, const double* vhx,
@@ -411,9 +414,9 @@ nb_status nb_leapfrog_kick(nb_ctx* ctx, double* vx, double* vy, double* vz, cons
     if (n == 0) return NB_OK;
     if (!vhx || !vhy || !vhz || !vx || !vy || !vz || !ax || !ay || !az)
         return nb::set_error(NB_ERR_INVALID_ARG, "nb_leapfrog_kick: null array pointer");
-    kick_kernel<<<nb::ceil_div(n, EW_THREADS), EW_THREADS, 0, (cudaStream_t)stream>>>(
-        vx, vy, vz, vhx, vhy, vhz, ax, ay, az, n, dt);
-    return nb::check_launch("kick_kernel");
+    NB_CUDA_TRY(nb::launch_after(kick_kernel, nb::ceil_div(n, EW_THREADS), EW_THREADS, 0,
+                                 (cudaStream_t)stream, vx, vy, vz, vhx, vhy, vhz, ax, ay, az, n, dt));
+    return NB_OK;
 }
 
 nb_status nb_leapfrog_kick_kick_drift(nb_ctx* ctx, double* vx, double* vy, double* vz,
@@ -425,9 +428,9 @@ nb_status nb_leapfrog_kick_kick_drift(nb_ctx* ctx, double* vx, double* vy, doubl
     if (n == 0) return NB_OK;
     if (!vhx || !vhy || !vhz || !vx || !vy || !vz || !x || !y || !z || !ax || !ay || !az)
         return nb::set_error(NB_ERR_INVALID_ARG, "nb_leapfrog_kick_kick_drift: null pointer");
-    kick_kick_drift_kernel<<<nb::ceil_div(n, EW_THREADS), EW_THREADS, 0, (cudaStream_t)stream>>>(
-        vx, vy, vz, vhx, vhy, vhz, x, y, z, ax, ay, az, n, dt);
-    return nb::check_launch("kick_kick_drift_kernel");
+    NB_CUDA_TRY(nb::launch_after(kick_kick_drift_kernel, nb::ceil_div(n, EW_THREADS), EW_THREADS, 0,
+                                 (cudaStream_t)stream, vx, vy, vz, vhx, vhy, vhz, x, y, z, ax, ay, az, n, dt));
+    return NB_OK;
 }
 
 nb_status nb_energy(nb_ctx* ctx, const double* m, const double* x, const double* y,

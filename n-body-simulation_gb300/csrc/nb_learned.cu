@@ -900,6 +900,15 @@ constexpr int TR_BLOCK = 256;
 constexpr int TR_CHUNK = 64;
 constexpr int TR_ROW = 36;
 
+// Zeroes the gradient and the loss; the gradient kernel computes meanwhile (two memsets before it and
+// ordinary launches: 18.8 us for gradient and Adam at 8,192 rows, this way 13.7).
+__global__ void mlp_zero_kernel(float* __restrict__ grad, float* __restrict__ loss) {
+    nb_grid_wait();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < P_COUNT) grad[k] = 0.f;
+    if (k == P_COUNT) *loss = 0.f;
+}
+
 __global__ void __launch_bounds__(TR_BLOCK)
 mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
                 const float* __restrict__ Y, const uint32_t* __restrict__ idx, uint32_t n,
@@ -911,7 +920,8 @@ mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
     static_assert(NF == 8 && P_B1 % 4 == 0 && P_W2 % 4 == 0 && P_B2 % 4 == 0 && P_W3 % 4 == 0,
                   "16-byte weight rows");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int k = tid; k < P_COUNT; k += TR_BLOCK) w[k] = P[k];
+    // this part runs while the kernel before this one does: it reads past L1
+    for (int k = tid; k < P_COUNT; k += TR_BLOCK) w[k] = __ldcg(P + k);
     const int s = tid >> 2, c0 = (tid & 3) * 8;  // sample of the chunk, first column
     const int ti = tid >> 4, to = tid & 15;      // tile of W2's gradient
     float g2[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, g1 = 0.f, gx = 0.f, lsum = 0.f;
@@ -919,19 +929,19 @@ mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
     auto row4 = [&](int at) { return *reinterpret_cast<const float4*>(&w[at]); };
     for (uint32_t first = blockIdx.x * TR_CHUNK; first < n; first += gridDim.x * TR_CHUNK) {
         const bool in = first + s < n;
-        const uint32_t row = in ? (idx ? idx[first + s] : first + s) : 0u;
+        const uint32_t row = in ? (idx ? __ldcg(idx + first + s) : first + s) : 0u;
         const float4* xr = reinterpret_cast<const float4*>(X + (size_t)row * NF);
         const bool wide = ((uintptr_t)X & 15) == 0;
         float x[8];
         if (wide) {
-            const float4 a = xr[0], b = xr[1];
+            const float4 a = __ldcg(xr), b = __ldcg(xr + 1);
             x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
             x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
         } else {
 #pragma unroll
-            for (int i = 0; i < NF; ++i) x[i] = X[(size_t)row * NF + i];
+            for (int i = 0; i < NF; ++i) x[i] = __ldcg(X + (size_t)row * NF + i);
         }
-        const float y = in ? Y[row] : 0.f;
+        const float y = in ? __ldcg(Y + row) : 0.f;
         __syncthreads();  // the weights are there, the last chunk's sums are done
         float h1[8], h2[8], d[8];
 #pragma unroll
@@ -1020,6 +1030,7 @@ mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
             gx += sdo[lane] + sdo[lane + 32];
         }
     }
+    nb_grid_wait();  // the sums are zeroed; what is read above was final before that kernel started
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
@@ -1040,6 +1051,7 @@ mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
 __global__ void mlp_adam_kernel(float* __restrict__ P, float* __restrict__ M, float* __restrict__ V,
                                 const float* __restrict__ grad, float lr, float b1, float b2,
                                 float eps, float c1, float c2) {
+    nb_grid_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= P_COUNT) return;
     const float g = grad[k];
@@ -1114,12 +1126,12 @@ nb_status nb_mlp_loss_grad(nb_ctx* ctx, const float* params, const float* X, con
     if (!params || !X || !Y || !grad || !loss || n == 0)
         return nb::set_error(NB_ERR_INVALID_ARG, "nb_mlp_loss_grad: bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
-    NB_CUDA_TRY(cudaMemsetAsync(grad, 0, P_COUNT * sizeof(float), s));
-    NB_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(float), s));
+    NB_CUDA_TRY(nb::launch_after(mlp_zero_kernel, nb::ceil_div(P_COUNT + 1, 256), 256, 0, s, grad, loss));
     int blocks = nb::ceil_div(n, TR_CHUNK);
     if (blocks > ctx->sm_count * 2) blocks = ctx->sm_count * 2;
-    mlp_grad_kernel<<<blocks, TR_BLOCK, 0, s>>>(params, X, Y, idx, n, grad, loss);
-    return nb::check_launch("mlp_grad_kernel");
+    NB_CUDA_TRY(nb::launch_after(mlp_grad_kernel, blocks, TR_BLOCK, 0, s, params, X, Y, idx, n, grad,
+                                 loss));
+    return NB_OK;
 }
 
 nb_status nb_mlp_adam(nb_ctx* ctx, float* params, float* m, float* v, const float* grad,
@@ -1130,9 +1142,10 @@ nb_status nb_mlp_adam(nb_ctx* ctx, float* params, float* m, float* v, const floa
         return nb::set_error(NB_ERR_INVALID_ARG, "nb_mlp_adam: bad arguments");
     const float c1 = 1.f / (1.f - powf(beta1, (float)step));
     const float c2 = 1.f / (1.f - powf(beta2, (float)step));
-    mlp_adam_kernel<<<nb::ceil_div(P_COUNT, 256), 256, 0, (cudaStream_t)stream>>>(
-        params, m, v, grad, lr, beta1, beta2, eps, c1, c2);
-    return nb::check_launch("mlp_adam_kernel");
+    NB_CUDA_TRY(nb::launch_after(mlp_adam_kernel, nb::ceil_div(P_COUNT, 256), 256, 0,
+                                 (cudaStream_t)stream, params, m, v, grad, lr, beta1, beta2, eps, c1,
+                                 c2));
+    return NB_OK;
 }
 
 nb_status nb_mlp_predict(nb_ctx* ctx, const float* params, const float* X, uint32_t n,

@@ -130,6 +130,7 @@ naive_fix_kernel(const double* __restrict__ m, const double* __restrict__ x,
                  uint32_t n, const uint32_t* __restrict__ targets, uint32_t i_begin, uint32_t n_t,
                  double G, double eps2, uint32_t chunk, double* __restrict__ part,
                  const uint32_t* __restrict__ k_part, uint32_t k_words) {
+    nb_grid_wait();
     __shared__ nbfix::FixRec src[FX_THREADS];
     __shared__ nbfix::Eps2Table e2;
     const int K = nbfix::block_scale(x, y, z, n, k_part, k_words);
@@ -185,6 +186,7 @@ naive_fix_cluster_kernel(const double* __restrict__ m, const double* __restrict_
                          const uint32_t* __restrict__ targets, uint32_t i_begin, uint32_t n_t,
                          double G, double eps2, const uint32_t* __restrict__ k_part,
                          uint32_t k_words) {
+    nb_grid_wait();
     namespace cg = cooperative_groups;
     __shared__ nbfix::FixRec src[FXC_THREADS];
     __shared__ nbfix::Eps2Table e2;
@@ -242,6 +244,7 @@ __global__ void __launch_bounds__(32 * CC_WARPS)
 chunk_combine_kernel(const double* __restrict__ part, uint32_t chunks, uint32_t i_begin,
                      uint32_t i_end, double* __restrict__ ax, double* __restrict__ ay,
                      double* __restrict__ az) {
+    nb_grid_wait();
     __shared__ double sum[CC_WARPS][3][32];
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, n_t = i_end - i_begin;
     const uint32_t t = blockIdx.x * 32 + lane;
@@ -551,9 +554,10 @@ nb_status naive_fix(nb_ctx* ctx, const double* m, const double* x, const double*
     uint32_t k_words = 0;
     NB_TRY(nb::launch_scale(x, y, z, n, k_part, &k_words, stream));
     if (n <= FXC_MAX_N) {
-        naive_fix_cluster_kernel<<<nb::ceil_div(n_t, 32) * FXC_CTAS, FXC_THREADS, 0, stream>>>(
-            m, x, y, z, ax, ay, az, n, targets, i_begin, n_t, G, eps2, k_part, k_words);
-        return nb::check_launch("naive_fix_cluster_kernel");
+        NB_CUDA_TRY(nb::launch_after(naive_fix_cluster_kernel, nb::ceil_div(n_t, 32) * FXC_CTAS,
+                                     FXC_THREADS, 0, stream, m, x, y, z, ax, ay, az, n, targets,
+                                     i_begin, n_t, G, eps2, k_part, k_words));
+        return NB_OK;
     }
     const int blocks = nb::ceil_div(n_t, FX_THREADS);
     uint32_t chunks = (uint32_t)std::min<long long>(
@@ -578,14 +582,14 @@ nb_status naive_fix(nb_ctx* ctx, const double* m, const double* x, const double*
         NB_TRY(nb::scratch(ctx, NB_SCRATCH_NAIVE_DF, part_bytes, &base));
         part = (double*)base;
     }
-    naive_fix_kernel<<<dim3(blocks, chunks), FX_THREADS, 0, stream>>>(
-        m, x, y, z, ax, ay, az, n, targets, i_begin, n_t, G, eps2, chunk, part, k_part, k_words);
-    NB_TRY(nb::check_launch("naive_fix_kernel"));
+    NB_CUDA_TRY(nb::launch_after(naive_fix_kernel, dim3(blocks, chunks), FX_THREADS, 0, stream, m, x,
+                                 y, z, ax, ay, az, n, targets, i_begin, n_t, G, eps2, chunk, part,
+                                 k_part, k_words));
     if (chunks == 1) return NB_OK;
     const uint32_t first = targets != nullptr ? 0 : i_begin;
-    chunk_combine_kernel<<<nb::ceil_div(n_t, 32), 32 * CC_WARPS, 0, stream>>>(part, chunks, first,
-                                                                     first + n_t, ax, ay, az);
-    return nb::check_launch("chunk_combine_kernel");
+    NB_CUDA_TRY(nb::launch_after(chunk_combine_kernel, nb::ceil_div(n_t, 32), 32 * CC_WARPS, 0, stream,
+                                 part, chunks, first, first + n_t, ax, ay, az));
+    return NB_OK;
 }
 
 nb_status naive_dispatch(nb_ctx* ctx, const double* m, const double* x, const double* y,
