@@ -84,10 +84,22 @@ def ptr(t) -> int:
     return t.data_ptr()
 
 
+_torch_cuda = None  # (torch.cuda, its calls for the current device and a device's current stream)
+
+
 def stream_ptr(stream=None):
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    """Handle of `stream`, or of torch's current stream on the current device: read directly (0.2 us),
+    since making torch's Stream object for it takes 3 us of a call's 10."""
+    if stream is not None:
+        return stream.cuda_stream
+    global _torch_cuda
+    if _torch_cuda is None:
+        import torch
+        _torch_cuda = torch.cuda, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+    cuda, device, raw_stream = _torch_cuda
+    if not cuda.is_initialized():
+        cuda.init()
+    return raw_stream(device())
 
 
 class Context:
