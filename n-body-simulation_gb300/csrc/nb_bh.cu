@@ -24,6 +24,8 @@
 //     (deepest level first), the cells reaching past their chunk (at most one per level) by tiers
 //     of blocks over 96 chunks each; children summed in octant order 0..7
 //     (bit-identical to BarnesHutOctree.cpp:304-311), node records written with the sums.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "nb_aabb.cuh"
@@ -472,14 +474,15 @@ __global__ void emit_kernel(uint32_t n, const uint32_t* __restrict__ ids,
             mask, base, key0, key1, T);
 }
 
-// Steps 1 to 6 for small systems in one block, sharing the device functions above: the chain of
-// launches costs 135 us at 777 bodies and 167 at 4,096, this one 28 and 98. Bound by latency: one
-// block's barriers and dependent instructions. (Key, body) pairs sort bitonically (ties by body id:
+// Steps 1 to 6 for small systems in one block, sharing the device functions above. Bound by latency:
+// one block's barriers and dependent instructions. (Key, body) pairs sort bitonically (ties by body id:
 // the stable order) in registers, with exchanges by shuffle within a warp; the cells' ranges come
 // from the splits' levels and their minima over powers of two, a halving walk over bytes in shared
-// memory; with all exchanges through shared memory and searches over the keys 41 and 115 us. The
-// DFS numbering is a block scan.
-constexpr uint32_t SB_MAX_N = 4096;
+// memory; with all exchanges through shared memory and searches over the keys it took 41 us at 777
+// bodies, this way 28. The DFS numbering is a block scan. The whole build, this way against the chain
+// of launches: 57 / 84 us at 777 bodies, 84 / 94 at 2,048; at 2,500 it would be 116 / 97, which is
+// where the line is.
+constexpr uint32_t SB_MAX_N = 2048;
 
 constexpr int small_log2(uint32_t v) { return v <= 1 ? 0 : 1 + small_log2(v / 2); }
 template <uint32_t CAP>
@@ -1026,7 +1029,6 @@ __device__ void cell_records(const ComArgs& A, uint32_t idx) {
 // rounding of that quotient), and the spread of a single body is 0.
 struct NodeSums {
     double x, y, z, m, q;
-    uint32_t count;
 };
 
 __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32_t b) {
@@ -1076,7 +1078,7 @@ __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32
     if (A.records & NB_REC_DF) {
         A.df_terms[idx] = df_terms_of(rcx, rcy, rcz, ox, oy, oz, A.G * mb, q.gm, massive);
     }
-    NodeSums sums{cx, cy, cz, mb, 0.0, 1};
+    NodeSums sums{cx, cy, cz, mb, 0.0};
     if (A.records & NB_REC_LEARNED) {  // spread sums and the FP32 body copies of the policy
         const double rx = bx - ox, ry = by - oy, rz = bz - oz;
         sums.q = mb * (rx * rx + ry * ry + rz * rz);
@@ -1204,10 +1206,21 @@ constexpr size_t chunk_smem_bytes(bool learned) {
     return (size_t)(2 * CW + CM_LEVELS) * ((learned ? 5 : 4) * sizeof(double));
 }
 
-template <int CW, int CH_THREADS>
-__global__ void __launch_bounds__(CH_THREADS, 1024 / CH_THREADS)
-com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
+// The CTAS blocks of a chunk (one, or a cluster) share its leaves and the records of its cells; the
+// sums are kept and added in the first one's shared memory.
+template <int CW, int CH_THREADS, int CTAS>
+__device__ __forceinline__ void com_chunk(const ComArgs& A, uint2* up, uint32_t* up_count) {
     static_assert(CW == CH_THREADS, "one leaf and at most one local cell per thread");
+    namespace cg = cooperative_groups;
+    auto all_sync = [] {
+        if constexpr (CTAS > 1) cg::this_cluster().sync();
+        else __syncthreads();
+    };
+    auto first_of = [](auto* ptr) {  // the same object in the chunk's first block
+        if constexpr (CTAS > 1) return cg::this_cluster().map_shared_rank(ptr, 0);
+        else return ptr;
+    };
+    const uint32_t rank = CTAS > 1 ? blockIdx.x % CTAS : 0u, chunk = blockIdx.x / CTAS;
     constexpr int CH_NODES = 2 * CW + CM_LEVELS;  // nodes starting in a chunk, at most
     extern __shared__ __align__(16) unsigned char com_smem[];
     const bool learned = (A.records & NB_REC_LEARNED) != 0;
@@ -1222,118 +1235,152 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
     __shared__ int deepest;
     __shared__ uint32_t cnt[CM_LEVELS], off[CM_LEVELS], fill[CM_LEVELS];
     __shared__ uint32_t n_found, n_up;
-    const uint32_t tid = threadIdx.x, P = blockIdx.x * CW;
+    uint32_t nf = 0, my = 0, nkids = 0;
+    bool cell = false;
+    const uint32_t tid = threadIdx.x, P = chunk * CW;
     nb_grid_wait();
     const uint32_t Pend = min(P + (uint32_t)CW, A.n);
     const uint32_t d0 = A.base[P], d1 = A.base[Pend];
     if (tid < CM_LEVELS) cnt[tid] = fill[tid] = 0;
     if (tid == 0) n_found = n_up = 0;
     if (d1 - d0 > (uint32_t)CH_NODES) {  // a consistent tree never gets here
-        if (tid == 0) {
+        if (tid == 0 && rank == 0) {
             atomicOr(A.err, NB_DEVERR_DEPTH);
-            up_count[blockIdx.x] = 0;
+            up_count[chunk] = 0;
         }
         return;
     }
-    __syncthreads();
-    if (const uint32_t p = P + tid; p < Pend) {
+    all_sync();  // the first block's memory is there
+    if (const uint32_t p = P + tid * CTAS + rank; p < Pend) {
         const uint32_t idx = A.base[p] + __popcll(A.mask[p]), k = idx - d0;
         const NodeSums s = leaf_sums(A, idx, p, A.ids[p]);
-        sx[k] = s.x;
-        sy[k] = s.y;
-        sz[k] = s.z;
-        sm[k] = s.m;
-        if (learned) sq[k] = s.q;
+        first_of(sx)[k] = s.x;
+        first_of(sy)[k] = s.y;
+        first_of(sz)[k] = s.z;
+        first_of(sm)[k] = s.m;
+        if (learned) first_of(sq)[k] = s.q;
     }
-    for (uint32_t idx = d0 + tid; idx < d1; idx += CH_THREADS) {
-        if (A.node_body[idx] != NB_NONE) continue;  // a leaf
-        const int l = min((int)A.node_level[idx], CM_LEVELS - 1);
-        if (A.node_last[idx] >= Pend) {  // reaches past the chunk: for the next tier
-            const uint32_t g = atomicAdd(&n_up, 1u);
-            if (g < (uint32_t)CM_LEVELS)
-                up[(size_t)blockIdx.x * CM_LEVELS + g] = make_uint2(idx, (uint32_t)l);
-            else
-                atomicOr(A.err, NB_DEVERR_DEPTH);  // more than one per level: inconsistent
-            continue;
-        }
-        const uint32_t slot = atomicAdd(&n_found, 1u);
-        if (slot < (uint32_t)CW) {
-            found[slot] = (uint16_t)(idx - d0);
-            flev[slot] = (uint8_t)l;
-            atomicAdd(&cnt[l], 1u);
-        } else {
-            atomicOr(A.err, NB_DEVERR_DEPTH);  // a consistent tree never gets here
-        }
-    }
-    __syncthreads();
-    const uint32_t nf = min(n_found, (uint32_t)CW);
-    if (tid == 0) up_count[blockIdx.x] = min(n_up, (uint32_t)CM_LEVELS);
-    level_offsets(cnt, off, &deepest);
-    __syncthreads();
-    for (uint32_t k = tid; k < nf; k += CH_THREADS) {
-        const uint32_t l = flev[k];
-        order[off[l] + atomicAdd(&fill[l], 1u)] = found[k];
-    }
-    __syncthreads();
-    // this thread's cell: its children in octant order as slots, and the compacted visit-order child
-    // list the learned traversal reads
-    const bool cell = tid < nf;
-    const uint32_t my = cell ? order[tid] : 0u;
-    uint32_t nkids = 0;
-    if (cell) {
-        uint32_t* cl = A.children + (size_t)(d0 + my) * 8;
-        const uint4 c0 = reinterpret_cast<const uint4*>(cl)[0],
-                    c1 = reinterpret_cast<const uint4*>(cl)[1];
-        const uint32_t vs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-        uint32_t nch = 0;
-#pragma unroll
-        for (int t = 0; t < 8; ++t)
-            if (vs[t] != NB_NONE) cl[nch++] = vs[t];
-        for (uint32_t t = nch; t < 8; ++t) cl[t] = NB_NONE;
-#pragma unroll
-        for (int o = 0; o < 8; ++o) {  // the reference's octant order 0..7
-            const uint32_t ch = vs[nb_visit_of_octant(o)];
-            if (ch != NB_NONE)
-                kids[tid][nkids++] = (uint16_t)min(ch - d0, (uint32_t)CH_NODES - 1);
-        }
-    }
-    // deepest level first
-    for (int l = deepest; l >= 0; --l) {
-        const uint32_t c = cnt[l], o0 = off[l];
-        if (c == 0) continue;  // uniform across the block
-        if (tid >= o0 && tid < o0 + c) {
-            // the reference's sums start at 0.0: 0.0 + c is c, with -0.0 as +0.0
-            const uint32_t k0 = kids[tid][0];
-            NodeSums s{plus_zero(sx[k0]), plus_zero(sy[k0]), plus_zero(sz[k0]), plus_zero(sm[k0]),
-                       learned ? 0.0 + sq[k0] : 0.0, 0};
-            for (uint32_t i = 1; i < nkids; ++i) {
-                const uint32_t k = kids[tid][i];
-                s.x = __dadd_rn(s.x, sx[k]);
-                s.y = __dadd_rn(s.y, sy[k]);
-                s.z = __dadd_rn(s.z, sz[k]);
-                s.m = __dadd_rn(s.m, sm[k]);
-                if (learned) s.q += sq[k];
+    if constexpr (CTAS > 1) all_sync();
+    if (rank == 0) {
+        for (uint32_t idx = d0 + tid; idx < d1; idx += CH_THREADS) {
+            if (A.node_body[idx] != NB_NONE) continue;  // a leaf
+            const int l = min((int)A.node_level[idx], CM_LEVELS - 1);
+            if (A.node_last[idx] >= Pend) {  // reaches past the chunk: for the next tier
+                const uint32_t g = atomicAdd(&n_up, 1u);
+                if (g < (uint32_t)CM_LEVELS)
+                    up[(size_t)chunk * CM_LEVELS + g] = make_uint2(idx, (uint32_t)l);
+                else
+                    atomicOr(A.err, NB_DEVERR_DEPTH);  // more than one per level: inconsistent
+                continue;
             }
-            sx[my] = s.x;
-            sy[my] = s.y;
-            sz[my] = s.z;
-            sm[my] = s.m;
-            if (learned) sq[my] = s.q;
+            const uint32_t slot = atomicAdd(&n_found, 1u);
+            if (slot < (uint32_t)CW) {
+                found[slot] = (uint16_t)(idx - d0);
+                flev[slot] = (uint8_t)l;
+                atomicAdd(&cnt[l], 1u);
+            } else {
+                atomicOr(A.err, NB_DEVERR_DEPTH);  // a consistent tree never gets here
+            }
         }
         __syncthreads();
+        nf = min(n_found, (uint32_t)CW);
+        if (tid == 0) n_found = nf;  // for the other blocks
+        if (tid == 0) up_count[chunk] = min(n_up, (uint32_t)CM_LEVELS);
+        level_offsets(cnt, off, &deepest);
+        __syncthreads();
+        for (uint32_t k = tid; k < nf; k += CH_THREADS) {
+            const uint32_t l = flev[k];
+            order[off[l] + atomicAdd(&fill[l], 1u)] = found[k];
+        }
+        __syncthreads();
+        // this thread's cell: its children in octant order as slots, and the compacted visit-order child
+        // list the learned traversal reads
+        cell = tid < nf;
+        my = cell ? order[tid] : 0u;
+        if (cell) {
+            uint32_t* cl = A.children + (size_t)(d0 + my) * 8;
+            const uint4 c0 = reinterpret_cast<const uint4*>(cl)[0],
+                        c1 = reinterpret_cast<const uint4*>(cl)[1];
+            const uint32_t vs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+            uint32_t nch = 0;
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+                if (vs[t] != NB_NONE) cl[nch++] = vs[t];
+            for (uint32_t t = nch; t < 8; ++t) cl[t] = NB_NONE;
+#pragma unroll
+            for (int o = 0; o < 8; ++o) {  // the reference's octant order 0..7
+                const uint32_t ch = vs[nb_visit_of_octant(o)];
+                if (ch != NB_NONE)
+                    kids[tid][nkids++] = (uint16_t)min(ch - d0, (uint32_t)CH_NODES - 1);
+            }
+        }
+        // deepest level first, four lanes per cell (x, y, z and mass; the first one the spread too), a
+        // cell's children read before the adds: a thread per cell with its children one after the other
+        // took 39 us instead of 31 at 1,024 bodies, 264 instead of 242 at 1,048,576 (the whole phase)
+        for (uint32_t t = nkids; t < 8; ++t) kids[tid][t] = 0xffff;
+        __syncthreads();
+        for (int l = deepest; l >= 0; --l) {
+            const uint32_t c = cnt[l], o0 = off[l];
+            if (c == 0) continue;  // uniform across the block
+            for (uint32_t pos = o0 + (tid >> 2); pos < o0 + c; pos += CH_THREADS / 4) {
+                const uint4 kk = *reinterpret_cast<const uint4*>(kids[pos]);
+                const uint32_t kw[4] = {kk.x, kk.y, kk.z, kk.w};
+                auto add_up = [&](double* sv) {
+                    double v[8];
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) {
+                        const uint32_t k = (kw[t >> 1] >> (16 * (t & 1))) & 0xffffu;
+                        v[t] = k != 0xffffu ? sv[k] : 0.0;
+                    }
+                    double sum = plus_zero(v[0]);  // 0.0 + v[0]
+#pragma unroll
+                    for (int t = 1; t < 8; ++t) {
+                        if (((kw[t >> 1] >> (16 * (t & 1))) & 0xffffu) == 0xffffu) break;
+                        sum = __dadd_rn(sum, v[t]);
+                    }
+                    sv[order[pos]] = sum;
+                };
+                add_up(sx + (tid & 3) * CH_NODES);
+                if (learned && (tid & 3) == 0) add_up(sq);
+            }
+            __syncthreads();
+        }
+    }
+    if constexpr (CTAS > 1) {
+        all_sync();  // every sum is final
+        nf = *first_of(&n_found);
+        cell = tid * CTAS + rank < nf;
+        my = cell ? first_of(order)[tid * CTAS + rank] : 0u;
     }
     if (cell) {
         const uint32_t idx = d0 + my;
-        A.comx[idx] = sx[my];
-        A.comy[idx] = sy[my];
-        A.comz[idx] = sz[my];
-        A.mass[idx] = sm[my];
-        if (learned) A.q[idx] = sq[my];
+        const double cx = first_of(sx)[my], cy = first_of(sy)[my], cz = first_of(sz)[my],
+                     cm = first_of(sm)[my], cq = learned ? first_of(sq)[my] : 0.0;
+        A.comx[idx] = cx;
+        A.comy[idx] = cy;
+        A.comz[idx] = cz;
+        A.mass[idx] = cm;
+        if (learned) A.q[idx] = cq;
         const uint32_t count = A.node_last[idx] - A.node_first[idx] + 1;
         A.node_count[idx] = count;
-        write_records(A, idx, sx[my], sy[my], sz[my], sm[my], learned ? sq[my] : 0.0, count,
-                      A.node_level[idx], A.node_skip[idx], NB_NONE);
+        write_records(A, idx, cx, cy, cz, cm, cq, count, A.node_level[idx], A.node_skip[idx], NB_NONE);
     }
+    if constexpr (CTAS > 1) all_sync();  // the first block's memory stays until all have read it
+}
+
+template <int CW, int CH_THREADS>
+__global__ void __launch_bounds__(CH_THREADS, 1024 / CH_THREADS)
+com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
+    com_chunk<CW, CH_THREADS, 1>(A, up, up_count);
+}
+
+// The whole of a system of 513 to CL_N bodies as one chunk of a cluster. In one block the leaves and
+// the cells' records took 33,000 of 63,000 cycles at 777 bodies (one SM's FP64 pipe); the cluster takes
+// 5 to 8 us off at 777 to 1,024 bodies, nothing at 500, and costs 3 at 100.
+constexpr int CL_N = 1024, CL_CTAS = 8;
+__global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_N, 1)
+com_cluster_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
+    com_chunk<CL_N, CL_N, CL_CTAS>(A, up, up_count);
 }
 
 // Tier of `span` sorted positions per block: the cells listed by the CM_FAN lower-tier chunks of the
@@ -1518,10 +1565,10 @@ nb_status allow_smem(K kernel, size_t bytes) {
 }
 nb_status build_prepare() {
     NB_TRY(allow_smem(build_small_kernel<1024, 1024>, small_smem_bytes<1024>()));
-    NB_TRY(allow_smem(build_small_kernel<2048, 1024>, small_smem_bytes<2048>()));
     NB_TRY(allow_smem(build_small_kernel<SB_MAX_N, 1024>, small_smem_bytes<SB_MAX_N>()));
     NB_TRY(allow_smem(com_tier_kernel, tier_smem_bytes(true)));
-    return allow_smem(com_chunk_kernel<1024, 1024>, chunk_smem_bytes<1024>(true));
+    NB_TRY(allow_smem(com_chunk_kernel<512, 512>, chunk_smem_bytes<512>(true)));
+    return allow_smem(com_cluster_kernel, chunk_smem_bytes<CL_N>(true));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1718,8 +1765,6 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
             NB_CUDA_TRY(go(build_small_kernel<512, 512>, 512, small_smem_bytes<512>()));
         else if (n <= 1024)
             NB_CUDA_TRY(go(build_small_kernel<1024, 1024>, 1024, small_smem_bytes<1024>()));
-        else if (n <= 2048)
-            NB_CUDA_TRY(go(build_small_kernel<2048, 1024>, 1024, small_smem_bytes<2048>()));
         else
             NB_CUDA_TRY(go(build_small_kernel<SB_MAX_N, 1024>, 1024, small_smem_bytes<SB_MAX_N>()));
     } else {
@@ -1796,15 +1841,18 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     A.sorted4lo = t->sorted4lo;
     {
         const bool learned = (t->records & NB_REC_LEARNED) != 0;
-        // one chunk for the smallest systems (no tier pass), else 256 positions per chunk
-        const uint32_t cw = n <= 1024 ? 1024 : 256;
+        // one chunk for the smallest systems (no tier pass: 4 chunks and a tier cost 9 us more at 300
+        // bodies and the same at 777), else 256 positions per chunk
+        const uint32_t cw = n <= 512 ? 512 : n <= (uint32_t)CL_N ? CL_N : 256;
         uint32_t chunks = (uint32_t)nb::ceil_div(n, cw);
-        auto go = [&](auto kernel, size_t smem) {
-            return nb::launch_after(kernel, chunks, cw, smem, s, A, t->tier_cells[0],
+        auto go = [&](auto kernel, uint32_t blocks, size_t smem) {
+            return nb::launch_after(kernel, blocks, cw, smem, s, A, t->tier_cells[0],
                                     t->tier_count[0]);
         };
-        NB_CUDA_TRY(cw == 1024 ? go(com_chunk_kernel<1024, 1024>, chunk_smem_bytes<1024>(learned))
-                               : go(com_chunk_kernel<256, 256>, chunk_smem_bytes<256>(learned)));
+        NB_CUDA_TRY(cw == CL_N ? go(com_cluster_kernel, CL_CTAS, chunk_smem_bytes<CL_N>(learned))
+                    : cw == 512 ? go(com_chunk_kernel<512, 512>, 1, chunk_smem_bytes<512>(learned))
+                                : go(com_chunk_kernel<256, 256>, chunks,
+                                     chunk_smem_bytes<256>(learned)));
         uint64_t span = cw;
         int in = 0;
         for (int tier = 1; tier <= CM_TIERS && chunks > 1; ++tier) {

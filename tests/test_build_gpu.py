@@ -1,6 +1,6 @@
-"""Octree build at the edges of its kernels -- the one-block build (up to 4,096 bodies, two sizes of
-it), the centre-of-mass chunks (1,024 positions, or 256 and tiers of 96 chunks) -- and of its
-division-free quotients: every cell equal to the oracle's, bit for bit, and the accelerations of the
+"""Octree build at the edges of its kernels -- the one-block build (up to 2,048 bodies, three sizes of
+it), the centre-of-mass chunks (one of up to 512 or 1,024 positions, or 256 and tiers of 96 chunks) --
+and of its division-free quotients: every cell equal to the oracle's, bit for bit, and the accelerations of the
 IEEE traversal (which read the quotients) too."""
 
 import numpy as np
