@@ -304,7 +304,7 @@ typedef struct nb_bh_ref_layout {
 } nb_bh_ref_layout;
 
 nb_status nb_bh_params_default(nb_bh_params* out);
-/* Allocates a tree for up to n_max bodies (device memory, ~0.5 KB per body). */
+/* Allocates a tree for up to n_max bodies (device memory, ~0.65 KB per body). */
 nb_status nb_bh_tree_create(nb_ctx* ctx, uint32_t n_max, const nb_bh_params* params,
                             nb_bh_tree** out);
 nb_status nb_bh_tree_destroy(nb_bh_tree* tree);
@@ -313,8 +313,9 @@ nb_status nb_bh_tree_set_theta(nb_bh_tree* tree, double theta);
 /* Node records later builds compute (no reference counterpart: the reference keeps only the
  * sums). The FP32 records (centres relative to the box centre, G*mass, edge^2) are always built;
  * further sets by bit:
- *   NB_REC_FP64    FP64 centres (the IEEE quotients of the reference's sums), masses, edges: the
- *                  per-body rule in NB_F64_IEEE, NB_F64 and NB_DF64, the FP64 group rule,
+ *   NB_REC_FP64    FP64 centres (the IEEE quotients of the reference's sums), masses, edges, and the
+ *                  same in fixed point for the NB_F64 monopoles: the per-body rule in
+ *                  NB_F64_IEEE, NB_F64 and NB_DF64, the FP64 group rule,
  *                  nb_bh_count_interactions and nb_bh_generate_pairs;
  *   NB_REC_DF      the further FP32 terms of centres and G*mass (exact triple-floats): NB_DF64;
  *   NB_REC_LEARNED per-node spread, count and first body, FP32 body copies in tree order:
