@@ -1330,7 +1330,7 @@ __device__ __forceinline__ void com_chunk(const ComArgs& A, uint2* up, uint32_t*
 #pragma unroll
                     for (int t = 0; t < 8; ++t) {
                         const uint32_t k = (kw[t >> 1] >> (16 * (t & 1))) & 0xffffu;
-                        v[t] = k != 0xffffu ? sv[k] : 0.0;
+    v[t] = sv[min(k, (uint32_t)CH_NODES - 1)];  // unused where there is no child
                     }
                     double sum = plus_zero(v[0]);  // 0.0 + v[0]
 #pragma unroll
@@ -1392,8 +1392,9 @@ com_cluster_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
 // (tier_slot finds a child's place in the block's list; what it names is checked, so that whatever an
 // earlier launch left there does not matter), and four lanes take a cell's four components. With the
 // children's sums read from global memory level by level, as for more cells than that, a level took
-// 5,300 cycles; this way the whole centre-of-mass phase takes 49 us instead of 64 at 16,411 bodies (one
-// tier), 80 instead of 106 at 131,101 (two).
+// 5,300 cycles and the kernel 66,000 at 16,411 bodies (9 levels, 201 cells); this way 1,300 and 35,000:
+// children packed to the front and read without branches (2,000 a level otherwise), the records'
+// other inputs requested before the levels.
 constexpr int CM_KEPT = 512;
 constexpr size_t tier_smem_bytes(bool learned) {
     return (size_t)CM_TIER_MAX * sizeof(uint32_t) +
@@ -1478,7 +1479,8 @@ com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
     // the children: their places in the list, or their sums
     constexpr int AHEAD = 4;
     double* const sums[5] = {A.comx, A.comy, A.comz, A.mass, A.q};
-    for (uint32_t e0 = tid; e0 < nf * 8; e0 += CC_THREADS * AHEAD) {
+    // a cell's eight children by eight neighbouring lanes, the ones that exist packed to the front
+    for (uint32_t e0 = tid; e0 - (tid & 31) < nf * 8; e0 += CC_THREADS * AHEAD) {
         uint32_t ch[AHEAD], at[AHEAD];
         double v[AHEAD][5];
 #pragma unroll
@@ -1498,16 +1500,19 @@ com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
 #pragma unroll
         for (int r = 0; r < AHEAD; ++r) {
             const uint32_t e = e0 + r * CC_THREADS;
+            const uint32_t group = tid & 24u;  // the cell's first lane
+            const uint32_t have = (__ballot_sync(0xffffffffu, ch[r] != NB_NONE) >> group) & 0xffu;
             if (e >= nf * 8) continue;
-            if (ch[r] == NB_NONE) {
-                kid[e] = (uint16_t)KID_NONE;
-            } else if (at[r] < nf && nodes[at[r]] == ch[r]) {
-                kid[e] = (uint16_t)at[r];
+            if ((e & 7) >= (uint32_t)__popc(have)) kid[e] = (uint16_t)KID_NONE;
+            if (ch[r] == NB_NONE) continue;
+            const uint32_t to = (e & ~7u) + __popc(have & ((1u << (e & 7)) - 1u));
+            if (at[r] < nf && nodes[at[r]] == ch[r]) {
+                kid[to] = (uint16_t)at[r];
             } else {
-                kid[e] = (uint16_t)KID_OUTSIDE;
+                kid[to] = (uint16_t)KID_OUTSIDE;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) val[c * (CM_KEPT * 8) + e] = v[r][c];
-                if (learned) val[4 * (CM_KEPT * 8) + e] = v[r][4];
+                for (int c = 0; c < 4; ++c) val[c * (CM_KEPT * 8) + to] = v[r][c];
+                if (learned) val[4 * (CM_KEPT * 8) + to] = v[r][4];
             }
         }
     }
@@ -1522,14 +1527,27 @@ com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
 #pragma unroll
         for (int o = 0; o < 8; ++o) {
             k[o] = (kw[o >> 1] >> (16 * (o & 1))) & 0xffffu;
-            v[o] = k[o] < (uint32_t)CM_KEPT ? kc[k[o]] : (k[o] == KID_OUTSIDE ? vc[o] : 0.0);
+            const double* const from = k[o] < (uint32_t)CM_KEPT ? kc + k[o] : vc + o;
+            v[o] = *from;  // unused where there is no child
         }
         double sum = 0.0;
 #pragma unroll
-        for (int o = 0; o < 8; ++o)
-            if (k[o] != KID_NONE) sum = __dadd_rn(sum, v[o]);  // absent children add nothing
+        for (int o = 0; o < 8; ++o) {
+            if (k[o] == KID_NONE) break;  // absent children add nothing
+            sum = __dadd_rn(sum, v[o]);
+        }
         kept[comp * CM_KEPT + pos] = sum;
     };
+    // what this thread's record needs besides the sums, requested before the levels
+    static_assert(CM_KEPT <= CC_THREADS, "one record per thread");
+    uint32_t idx = NB_NONE, pos0 = 0, pos1 = 0, skip = 0, level = 0;
+    if (tid < nf) {
+        idx = nodes[tid];
+        pos0 = A.node_first[idx];
+        pos1 = A.node_last[idx];
+        skip = A.node_skip[idx];
+        level = A.node_level[idx];
+    }
     for (int l = deepest; l >= 0; --l) {
         const uint32_t c = cnt[l], o0 = off[l];
         if (c == 0) continue;  // uniform across the block
@@ -1539,8 +1557,8 @@ com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
         }
         __syncthreads();
     }
-    for (uint32_t k = tid; k < nf; k += CC_THREADS) {
-        const uint32_t idx = nodes[k];
+    if (idx != NB_NONE) {
+        const uint32_t k = tid, count = pos1 - pos0 + 1;
         const double sx = kept[k], sy = kept[CM_KEPT + k], sz = kept[2 * CM_KEPT + k],
                      sm = kept[3 * CM_KEPT + k], sq = learned ? kept[4 * CM_KEPT + k] : 0.0;
         A.comx[idx] = sx;
@@ -1548,11 +1566,9 @@ com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
         A.comz[idx] = sz;
         A.mass[idx] = sm;
         if (learned) A.q[idx] = sq;
-        const uint32_t count = A.node_last[idx] - A.node_first[idx] + 1;
         A.node_count[idx] = count;
         compact_children(A, idx);
-        write_records(A, idx, sx, sy, sz, sm, sq, count, A.node_level[idx], A.node_skip[idx],
-                      NB_NONE);
+        write_records(A, idx, sx, sy, sz, sm, sq, count, (int)level, skip, NB_NONE);
     }
 }
 
