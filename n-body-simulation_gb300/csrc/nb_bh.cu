@@ -1114,7 +1114,8 @@ __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32
 //    Bound: per level a barrier and a chain of FP64 additions (68 cycles each) in the reference's
 //    order. Against a leaf kernel and level sums through L2 by blocks of 4,096 positions
 //    (~1,200 cycles per level): 777 bodies 53 -> 35 us, 16,411 127 -> 63, 131,101 145 -> 104,
-//    1,048,576 332 -> 309.
+//    1,048,576 332 -> 309; with four lanes per cell, the cluster and the tiers from shared memory
+//    25, 43, 72 and 242 (the whole phase).
 //  * com_tier_kernel: one block per span of CM_FAN lower-tier chunks, same scheme on the listed
 //    cells.
 constexpr int CW_MIN = 256;                       // sorted positions per chunk, at least
