@@ -170,7 +170,9 @@ cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();  // reported here, not by a later check_launch
+    return e;
 }
 }  // namespace nb
 
