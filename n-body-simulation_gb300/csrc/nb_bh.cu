@@ -18,8 +18,8 @@
 // What later launches want zeroed or filled is written by earlier ones (keys: the sort's counters,
 // second key words and level masks; splits: the child lists), the digit offsets are summed by the
 // sort's passes and the node counts by the scan: 18 launches, where separate ones took 26 and 22 us
-// more at 16,411 bodies. Each launch of the chain may start while the one before it ends (nb_grid_wait):
-// 122 us for that build instead of 162.
+// more at 16,411 bodies. Each launch of the chain may start while the one before it ends
+// (nb_grid_wait): 122 us for that build instead of 162.
 //  7. bottom-up centre of mass: leaves and cells by blocks over chunks of 256 sorted positions
 //     (deepest level first), the cells reaching past their chunk (at most one per level) by tiers
 //     of blocks over 96 chunks each; children summed in octant order 0..7
@@ -474,14 +474,14 @@ __global__ void emit_kernel(uint32_t n, const uint32_t* __restrict__ ids,
             mask, base, key0, key1, T);
 }
 
-// Steps 1 to 6 for small systems in one block, sharing the device functions above. Bound by latency:
-// one block's barriers and dependent instructions. (Key, body) pairs sort bitonically (ties by body id:
-// the stable order) in registers, with exchanges by shuffle within a warp; the cells' ranges come
-// from the splits' levels and their minima over powers of two, a halving walk over bytes in shared
-// memory; with all exchanges through shared memory and searches over the keys it took 41 us at 777
-// bodies, this way 28. The DFS numbering is a block scan. The whole build, this way against the chain
-// of launches: 57 / 84 us at 777 bodies, 84 / 94 at 2,048; at 2,500 it would be 116 / 97, which is
-// where the line is.
+// Steps 1 to 6 for small systems in one block, sharing the device functions above. Bound by
+// latency: one block's barriers and dependent instructions. (Key, body) pairs sort bitonically
+// (ties by body id: the stable order) in registers, with exchanges by shuffle within a warp; the
+// cells' ranges come from the splits' levels and their minima over powers of two, a halving walk
+// over bytes in shared memory; with all exchanges through shared memory and searches over the keys
+// it took 41 us at 777 bodies, this way 28. The DFS numbering is a block scan. The whole build,
+// this way against the chain of launches: 57 / 84 us at 777 bodies, 84 / 94 at 2,048; at 2,500 it
+// would be 116 / 97, which is where the line is.
 constexpr uint32_t SB_MAX_N = 2048;
 
 constexpr int small_log2(uint32_t v) { return v <= 1 ? 0 : 1 + small_log2(v / 2); }
@@ -595,8 +595,8 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
         if (lane == 0 && !quantized) grid_s = fixed_grid(sbox);
     }
     __syncthreads();
-    // (key, body) number e = tid * PER + h in registers; exchanges within a thread, by shuffles within
-    // a warp, and through shared memory beyond
+    // (key, body) number e = tid * PER + h in registers; exchanges within a thread, by shuffles
+    // within a warp, and through shared memory beyond
     uint64_t key[PER];
     uint32_t id[PER];
 #pragma unroll
@@ -674,9 +674,9 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
     for (uint32_t p = tid; p < n; p += THREADS)
         fix_run(p, x, y, z, n, sbox, key0, key1, ids, err, quantized);
     __syncthreads();
-    // the splits' levels and their minima over powers of two, then the cells' ranges: a cell of level
-    // L reaches from its split as far as no split is below L, and the split whose left side has none
-    // at L stands for the cell (split_at's rules)
+    // the splits' levels and their minima over powers of two, then the cells' ranges: a cell of
+    // level L reaches from its split as far as no split is below L, and the split whose left side
+    // has none at L stands for the cell (split_at's rules)
     const int log = __ffs((int)m) - 1;
     for (uint32_t p = tid; p < m; p += THREADS) {
         int L = 0;  // past the last split: below or at every level, never crossed
@@ -795,11 +795,11 @@ __device__ __forceinline__ int biased_exp(double v) {
 
 // RN(c / m) for the rounded product c = RN(x * m) of a leaf (its centre-of-mass numerator over its
 // mass), without a division: c / m = x - err / m with err = x * m - c, the rounding error of the
-// product, exact in one FMA and at most half a unit in c's last place, so c / m lies within one unit
-// of x and rounds to x or to its neighbour on err's side. Which of them is decided by comparing
-// |err| 2^(53 - e(x)) with m (beyond half a unit; a tie goes to the even one), both positive normal
-// numbers, as integers. The IEEE division remains for x a power of two (whose units differ on its
-// two sides), subnormal or extreme values, and masses that are not positive.
+// product, exact in one FMA and at most half a unit in c's last place, so c / m lies within one
+// unit of x and rounds to x or to its neighbour on err's side. Which of them is decided by
+// comparing |err| 2^(53 - e(x)) with m (beyond half a unit; a tie goes to the even one), both
+// positive normal numbers, as integers. The IEEE division remains for x a power of two (whose units
+// differ on its two sides), subnormal or extreme values, and masses that are not positive.
 __device__ __forceinline__ double leaf_quotient(double x, double m, double c) {
     const long long xb = __double_as_longlong(x);
     const int ex = biased_exp(x), em = biased_exp(m), ec = biased_exp(c);
@@ -1106,11 +1106,11 @@ __device__ NodeSums leaf_sums(const ComArgs& A, uint32_t idx, uint32_t p, uint32
 // the rest up again, until one block spans all bodies. Every sum has its children's sums final
 // before it starts (kernel order, then levels deepest first within a block), so no thread waits
 // on another, and the FP64 work is spread over all SMs at every tier.
-//  * com_chunk_kernel: one block per chunk. Its leaves' sums go to shared memory (and, like all sums
-//    and records, to global memory), the local cells are sorted by level, each thread keeps its
-//    cells' children as slots of the shared sums, and the levels are summed from there; the cells'
-//    records follow in one sweep (FP64 work with full warps: on this part an FP64 warp instruction
-//    costs the FP64 pipe the same time however few of its lanes are active).
+//  * com_chunk_kernel: one block per chunk. Its leaves' sums go to shared memory (and, like all
+//    sums and records, to global memory), the local cells are sorted by level, each thread keeps
+//    its cells' children as slots of the shared sums, and the levels are summed from there; the
+//    cells' records follow in one sweep (FP64 work with full warps: on this part an FP64 warp
+//    instruction costs the FP64 pipe the same time however few of its lanes are active).
 //    Bound: per level a barrier and a chain of FP64 additions (68 cycles each) in the reference's
 //    order. Against a leaf kernel and level sums through L2 by blocks of 4,096 positions
 //    (~1,200 cycles per level): 777 bodies 53 -> 35 us, 16,411 127 -> 63, 131,101 145 -> 104,
@@ -1294,8 +1294,8 @@ __device__ __forceinline__ void com_chunk(const ComArgs& A, uint2* up, uint32_t*
             order[off[l] + atomicAdd(&fill[l], 1u)] = found[k];
         }
         __syncthreads();
-        // this thread's cell: its children in octant order as slots, and the compacted visit-order child
-        // list the learned traversal reads
+        // this thread's cell: its children in octant order as slots, and the compacted visit-order
+        // child list the learned traversal reads
         cell = tid < nf;
         my = cell ? order[tid] : 0u;
         if (cell) {
@@ -1315,9 +1315,10 @@ __device__ __forceinline__ void com_chunk(const ComArgs& A, uint2* up, uint32_t*
                     kids[tid][nkids++] = (uint16_t)min(ch - d0, (uint32_t)CH_NODES - 1);
             }
         }
-        // deepest level first, four lanes per cell (x, y, z and mass; the first one the spread too), a
-        // cell's children read before the adds: a thread per cell with its children one after the other
-        // took 39 us instead of 31 at 1,024 bodies, 264 instead of 242 at 1,048,576 (the whole phase)
+        // deepest level first, four lanes per cell (x, y, z and mass; the first one the spread
+        // too), a cell's children read before the adds: a thread per cell with its children one
+        // after the other took 39 us instead of 31 at 1,024 bodies, 264 instead of 242 at 1,048,576
+        // (the whole phase)
         for (uint32_t t = nkids; t < 8; ++t) kids[tid][t] = 0xffff;
         __syncthreads();
         for (int l = deepest; l >= 0; --l) {
@@ -1375,27 +1376,27 @@ com_chunk_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
     com_chunk<CW, CH_THREADS, 1>(A, up, up_count);
 }
 
-// The whole of a system of 513 to CL_N bodies as one chunk of a cluster. In one block the leaves and
-// the cells' records took 33,000 of 63,000 cycles at 777 bodies (one SM's FP64 pipe); the cluster takes
-// 5 to 8 us off at 777 to 1,024 bodies, nothing at 500, and costs 3 at 100.
+// The whole of a system of 513 to CL_N bodies as one chunk of a cluster. In one block the leaves
+// and the cells' records took 33,000 of 63,000 cycles at 777 bodies (one SM's FP64 pipe); the
+// cluster takes 5 to 8 us off at 777 to 1,024 bodies, nothing at 500, and costs 3 at 100.
 constexpr int CL_N = 1024, CL_CTAS = 8;
 __global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_N, 1)
 com_cluster_kernel(ComArgs A, uint2* up, uint32_t* up_count) {
     com_chunk<CL_N, CL_N, CL_CTAS>(A, up, up_count);
 }
 
-// Tier of `span` sorted positions per block: the cells listed by the CM_FAN lower-tier chunks of the
-// span (in[c * CM_LEVELS + k], k < in_count[c]) that end inside it are summed here; the others go to
-// up[] for the next tier (up == nullptr: the last tier, whose single block spans all bodies).
-// Bound by latency: a block has a few hundred cells over 8 to 12 levels and a level waits for the one
-// below. Up to CM_KEPT cells therefore sum from shared memory: all children outside the tier, which
-// are final, are read ahead of the first level, the sums of the tier's own cells stay in shared memory
-// (tier_slot finds a child's place in the block's list; what it names is checked, so that whatever an
-// earlier launch left there does not matter), and four lanes take a cell's four components. With the
-// children's sums read from global memory level by level, as for more cells than that, a level took
-// 5,300 cycles and the kernel 66,000 at 16,411 bodies (9 levels, 201 cells); this way 1,300 and 35,000:
-// children packed to the front and read without branches (2,000 a level otherwise), the records'
-// other inputs requested before the levels.
+// Tier of `span` sorted positions per block: the cells listed by the CM_FAN lower-tier chunks of
+// the span (in[c * CM_LEVELS + k], k < in_count[c]) that end inside it are summed here; the others
+// go to up[] for the next tier (up == nullptr: the last tier, whose single block spans all bodies).
+// Bound by latency: a block has a few hundred cells over 8 to 12 levels and a level waits for the
+// one below. Up to CM_KEPT cells therefore sum from shared memory: all children outside the tier,
+// which are final, are read ahead of the first level, the sums of the tier's own cells stay in
+// shared memory (tier_slot finds a child's place in the block's list; what it names is checked, so
+// that whatever an earlier launch left there does not matter), and four lanes take a cell's four
+// components. With the children's sums read from global memory level by level, as for more cells
+// than that, a level took 5,300 cycles and the kernel 66,000 at 16,411 bodies (9 levels, 201
+// cells); this way 1,300 and 35,000: children packed to the front and read without branches (2,000
+// a level otherwise), the records' other inputs requested before the levels.
 constexpr int CM_KEPT = 512;
 constexpr size_t tier_smem_bytes(bool learned) {
     return (size_t)CM_TIER_MAX * sizeof(uint32_t) +
@@ -1573,7 +1574,8 @@ com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
     }
 }
 
-// The kernels whose dynamic shared memory is above the default limit (before any capture of a build).
+// The kernels whose dynamic shared memory is above the default limit (before any capture of a
+// build).
 template <typename K>
 nb_status allow_smem(K kernel, size_t bytes) {
     NB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1858,8 +1860,8 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     A.sorted4lo = t->sorted4lo;
     {
         const bool learned = (t->records & NB_REC_LEARNED) != 0;
-        // one chunk for the smallest systems (no tier pass: 4 chunks and a tier cost 9 us more at 300
-        // bodies and the same at 777), else 256 positions per chunk
+        // one chunk for the smallest systems (no tier pass: 4 chunks and a tier cost 9 us more at
+        // 300 bodies and the same at 777), else 256 positions per chunk
         const uint32_t cw = n <= 512 ? 512 : n <= (uint32_t)CL_N ? CL_N : 256;
         uint32_t chunks = (uint32_t)nb::ceil_div(n, cw);
         auto go = [&](auto kernel, uint32_t blocks, size_t smem) {

@@ -30,7 +30,8 @@ struct __align__(16) NodeRec32 {
     uint32_t skip, body, level;
 };
 
-// Further FP32 terms of rec32's centre (with them a triple-float: exact) and G*mass (a double-float).
+// Further FP32 terms of rec32's centre (with them a triple-float: exact) and G*mass (a
+// double-float).
 struct __align__(32) DfTerms {
     float mx, my, mz, gl;  // second terms of the centre and of G * mass
     float lx, ly, lz, pad;  // third terms of the centre

@@ -223,11 +223,11 @@ __device__ __forceinline__ float margin_floor(float th2, float edge) {
 // FP32 error bound of d^2 with positions rounded relative to the box centre (|c-a|, |p-a| <=
 // E/2 per axis, u = 2^-24): |d2f - d2| <= u d^2 (2*sqrt(3) E/d + 5) + 3 u^2 E^2; the test below
 // widens it by 4x (the last term to 4 u^2 E^2: it decides only where d2f is far below u^2 E^2, when
-// one axis resolves less than the others) and adds the roundings of edge^2 and theta^2*d2f. Accumulation order per body is the
-// reference's DFS order, so MODE IEEE64 stays bit-identical. Warps take groups of 32 sorted
-// positions; with `order` != nullptr the bodies of the positions come from it (the previous
-// walk's lengths regrouped within windows, regroup_kernel) instead of from ids. Each body's
-// accepted-cell count goes to walk_len[body].
+// one axis resolves less than the others) and adds the roundings of edge^2 and theta^2*d2f.
+// Accumulation order per body is the reference's DFS order, so MODE IEEE64 stays bit-identical.
+// Warps take groups of 32 sorted positions; with `order` != nullptr the bodies of the positions
+// come from it (the previous walk's lengths regrouped within windows, regroup_kernel) instead of
+// from ids. Each body's accepted-cell count goes to walk_len[body].
 __global__ void __launch_bounds__(TR_THREADS)
 bh_theta_lane_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __restrict__ rec64,
                      const uint32_t* __restrict__ info, const uint32_t* __restrict__ ids,
@@ -570,8 +570,8 @@ regroup_kernel(const uint32_t* __restrict__ ids, const uint32_t* __restrict__ wa
     if (p < n) order[p] = ids[blockIdx.x * RG_WINDOW + (uint32_t)(key[i] & 0xffffffffu)];
 }
 
-// Per-body reference rule with FP64-accurate double-float monopoles (NB_DF64, systems of one lane per
-// body; smaller ones take bh_theta_team_kernel's fixed point, which is faster there and more
+// Per-body reference rule with FP64-accurate double-float monopoles (NB_DF64, systems of one lane
+// per body; smaller ones take bh_theta_team_kernel's fixed point, which is faster there and more
 // accurate). The walk, the decisions and the lists are those of bh_theta_fix_kernel, so each body
 // accepts exactly the reference's cells; the accepted monopoles are evaluated in double-float
 // arithmetic on the FP32 pipe (~2^-48 relative per operation). Centres and the body are exact

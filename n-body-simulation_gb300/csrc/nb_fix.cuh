@@ -9,11 +9,12 @@
 //    coordinate is below 2^K. A double above 2^(K - 40) is represented exactly, a smaller one to
 //    2^(K - 94).
 //  * A pair: the three exact differences as magnitudes, shifted left by a common `sh` until the
-//    largest is in [2^29, 2^30) by its first word; r^2 + eps^2 as a 64-bit integer D in [2^60, 2^64)
-//    (truncation errors below 2^-55 of it, centred); r^-3 from an estimate Y of D^(-1/2) good to
-//    2^-28 (MUFU and one Newton step), its residual e = 1 - D Y^2, of which 32 bits remain, and
-//    Y^3 (1 + 3e/2) (dropped terms below 2^-55), times the mass's 53 bits, rounded once to a double.
-//    In all within 2^-52.2 of exact, root mean square 2^-54.2 (the final rounding alone: 2^-54.4).
+//    largest is in [2^29, 2^30) by its first word; r^2 + eps^2 as a 64-bit integer D in [2^60,
+//    2^64) (truncation errors below 2^-55 of it, centred); r^-3 from an estimate Y of D^(-1/2) good
+//    to 2^-28 (MUFU and one Newton step), its residual e = 1 - D Y^2, of which 32 bits remain, and
+//    Y^3 (1 + 3e/2) (dropped terms below 2^-55), times the mass's 53 bits, rounded once to a
+//    double. In all within 2^-52.2 of exact, root mean square 2^-54.2 (the final rounding alone:
+//    2^-54.4).
 //  * What the integers cannot hold is left to the caller's FP64 expressions: a pair closer than
 //    2^(K - 29), masses that are not positive normal numbers, coordinates outside 2^K, scales
 //    beyond the exponent range, eps^2 too large for the scale.
@@ -402,9 +403,9 @@ __device__ __forceinline__ bool term(const FixRec& f, const Fix3& p, int K, cons
     return ok;
 }
 
-// Whether a pair that term() refuses adds exactly 0 in the FP64 expressions too: a massless source, or
-// a body paired with itself (`self`), whose separation is 0, with a finite factor either way (eps^2
-// and the mass far from the exponent limits). The target fits the fixed point (sh_max >= 0).
+// Whether a pair that term() refuses adds exactly 0 in the FP64 expressions too: a massless source,
+// or a body paired with itself (`self`), whose separation is 0, with a finite factor either way
+// (eps^2 and the mass far from the exponent limits). The target fits the fixed point (sh_max >= 0).
 __device__ __forceinline__ bool adds_nothing(const FixRec& f, bool self, int K, int sh_max,
                                              double eps2) {
     return sh_max >= 0 && eps2 > 1e-60 &&

@@ -147,11 +147,12 @@ __device__ __forceinline__ float nb_rsqrt_f32(float x) {
 }
 
 // Packed FP32x2 arithmetic (sm_100+ f32x2 instructions): one instruction, two lanes.
-// Dependent launches. A kernel launched with nb::launch_after may start while the kernel before it in
-// the stream still runs; nb_grid_wait, which such a kernel calls before it touches memory that earlier
-// launches write, returns when that kernel has finished and its writes are visible, and lets the next
-// dependent launch start in turn. (So everything before the preceding kernel has finished already
-// when a dependent one starts.) Saves the gap between the short launches of a chain, 1 to 1.5 us each.
+// Dependent launches. A kernel launched with nb::launch_after may start while the kernel before it
+// in the stream still runs; nb_grid_wait, which such a kernel calls before it touches memory that
+// earlier launches write, returns when that kernel has finished and its writes are visible, and
+// lets the next dependent launch start in turn. (So everything before the preceding kernel has
+// finished already when a dependent one starts.) Saves the gap between the short launches of a
+// chain, 1 to 1.5 us each.
 __device__ __forceinline__ void nb_grid_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -468,7 +468,8 @@ bh_learned_kernel(const NodeRec32* __restrict__ rec, const NodeAux* __restrict__
     // the group's positions as packed pairs (bodies 2j, 2j+1) per axis, for the gap loop
     __shared__ nb_f2 gpx[LT_WARPS][16], gpy[LT_WARPS][16], gpz[LT_WARPS][16];
     __shared__ float4 ilist[LT_WARPS][LT_LIST];
-    // per step: the lane whose cell fills each new list slot (0xff: a monopole, written by its lane)
+    // per step: the lane whose cell fills each new list slot (0xff: a monopole, written by its
+    // lane)
     __shared__ uint8_t slot_lane[LT_WARPS][LT_BATCH * LT_DIRECT];
     __shared__ __align__(16) uint32_t wfrag[32 * MF_WS];
     __shared__ __align__(16) float bfrag[32 * MF_BS];
@@ -892,16 +893,17 @@ pairs_label_kernel(const NodeRec32* __restrict__ rec, const NodeRec64* __restric
 // One block per chunk of 64 samples (two chunks per SM and then loops). Forward and backward: four
 // threads per sample, each with 8 of the 32 columns of a layer, the samples' activations in shared
 // memory in rows of 36 words (16-byte loads of 8 samples meet 8 different bank groups). Gradients:
-// thread (i, o) of a 16 x 16 grid owns a 2 x 2 tile of W2's gradient and one entry of W1's, the first
-// warps the bias and output-layer entries; one atomic per entry and block.
+// thread (i, o) of a 16 x 16 grid owns a 2 x 2 tile of W2's gradient and one entry of W1's, the
+// first warps the bias and output-layer entries; one atomic per entry and block.
 //  Bound: latency (8,192 rows fill 128 of 152 SMs once, ~1,000 dependent FMAs per thread) and the
-//  launches around it. With one thread per sample and 32 blocks: 80 us per 8,192 rows; now 12 us (65,536 rows: 55).
+//  launches around it. With one thread per sample and 32 blocks: 80 us per 8,192 rows; now 12 us
+//  (65,536 rows: 55).
 constexpr int TR_BLOCK = 256;
 constexpr int TR_CHUNK = 64;
 constexpr int TR_ROW = 36;
 
-// Zeroes the gradient and the loss; the gradient kernel computes meanwhile (two memsets before it and
-// ordinary launches: 18.8 us for gradient and Adam at 8,192 rows, this way 13.7).
+// Zeroes the gradient and the loss; the gradient kernel computes meanwhile (two memsets before it
+// and ordinary launches: 18.8 us for gradient and Adam at 8,192 rows, this way 13.7).
 __global__ void mlp_zero_kernel(float* __restrict__ grad, float* __restrict__ loss) {
     nb_grid_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;

@@ -81,9 +81,9 @@ naive_ieee_kernel(const double* __restrict__ m, const double* __restrict__ x,
     }
 }
 
-// Adds the pair (source record f, body q) seen from body i at p to the sums: NB_F64's arithmetic. The
-// pairs the fixed point cannot hold take the FP64 expressions; the self pair (its separation is 0)
-// and massless sources mostly add nothing.
+// Adds the pair (source record f, body q) seen from body i at p to the sums: NB_F64's arithmetic.
+// The pairs the fixed point cannot hold take the FP64 expressions; the self pair (its separation is
+// 0) and massless sources mostly add nothing.
 struct FixSums {
     double x, y, z;
 };
@@ -108,17 +108,19 @@ __device__ __forceinline__ void fix_pair(const nbfix::FixRec& f, uint32_t q, uin
     a.z = fma(w, dz, a.z);
 }
 
-// NB_F64, one-sided: target ranges, listed targets, systems below the symmetric kernel's sizes. One thread per target; the
-// sources of a tile are converted to the fixed point of nb_fix.cuh by the block as it loads them,
-// and a pair costs ~115 integer instructions and 3 FP64 ones instead of 16 FP64 ones. blockIdx.y selects a chunk of `chunk` sources; with more than one chunk the partial sums (times
-// G) go to part[(chunk index * targets + target) * 3 + axis].
+// NB_F64, one-sided: target ranges, listed targets, systems below the symmetric kernel's sizes. One
+// thread per target; the sources of a tile are converted to the fixed point of nb_fix.cuh by the
+// block as it loads them, and a pair costs ~115 integer instructions and 3 FP64 ones instead of 16
+// FP64 ones. blockIdx.y selects a chunk of `chunk` sources; with more than one chunk the partial
+// sums (times G) go to part[(chunk index * targets + target) * 3 + axis].
 //  Bound: the FP64 pipe (81% busy at 3 FMAs per pair) and dispatch. 8,192 bodies 2.16 -> 0.50 ms
-//  (31 -> 133 Gpairs/s), 4,096 0.53 -> 0.15. 32 warps per SM in blocks of 256 (blocks of 128: 3% slower, of 64: 16%).
+//  (31 -> 133 Gpairs/s), 4,096 0.53 -> 0.15. 32 warps per SM in blocks of 256 (blocks of 128: 3%
+//  slower, of 64: 16%).
 constexpr int FX_THREADS = 256;
 constexpr int FX_BLOCKS_PER_SM = 4;
-// Source chunks: 32 blocks per SM in all (fewer leave a longer last wave: 16 are 4% slower at 16,384
-// bodies, 8 8%), but at most 128 chunks and at least 4 sources each, since every pair of a lone
-// block's chain of tiles is ~0.5 us while its start and the combine pass are ~2 us each.
+// Source chunks: 32 blocks per SM in all (fewer leave a longer last wave: 16 are 4% slower at
+// 16,384 bodies, 8 8%), but at most 128 chunks and at least 4 sources each, since every pair of a
+// lone block's chain of tiles is ~0.5 us while its start and the combine pass are ~2 us each.
 constexpr long long FX_GRID_PER_SM = 32;
 constexpr uint32_t FX_CHUNKS_MAX = 128, FX_CHUNK_MIN = 4;
 static_assert(NB_COUNTER_WORDS - NB_COUNTER_SCALE >= (int)nbfix::SCALE_WORDS, "scale words");
@@ -168,9 +170,9 @@ naive_fix_kernel(const double* __restrict__ m, const double* __restrict__ x,
 }
 
 // The same for systems of up to FXC_MAX_N bodies, where one launch without global partials counts:
-// a cluster of 8 CTAs per 32 targets, the sources split over the CTAs and each CTA's share over its 8
-// warps. The warps' sums are added in warp order in shared memory, the CTAs' sums in rank order by
-// rank 0 through distributed shared memory.
+// a cluster of 8 CTAs per 32 targets, the sources split over the CTAs and each CTA's share over its
+// 8 warps. The warps' sums are added in warp order in shared memory, the CTAs' sums in rank order
+// by rank 0 through distributed shared memory.
 //  Bound: the ~0.5 us latency of each of the n / 64 pairs a warp evaluates one after the other, and
 //  ~4 us of start and reductions. 1,009 bodies: 48 us (FP64, chunks and a combine pass) -> 19 us;
 //  2,048: 144 -> 50. At 3,000 bodies the chunked kernel above is 8% faster.
@@ -307,8 +309,8 @@ nb_status naive_sym(nb_ctx* ctx, int form, const double* m, const double* x, con
     if (g_naive_sym_mode == 0) return NB_OK;
     // candidate shapes: the configured one, except in the automatic mode of the FP64 and
     // double-float forms, which take shape 0 (4,2,64) with 256-body I-blocks (fewer registers per
-    // thread); where its partials do not fit, double-float takes shape 1 (4,4,64) with 512, FP64 the
-    // one-sided kernel (as fast as its shape 1)
+    // thread); where its partials do not fit, double-float takes shape 1 (4,4,64) with 512, FP64
+    // the one-sided kernel (as fast as its shape 1)
     int cand[2] = {g_naive_sym_cfg[form], -1};
     if (g_naive_sym_mode == 1 && form != nb::SYM_F32) {
         cand[0] = 0;
