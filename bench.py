@@ -37,7 +37,7 @@ DT = 1.0 / 24
 EPS2 = 1e-22
 SEED = 1
 def launches_per_step(n: int) -> int:
-    """Kernels of ours launched per step (above 73,000 bodies): kick_drift 1, build (aabb 1, keys 1,
+    """Kernels of ours launched per step (above 36,480 bodies): kick_drift 1, build (aabb 1, keys 1,
     sort 9: one histogram of all digits and 8 look-back passes, runs 1, splits 1, scan 2 or, above
     8.4M bodies, 3, emit 1, centre of mass: chunks of 256 bodies 1, one tier per factor of 96 above
     the chunk until one block spans all bodies), walk order from the last walk lengths 1,

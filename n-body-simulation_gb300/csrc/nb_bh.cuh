@@ -73,6 +73,7 @@ struct nb_bh_tree {
     // the walk order the next one takes from them; walk_n = bodies they were recorded for (0: none)
     uint32_t* walk_len = nullptr;
     uint32_t* walk_ids = nullptr;
+    uint32_t* walk_cost = nullptr;  // longest of each group of 32 in that order
     mutable uint32_t walk_n = 0;
     cudaEvent_t phase_ev[6] = {};  // build phase boundaries (nb_bh_set_phase_timing)
     bool phase_timing = false;

@@ -213,3 +213,27 @@ def test_naive_in_a_capture_without_scratch():
     ref = naive(c, d, 1e-6, "f64_ieee")
     assert rel_err(*[host(v) for v in a], *ref).max() <= 1e-12
     c.close()
+
+
+@pytest.mark.parametrize("n", [36480, 36481, 36512, 70001])
+def test_groups_in_cost_order(ctx, n):
+    """The last size of the teams and one lane per body: later calls walk the groups by cost class
+    (uneven walks; the last group full, with one body, in part), each once, to the same bits."""
+    import torch
+    from nbody.lib import BHTree
+    d = bodies("plummer", n, seed=n)
+    both(ctx, d, 0.9, 1e-6)
+    t = [dev(d[k]) for k in ("m", "x", "y", "z")]
+    tree = BHTree(ctx, n, theta=0.9)
+    tree.build(*t, d["G"])
+    runs = []
+    for _ in range(3):
+        a = [torch.full((n,), np.nan, dtype=torch.float64, device="cuda") for _ in range(3)]
+        tree.accel(*t[1:], *a, d["G"], 1e-6, "theta", "df64")
+        ctx.sync()
+        runs.append([host(v) for v in a])
+    for r in runs[1:]:
+        for u, v in zip(r, runs[0]):
+            np.testing.assert_array_equal(u, v)
+    assert not np.isnan(np.stack(runs[0])).any()
+    tree.close()
