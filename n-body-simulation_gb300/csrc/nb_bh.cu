@@ -143,20 +143,9 @@ __device__ uint64_t key_word_quantized(const double* __restrict__ box, double px
     return (spread3(hy) << 2) | (spread3(~hz & m) << 1) | spread3(~hx & m);
 }
 
-// Box entries beyond the AABB, by the first threads of the keys kernels: the centre, for the node
-// records, and the scale exponent of the fixed-point records.
-__device__ __forceinline__ void box_extras(double* __restrict__ box, uint32_t i) {
-    if (i < 3) box[7 + i] = box[i] + box[6] / 2;
-    if (i == 3) {
-        long long v = 0;
-        for (int k = 0; k < 6; ++k)
-            v = max(v, __double_as_longlong(box[k]) & 0x7fffffffffffffffll);
-        const int K = nbfix::k_of(__longlong_as_double(v));
-        box[10] = (double)K;
-        // K and (float)(edge^2) as bits, for the record writers
-        box[11] = __hiloint2double(K, __float_as_int((float)(box[6] * box[6])));
-    }
-}
+// Box entries beyond the AABB, by the first four threads of the keys kernels.
+using nbfix::box_extras;
+using nbfix::BOX_WORDS;
 
 // Zeroes what the launches after the keys count on: the sort's counters, the second key words and
 // the level masks, by all threads of the grid.
@@ -534,7 +523,7 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
     uint8_t* split_level = level_min[0];
     __shared__ long long wmin[3][32], wmax[3][32];
     __shared__ uint32_t warp_sums[32];
-    __shared__ double sbox[11];
+    __shared__ double sbox[BOX_WORDS];
     __shared__ FixedGrid grid_s;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // children lists start empty; written before the barriers below, filled after them
@@ -591,7 +580,7 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
         __syncwarp();
         box_extras(sbox, lane);
         __syncwarp();
-        if (lane < 12) box[lane] = sbox[lane];
+        if (lane < BOX_WORDS) box[lane] = sbox[lane];
         if (lane == 0 && !quantized) grid_s = fixed_grid(sbox);
     }
     __syncthreads();
@@ -1607,7 +1596,7 @@ struct Carver {
 
 void carve(nb_bh_tree* t, Carver& c) {
     const size_t n = t->n_max, cap = t->node_cap;
-    t->box = c.take<double>(16);
+    t->box = c.take<double>(BOX_WORDS);
     t->info = c.take<uint32_t>(16);
     t->work = c.take<uint32_t>(16);
     t->sched = c.take<uint32_t>(32);

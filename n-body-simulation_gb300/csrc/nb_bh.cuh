@@ -55,9 +55,7 @@ struct nb_bh_tree {
     double G = 0;
     int device = 0;
 
-    double* box = nullptr;  // [0..6] AABB (min xyz, max xyz, edge), [7..9] box centre, [10] the
-                            // scale exponent K of the fixed-point records (nb_fix.cuh), [11] K and
-                            // (float) edge^2 as bits
+    double* box = nullptr;  // nbfix::BOX_WORDS entries: see nbfix::box_extras
     uint32_t* info = nullptr;  // [0] node count (copy of base[n])
     uint2* tier_cells[2] = {};      // centre-of-mass tiers: cells passed up, (node, level)
     uint32_t* tier_count[2] = {};   // their count per chunk

@@ -81,6 +81,15 @@ NB_FIX_FN double double_of(uint32_t hi, uint32_t lo) {
     return v;
 #endif
 }
+NB_FIX_FN uint32_t float_bits(float v) {
+#if NB_FIX_DEV
+    return __float_as_uint(v);
+#else
+    uint32_t u;
+    std::memcpy(&u, &v, 4);
+    return u;
+#endif
+}
 // the high word of (hi:lo) << (s & 31)
 NB_FIX_FN uint32_t fsl(uint32_t lo, uint32_t hi, uint32_t s) {
 #if NB_FIX_DEV
@@ -141,6 +150,24 @@ NB_FIX_FN void sub96(uint32_t a2, uint32_t a1, uint32_t a0, uint32_t b2, uint32_
 // Outside +-K_MAX the scale is unusable.
 NB_FIX_FN int k_of(double v_max) { return (int)((bits_of(v_max) >> 52) & 0x7ff) - 1022; }
 NB_FIX_FN bool k_usable(int K) { return K >= -K_MAX && K <= K_MAX; }
+
+// A tree's box: [0..6] its AABB (nb_aabb), [7..9] the centre and [10], [11] the scale of its records:
+// K, and K again with the FP32 edge^2 as the bits of one double. From the AABB, by calls 0 to 3 (of
+// four threads: none reads what another writes).
+constexpr int BOX_WORDS = 12;
+NB_FIX_FN void box_extras(double* box, uint32_t i) {
+    if (i < 3) box[7 + i] = box[i] + box[6] / 2;
+    if (i == 3) {
+        uint64_t v = 0;  // the largest |coordinate|
+        for (int k = 0; k < 6; ++k) {
+            const uint64_t u = bits_of(box[k]) & 0x7fffffffffffffffull;
+            v = u > v ? u : v;
+        }
+        const int K = k_of(double_of((uint32_t)(v >> 32), (uint32_t)v));
+        box[10] = (double)K;
+        box[11] = double_of((uint32_t)K, float_bits((float)(box[6] * box[6])));
+    }
+}
 
 // The words of v as a multiple of 2^(K - 93) (rounded to nearest where v has lower bits); false
 // when v is not finite or beyond 2^K.
