@@ -11,7 +11,7 @@
 //  * A pair: the three exact differences as magnitudes, shifted left by a common `sh` until the
 //    largest is in [2^29, 2^30) by its first word; r^2 + eps^2 as a 64-bit integer D in [2^60,
 //    2^64) (truncation errors below 2^-55 of it, centred); r^-3 from an estimate Y of D^(-1/2) good
-//    to 2^-28 (MUFU and one Newton step), its residual e = 1 - D Y^2, of which 32 bits remain, and
+//    to 2^-30 (MUFU and one Newton step), its residual e = 1 - D Y^2, of which 32 bits remain, and
 //    Y^3 (1 + 3e/2) (dropped terms below 2^-55), times the mass's 53 bits, rounded once to a
 //    double. In all within 2^-52.2 of exact, root mean square 2^-54.2 (the final rounding alone:
 //    2^-54.4).
@@ -283,8 +283,10 @@ NB_FIX_FN uint64_t norm2(const Sep& s) {
     return (r << 2) + ((uint64_t)h << 3);
 }
 
-// Y ~ 2^61 D^(-1/2) to 2^-28 and e = 1 - D Y^2 / 2^122 in units 2^-58 (|e| < 2^31); W = Y^2.
-// D Y^2 is so near 2^122 that of its upper half only the low 32 bits are formed.
+// Y ~ 2^61 D^(-1/2), within 2^-30 of it and below 2^31 (the rounded estimate reaches 2^31 for D up to
+// 2^60 + 2^32, where one unit less is as good: its users multiply it as a signed word), and
+// e = 1 - D Y^2 / 2^122 in units 2^-58 (|e| < 2^30); W = Y^2. D Y^2 is so near 2^122 that of its upper
+// half only the low 32 bits are formed.
 NB_FIX_FN int rsqrt_residual(uint64_t D, uint32_t& Y, uint64_t& W) {
     const uint32_t dh = (uint32_t)(D >> 32), dl = (uint32_t)D;
     const float f = rsqrt_est((float)dh) * 35184372088832.0f;  // 2^45: at most 2^31
@@ -298,6 +300,7 @@ NB_FIX_FN int rsqrt_residual(uint64_t D, uint32_t& Y, uint64_t& W) {
     const uint64_t p = (uint64_t)dh * (uint32_t)(w0 >> 32) + mul_hi(dh, (uint32_t)w0);
     const int ne0 = (int)(fsl((uint32_t)p, (uint32_t)(p >> 32), 5) ^ 0x80000000u);  // -e0 2^31
     Y = (uint32_t)(y0 - (int)(((int64_t)y0 * ne0 + 0x80000000ll) >> 32));  // rounded
+    Y = Y < 0x7fffffffu ? Y : 0x7fffffffu;
     W = (uint64_t)Y * Y;
     const uint32_t wh = (uint32_t)(W >> 32), wl = (uint32_t)W;
     return -(int)(dh * wh + mul_hi(dh, wl) + mul_hi(dl, wh) + 1u);

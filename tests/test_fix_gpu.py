@@ -237,3 +237,38 @@ def test_groups_in_cost_order(ctx, n):
             np.testing.assert_array_equal(u, v)
     assert not np.isnan(np.stack(runs[0])).any()
     tree.close()
+
+
+# -- separations whose squares are powers of four (the largest estimate of 1/r) --------------------
+# Every term of a body's sum is within 2^-52 of exact on either side and the FP64 sums of n terms
+# within n 2^-53 of the sum of the terms' magnitudes each: (n + 4) 2^-52 of that sum.
+@pytest.mark.parametrize("side", [2, 8, 13])
+@pytest.mark.parametrize("eps2", [1e-22, 1e-9])
+def test_unit_lattice(ctx, side, eps2):
+    import oracle
+    import torch
+    from nbody.lib import SYM_ALWAYS, SYM_AUTO, SYM_NEVER, set_naive_symmetric
+    p = np.stack(np.meshgrid(*[np.arange(float(side))] * 3, indexing="ij")).reshape(3, -1)
+    n = p.shape[1]
+    d = dict(zip("xyz", np.ascontiguousarray(p)), m=np.ones(n), G=1.0)
+    q = p[:, :, None] - p[:, None, :]
+    r2 = (q ** 2).sum(axis=0) + eps2
+    np.fill_diagonal(r2, np.inf)
+    bound = (n + 4) * 2.0 ** -52 * (np.abs(q) / r2 ** 1.5).sum(axis=2)
+    ref = naive(ctx, d, eps2, "f64_ieee")
+    try:
+        for mode in (SYM_NEVER, SYM_ALWAYS):
+            set_naive_symmetric(mode)
+            for g, r, b in zip(naive(ctx, d, eps2, "f64"), ref, bound):
+                assert (np.abs(g - r) <= b).all()
+    finally:
+        set_naive_symmetric(SYM_AUTO)
+    got, ref = both(ctx, d, 0.0, eps2)  # every body against every other
+    for g, r, b in zip(got, ref, bound):
+        assert (np.abs(g - r) <= b).all()
+    zero = np.zeros(n)
+    out = torch.zeros(4, dtype=torch.float64, device="cuda")
+    ctx.energy(*[dev(d[k]) for k in ("m", "x", "y", "z")], *[dev(zero)] * 3, 1.0, out)
+    ctx.sync()
+    o = oracle.energy(*[d[k] for k in ("m", "x", "y", "z")], zero, zero, zero, 1.0)
+    assert abs(out[1].item() - o["potential"]) <= 1e-12 * abs(o["potential"])
