@@ -931,15 +931,17 @@ mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
     auto row4 = [&](int at) { return *reinterpret_cast<const float4*>(&w[at]); };
     for (uint32_t first = blockIdx.x * TR_CHUNK; first < n; first += gridDim.x * TR_CHUNK) {
         const bool in = first + s < n;
+        // past the end: an all-zero sample whose activations are zero too, so that whatever the rows
+        // and the weights hold, it adds nothing
         const uint32_t row = in ? (idx ? __ldcg(idx + first + s) : first + s) : 0u;
         const float4* xr = reinterpret_cast<const float4*>(X + (size_t)row * NF);
         const bool wide = ((uintptr_t)X & 15) == 0;
-        float x[8];
-        if (wide) {
+        float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (in && wide) {
             const float4 a = __ldcg(xr), b = __ldcg(xr + 1);
             x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
             x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
-        } else {
+        } else if (in) {
 #pragma unroll
             for (int i = 0; i < NF; ++i) x[i] = __ldcg(X + (size_t)row * NF + i);
         }
@@ -957,7 +959,7 @@ mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
         }
 #pragma unroll
         for (int o = 0; o < 8; ++o) {
-            h1[o] = fmaxf(h1[o], 0.f);
+            h1[o] = in ? fmaxf(h1[o], 0.f) : 0.f;
             sh1[s][c0 + o] = h1[o];
         }
         if ((tid & 3) == 0) {
@@ -983,14 +985,14 @@ mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
         float out = 0.f;
 #pragma unroll
         for (int o = 0; o < 8; ++o) {
-            h2[o] = fmaxf(h2[o], 0.f);
+            h2[o] = in ? fmaxf(h2[o], 0.f) : 0.f;
             out = fmaf(h2[o], w[P_W3 + c0 + o], out);
         }
         out += __shfl_xor_sync(0xffffffffu, out, 1);
         out += __shfl_xor_sync(0xffffffffu, out, 2);
         const float e = in ? out + w[P_B3] - y : 0.f;
         if ((tid & 3) == 0) lsum = fmaf(e, e, lsum);
-        const float dout = 2.f * e * inv_n;  // 0 for rows past the end: they add nothing below
+        const float dout = 2.f * e * inv_n;  // 0 past the end
 #pragma unroll
         for (int o = 0; o < 8; ++o) {
             sh2[s][c0 + o] = h2[o];

@@ -233,3 +233,28 @@ def test_group_order_does_not_change_the_result(ctx, n):
     for a, b in zip(*res):
         np.testing.assert_array_equal(a, b)
     tree.close()
+
+
+@pytest.mark.parametrize("n", [1, 63, 100, 129])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_gradient_ignores_rows_outside_the_batch(ctx, n, bad, offset):
+    """A row that the index list leaves out may hold anything, also where the last chunk of samples is
+    not full; X on and off a 16-byte boundary. Tolerance as above."""
+    import torch
+    from nbody.lib import mlp_loss_grad
+    p, X, Y = _rand(n, n + 20)
+    X[0] = bad
+    Y[0] = bad
+    rows = 1 + np.random.default_rng(4).permutation(n + 19)[:n].astype(np.int32)
+    grad = torch.zeros(omlp.COUNT, dtype=torch.float32, device="cuda")
+    loss = torch.zeros(1, dtype=torch.float32, device="cuda")
+    tX = torch.zeros(X.size + offset, dtype=torch.float32, device="cuda")[offset:].view(X.shape)
+    tX.copy_(torch.as_tensor(X))
+    tp, tY, tidx = (torch.as_tensor(a, device="cuda") for a in (p, Y, rows))
+    mlp_loss_grad(ctx, tp, tX, tY, tidx, n, grad, loss)
+    ctx.sync()
+    l_ref, g_ref = omlp.loss_grad(p.astype(np.float64), X[rows], Y[rows])
+    assert loss.item() == pytest.approx(l_ref, rel=1e-4)
+    g = grad.cpu().numpy().astype(np.float64)
+    assert np.max(np.abs(g - g_ref)) <= 1e-4 * np.abs(g_ref).max()
