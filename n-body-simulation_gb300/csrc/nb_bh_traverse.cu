@@ -424,7 +424,8 @@ bh_theta_fix_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __rest
             pre = pretest_of(box, px, py, pz, theta);
             body = fix_body<FAST64>(px, py, pz, K, e2);
         }
-        uint32_t accepted = 0, k = valid ? 0u : nn;
+        // bit 31 keeps the body's mark of rounded coordinates (a register less through the walk)
+        uint32_t accepted = body.p.rounded << 31, k = valid ? 0u : nn;
         double acx = 0, acy = 0, acz = 0;
         for (;;) {
             int cnt = 0;
@@ -443,6 +444,7 @@ bh_theta_fix_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __rest
             FixRec next = load_fix(fix_hi, fix_lo, cnt > 0 ? list[0][tid] : 0u);
             for (int i = 0; i < most; ++i) {
                 const FixRec f = next;
+                body.p.rounded = accepted >> 31;
                 if (i + 1 < cnt) next = load_fix(fix_hi, fix_lo, list[i + 1][tid]);
                 if (i < cnt)
                     fix_monopole(f, rec64, list[i][tid], body, K, e2, x, y, z, me, eps2, acx, acy,
@@ -453,7 +455,7 @@ bh_theta_fix_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __rest
             ax[me] = acx * G;
             ay[me] = acy * G;
             az[me] = acz * G;
-            walk_len[me] = accepted;
+            walk_len[me] = accepted & 0x7fffffffu;
         }
     }
 }

@@ -6,8 +6,8 @@
 // (one DFMA per axis) stay on the FP64 pipe.
 //
 //  * Coordinates: 96-bit two's complement multiples of 2^(K - 93), K chosen so that every
-//    coordinate is below 2^K. A double above 2^(K - 40) is represented exactly, a smaller one to
-//    2^(K - 94).
+//    coordinate is below 2^K. A double above 2^(K - 41) is represented exactly, a smaller one is
+//    rounded to 2^(K - 94) where it has lower bits, and marked.
 //  * A pair: the three exact differences as magnitudes, shifted left by a common `sh` until the
 //    largest is in [2^29, 2^30) by its first word; r^2 + eps^2 as a 64-bit integer D in [2^60,
 //    2^64) (truncation errors below 2^-55 of it, centred); r^-3 from an estimate Y of D^(-1/2) good
@@ -16,8 +16,10 @@
 //    double. In all within 2^-52.2 of exact, root mean square 2^-54.2 (the final rounding alone:
 //    2^-54.4).
 //  * What the integers cannot hold is left to the caller's FP64 expressions: a pair closer than
-//    2^(K - 29), masses that are not positive normal numbers, coordinates outside 2^K, scales
-//    beyond the exponent range, eps^2 too large for the scale.
+//    2^(K - 29), a component below 2^(K - 38) between bodies one of which is marked as rounded (so
+//    small components keep their own relative accuracy), masses that are not positive normal
+//    numbers, coordinates outside 2^K, scales beyond the exponent range, eps^2 too large for the
+//    scale.
 //
 // Everything up to the device-only part also compiles as plain C++, for the CPU tests.
 #pragma once
@@ -43,8 +45,9 @@ constexpr int ZERO_MASS = NO_EXP + 1;  // FixRec::e of a massless source with fi
 constexpr int K_MAX = 300;          // |K| beyond this: FP64 expressions for everything
 constexpr int SH_MAX = 29;          // largest common shift
 
-// A source: coordinate words (most significant first), the mass's mantissa (64 bits, top bit set)
-// and its biased exponent - 3 K.
+// A source: coordinate words (most significant first), the mass's mantissa (64 bits, top bit set,
+// the lowest 11 clear but for bit 0, which marks rounded coordinates; it moves the truncated mass
+// product by less than 1/8 of its last unit) and its biased exponent - 3 K.
 struct alignas(16) FixRec {
     uint32_t x2, y2, z2, mh;
     uint32_t x1, y1, z1, ml;
@@ -60,6 +63,7 @@ struct alignas(32) FixHi {
 
 struct Fix3 {
     uint32_t x2, y2, z2, x1, y1, z1, x0, y0, z0;
+    uint32_t rounded;  // bit 0: a coordinate has bits below the last word's
 };
 
 NB_FIX_FN uint64_t bits_of(double v) {
@@ -169,9 +173,9 @@ NB_FIX_FN void box_extras(double* box, uint32_t i) {
     }
 }
 
-// The words of v as a multiple of 2^(K - 93) (rounded to nearest where v has lower bits); false
-// when v is not finite or beyond 2^K.
-NB_FIX_FN bool split96(double v, int K, uint32_t& w2, uint32_t& w1, uint32_t& w0) {
+// The words of v as a multiple of 2^(K - 93), rounded to nearest where v has lower bits, which are
+// or'ed into `lost`; false when v is not finite or beyond 2^K.
+NB_FIX_FN bool split96(double v, int K, uint32_t& w2, uint32_t& w1, uint32_t& w0, uint32_t& lost) {
     const uint64_t u = bits_of(v);
     const uint32_t uh = (uint32_t)(u >> 32), ul = (uint32_t)u;
     const int be = (int)((uh >> 20) & 0x7ff);
@@ -186,6 +190,7 @@ NB_FIX_FN bool split96(double v, int K, uint32_t& w2, uint32_t& w1, uint32_t& w0
     w1 = q == 1 ? a2 : q == 2 ? a1 : q == 3 ? a0 : 0u;
     w2 = q == 2 ? a2 : q == 3 ? a1 : 0u;
     const uint32_t half = (q == 0 ? a1 : q == 1 ? a0 : 0u) >> 31;
+    lost |= q == 0 ? a0 | a1 : q == 1 ? a0 : in ? 0u : (uh << 1) | ul;
     // plus the half; negative values as the complement plus one
     const uint32_t neg = (uint32_t)((int)uh >> 31);
     const uint64_t t = (uint64_t)w0 + half;
@@ -199,9 +204,11 @@ NB_FIX_FN bool split96(double v, int K, uint32_t& w2, uint32_t& w1, uint32_t& w0
 }
 
 NB_FIX_FN bool split3(double x, double y, double z, int K, Fix3& f) {
-    const bool a = split96(x, K, f.x2, f.x1, f.x0);
-    const bool b = split96(y, K, f.y2, f.y1, f.y0);
-    const bool c = split96(z, K, f.z2, f.z1, f.z0);
+    uint32_t lost = 0;
+    const bool a = split96(x, K, f.x2, f.x1, f.x0, lost);
+    const bool b = split96(y, K, f.y2, f.y1, f.y0, lost);
+    const bool c = split96(z, K, f.z2, f.z1, f.z0, lost);
+    f.rounded = lost != 0 ? 1u : 0u;
     return a && b && c && k_usable(K);
 }
 
@@ -221,6 +228,7 @@ NB_FIX_FN FixRec make_rec(double x, double y, double z, double m, int K) {
     int be;
     const bool ok = split3(x, y, z, K, f);
     const bool mk = split_mass(m, r.mh, r.ml, be);
+    r.ml |= f.rounded;
     r.x2 = f.x2;
     r.y2 = f.y2;
     r.z2 = f.z2;
@@ -385,8 +393,17 @@ NB_FIX_FN double axis_small(uint32_t s, uint32_t h, uint32_t l, uint32_t x, int 
     return double_of(hi | (s & 0x80000000u), (mh << 21) | (ml >> 11));
 }
 
-NB_FIX_FN void axes(const Sep& s, int K, double& dx, double& dy, double& dz) {
+// Whether a component is below 2^55 units: then a rounded coordinate may have cost it bits that a
+// double holds.
+NB_FIX_FN bool axis_tiny(uint32_t h, uint32_t l, int sh) {
+    return ((((uint64_t)h << 32) | l) >> (23 + sh)) == 0;
+}
+
+// False when a component needs the coordinates' own bits (`rounded`: either body's mark).
+NB_FIX_FN bool axes(const Sep& s, int K, double& dx, double& dy, double& dz,
+                    uint32_t rounded = 0) {
     const int base = 1025 + K - s.sh;
+    bool fits = true;
     uint32_t least = s.xh < s.yh ? s.xh : s.yh;
     least = least < s.zh ? least : s.zh;
     if (least >= AXIS_TWO_WORDS) {
@@ -394,10 +411,14 @@ NB_FIX_FN void axes(const Sep& s, int K, double& dx, double& dy, double& dz) {
         dy = axis(s.ys, s.yh, s.yl, base);
         dz = axis(s.zs, s.zh, s.zl, base);
     } else {
+        if (rounded != 0)
+            fits = !(axis_tiny(s.xh, s.xl, s.sh) || axis_tiny(s.yh, s.yl, s.sh) ||
+                     axis_tiny(s.zh, s.zl, s.sh));
         dx = axis_small(s.xs, s.xh, s.xl, (s.x0 << s.sh) ^ s.xs, base);
         dy = axis_small(s.ys, s.yh, s.yl, (s.y0 << s.sh) ^ s.ys, base);
         dz = axis_small(s.zs, s.zh, s.zl, (s.z0 << s.sh) ^ s.zs, base);
     }
+    return fits;
 }
 
 #ifdef __CUDACC__
@@ -429,8 +450,8 @@ __device__ __forceinline__ bool term(const FixRec& f, const Fix3& p, int K, cons
     const uint64_t D = norm2(s) + t.units[s.sh];  // with norm2's bias
     bool ok;
     w = mass_rinv3(rinv3(D), f.mh, f.ml, f.e, s.sh, ok);
-    axes(s, K, dx, dy, dz);
-    return ok;
+    const bool fits = axes(s, K, dx, dy, dz, (f.ml | p.rounded) & 1u);
+    return ok && fits;
 }
 
 // Whether a pair that term() refuses adds exactly 0 in the FP64 expressions too: a massless source,

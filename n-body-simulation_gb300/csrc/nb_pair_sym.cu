@@ -385,7 +385,7 @@ pair_sym_fix_kernel(SymPlan S, const nbfix::FixRec* __restrict__ src,
     // the one-sided arithmetic: the pairs the loop below leaves.
     auto one_side = [&](const nbfix::FixRec& f, uint32_t b, const nbfix::FixRec& t, uint32_t at,
                         double& sx, double& sy, double& sz) {
-        const nbfix::Fix3 p{t.x2, t.y2, t.z2, t.x1, t.y1, t.z1, t.x0, t.y0, t.z0};
+        const nbfix::Fix3 p{t.x2, t.y2, t.z2, t.x1, t.y1, t.z1, t.x0, t.y0, t.z0, t.ml & 1u};
         const int lim = t.e == nbfix::NO_EXP ? -1 : sh_max;
         double w, dx, dy, dz;
         if (lim < 0 || !nbfix::term(f, p, K, e2, lim, w, dx, dy, dz)) {
@@ -444,8 +444,9 @@ pair_sym_fix_kernel(SymPlan S, const nbfix::FixRec* __restrict__ src,
                             const double si = nbfix::mass_rinv3(inv3, I[k].mh, I[k].ml, I[k].e,
                                                                 sep.sh, oi);
                             double dx, dy, dz;
-                            nbfix::axes(sep, K, dx, dy, dz);
-                            ok = oj && oi;
+                            const bool fits =
+                                nbfix::axes(sep, K, dx, dy, dz, (J.ml | I[k].ml) & 1u);
+                            ok = oj && oi && fits;
                             if (ok) {
                                 tx[k] = fma(dx, sj, tx[k]);
                                 ty[k] = fma(dy, sj, ty[k]);

@@ -34,9 +34,9 @@ extern "C" int fix_pair(const double* c, const double* p, double m, double eps2,
     const uint64_t D = norm2(s) + (uint64_t)(eps2_units(eps2, K, s.sh) + 0.5) + NORM2_BIAS;
     bool ok;
     out[0] = mass_rinv3(rinv3(D), r.mh, r.ml, r.e, s.sh, ok);
-    axes(s, K, out[1], out[2], out[3]);
+    const bool fits = axes(s, K, out[1], out[2], out[3], (r.ml | P.rounded) & 1u);
     out[4] = scaled_double(rinv1(D), 1023 - K + s.sh);
-    return ok;
+    return ok && fits;
 }
 """
 
@@ -95,3 +95,35 @@ def test_pairs_at_powers_of_two(fix):
         assert got is not None
         assert abs(Decimal(got[0]) * r2 * r2.sqrt() / Decimal(1.25) - 1) <= Decimal(2.0 ** -52.4), (d, eps2)
         assert abs(Decimal(got[4]) * r2.sqrt() - 1) <= Decimal(2.0 ** -52.4), (d, eps2)
+
+
+@pytest.mark.parametrize("size", [1e-8, 1e-11, 1e-13, 1e-16, 1e-20, 1e-27, 1e-40, 1e-320])
+@pytest.mark.parametrize("eps2", [0.0, 1e-6])
+def test_small_components(fix, size, eps2):
+    """A box of 30 whose z coordinates are of the given size on one or both sides: the component keeps
+    its 53 bits or the pair is left to FP64 -- which pairs with one z of ordinary size never are, nor
+    those of a plane (z exactly 0)."""
+    rng = random.Random(3)
+    left = 0
+    for i in range(400):
+        c, p = ([rng.uniform(-1.0, 1.0) * 15.0 for _ in range(3)] for _ in range(2))
+        one_side = i % 4 == 0
+        c[2] = rng.uniform(-1.0, 1.0) * size
+        if not one_side:
+            p[2] = rng.choice((rng.uniform(-1.0, 1.0) * size, 0.0, c[2] * (1.0 + 2.0 ** -20)))
+        if i % 2:
+            c, p = p, c
+        got = pair(fix, c, p, 1.5, eps2, 15.0)
+        if got is None:
+            left += 1
+            assert not one_side and size < 1e-10
+            continue
+        d = [Decimal(a) - Decimal(b) for a, b in zip(c, p)]
+        for g, v in zip(got[1:], d):
+            # 2^-52 for the truncation to 53 bits and 2 half units of 2^-55 for the coordinates
+            assert abs(Decimal(g) - v) <= abs(v) * Decimal(2.0 ** -52 + 2.0 ** -55)
+        r2 = sum(v * v for v in d) + Decimal(eps2)
+        assert abs(Decimal(got[0]) * r2 * r2.sqrt() / Decimal(1.5) - 1) <= Decimal(2.0 ** -52.4)
+    assert left == 0 if size >= 1e-8 else left > 0 if size <= 1e-13 else True
+    c[2] = p[2] = 0.0
+    assert pair(fix, c, p, 1.5, eps2, 15.0) is not None

@@ -272,3 +272,36 @@ def test_unit_lattice(ctx, side, eps2):
     ctx.sync()
     o = oracle.energy(*[d[k] for k in ("m", "x", "y", "z")], zero, zero, zero, 1.0)
     assert abs(out[1].item() - o["potential"]) <= 1e-12 * abs(o["potential"])
+
+
+# -- sheets far thinner than the fixed point's grid resolves ----------------------------------------
+@pytest.mark.parametrize("thickness", [1e-11, 1e-14, 1e-18, 1e-25, 1e-32])
+@pytest.mark.parametrize("n", [700, 2500])
+def test_thin_sheet(ctx, n, thickness):
+    """The force across the sheet keeps its own relative accuracy (bound of test_thin_disc_component);
+    a few bodies of the plane itself (z exactly 0) and a few far from it."""
+    from nbody.lib import SYM_ALWAYS, SYM_AUTO, SYM_NEVER, set_naive_symmetric
+    d = bodies("plummer", n, seed=8)
+    d["z"] = d["z"] * thickness
+    d["z"][::50] = 0.0
+    eps2 = 1e-6
+    ref = naive(ctx, d, eps2, "f64_ieee")
+    scale = np.sqrt((ref[2] ** 2).mean())
+    got = []
+    try:
+        for mode in (SYM_NEVER, SYM_ALWAYS):
+            set_naive_symmetric(mode)
+            got.append(naive(ctx, d, eps2, "f64"))
+    finally:
+        set_naive_symmetric(SYM_AUTO)
+    got.append(naive(ctx, d, eps2, "f64", targets=np.arange(n)))
+    for g in got:
+        assert np.sqrt(((g[2] - ref[2]) ** 2).mean()) <= 1e-13 * scale
+        assert rel_err(*g, *ref).max() <= 1e-12
+    d["z"][1::40] = 0.5  # a pair's other components and its factor stay in the fixed point
+    got, ref = both(ctx, d, 0.5, eps2)
+    assert rel_err(*got, *ref).max() <= 1e-12
+    d["z"][1::40] = 0.0
+    got, ref = both(ctx, d, 0.5, eps2)
+    scale = np.sqrt((ref[2] ** 2).mean())
+    assert np.sqrt(((got[2] - ref[2]) ** 2).mean()) <= 1e-13 * scale
