@@ -127,3 +127,30 @@ def test_small_components(fix, size, eps2):
     assert left == 0 if size >= 1e-8 else left > 0 if size <= 1e-13 else True
     c[2] = p[2] = 0.0
     assert pair(fix, c, p, 1.5, eps2, 15.0) is not None
+
+
+def test_components_are_rounded(fix):
+    """Differences that doubles hold are exact, with either sign (of the words kept, those of a negative
+    one fall short by a unit); others are within half a unit in the last place where the two words have
+    four bits and more beyond it (2^-53, and 2^-57 twice for those words' own truncation)."""
+    rng = random.Random(17)
+    for i in range(2000):
+        c, p = ([float(rng.randint(-12, 12)) * 2.0 ** -rng.randint(0, 6) for _ in range(3)]
+                for _ in range(2))
+        got = pair(fix, c, p, 1.0, 1e-9, 15.0)
+        d = [a - b for a, b in zip(c, p)]
+        if got is None:
+            assert max(map(abs, d)) < 2.0 ** -25
+            continue
+        most = max(map(abs, d))
+        for g, v in zip(got[1:], d):
+            if abs(v) >= most * 2.0 ** -6 or v == 0.0:
+                assert g == v
+    for i in range(4000):
+        f = 2.0 ** -rng.uniform(0, 20)
+        p = [rng.uniform(-1.0, 1.0) * 14.0 for _ in range(3)]
+        c = [v + rng.uniform(0.03, 1.0) * rng.choice((-1, 1)) * f for v in p]
+        got = pair(fix, c, p, 1.0, 1e-9, 15.0)
+        for g, a, b in zip(got[1:], c, p):
+            v = Decimal(a) - Decimal(b)
+            assert abs(Decimal(g) - v) <= abs(v) * Decimal(2.0 ** -53 + 2.0 ** -56)
