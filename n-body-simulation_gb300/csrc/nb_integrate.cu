@@ -115,7 +115,7 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
     while ((uint64_t)q * (row + 1) * (row + 2) / 2 <= u0) ++row;
     uint32_t t = (uint32_t)(u0 - (uint64_t)q * row * (row + 1) / 2);  // tile of the row
     uint32_t j = 0;
-    bool active = false;
+    bool active = false, paired = false;  // paired: the row so far has pairs for this target
     nbfix::Fix3 p{};
     double mj = 0, ek = 0, ep = 0, acc = 0;
     bool load = true;
@@ -133,6 +133,7 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
                 }
             }
             acc = 0;
+            paired = false;
         }
         const uint32_t i0 = t * tile;
         __syncthreads();
@@ -147,6 +148,7 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
         }
         __syncthreads();
         const uint32_t cnt = active && j > i0 ? min(tile, j - i0) : 0u;
+        paired = paired || cnt != 0;
 #pragma unroll 1
         for (uint32_t ii = 0; ii < cnt; ++ii) {
             const nbfix::FixRec f = src[ii];
@@ -164,7 +166,7 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
             acc = fma(__hiloint2double((int)f.mh, (int)f.ml), inv, acc);
         }
         if (++t == q * (row + 1) || u + 1 == u1) {  // the row (or the CTA's range) ends
-            if (active) ep = fma(G * mj, acc, ep);
+            if (paired) ep = fma(G * mj, acc, ep);  // without pairs a mass of infinity adds nothing
             t = 0;
             ++row;
             load = true;

@@ -305,3 +305,18 @@ def test_thin_sheet(ctx, n, thickness):
     got, ref = both(ctx, d, 0.5, eps2)
     scale = np.sqrt((ref[2] ** 2).mean())
     assert np.sqrt(((got[2] - ref[2]) ** 2).mean()) <= 1e-13 * scale
+
+
+def test_energy_that_is_not_finite(ctx):
+    import torch
+    d = bodies("plummer", 400, seed=3)
+    keys = ("m", "x", "y", "z", "vx", "vy", "vz")
+    for what, value in (("vx", np.inf), ("vx", np.nan), ("m", np.inf)):
+        e = {k: d[k].copy() for k in keys}
+        e[what][7] = value
+        out = torch.zeros(4, dtype=torch.float64, device="cuda")
+        ctx.energy(*[dev(e[k]) for k in keys], 1.0, out)
+        ctx.sync()
+        k, u = out[0].item(), out[1].item()
+        assert np.isnan(k) if np.isnan(value) else k == np.inf
+        assert u == -np.inf if what == "m" else np.isfinite(u)
