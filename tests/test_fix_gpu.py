@@ -307,6 +307,31 @@ def test_thin_sheet(ctx, n, thickness):
     assert np.sqrt(((got[2] - ref[2]) ** 2).mean()) <= 1e-13 * scale
 
 
+@pytest.mark.parametrize("n,noalloc", [(2700, False), (5000, False), (20000, True), (60001, False)])
+def test_energy_adds_partials_without_loss(ctx, n, noalloc):
+    """One body with a kinetic energy of 1 and the rows (of 128 bodies) that its CTA takes to itself; the
+    other rows' bodies hold a few units of 2^-60, exact within a CTA: what remains is the one rounding of
+    the whole (half a unit in its last place, and the bits dropped 2^-111 below)."""
+    import torch
+    from fractions import Fraction
+    from nbody.lib import check, ptr, stream_ptr
+    d = bodies("plummer", n, seed=2)
+    for seed in range(12):
+        k = np.random.default_rng(seed).integers(0, 4, n).astype(np.float64)
+        k[:2560] = 0.0
+        vx = k * 2.0 ** -30
+        vx[0] = 1.0
+        out = torch.zeros(4, dtype=torch.float64, device="cuda")
+        t = [dev(np.full(n, 2.0))] + [dev(d[q]) for q in "xyz"] + [dev(vx), dev(k * 0), dev(k * 0)]
+        if noalloc:
+            check(ctx.lib.nb_energy_noalloc(*[ptr(v) for v in t], n, 0.0, ptr(out), stream_ptr()))
+        else:
+            ctx.energy(*t, 0.0, out)
+        ctx.sync()
+        exact = 1 + Fraction(int((k * k).sum()), 2 ** 60)
+        assert abs(Fraction(out[0].item()) - exact) <= Fraction(1, 2 ** 53) + Fraction(1, 2 ** 100)
+
+
 def test_energy_that_is_not_finite(ctx):
     import torch
     d = bodies("plummer", 400, seed=3)
