@@ -324,7 +324,8 @@ pair_sym_kernel(SymPlan S, const float4* __restrict__ src, float eps2,
 
 // FP64 form: the pair's separation, r^2 + eps^2 and r^-3 in fixed point (nb_fix.cuh), shared by the
 // two bodies, and a mass product each; FP64 sums, kept in registers for a whole row segment (i) or
-// rotated through the lanes (j). Pairs the fixed point cannot hold are added one side at a time.
+// rotated through the lanes (j). Pairs the fixed point cannot hold take the FP64 expressions, once for
+// both bodies; those with a massless body are added one side at a time.
 //  Bound: the FP64 pipe, 92% busy with 3 FMAs per ordered pair (10 FP64 operations before).
 //  65,536 bodies 76.8 -> 26.7 ms (56 -> 161 Gpairs/s), 16,384 4.96 -> 1.72 ms. Registers for 20
 //  warps per SM: 12, 16 and 24 warps measured 15%, 3% and 2% slower.
@@ -381,8 +382,8 @@ pair_sym_fix_kernel(SymPlan S, const nbfix::FixRec* __restrict__ src,
     const int sh_max = e2.sh_max;
     nbfix::FixRec I[P];
     double tx[P], ty[P], tz[P];
-    // Adds the pair (source at record f, body b) seen from the body `at` (record t) in FP64 or by
-    // the one-sided arithmetic: the pairs the loop below leaves.
+    // Adds the pair (source at record f, body b) seen from the body `at` (record t) by the one-sided
+    // arithmetic: pairs in which one body is massless.
     auto one_side = [&](const nbfix::FixRec& f, uint32_t b, const nbfix::FixRec& t, uint32_t at,
                         double& sx, double& sy, double& sz) {
         const nbfix::Fix3 p{t.x2, t.y2, t.z2, t.x1, t.y1, t.z1, t.x0, t.y0, t.z0, t.ml & 1u};
@@ -459,9 +460,23 @@ pair_sym_fix_kernel(SymPlan S, const nbfix::FixRec* __restrict__ src,
                         if (!ok) {  // pads, and what the fixed point cannot hold
                             const uint32_t li = a * IB + (w * P + k) * 32 + lane,
                                            lj = jt * JT + g * 32 + ((lane + s) & 31);
-                            if (li < count && lj < count) {
-                                one_side(J, off + lj, I[k], off + li, tx[k], ty[k], tz[k]);
-                                one_side(I[k], off + li, J, off + lj, jx, jy, jz);
+                            const uint32_t bi = off + li, bj = off + lj;
+                            if (li >= count || lj >= count) {
+                            } else if (sh_max >= 0 && min(J.e, I[k].e) == nbfix::ZERO_MASS) {
+                                one_side(J, bj, I[k], bi, tx[k], ty[k], tz[k]);
+                                one_side(I[k], bi, J, bj, jx, jy, jz);
+                            } else if (!nbfix::adds_nothing(J, bi == bj, K, sh_max, eps2)) {
+                                const double dx = x[bj] - x[bi], dy = y[bj] - y[bi],
+                                             dz = z[bj] - z[bi];
+                                const double c = nb_m_rinv3_f64(
+                                    1.0, fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
+                                const double sj = m[bj] * c, si = m[bi] * c;
+                                tx[k] = fma(dx, sj, tx[k]);
+                                ty[k] = fma(dy, sj, ty[k]);
+                                tz[k] = fma(dz, sj, tz[k]);
+                                jx = fma(-dx, si, jx);
+                                jy = fma(-dy, si, jy);
+                                jz = fma(-dz, si, jz);
                             }
                         }
                     }

@@ -345,3 +345,35 @@ def test_energy_that_is_not_finite(ctx):
         k, u = out[0].item(), out[1].item()
         assert np.isnan(k) if np.isnan(value) else k == np.inf
         assert u == -np.inf if what == "m" else np.isfinite(u)
+
+
+@pytest.mark.parametrize("what", ["negative", "massless", "subnormal", "outlier", "softening"])
+def test_symmetric_pairs_outside_the_fixed_point(ctx, what):
+    """What the symmetric kernel leaves to FP64: everything, or the pairs of some bodies. Bound as for the
+    lattice (the FP64 factor is within 2^-51, the sums within n 2^-53 of the terms' magnitudes)."""
+    from nbody.lib import SYM_ALWAYS, SYM_AUTO, set_naive_symmetric
+    n, eps2 = 700, 1e-6
+    d = bodies("plummer", n, seed=9)
+    if what == "negative":
+        d["m"][::3] *= -1.0
+    elif what == "massless":
+        d["m"][::2] = 0.0
+        d["m"][1::10] = -0.0
+    elif what == "subnormal":
+        d["m"][::3] = 1e-310
+    elif what == "outlier":
+        d["x"][5] = 1e14
+    else:
+        eps2 = 1e9
+    p = np.stack([d[k] for k in "xyz"])
+    q = p[:, None, :] - p[:, :, None]
+    r2 = (q ** 2).sum(axis=0) + eps2
+    bound = (n + 8) * 2.0 ** -52 * d["G"] * (np.abs(d["m"] * q) / (r2 * np.sqrt(r2))).sum(axis=2)
+    try:
+        set_naive_symmetric(SYM_ALWAYS)
+        got = naive(ctx, d, eps2, "f64")
+    finally:
+        set_naive_symmetric(SYM_AUTO)
+    ref = naive(ctx, d, eps2, "f64_ieee")
+    for g, r, b in zip(got, ref, bound):
+        assert np.isfinite(r).all() and (np.abs(g - r) <= b).all()
