@@ -808,14 +808,16 @@ __device__ __forceinline__ double leaf_quotient(double x, double m, double c) {
 // functions on the IBM RISC System/6000 processor", 1990): y = RN(1 / m) by Newton steps from the
 // hardware estimate (m's mantissa not all ones); q1 = q0 + r0 y is within one unit of the quotient
 // and q1 + r1 y with the exact remainder r1 = c - m q1 rounds to it. The IEEE division remains
-// outside a range in which every intermediate is normal.
+// outside a range in which every intermediate is normal, the quotients included (a subnormal one can
+// lie halfway between two doubles, where the last step's own rounding decides).
 __device__ __forceinline__ void exact_quotients(double cx, double cy, double cz, double m,
                                                 double& qx, double& qy, double& qz) {
     const int em = biased_exp(m);
     const uint64_t mant = (uint64_t)__double_as_longlong(m) & 0xfffffffffffffull;
     auto fits = [&](double c) {
         const int e = biased_exp(c);
-        return (e >= 300 && e <= 1700) || ((__double_as_longlong(c) << 1) == 0);
+        return (e >= 300 && e <= 1700 && abs(e - em) < 960) ||
+               ((__double_as_longlong(c) << 1) == 0);
     };
     if (em < 300 || em > 1700 || mant == 0xfffffffffffffull || !fits(cx) || !fits(cy) ||
         !fits(cz)) {

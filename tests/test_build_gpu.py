@@ -144,3 +144,17 @@ def test_many_cells_across_chunks(ctx, clumps):
     and one below; one and two tiers. The clumps' cores are smaller than the FP32 records resolve, so
     the walk's opening tests there have to be left to FP64."""
     check(ctx, _nested(clumps, 28, 9, clumps), storage=512)
+
+
+def test_subnormal_quotients(ctx):
+    """Cells whose centre's z lies halfway between two subnormal numbers: (4 * 1 + 1 * 5) / 6 of the
+    smallest one and the like, with masses that keep the numerators normal."""
+    tiny = 2.0 ** -1074
+    rng = np.random.default_rng(6)
+    rows = []
+    for i, (a, b) in enumerate([(4, 1), (13, 1), (7, 10), (1, 4), (2, 5), (16, 13), (21, 0), (0, 3)]):
+        x, y = -1.5 + 0.4 * i, rng.uniform(-1.0, 1.0)
+        rows += [(2.0 ** 400, x, y, a * tiny), (5 * 2.0 ** 400, x + 2.0 ** -11, y, b * tiny),
+                 (1.0, x + 0.1, y + 0.2, 0.0)]
+    m, x, y, z = np.array(rows).T.copy()
+    check(ctx, {"m": m, "x": x, "y": y, "z": z, "G": 1.0}, storage=64)
