@@ -29,20 +29,36 @@ nb_status check_launch(const char* what) {
     return NB_OK;
 }
 
-nb_status scratch(nb_ctx* ctx, int slot, size_t bytes, void** out) {
+bool is_capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        cudaGetLastError();  // the legacy stream beside another stream's capture
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
+nb_status scratch(nb_ctx* ctx, int slot, size_t bytes, cudaStream_t stream, void** out) {
     nb_scratch_buf& b = ctx->scratch[slot];
     if (b.bytes < bytes) {
-        if (b.ptr) {
+        if (b.ptr && b.captured) {
+            try {
+                ctx->outgrown.push_back(b.ptr);
+            } catch (...) {
+                return set_error(NB_ERR_OOM, "scratch: no host memory");
+            }
+            b = nb_scratch_buf{};
+        } else if (b.ptr) {
             // the previous user of this slot may still be running on some stream
             NB_CUDA_TRY(cudaDeviceSynchronize());
             NB_CUDA_TRY(cudaFree(b.ptr));
-            b.ptr = nullptr;
-            b.bytes = 0;
+            b = nb_scratch_buf{};
         }
         size_t want = bytes < 256 ? 256 : bytes;
         NB_CUDA_TRY(cudaMalloc(&b.ptr, want));
         b.bytes = want;
     }
+    if (!b.captured) b.captured = is_capturing(stream);
     *out = b.ptr;
     return NB_OK;
 }
@@ -87,6 +103,7 @@ nb_status nb_ctx_destroy(nb_ctx* ctx) {
         if (b.ptr) cudaFree(b.ptr);
         b.ptr = nullptr;
     }
+    for (void* p : ctx->outgrown) cudaFree(p);
     if (ctx->dev_error) cudaFree(ctx->dev_error);
     if (ctx->dev_counter) cudaFree(ctx->dev_counter);
     delete ctx;

@@ -454,7 +454,8 @@ nb_status launch_aabb(nb_ctx* ctx, const double* x, const double* y, const doubl
     if (blocks > ctx->sm_count * 4) blocks = ctx->sm_count * 4;
     if (blocks < 1) blocks = 1;
     void* part = nullptr;
-    NB_TRY(nb::scratch(ctx, NB_SCRATCH_AABB, (size_t)blocks * sizeof(MinMax6), &part));
+    NB_TRY(nb::scratch(ctx, NB_SCRATCH_AABB, (size_t)blocks * sizeof(MinMax6), stream,
+                       &part));
     NB_CUDA_TRY(nb::launch_after(aabb_kernel, blocks, AABB_THREADS, 0, stream, x, y, z, n,
                                  (MinMax6*)part, ctx->dev_counter + 0, out_dev));
     return NB_OK;
@@ -514,7 +515,8 @@ nb_status nb_energy(nb_ctx* ctx, const double* m, const double* x, const double*
     const EnergyShape e = energy_shape(n, ctx->sm_count, 0xffffffffu);
     const size_t part_bytes = (size_t)e.ctas * sizeof(double2);
     void* part = nullptr;
-    NB_TRY(nb::scratch(ctx, NB_SCRATCH_ENERGY, part_bytes + nbfix::SCALE_WORDS * sizeof(uint32_t), &part));
+    NB_TRY(nb::scratch(ctx, NB_SCRATCH_ENERGY, part_bytes + nbfix::SCALE_WORDS * sizeof(uint32_t),
+                       (cudaStream_t)stream, &part));
     return energy_launch(e, m, x, y, z, vx, vy, vz, n, G, (uint32_t*)((char*)part + part_bytes),
                          (double2*)part, out_dev, (cudaStream_t)stream);
 }

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <string>
+#include <vector>
 
 #include "nbody.h"
 
@@ -28,6 +29,7 @@ constexpr unsigned long long NB_WAIT_LIMIT_DEFAULT = 1ull << 22;
 struct nb_scratch_buf {
     void* ptr = nullptr;
     size_t bytes = 0;
+    bool captured = false;  // a captured graph holds its address
 };
 
 enum nb_scratch_slot : int {
@@ -61,6 +63,7 @@ struct nb_ctx {
     uint32_t* dev_error = nullptr;  // device error word (NB_DEVERR_* bits)
     unsigned int* dev_counter = nullptr;  // last-block-done counters for fused grid reductions
     nb_scratch_buf scratch[NB_SCRATCH_COUNT];
+    std::vector<void*> outgrown;  // captured scratch that a larger buffer has replaced
     // failure-path test hooks (nb_ctx_set_fault_hooks)
     unsigned long long wait_limit = NB_WAIT_LIMIT_DEFAULT;
     unsigned int fault_flags = 0;
@@ -73,8 +76,11 @@ namespace nb {
 
 nb_status set_error(nb_status st, const char* fmt, ...);
 nb_status cuda_error(cudaError_t err, const char* what);
-// Grows scratch slot `slot` of the context to at least `bytes` (cudaMalloc; synchronous).
-nb_status scratch(nb_ctx* ctx, int slot, size_t bytes, void** out);
+// Grows scratch slot `slot` of the context to at least `bytes` (cudaMalloc; synchronous) for work on
+// `stream`. A buffer handed out during a capture stays allocated until the context is destroyed, since
+// graphs that replay on it may live as long.
+nb_status scratch(nb_ctx* ctx, int slot, size_t bytes, cudaStream_t stream, void** out);
+bool is_capturing(cudaStream_t stream);
 nb_status check_launch(const char* what);
 
 // Enqueues the words of nbfix::block_scale for a system's coordinates: k_part has room for

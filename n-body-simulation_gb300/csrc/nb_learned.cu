@@ -1197,7 +1197,7 @@ nb_status nb_bh_generate_pairs(nb_ctx* ctx, const nb_bh_tree* t, const double* m
         return nb::set_error(NB_ERR_INVALID_ARG, "nb_bh_generate_pairs: bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
     void* buf = nullptr;
-    NB_TRY(nb::scratch(ctx, NB_SCRATCH_LABELS, (size_t)max_pairs * sizeof(uint2), &buf));
+    NB_TRY(nb::scratch(ctx, NB_SCRATCH_LABELS, (size_t)max_pairs * sizeof(uint2), s, &buf));
     NB_CUDA_TRY(cudaMemsetAsync(count_dev, 0, sizeof(uint32_t), s));
     const uint32_t warps = (t->n + 31) / 32;
     const uint32_t threshold = (uint32_t)(sample_fraction * 4294967295.0);

@@ -337,7 +337,7 @@ nb_status naive_sym(nb_ctx* ctx, int form, const double* m, const double* x, con
     const size_t pi_bytes = al(nb::sym_part_i_bytes(form, cfg, hp.ctas, hp.n_blocks));
     void* base = nullptr;
     NB_TRY(nb::scratch(ctx, NB_SCRATCH_PAIR_SYM, table_bytes + src_bytes + pi_bytes + pj_bytes,
-                       &base));
+                       stream, &base));
     char* b = (char*)base;
     nbsym::SymSys* table = (nbsym::SymSys*)b;
     NB_TRY(nb::sym_single_table(table, hp, stream));
@@ -387,7 +387,7 @@ nb_status naive_f32c(nb_ctx* ctx, const double* m, const double* x, const double
     const size_t part_bytes = nb::pair_partial_floats(cfg, (uint32_t)ctas, n_ib) * sizeof(float);
     void* base = nullptr;
     NB_TRY(nb::scratch(ctx, NB_SCRATCH_NAIVE_F32, plan_bytes + src_bytes + tgt_bytes + part_bytes,
-                       &base));
+                       stream, &base));
     char* b = (char*)base;
     uint64_t* unit_off = (uint64_t*)b;
     uint32_t* sys_off = (uint32_t*)(b + 64);
@@ -532,7 +532,7 @@ nb_status naive_df64(nb_ctx* ctx, const double* m, const double* x, const double
     const size_t src_bytes = ((size_t)n * sizeof(SrcTF) + 255) & ~(size_t)255;
     const size_t part_bytes = chunks > 1 ? (size_t)chunks * n_t * 3 * sizeof(double) : 0;
     void* base = nullptr;
-    NB_TRY(nb::scratch(ctx, NB_SCRATCH_NAIVE_DF, src_bytes + part_bytes, &base));
+    NB_TRY(nb::scratch(ctx, NB_SCRATCH_NAIVE_DF, src_bytes + part_bytes, stream, &base));
     SrcTF* src = (SrcTF*)base;
     double* part = (double*)((char*)base + src_bytes);
     df_prepare_kernel<<<nb::ceil_div(n, 256), 256, 0, stream>>>(m, x, y, z, n, G, src);
@@ -567,23 +567,18 @@ nb_status naive_fix(nb_ctx* ctx, const double* m, const double* x, const double*
     uint32_t chunk = std::max<uint32_t>((uint32_t)nb::ceil_div(n, chunks), FX_CHUNK_MIN);
     if (chunk > FX_THREADS) chunk = (uint32_t)nb::ceil_div(chunk, FX_THREADS) * FX_THREADS;
     chunks = (uint32_t)nb::ceil_div(n, chunk);
-    size_t part_bytes = chunks > 1 ? (size_t)chunks * n_t * 3 * sizeof(double) : 0;
-    if (part_bytes > ctx->scratch[NB_SCRATCH_NAIVE_DF].bytes) {
-        // a stream being captured cannot wait for an allocation: one chunk needs none
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        NB_CUDA_TRY(cudaStreamIsCapturing(stream, &capture));
-        if (capture != cudaStreamCaptureStatusNone) {
-            chunk = (uint32_t)nb::ceil_div(n, FX_THREADS) * FX_THREADS;
-            chunks = 1;
-            part_bytes = 0;
-        }
+    // A capture that finds no scratch large enough cannot wait for an allocation: the partials are then
+    // the graph's own memory. (So the chunks, and with them the sums' order, never depend on what ran
+    // before.)
+    const size_t part_bytes = chunks > 1 ? (size_t)chunks * n_t * 3 * sizeof(double) : 0;
+    const bool own = part_bytes > ctx->scratch[NB_SCRATCH_NAIVE_DF].bytes && nb::is_capturing(stream);
+    void* base = nullptr;
+    if (own) {
+        NB_CUDA_TRY(cudaMallocAsync(&base, part_bytes, stream));
+    } else if (chunks > 1) {
+        NB_TRY(nb::scratch(ctx, NB_SCRATCH_NAIVE_DF, part_bytes, stream, &base));
     }
-    double* part = nullptr;
-    if (chunks > 1) {
-        void* base = nullptr;
-        NB_TRY(nb::scratch(ctx, NB_SCRATCH_NAIVE_DF, part_bytes, &base));
-        part = (double*)base;
-    }
+    double* part = (double*)base;
     NB_CUDA_TRY(nb::launch_after(naive_fix_kernel, dim3(blocks, chunks), FX_THREADS, 0, stream, m, x,
                                  y, z, ax, ay, az, n, targets, i_begin, n_t, G, eps2, chunk, part,
                                  k_part, k_words));
@@ -591,6 +586,7 @@ nb_status naive_fix(nb_ctx* ctx, const double* m, const double* x, const double*
     const uint32_t first = targets != nullptr ? 0 : i_begin;
     NB_CUDA_TRY(nb::launch_after(chunk_combine_kernel, nb::ceil_div(n_t, 32), 32 * CC_WARPS, 0, stream,
                                  part, chunks, first, first + n_t, ax, ay, az));
+    if (own) NB_CUDA_TRY(cudaFreeAsync(base, stream));
     return NB_OK;
 }
 
