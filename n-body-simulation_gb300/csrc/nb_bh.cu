@@ -164,8 +164,8 @@ __device__ __forceinline__ void build_zero(const BuildZero& Z, uint32_t i, uint3
     }
 }
 
-__global__ void keys_quantized_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                                      const double* __restrict__ z, uint32_t n,
+__global__ void keys_quantized_kernel(const double* x, const double* y,
+                                      const double* z, uint32_t n,
                                       double* __restrict__ box, uint64_t* __restrict__ key0,
                                       uint32_t* __restrict__ ids, BuildZero Z) {
     nb_grid_wait();
@@ -237,8 +237,8 @@ __device__ __forceinline__ uint64_t exact_key(const double* __restrict__ box, co
 }
 
 __global__ void __launch_bounds__(BH_THREADS)
-keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
-            const double* __restrict__ z, uint32_t n, double* __restrict__ box,
+keys_kernel(const double* x, const double* y,
+            const double* z, uint32_t n, double* __restrict__ box,
             uint64_t* __restrict__ key0, uint32_t* __restrict__ ids, BuildZero Z) {
     __shared__ FixedGrid grid_s;  // once per block: it takes an FP64 division
     nb_grid_wait();
@@ -288,9 +288,9 @@ __device__ __forceinline__ void fix_run(uint32_t p, const double* __restrict__ x
     }
 }
 
-__global__ void runs_fixup_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                                  const double* __restrict__ z, uint32_t n,
-                                  const double* __restrict__ box, const uint64_t* __restrict__ key0,
+__global__ void runs_fixup_kernel(const double* x, const double* y,
+                                  const double* z, uint32_t n,
+                                  const double* box, const uint64_t* key0,
                                   uint64_t* __restrict__ key1, uint32_t* __restrict__ ids,
                                   uint32_t* __restrict__ err, int quantized) {
     nb_grid_wait();
@@ -364,7 +364,7 @@ __device__ __forceinline__ void split_at(uint32_t j, const uint64_t* __restrict_
     atomicOr(&mask[a], 1ull << L);
 }
 
-__global__ void splits_kernel(const uint64_t* __restrict__ key0, const uint64_t* __restrict__ key1,
+__global__ void splits_kernel(const uint64_t* key0, const uint64_t* key1,
                               uint32_t n, uint8_t* __restrict__ split_level,
                               uint32_t* __restrict__ split_start, uint32_t* __restrict__ split_end,
                               unsigned long long* __restrict__ mask, uint32_t* __restrict__ children,
@@ -451,13 +451,13 @@ __device__ __forceinline__ void emit_at(uint32_t p, uint32_t n, const uint32_t* 
     }
 }
 
-__global__ void emit_kernel(uint32_t n, const uint32_t* __restrict__ ids,
-                            const uint8_t* __restrict__ split_level,
-                            const uint32_t* __restrict__ split_start,
-                            const uint32_t* __restrict__ split_end,
-                            const unsigned long long* __restrict__ mask,
-                            const uint32_t* __restrict__ base, const uint64_t* __restrict__ key0,
-                            const uint64_t* __restrict__ key1, NodeTable T) {
+__global__ void emit_kernel(uint32_t n, const uint32_t* ids,
+                            const uint8_t* split_level,
+                            const uint32_t* split_start,
+                            const uint32_t* split_end,
+                            const unsigned long long* mask,
+                            const uint32_t* base, const uint64_t* key0,
+                            const uint64_t* key1, NodeTable T) {
     nb_grid_wait();
     emit_at(blockIdx.x * blockDim.x + threadIdx.x, n, ids, split_level, split_start, split_end,
             mask, base, key0, key1, T);
@@ -502,8 +502,8 @@ __device__ __forceinline__ uint32_t small_block_scan(uint32_t v, uint32_t* warp_
 
 template <uint32_t CAP, uint32_t THREADS>
 __global__ void __launch_bounds__(THREADS)
-build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                   const double* __restrict__ z, uint32_t n, double* __restrict__ box,
+build_small_kernel(const double* x, const double* y,
+                   const double* z, uint32_t n, double* __restrict__ box,
                    uint64_t* __restrict__ key0_out, uint64_t* __restrict__ key1_out,
                    uint32_t* __restrict__ ids_out, unsigned long long* __restrict__ mask_out,
                    uint32_t* __restrict__ base_out, NodeTable T, uint32_t* __restrict__ err,
@@ -526,9 +526,6 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
     __shared__ double sbox[BOX_WORDS];
     __shared__ FixedGrid grid_s;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // children lists start empty; written before the barriers below, filled after them
-    for (uint32_t k = tid; k < 4 * n; k += THREADS)
-        reinterpret_cast<uint4*>(T.children)[k] = make_uint4(NB_NONE, NB_NONE, NB_NONE, NB_NONE);
     // box, with the reference's zero-initialised bounds
     double px[PER], py[PER], pz[PER];
     const long long zero = nbaabb::ord_of(0.0);
@@ -540,6 +537,13 @@ build_small_kernel(const double* __restrict__ x, const double* __restrict__ y,
         px[h] = in ? x[i] : 0.0;
         py[h] = in ? y[i] : 0.0;
         pz[h] = in ? z[i] : 0.0;
+    }
+    // children lists start empty; written before the barriers below, filled after them
+    for (uint32_t k = tid; k < 4 * n; k += THREADS)
+        reinterpret_cast<uint4*>(T.children)[k] = make_uint4(NB_NONE, NB_NONE, NB_NONE, NB_NONE);
+#pragma unroll
+    for (int h = 0; h < PER; ++h) {
+        const bool in = tid * PER + h < n;
         const long long o[3] = {nbaabb::ord_of(px[h]), nbaabb::ord_of(py[h]),
                                 nbaabb::ord_of(pz[h])};
 #pragma unroll
@@ -1396,8 +1400,8 @@ constexpr size_t tier_smem_bytes(bool learned) {
 constexpr uint32_t KID_NONE = 0xffff, KID_OUTSIDE = 0xfffe;  // else a place in the tier's list
 
 __global__ void __launch_bounds__(CC_THREADS)
-com_tier_kernel(ComArgs A, uint32_t span, const uint2* __restrict__ in,
-                const uint32_t* __restrict__ in_count, uint32_t in_chunks, uint2* up,
+com_tier_kernel(ComArgs A, uint32_t span, const uint2* in,
+                const uint32_t* in_count, uint32_t in_chunks, uint2* up,
                 uint32_t* up_count) {
     extern __shared__ __align__(16) unsigned char com_smem[];
     const bool learned = (A.records & NB_REC_LEARNED) != 0;

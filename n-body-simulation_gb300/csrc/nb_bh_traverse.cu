@@ -77,22 +77,38 @@ struct Arith<FAST64> {
 
 using nbfix::FixRec;
 
-// 32-byte loads (one instruction of the load pipe instead of two).
-__device__ __forceinline__ NodeRec32 load_rec32(const NodeRec32* __restrict__ p) {
+// 32-byte loads (one instruction of the load pipe instead of two). READ_ONLY: of memory that nothing
+// writes while the kernel runs; otherwise (dependent launches) volatile, as the wait before them.
+template <bool READ_ONLY = true>
+__device__ __forceinline__ NodeRec32 load_rec32(const NodeRec32* p) {
     NodeRec32 r;
-    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(r.cx), "=f"(r.cy), "=f"(r.cz), "=f"(r.gm), "=f"(r.edge2), "=r"(r.skip),
-          "=r"(r.body), "=r"(r.level)
-        : "l"(p));
+    if constexpr (READ_ONLY)
+        asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(r.cx), "=f"(r.cy), "=f"(r.cz), "=f"(r.gm), "=f"(r.edge2), "=r"(r.skip),
+              "=r"(r.body), "=r"(r.level)
+            : "l"(p));
+    else
+        asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(r.cx), "=f"(r.cy), "=f"(r.cz), "=f"(r.gm), "=f"(r.edge2), "=r"(r.skip),
+                       "=r"(r.body), "=r"(r.level)
+                     : "l"(p)
+                     : "memory");
     return r;
 }
-__device__ __forceinline__ FixRec load_fix(const nbfix::FixHi* __restrict__ hi,
-                                           const uint4* __restrict__ lo, uint32_t k) {
+template <bool READ_ONLY = true>
+__device__ __forceinline__ FixRec load_fix(const nbfix::FixHi* hi, const uint4* lo, uint32_t k) {
     FixRec r;
-    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(r.x2), "=r"(r.y2), "=r"(r.z2), "=r"(r.mh), "=r"(r.x1), "=r"(r.y1), "=r"(r.z1),
-          "=r"(r.e)
-        : "l"(hi + k));
+    if constexpr (READ_ONLY)
+        asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(r.x2), "=r"(r.y2), "=r"(r.z2), "=r"(r.mh), "=r"(r.x1), "=r"(r.y1), "=r"(r.z1),
+              "=r"(r.e)
+            : "l"(hi + k));
+    else
+        asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r.x2), "=r"(r.y2), "=r"(r.z2), "=r"(r.mh), "=r"(r.x1), "=r"(r.y1),
+                       "=r"(r.z1), "=r"(r.e)
+                     : "l"(hi + k)
+                     : "memory");
     const uint4 l = lo[k];
     r.x0 = l.x;
     r.y0 = l.y;
@@ -475,11 +491,11 @@ constexpr int TEAM_BLOCKS_PER_SM = 5;
 
 template <int T>
 __global__ void __launch_bounds__(TR_THREADS, TEAM_BLOCKS_PER_SM)
-bh_theta_team_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __restrict__ rec64,
-                     const nbfix::FixHi* __restrict__ fix_hi, const uint4* __restrict__ fix_lo,
-                     const uint32_t* __restrict__ info, const uint32_t* __restrict__ ids,
-                     const double* __restrict__ x, const double* __restrict__ y,
-                     const double* __restrict__ z, const double* __restrict__ box, uint32_t n,
+bh_theta_team_kernel(const NodeRec32* rec32, const NodeRec64* rec64,
+                     const nbfix::FixHi* fix_hi, const uint4* fix_lo,
+                     const uint32_t* info, const uint32_t* ids,
+                     const double* x, const double* y,
+                     const double* z, const double* box, uint32_t n,
                      Theta theta, double eps2, double G, double* __restrict__ ax,
                      double* __restrict__ ay, double* __restrict__ az,
                      uint32_t* __restrict__ walk_len) {
@@ -517,7 +533,7 @@ bh_theta_team_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
             bool take = false;
             uint32_t end = 0;  // inclusive prefix maximum of the accepted nodes' skip links
             if (active && idx >= k && idx < nn) {
-                const NodeRec32 r = load_rec32(rec32 + idx);
+                const NodeRec32 r = load_rec32<false>(rec32 + idx);
                 const bool accept = accepts(r, pre, rec64, idx, x, y, z, me, theta);
                 take = accept && r.body != me;
                 if (accept) end = r.skip;
@@ -540,10 +556,10 @@ bh_theta_team_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
         if (most == 0) break;
         __syncwarp();
         int i = (j - ord) & (T - 1);
-        FixRec next = load_fix(fix_hi, fix_lo, i < cnt ? list[i] : 0u);
+        FixRec next = load_fix<false>(fix_hi, fix_lo, i < cnt ? list[i] : 0u);
         for (int c = 0; c < most; c += T, i += T) {
             const FixRec f = next;
-            if (i + T < cnt) next = load_fix(fix_hi, fix_lo, list[i + T]);
+            if (i + T < cnt) next = load_fix<false>(fix_hi, fix_lo, list[i + T]);
             if (i < cnt)
                 fix_monopole(f, rec64, list[i], body, K, e2, x, y, z, me, eps2, acx, acy, acz);
         }

@@ -13,40 +13,43 @@ constexpr int EW_THREADS = 256;
 // NaiveAlgorithm.cpp:154-163 / BarnesHutAlgorithm.cpp:171-181. Each statement is a separately
 // rounded multiply and add, exactly as the reference writes it.
 __global__ void kick_drift_kernel(double* __restrict__ vhx, double* __restrict__ vhy,
-                                  double* __restrict__ vhz, const double* __restrict__ vx,
-                                  const double* __restrict__ vy, const double* __restrict__ vz,
+                                  double* __restrict__ vhz, const double* vx,
+                                  const double* vy, const double* vz,
                                   double* __restrict__ x, double* __restrict__ y,
-                                  double* __restrict__ z, const double* __restrict__ ax,
-                                  const double* __restrict__ ay, const double* __restrict__ az,
+                                  double* __restrict__ z, const double* ax,
+                                  const double* ay, const double* az,
                                   uint32_t n, double dt) {
     nb_grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double h = dt / 2.0;
+    const double h = dt / 2.0, px = x[i], py = y[i], pz = z[i];
     const double hx = __dadd_rn(vx[i], __dmul_rn(ax[i], h));
     const double hy = __dadd_rn(vy[i], __dmul_rn(ay[i], h));
     const double hz = __dadd_rn(vz[i], __dmul_rn(az[i], h));
     vhx[i] = hx;
     vhy[i] = hy;
     vhz[i] = hz;
-    x[i] = __dadd_rn(x[i], __dmul_rn(hx, dt));
-    y[i] = __dadd_rn(y[i], __dmul_rn(hy, dt));
-    z[i] = __dadd_rn(z[i], __dmul_rn(hz, dt));
+    x[i] = __dadd_rn(px, __dmul_rn(hx, dt));
+    y[i] = __dadd_rn(py, __dmul_rn(hy, dt));
+    z[i] = __dadd_rn(pz, __dmul_rn(hz, dt));
 }
 
 // NaiveAlgorithm.cpp:217-221 / BarnesHutAlgorithm.cpp:234-238.
 __global__ void kick_kernel(double* __restrict__ vx, double* __restrict__ vy,
-                            double* __restrict__ vz, const double* __restrict__ vhx,
-                            const double* __restrict__ vhy, const double* __restrict__ vhz,
-                            const double* __restrict__ ax, const double* __restrict__ ay,
-                            const double* __restrict__ az, uint32_t n, double dt) {
+                            double* __restrict__ vz, const double* vhx,
+                            const double* vhy, const double* vhz,
+                            const double* ax, const double* ay,
+                            const double* az, uint32_t n, double dt) {
     nb_grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double h = dt / 2.0;
-    vx[i] = __dadd_rn(vhx[i], __dmul_rn(ax[i], h));
-    vy[i] = __dadd_rn(vhy[i], __dmul_rn(ay[i], h));
-    vz[i] = __dadd_rn(vhz[i], __dmul_rn(az[i], h));
+    const double nvx = __dadd_rn(vhx[i], __dmul_rn(ax[i], h));
+    const double nvy = __dadd_rn(vhy[i], __dmul_rn(ay[i], h));
+    const double nvz = __dadd_rn(vhz[i], __dmul_rn(az[i], h));
+    vx[i] = nvx;
+    vy[i] = nvy;
+    vz[i] = nvz;
 }
 
 // Part 2 of one step followed by part 1 of the next: v = vh + a*dt/2; vh = v + a*dt/2;
@@ -55,13 +58,13 @@ __global__ void kick_kick_drift_kernel(double* __restrict__ vx, double* __restri
                                        double* __restrict__ vz, double* __restrict__ vhx,
                                        double* __restrict__ vhy, double* __restrict__ vhz,
                                        double* __restrict__ x, double* __restrict__ y,
-                                       double* __restrict__ z, const double* __restrict__ ax,
-                                       const double* __restrict__ ay,
-                                       const double* __restrict__ az, uint32_t n, double dt) {
+                                       double* __restrict__ z, const double* ax,
+                                       const double* ay,
+                                       const double* az, uint32_t n, double dt) {
     nb_grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double h = dt / 2.0;
+    const double h = dt / 2.0, px = x[i], py = y[i], pz = z[i];
     const double kx = __dmul_rn(ax[i], h), ky = __dmul_rn(ay[i], h), kz = __dmul_rn(az[i], h);
     const double nvx = __dadd_rn(vhx[i], kx), nvy = __dadd_rn(vhy[i], ky),
                  nvz = __dadd_rn(vhz[i], kz);
@@ -72,9 +75,9 @@ __global__ void kick_kick_drift_kernel(double* __restrict__ vx, double* __restri
     vhx[i] = hx;
     vhy[i] = hy;
     vhz[i] = hz;
-    x[i] = __dadd_rn(x[i], __dmul_rn(hx, dt));
-    y[i] = __dadd_rn(y[i], __dmul_rn(hy, dt));
-    z[i] = __dadd_rn(z[i], __dmul_rn(hz, dt));
+    x[i] = __dadd_rn(px, __dmul_rn(hx, dt));
+    y[i] = __dadd_rn(py, __dmul_rn(hy, dt));
+    z[i] = __dadd_rn(pz, __dmul_rn(hz, dt));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -346,8 +349,8 @@ scale_kernel(const double* __restrict__ x, const double* __restrict__ y,
 }
 
 __global__ void __launch_bounds__(AABB_THREADS)
-aabb_kernel(const double* __restrict__ x, const double* __restrict__ y,
-            const double* __restrict__ z, uint32_t n, MinMax6* __restrict__ part,
+aabb_kernel(const double* x, const double* y,
+            const double* z, uint32_t n, MinMax6* __restrict__ part,
             unsigned int* __restrict__ counter, double* __restrict__ out) {
     nb_grid_wait();
     const long long zero = ord_of(0.0);

@@ -158,7 +158,9 @@ __device__ __forceinline__ float nb_rsqrt_f32(float x) {
 // earlier launches write, returns when that kernel has finished and its writes are visible, and
 // lets the next dependent launch start in turn. (So everything before the preceding kernel has
 // finished already when a dependent one starts.) Saves the gap between the short launches of a
-// chain, 1 to 1.5 us each.
+// chain, 1 to 1.5 us each. Since what it reads is written while it may run already, such a kernel has
+// no const __restrict__ parameters and no ld.global.nc: read-only loads are for memory that nothing
+// writes during the kernel, and the compiler need not keep them behind the wait.
 __device__ __forceinline__ void nb_grid_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -912,8 +912,8 @@ __global__ void mlp_zero_kernel(float* __restrict__ grad, float* __restrict__ lo
 }
 
 __global__ void __launch_bounds__(TR_BLOCK)
-mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
-                const float* __restrict__ Y, const uint32_t* __restrict__ idx, uint32_t n,
+mlp_grad_kernel(const float* P, const float* X,
+                const float* Y, const uint32_t* idx, uint32_t n,
                 float* __restrict__ grad, float* __restrict__ loss) {
     __shared__ __align__(16) float w[(P_COUNT + 3) / 4 * 4];
     __shared__ __align__(16) float sx[TR_CHUNK][NF], sh1[TR_CHUNK][TR_ROW], sh2[TR_CHUNK][TR_ROW];
@@ -1053,7 +1053,7 @@ mlp_grad_kernel(const float* __restrict__ P, const float* __restrict__ X,
 }
 
 __global__ void mlp_adam_kernel(float* __restrict__ P, float* __restrict__ M, float* __restrict__ V,
-                                const float* __restrict__ grad, float lr, float b1, float b2,
+                                const float* grad, float lr, float b1, float b2,
                                 float eps, float c1, float c2) {
     nb_grid_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;

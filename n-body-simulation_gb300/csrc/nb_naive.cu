@@ -126,12 +126,12 @@ constexpr uint32_t FX_CHUNKS_MAX = 128, FX_CHUNK_MIN = 4;
 static_assert(NB_COUNTER_WORDS - NB_COUNTER_SCALE >= (int)nbfix::SCALE_WORDS, "scale words");
 
 __global__ void __launch_bounds__(FX_THREADS, FX_BLOCKS_PER_SM)
-naive_fix_kernel(const double* __restrict__ m, const double* __restrict__ x,
-                 const double* __restrict__ y, const double* __restrict__ z,
+naive_fix_kernel(const double* m, const double* x,
+                 const double* y, const double* z,
                  double* __restrict__ ax, double* __restrict__ ay, double* __restrict__ az,
-                 uint32_t n, const uint32_t* __restrict__ targets, uint32_t i_begin, uint32_t n_t,
+                 uint32_t n, const uint32_t* targets, uint32_t i_begin, uint32_t n_t,
                  double G, double eps2, uint32_t chunk, double* __restrict__ part,
-                 const uint32_t* __restrict__ k_part, uint32_t k_words) {
+                 const uint32_t* k_part, uint32_t k_words) {
     nb_grid_wait();
     __shared__ nbfix::FixRec src[FX_THREADS];
     __shared__ nbfix::Eps2Table e2;
@@ -179,14 +179,15 @@ naive_fix_kernel(const double* __restrict__ m, const double* __restrict__ x,
 constexpr int FXC_CTAS = 8, FXC_WARPS = 8, FXC_THREADS = 32 * FXC_WARPS;
 constexpr uint32_t FXC_MAX_N = 2048;
 static_assert(FXC_MAX_N <= nbfix::SCALE_SCAN_N, "one launch");
+static_assert(FXC_MAX_N <= FXC_CTAS * FXC_THREADS, "a CTA's share of the sources is one tile");
 
 __global__ void __cluster_dims__(FXC_CTAS, 1, 1) __launch_bounds__(FXC_THREADS)
-naive_fix_cluster_kernel(const double* __restrict__ m, const double* __restrict__ x,
-                         const double* __restrict__ y, const double* __restrict__ z,
+naive_fix_cluster_kernel(const double* m, const double* x,
+                         const double* y, const double* z,
                          double* __restrict__ ax, double* __restrict__ ay,
                          double* __restrict__ az, uint32_t n,
-                         const uint32_t* __restrict__ targets, uint32_t i_begin, uint32_t n_t,
-                         double G, double eps2, const uint32_t* __restrict__ k_part,
+                         const uint32_t* targets, uint32_t i_begin, uint32_t n_t,
+                         double G, double eps2, const uint32_t* k_part,
                          uint32_t k_words) {
     nb_grid_wait();
     namespace cg = cooperative_groups;
@@ -196,27 +197,30 @@ naive_fix_cluster_kernel(const double* __restrict__ m, const double* __restrict_
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank();
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int K = nbfix::block_scale(x, y, z, n, k_part, k_words);
-    nbfix::fill_eps2(e2, eps2, K);
-    __syncthreads();
     const uint32_t t = (blockIdx.x / FXC_CTAS) * 32 + lane;
     const bool active = t < n_t;
     const uint32_t i = active ? (targets != nullptr ? targets[t] : i_begin + t) : 0u;
-    nbfix::Fix3 p;
-    const int sh_max = nbfix::split3(x[i], y[i], z[i], K, p) ? e2.sh_max : -1;
-    FixSums acc{0.0, 0.0, 0.0};
     const uint32_t share = (n + FXC_CTAS - 1) / FXC_CTAS;
-    const uint32_t j0 = min(n, rank * share), j1 = min(n, j0 + share);
-    for (uint32_t k = j0; k < j1; k += FXC_THREADS) {
-        const uint32_t j = k + threadIdx.x;
-        __syncthreads();
-        if (j < j1) src[threadIdx.x] = nbfix::make_rec(x[j], y[j], z[j], m[j], K);
-        __syncthreads();
-        const uint32_t cnt = min((uint32_t)FXC_THREADS, j1 - k);
-#pragma unroll 1
-        for (uint32_t jj = w; jj < cnt; jj += FXC_WARPS)
-            fix_pair(src[jj], k + jj, i, p, K, e2, sh_max, eps2, m, x, y, z, acc);
+    const uint32_t j0 = min(n, rank * share), j1 = min(n, j0 + share), j = j0 + threadIdx.x;
+    // the target and this thread's source, requested before the scan for the scale
+    const double px = x[i], py = y[i], pz = z[i];
+    double jx = 0.0, jy = 0.0, jz = 0.0, jm = 0.0;
+    if (j < j1) {
+        jx = x[j];
+        jy = y[j];
+        jz = z[j];
+        jm = m[j];
     }
+    const int K = nbfix::block_scale(x, y, z, n, k_part, k_words);
+    nbfix::fill_eps2(e2, eps2, K);
+    if (j < j1) src[threadIdx.x] = nbfix::make_rec(jx, jy, jz, jm, K);
+    __syncthreads();
+    nbfix::Fix3 p;
+    const int sh_max = nbfix::split3(px, py, pz, K, p) ? e2.sh_max : -1;
+    FixSums acc{0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (uint32_t jj = w; jj < j1 - j0; jj += FXC_WARPS)
+        fix_pair(src[jj], j0 + jj, i, p, K, e2, sh_max, eps2, m, x, y, z, acc);
     sums[w][0][lane] = acc.x;
     sums[w][1][lane] = acc.y;
     sums[w][2][lane] = acc.z;
@@ -243,7 +247,7 @@ naive_fix_cluster_kernel(const double* __restrict__ m, const double* __restrict_
 constexpr int CC_WARPS = 8;
 
 __global__ void __launch_bounds__(32 * CC_WARPS)
-chunk_combine_kernel(const double* __restrict__ part, uint32_t chunks, uint32_t i_begin,
+chunk_combine_kernel(const double* part, uint32_t chunks, uint32_t i_begin,
                      uint32_t i_end, double* __restrict__ ax, double* __restrict__ ay,
                      double* __restrict__ az) {
     nb_grid_wait();

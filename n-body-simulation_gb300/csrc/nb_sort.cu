@@ -94,7 +94,7 @@ scan_sums_kernel(uint32_t* __restrict__ sums, uint32_t nb) {
 template <class Items>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_apply_kernel(Items in, uint32_t* __restrict__ out, uint32_t n,
-                  const uint32_t* __restrict__ sums, int write_total, int summed) {
+                  const uint32_t* sums, int write_total, int summed) {
     nb_grid_wait();
     const uint32_t base = blockIdx.x * SCAN_TILE;
     uint32_t before = 0;
@@ -151,7 +151,7 @@ static_assert(RS_THREADS == RS_BINS, "the look-back and the digit scan run one t
 
 // hist[p][d]: keys whose digit of pass p is d, for all passes in one read.
 __global__ void __launch_bounds__(RS_THREADS)
-radix_hist_all_kernel(const uint64_t* __restrict__ keys, uint32_t n, int begin_bit, int passes,
+radix_hist_all_kernel(const uint64_t* keys, uint32_t n, int begin_bit, int passes,
                       uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[RS_MAX_PASSES][RS_BINS];
     for (int e = threadIdx.x; e < RS_MAX_PASSES * RS_BINS; e += RS_THREADS) (&h[0][0])[e] = 0;
@@ -185,9 +185,9 @@ constexpr int RS_REORDER_BYTES = RS_THREADS * RS_ITEMS * (int)(sizeof(uint64_t) 
 // placed at digit offset + keys of the digit in earlier tiles + rank.
 template <int RS_ITEMS>
 __global__ void __launch_bounds__(RS_THREADS)
-radix_pass_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+radix_pass_kernel(const uint64_t* keys_in, const uint32_t* vals_in,
                   uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
-                  int shift, const uint32_t* __restrict__ hist, uint32_t* __restrict__ lb,
+                  int shift, const uint32_t* hist, uint32_t* __restrict__ lb,
                   uint32_t* __restrict__ ticket, uint32_t* __restrict__ err,
                   unsigned long long wait_limit, int drop_first) {
     constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
