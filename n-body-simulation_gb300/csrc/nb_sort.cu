@@ -1,6 +1,7 @@
 // nb_sort.cu -- device-wide exclusive scan (u32) and stable LSD radix sort of (u64 key, u32 value)
 // pairs, used by the octree build. Deterministic: no result depends on thread timing.
 #include <algorithm>
+#include <atomic>
 
 #include "nb_sort.cuh"
 
@@ -360,7 +361,7 @@ static uint32_t radix_tiles(uint32_t n) {
 }
 
 nb_status radix_prepare() {
-    static bool done[64] = {};
+    static std::atomic<bool> done[64];
     int dev = 0;
     NB_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || done[dev]) return NB_OK;
