@@ -132,9 +132,8 @@ nb_status nb_naive_set_pair_config(int config);
  * (4,12,128), (4,16,128), (8,8,256), (4,8,256), (8,6,256), (2,12,128); config_f64
  * 0..NB_SYM64_CONFIG_COUNT-1 = (4,2,64), (4,4,64), (8,2,64), (4,2,128); config_df
  * 0..NB_SYMDF_CONFIG_COUNT-1 = (4,2,64), (4,4,64). In mode 1 the FP64 and double-float shapes
- * are chosen by the library ((4,2,64); double-float (4,4,64) when its partials exceed the cap).
- * Process-wide; nb_naive_accel_range
- * with a partial range always uses the one-sided kernels. */
+ * are chosen by the library ((4,2,64), or (4,4,64) when its partials exceed the cap). Process-wide;
+ * nb_naive_accel_range with a partial range always uses the one-sided kernels. */
 #define NB_SYM_CONFIG_COUNT 8
 #define NB_SYM64_CONFIG_COUNT 4
 #define NB_SYMDF_CONFIG_COUNT 2

@@ -313,12 +313,14 @@ nb_status naive_sym(nb_ctx* ctx, int form, const double* m, const double* x, con
     if (g_naive_sym_mode == 0) return NB_OK;
     // candidate shapes: the configured one, except in the automatic mode of the FP64 and
     // double-float forms, which take shape 0 (4,2,64) with 256-body I-blocks (fewer registers per
-    // thread); where its partials do not fit, double-float takes shape 1 (4,4,64) with 512, FP64
-    // the one-sided kernel (as fast as its shape 1)
+    // thread) and, where its partials do not fit, shape 1 (4,4,64) with 512 and half the partials.
+    // FP64, shape 0 against 1: 157 / 146 Gpairs/s at 16,384 bodies, 161 / 159 at 32,768, 164 / 162
+    // from 98,304 on; at 320,000, where shape 0 needs 4.4 GiB of partials, 165 / 163 and 149
+    // one-sided.
     int cand[2] = {g_naive_sym_cfg[form], -1};
     if (g_naive_sym_mode == 1 && form != nb::SYM_F32) {
         cand[0] = 0;
-        cand[1] = form == nb::SYM_DF ? 1 : -1;
+        cand[1] = 1;
     }
     const uint64_t min_units = form == nb::SYM_F64 ? SYM_MIN_UNITS_F64 : SYM_MIN_UNITS_PER_CTA;
     int cfg = -1;

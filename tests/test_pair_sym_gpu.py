@@ -163,3 +163,24 @@ def test_symmetric_df64_selected_and_deterministic(ctx):
     diff = np.sqrt(sum((f - o) ** 2 for f, o in zip(first, one)))
     assert (diff / np.maximum(mag, np.median(mag))).max() <= 1e-11
     assert any(np.any(f != o) for f, o in zip(first, one))  # a different kernel ran
+
+
+def test_f64_shape_with_fewer_partials(ctx):
+    """From about 304,000 bodies on the partials of the automatic FP64 shape exceed the cap: the shape with
+    half of them is taken (its bits), not the one-sided kernel."""
+    import torch
+    from nbody import generators
+    from nbody.lib import SYM_ALWAYS, SYM_AUTO, set_naive_symmetric
+    n = 306000
+    d = generators.plummer(n, seed=1)
+    t = [dev(d[k]) for k in ("m", "x", "y", "z")]
+    a, b = ([torch.empty(n, dtype=torch.float64, device="cuda") for _ in range(3)] for _ in range(2))
+    ctx.naive_accel(*t, *a, d["G"], 1e-6, "f64")
+    try:
+        set_naive_symmetric(SYM_ALWAYS, 0, 1, 0)
+        ctx.naive_accel(*t, *b, d["G"], 1e-6, "f64")
+    finally:
+        set_naive_symmetric(SYM_AUTO)
+    ctx.sync()
+    for u, v in zip(a, b):
+        assert torch.equal(u, v)
