@@ -152,8 +152,9 @@ __device__ __forceinline__ void fix_monopole(const FixRec& f, const NodeRec64* _
     acz = fma(w, dz, acz);
 }
 
-// Per-body reference rule, FP64 (IEEE64 bit-identical to the host evaluation; FAST64 with FMAs).
-template <int MODE>
+// Per-body reference rule, FP64 (IEEE64 bit-identical to the host evaluation; FAST64: NB_F64's
+// arithmetic, with the TEAM partial sums of the default schedule's lanes in turn).
+template <int MODE, int TEAM>
 __global__ void __launch_bounds__(TR_THREADS)
 bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const nbfix::FixHi* __restrict__ fix_hi,
                     const uint4* __restrict__ fix_lo,
@@ -161,8 +162,7 @@ bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const nbfix::FixHi* __res
                     const uint32_t* __restrict__ ids, const double* __restrict__ x,
                     const double* __restrict__ y, const double* __restrict__ z,
                     const double* __restrict__ box, uint32_t n,
-                    double theta, double eps2, double G, int team,
-                    double* __restrict__ ax,
+                    double theta, double eps2, double G, double* __restrict__ ax,
                     double* __restrict__ ay, double* __restrict__ az) {
     using A = Arith<MODE>;
     __shared__ nbfix::Eps2Table e2;
@@ -182,9 +182,7 @@ bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const nbfix::FixHi* __res
         pz = z[me];
     }
     const FixBody me_fix = fix_body<MODE>(px, py, pz, K, e2);
-    // NB_F64: `team` partial sums in turn, as bh_theta_team_kernel
-    constexpr int TEAM_MAX = MODE == FAST64 ? 32 : 1;
-    double acx[TEAM_MAX] = {}, acy[TEAM_MAX] = {}, acz[TEAM_MAX] = {};
+    double acx[TEAM] = {}, acy[TEAM] = {}, acz[TEAM] = {};
     uint32_t ord = 0;
     uint32_t kl = valid ? 0u : nn;
     for (;;) {
@@ -198,7 +196,7 @@ bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const nbfix::FixHi* __res
             const double cur = A::mul(r.edge, A::rsqrt(d2));  // :355-357
             if (cur < theta || r.body != NB_NONE) {           // :359
                 if constexpr (MODE == FAST64) {
-                    const uint32_t c = ord++ & (uint32_t)(team - 1);
+                    const uint32_t c = ord++ & (uint32_t)(TEAM - 1);
                     fix_monopole(load_fix(fix_hi, fix_lo, k), rec, k, me_fix, K, e2, x, y, z, me,
                                  eps2, acx[c], acy[c], acz[c]);
                 } else {
@@ -212,14 +210,13 @@ bh_theta_f64_kernel(const NodeRec64* __restrict__ rec, const nbfix::FixHi* __res
             kl = r.skip;
         }
     }
-    if constexpr (MODE == FAST64) {
-        for (int o = team / 2; o > 0; o >>= 1)
-            for (int c = 0; c < o; ++c) {
-                acx[c] += acx[c + o];
-                acy[c] += acy[c + o];
-                acz[c] += acz[c + o];
-            }
-    }
+#pragma unroll
+    for (int o = TEAM / 2; o > 0; o >>= 1)
+        for (int c = 0; c < o; ++c) {
+            acx[c] += acx[c + o];
+            acy[c] += acy[c + o];
+            acz[c] += acz[c + o];
+        }
     if (valid) {
         ax[me] = A::mul(acx[0], G);
         ay[me] = A::mul(acy[0], G);
@@ -1097,6 +1094,27 @@ nb_status launch_f64(nb_ctx* ctx, const nb_bh_tree* t, nb_precision prec, const 
     return NB_OK;
 }
 
+// NB_F64 and NB_F64_IEEE in lockstep (nb_bh_set_schedule).
+nb_status launch_lockstep(nb_ctx* ctx, const nb_bh_tree* t, nb_precision prec, const double* x,
+                          const double* y, const double* z, double* ax, double* ay, double* az,
+                          double G, double eps2, cudaStream_t s) {
+    auto go = [&](auto kernel) {
+        kernel<<<nb::ceil_div(t->n, TR_THREADS), TR_THREADS, 0, s>>>(
+            t->rec64, t->fix_hi, t->fix_lo, t->info, t->ids, x, y, z, t->box, t->n, t->params.theta,
+            eps2, G, ax, ay, az);
+        return nb::check_launch("bh_theta_f64_kernel");
+    };
+    if (prec == NB_F64_IEEE) return go(bh_theta_f64_kernel<IEEE64, 1>);
+    switch (team_lanes(ctx, t->n)) {
+        case 1: return go(bh_theta_f64_kernel<FAST64, 1>);
+        case 2: return go(bh_theta_f64_kernel<FAST64, 2>);
+        case 4: return go(bh_theta_f64_kernel<FAST64, 4>);
+        case 8: return go(bh_theta_f64_kernel<FAST64, 8>);
+        case 16: return go(bh_theta_f64_kernel<FAST64, 16>);
+        default: return go(bh_theta_f64_kernel<FAST64, 32>);
+    }
+}
+
 }  // namespace
 
 namespace nb {
@@ -1125,26 +1143,17 @@ nb_status nb_bh_accel(nb_ctx* ctx, const nb_bh_tree* t, const double* x, const d
     const uint32_t n = t->n;
     const int grid = nb::ceil_div(n, TR_THREADS);
     const double theta = t->params.theta;
-    const int team = team_lanes(ctx, n);
     if (opening == NB_OPEN_THETA) {
         switch (prec) {
             case NB_F64_IEEE:
                 NB_TRY(nb_need_records(t, NB_REC_FP64, "nb_bh_accel"));
-                if (g_lockstep) {
-                    bh_theta_f64_kernel<IEEE64><<<grid, TR_THREADS, 0, s>>>(
-                        t->rec64, t->fix_hi, t->fix_lo, t->info, t->ids, x, y, z, t->box, n, theta,
-                        eps2, G, team, ax, ay, az);
-                    return nb::check_launch("bh_theta_f64_kernel<ieee>");
-                }
+                if (g_lockstep)
+                    return launch_lockstep(ctx, t, prec, x, y, z, ax, ay, az, G, eps2, s);
                 return launch_lane(ctx, t, prec, x, y, z, ax, ay, az, G, eps2, s);
             case NB_F64:
                 NB_TRY(nb_need_records(t, NB_REC_FP64, "nb_bh_accel"));
-                if (g_lockstep) {
-                    bh_theta_f64_kernel<FAST64><<<grid, TR_THREADS, 0, s>>>(
-                        t->rec64, t->fix_hi, t->fix_lo, t->info, t->ids, x, y, z, t->box, n, theta,
-                        eps2, G, team, ax, ay, az);
-                    return nb::check_launch("bh_theta_f64_kernel");
-                }
+                if (g_lockstep)
+                    return launch_lockstep(ctx, t, prec, x, y, z, ax, ay, az, G, eps2, s);
                 return launch_f64(ctx, t, prec, x, y, z, ax, ay, az, G, eps2, s);
             case NB_DF64:
                 NB_TRY(nb_need_records(t, NB_REC_FP64 | NB_REC_DF, "nb_bh_accel"));
