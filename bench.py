@@ -132,6 +132,34 @@ def measured_hbm_peak():
         return 6800.0, "fallback"
 
 
+# What the result line carries besides the metric's own keys; the rest goes to stderr (and --detail):
+# with all of it the line has 20,000 characters, which a reader of the output's last few thousand loses.
+LINE_LEFT_OUT = {"also": (), "roofline_build": (), "tree": (), "roofline": ("note", "work"),
+                 "cpu_baseline": ("build_s", "traversal_s")}
+
+
+def short_line(record: dict) -> dict:
+    """The record without the keys of LINE_LEFT_OUT (whole, or the named ones inside)."""
+    line = {}
+    for key, value in record.items():
+        inside = LINE_LEFT_OUT.get(key)
+        if inside == ():
+            continue
+        if inside and isinstance(value, dict):
+            value = {k: v for k, v in value.items() if k not in inside}
+        line[key] = value
+    return line
+
+
+def print_result(record: dict, detail_path) -> None:
+    """The whole record to stderr (and a file), the result line to stdout."""
+    print(json.dumps(record), file=sys.stderr, flush=True)
+    if detail_path:
+        with open(detail_path, "w") as f:
+            json.dump(record, f)
+    print(json.dumps(short_line(record)), flush=True)
+
+
 def headline_config(ws: int) -> dict:
     """The workload both arms (ours and --impl reference) report, as one dict."""
     return {"workload": f"barnes-hut fp64 theta={THETA}, {N_BODIES:,}-body heliocentric disc "
@@ -449,7 +477,7 @@ def run_ours(args):
             "cpu_baseline": cpu,
             "also": also,
         }
-        print(json.dumps(line), flush=True)
+        print_result(line, args.detail)
     tree.close()
     ctx.close()
     if dist is not None:
@@ -833,6 +861,8 @@ def main():
     ap.add_argument("--impl", choices=("ours", "reference"), default="ours")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--quick", action="store_true", help="skip the secondary measurements")
+    ap.add_argument("--detail", metavar="FILE",
+                    help="also write the whole record (build phases, other workloads) to a file")
     ap.add_argument("--bodies", type=int, default=N_BODIES,
                     help="bodies of the disc (default 1,048,576; smaller only for profiling)")
     ap.add_argument("--case", nargs="+", metavar=("NAME", "ARG"),
