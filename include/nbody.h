@@ -44,8 +44,10 @@ typedef enum nb_status {
 /* Arithmetic of the pair interactions. Positions, velocities, integration, AABB and energy sums
  * are FP64 in every mode. */
 typedef enum nb_precision {
-    NB_F64 = 0,       /* FP64 pair math with fused multiply-adds and a Newton-refined rsqrt
-                         (relative difference to the reference's FP64 sum ~1e-15) */
+    NB_F64 = 0,       /* FP64-accurate pairs: separation, r^2 + eps^2 and m r^-3 in fixed point (96-bit
+                         coordinates), FP64 sums; pairs that do not fit it (very close ones, small
+                         components of coordinates below 2^-41 of the box, boxes beyond 2^+-300)
+                         in FP64 (relative difference to the reference's FP64 sum ~1e-15) */
     NB_F64_IEEE = 1,  /* FP64, every operation separately and correctly rounded in the reference's
                          order (1/sqrt for sycl::rsqrt): bit-identical to a host FP64 evaluation
                          of the reference's formula */

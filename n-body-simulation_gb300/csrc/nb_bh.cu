@@ -746,8 +746,7 @@ build_small_kernel(const double* x, const double* y,
 
 struct ComArgs {
     uint32_t n;
-    uint32_t* err;  // device error word
-
+    uint32_t* err;      // device error word
     uint32_t records;  // NB_REC_* sets to compute
     const double *m, *x, *y, *z;
     const double* box;
@@ -1328,7 +1327,7 @@ __device__ __forceinline__ void com_chunk(const ComArgs& A, uint2* up, uint32_t*
 #pragma unroll
                     for (int t = 0; t < 8; ++t) {
                         const uint32_t k = (kw[t >> 1] >> (16 * (t & 1))) & 0xffffu;
-    v[t] = sv[min(k, (uint32_t)CH_NODES - 1)];  // unused where there is no child
+                        v[t] = sv[min(k, (uint32_t)CH_NODES - 1)];  // unused where there is no child
                     }
                     double sum = plus_zero(v[0]);  // 0.0 + v[0]
 #pragma unroll
@@ -1842,7 +1841,6 @@ nb_status nb_bh_build(nb_ctx* ctx, nb_bh_tree* t, const double* m, const double*
     A.node_last = t->node_last;
     A.node_skip = t->node_skip;
     A.err = ctx->dev_error;
-
     A.node_body = t->node_body;
     A.tier_slot = t->tier_slot;
     A.node_count = t->node_count;

@@ -331,9 +331,6 @@ bh_theta_lane_kernel(const NodeRec32* __restrict__ rec32, const NodeRec64* __res
     }
 }
 
-// Decision of the reference's opening rule for node `idx` seen from a body: true = accepted (a
-// leaf, or certainly below theta), by the FP32 test where its margin allows (see
-// bh_theta_lane_kernel), else by the FP64 expression.
 // Opening parameter as a kernel argument: its FP32 square stays in the constant bank.
 struct Theta {
     double value;
@@ -343,6 +340,9 @@ struct Theta {
 struct Pretest {
     float px, py, pz, edge, floor2;  // body relative to the box centre, box edge, margin_floor
 };
+// Decision of the reference's opening rule for node `idx` seen from a body: true = accepted (a
+// leaf, or certainly below theta), by the FP32 test where its margin allows (see
+// bh_theta_lane_kernel), else by the FP64 expression.
 __device__ __forceinline__ bool accepts(const NodeRec32& r, const Pretest& b,
                                         const NodeRec64* __restrict__ rec64, uint32_t idx,
                                         const double* __restrict__ x,
@@ -691,7 +691,8 @@ bh_theta_df_kernel(const NodeRec32* __restrict__ rec32, const DfTerms* __restric
                    const double* __restrict__ box, uint32_t n, Theta theta, double eps2,
                    double gscale, double* __restrict__ ax, double* __restrict__ ay,
                    double* __restrict__ az, uint32_t* __restrict__ next_group,
-                   const uint32_t* __restrict__ order, uint32_t* __restrict__ walk_len, const uint32_t* __restrict__ cost,
+                   const uint32_t* __restrict__ order, uint32_t* __restrict__ walk_len,
+                   const uint32_t* __restrict__ cost,
                    const unsigned long long* __restrict__ cost_sum) {
     __shared__ uint32_t list[FIX_LIST][TR_THREADS];
     const uint32_t n_groups = (n + 31) / 32, nn = info[0];

@@ -11,7 +11,7 @@
 //  * A pair: the three exact differences as magnitudes, shifted left by a common `sh` until the
 //    largest is in [2^29, 2^30) by its first word; r^2 + eps^2 as a 64-bit integer D in [2^60,
 //    2^64) (truncation errors below 2^-55 of it, centred); r^-3 from an estimate Y of D^(-1/2) good
-//    to 2^-30 (MUFU and one Newton step), its residual e = 1 - D Y^2, of which 32 bits remain, and
+//    to 2^-28 (MUFU and one Newton step), its residual e = 1 - D Y^2, of which 32 bits remain, and
 //    Y^3 (1 + 3e/2) (dropped terms below 2^-55), times the mass's 53 bits, rounded once to a
 //    double. In all within 2^-52.2 of exact, root mean square 2^-54.2 (the final rounding alone:
 //    2^-54.4).
@@ -301,9 +301,9 @@ NB_FIX_FN uint64_t norm2(const Sep& s) {
     return (r << 2) + ((uint64_t)h << 3);
 }
 
-// Y ~ 2^61 D^(-1/2), within 2^-30 of it and below 2^31 (the rounded estimate reaches 2^31 for D up to
+// Y ~ 2^61 D^(-1/2) to 2^-28 and below 2^31 (the rounded estimate reaches 2^31 for D up to
 // 2^60 + 2^32, where one unit less is as good: its users multiply it as a signed word), and
-// e = 1 - D Y^2 / 2^122 in units 2^-58 (|e| < 2^30); W = Y^2. D Y^2 is so near 2^122 that of its upper
+// e = 1 - D Y^2 / 2^122 in units 2^-58 (|e| < 2^31); W = Y^2. D Y^2 is so near 2^122 that of its upper
 // half only the low 32 bits are formed.
 NB_FIX_FN int rsqrt_residual(uint64_t D, uint32_t& Y, uint64_t& W) {
     const uint32_t dh = (uint32_t)(D >> 32), dl = (uint32_t)D;

@@ -88,7 +88,7 @@ __global__ void kick_kick_drift_kernel(double* __restrict__ vx, double* __restri
 // the units of all rows form one sequence that the CTAs split into equal contiguous ranges, so the
 // triangle's rows of unequal length load the SMs evenly. 1/r comes from the fixed point of
 // nb_fix.cuh (within one rounding of exact); of a pair's work only the sum, m_i * (1/r), is on the
-// FP64 pipe. Pairs the fixed point cannot hold (closer than 2^(K-30), or coordinates beyond its
+// FP64 pipe. Pairs the fixed point cannot hold (closer than 2^(K-29), or coordinates beyond its
 // exponent range) take the FP64 expression.
 //  Bound: dispatch of 104 instructions per unordered pair, half of them 64-bit (issue 58%, integer
 //  pipe 54%, wide multiplies 57%, FP64 pipe 38% of cycles), against 14 FP64 operations at 1/75 of
@@ -336,7 +336,7 @@ using nbaabb::val_of;
 // One word per block for nbfix::block_scale.
 __global__ void __launch_bounds__(256)
 scale_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                    const double* __restrict__ z, uint32_t n, uint32_t* __restrict__ out) {
+             const double* __restrict__ z, uint32_t n, uint32_t* __restrict__ out) {
     __shared__ uint32_t most;
     if (threadIdx.x == 0) most = 0;
     __syncthreads();
@@ -540,8 +540,8 @@ nb_status nb_aabb(nb_ctx* ctx, const double* x, const double* y, const double* z
 // GPU's memory up front for its own pool and forbids later cudaMalloc calls, or a time-critical
 // loop that cannot pay for cudaMalloc's device-wide synchronisation and unpredictable latency.
 // nb_energy needs a context (whose creation allocates) and grows per-block scratch on demand;
-// nb_energy_noalloc runs the same two kernels with their per-block partial sums in the fixed
-// array below instead. Nothing in the array needs clearing between calls: every call writes each
+// nb_energy_noalloc runs the same kernels with their per-block partial sums and scale words in the
+// fixed array below instead. Nothing in the array needs clearing between calls: every call writes each
 // partial it later reads. All calls share the array, so calls that overlap on the GPU (two
 // streams, two host threads) race and must be serialised by the caller.
 // ---------------------------------------------------------------------------------------------

@@ -152,7 +152,6 @@ __device__ __forceinline__ float nb_rsqrt_f32(float x) {
     return y;
 }
 
-// Packed FP32x2 arithmetic (sm_100+ f32x2 instructions): one instruction, two lanes.
 // Dependent launches. A kernel launched with nb::launch_after may start while the kernel before it
 // in the stream still runs; nb_grid_wait, which such a kernel calls before it touches memory that
 // earlier launches write, returns when that kernel has finished and its writes are visible, and
@@ -185,6 +184,7 @@ cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
 }
 }  // namespace nb
 
+// Packed FP32x2 arithmetic (sm_100+ f32x2 instructions): one instruction, two lanes.
 typedef unsigned long long nb_f2;
 __device__ __forceinline__ nb_f2 f2_pack(float lo, float hi) {
     nb_f2 r;

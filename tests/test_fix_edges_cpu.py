@@ -62,9 +62,10 @@ def pair(fix, c, p, m, eps2, v_max):
     return list(out) if ok else None
 
 
-# D^(-3/2) and D^(-1/2): the estimate is rounded to an integer of at least 2^29 (or clamped one unit
-# below 2^31), so its residual is below 2^-29 and the dropped terms below 2 x 2^-58; D^(-3/2) 2^151 is
-# at least 2^55 and truncated by less than 4 units, D^(-1/2) 2^93 at least 2^61 and by one.
+# D^(-3/2) and D^(-1/2): the estimate leaves D's low word out (2^-29 of it) and is rounded to an integer
+# of at least 2^29 (or clamped one unit below 2^31), so its residual is about 2^-28 and the dropped terms
+# 15/8 and 3/8 of 2^-56; D^(-3/2) 2^151 is at least 2^55 and truncated by less than 3 units, D^(-1/2) 2^93
+# at least 2^61 and by one.
 @pytest.mark.parametrize("base", [1 << 60, (1 << 60) + (1 << 32), 1 << 61, 1 << 62, 3 << 62, (1 << 64) - 1])
 def test_inverse_powers_at_the_limits(fix, base):
     rng = random.Random(base)
