@@ -396,10 +396,10 @@ __device__ __forceinline__ uint32_t next_walk(uint32_t* __restrict__ next_group,
 // cell's record loaded while the current one is computed.
 //  Bound: the load pipe (75% of its wavefronts: every lane reads its own 32-byte walk record per
 //  visited and 48-byte fixed-point record per accepted cell) and issue (61% of cycles). The
-//  monopole is ~130 instructions with 3 FP64 ones (nb_fix.cuh) against 16 FP64 operations before,
+//  monopole is ~137 instructions with 3 FP64 ones (nb_fix.cuh) against 16 FP64 operations before,
 //  whose pipe was 82% busy; 256-bit loads halve the load instructions (14.6 -> 13.45 ms), the
 //  lists (against one accepted cell at a time) keep 30.9 of 32 lanes active (17.2 -> 14.6 ms with
-//  the record prefetch). Step at 1,048,576 bodies (disc, theta = 0.5): 35.5 -> 13.1 ms. 24 warps
+//  the record prefetch). Step at 1,048,576 bodies (disc, theta = 0.5): 35.5 -> 13.2 ms. 24 warps
 //  per SM: 20 measured 4%, 28 2.5% and 32 4% slower; lists of 8 2% slower.
 constexpr int FIX_LIST = 16;
 constexpr int FIX_BLOCKS_PER_SM = 6;

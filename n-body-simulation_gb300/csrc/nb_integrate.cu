@@ -90,9 +90,9 @@ __global__ void kick_kick_drift_kernel(double* __restrict__ vx, double* __restri
 // nb_fix.cuh (within one rounding of exact); of a pair's work only the sum, m_i * (1/r), is on the
 // FP64 pipe. Pairs the fixed point cannot hold (closer than 2^(K-29), or coordinates beyond its
 // exponent range) take the FP64 expression.
-//  Bound: dispatch of 104 instructions per unordered pair, half of them 64-bit (issue 58%, integer
+//  Bound: dispatch of 107 instructions per unordered pair, half of them 64-bit (issue 58%, integer
 //  pipe 54%, wide multiplies 57%, FP64 pipe 38% of cycles), against 14 FP64 operations at 1/75 of
-//  the FP32 rate before. 50,021 bodies: 49.2 -> 5.4 ms (25 -> 233 Gpairs/s). 48 warps per SM (24
+//  the FP32 rate before. 50,021 bodies: 49.2 -> 5.45 ms (25 -> 230 Gpairs/s). 48 warps per SM (24
 //  to 40: 1 to 7% slower).
 // ---------------------------------------------------------------------------------------------
 constexpr int EN_THREADS = 128;        // targets per row, sources per tile at most

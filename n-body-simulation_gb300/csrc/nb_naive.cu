@@ -110,11 +110,11 @@ __device__ __forceinline__ void fix_pair(const nbfix::FixRec& f, uint32_t q, uin
 
 // NB_F64, one-sided: target ranges, listed targets, systems below the symmetric kernel's sizes. One
 // thread per target; the sources of a tile are converted to the fixed point of nb_fix.cuh by the
-// block as it loads them, and a pair costs ~115 integer instructions and 3 FP64 ones instead of 16
+// block as it loads them, and a pair costs ~122 integer instructions and 3 FP64 ones instead of 16
 // FP64 ones. blockIdx.y selects a chunk of `chunk` sources; with more than one chunk the partial
 // sums (times G) go to part[(chunk index * targets + target) * 3 + axis].
-//  Bound: the FP64 pipe (81% busy at 3 FMAs per pair) and dispatch. 8,192 bodies 2.16 -> 0.50 ms
-//  (31 -> 133 Gpairs/s), 4,096 0.53 -> 0.15. 32 warps per SM in blocks of 256 (blocks of 128: 3%
+//  Bound: the FP64 pipe (77% busy at 3 FMAs per pair) and dispatch. 8,192 bodies 2.16 -> 0.54 ms
+//  (31 -> 125 Gpairs/s), 4,096 0.53 -> 0.16. 32 warps per SM in blocks of 256 (blocks of 128: 3%
 //  slower, of 64: 16%).
 constexpr int FX_THREADS = 256;
 constexpr int FX_BLOCKS_PER_SM = 4;
@@ -299,8 +299,9 @@ int g_naive_sym_cfg[3] = {0, 0, 0};
 // spread small systems better) and j-side partials (3 values per unit and tile body) below the
 // cap.
 constexpr uint64_t SYM_MIN_UNITS_PER_CTA = 7;
-// FP64: from 4 units per CTA on (~9,900 bodies). 12,000 bodies (5.8 units): 0.95 ms against 1.04
-// one-sided, 8,192 (2.8 units): 0.50 either way, 4,096: 0.23 against 0.15.
+// FP64: from 4 units per CTA on (~9,900 bodies). 12,000 bodies (5.8 units): 0.97 ms against 1.10
+// one-sided, 9,900: 0.76 / 0.77, 8,192 (2.8 units): 0.51 / 0.54, 4,096: 0.18 / 0.16; between the last
+// two the one-sided kernel stays, which also runs in a capture without scratch.
 constexpr uint64_t SYM_MIN_UNITS_F64 = 4;
 constexpr size_t SYM_PART_CAP_BYTES = (size_t)4 << 30;
 

@@ -326,8 +326,8 @@ pair_sym_kernel(SymPlan S, const float4* __restrict__ src, float eps2,
 // two bodies, and a mass product each; FP64 sums, kept in registers for a whole row segment (i) or
 // rotated through the lanes (j). Pairs the fixed point cannot hold take the FP64 expressions, once for
 // both bodies; those with a massless body are added one side at a time.
-//  Bound: the FP64 pipe, 92% busy with 3 FMAs per ordered pair (10 FP64 operations before).
-//  65,536 bodies 76.8 -> 26.7 ms (56 -> 161 Gpairs/s), 16,384 4.96 -> 1.72 ms. Registers for 20
+//  Bound: the FP64 pipe, 83 to 90% busy with 3 FMAs per ordered pair (10 FP64 operations before).
+//  65,536 bodies 76.8 -> 27.0 ms (56 -> 159 Gpairs/s), 16,384 4.96 -> 1.76 ms. Registers for 20
 //  warps per SM: 12, 16 and 24 warps measured 15%, 3% and 2% slower.
 constexpr int FIX_WARPS_PER_SM = 20;
 
