@@ -465,7 +465,7 @@ pair_sym_fix_kernel(SymPlan S, const nbfix::FixRec* __restrict__ src,
                             } else if (sh_max >= 0 && min(J.e, I[k].e) == nbfix::ZERO_MASS) {
                                 one_side(J, bj, I[k], bi, tx[k], ty[k], tz[k]);
                                 one_side(I[k], bi, J, bj, jx, jy, jz);
-                            } else if (!nbfix::adds_nothing(J, bi == bj, K, sh_max, eps2)) {
+                            } else if (bi != bj || !nbfix::adds_nothing(J, true, K, sh_max, eps2)) {
                                 const double dx = x[bj] - x[bi], dy = y[bj] - y[bi],
                                              dz = z[bj] - z[bi];
                                 const double c = nb_m_rinv3_f64(

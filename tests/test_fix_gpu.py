@@ -347,7 +347,7 @@ def test_energy_that_is_not_finite(ctx):
         assert u == -np.inf if what == "m" else np.isfinite(u)
 
 
-@pytest.mark.parametrize("what", ["negative", "massless", "subnormal", "outlier", "softening"])
+@pytest.mark.parametrize("what", ["negative", "massless", "mixed", "subnormal", "outlier", "softening"])
 def test_symmetric_pairs_outside_the_fixed_point(ctx, what):
     """What the symmetric kernel leaves to FP64: everything, or the pairs of some bodies. Bound as for the
     lattice (the FP64 factor is within 2^-51, the sums within n 2^-53 of the terms' magnitudes)."""
@@ -359,6 +359,10 @@ def test_symmetric_pairs_outside_the_fixed_point(ctx, what):
     elif what == "massless":
         d["m"][::2] = 0.0
         d["m"][1::10] = -0.0
+    elif what == "mixed":  # massless bodies beside masses that the fixed point refuses
+        d["m"][::2] = 0.0
+        d["m"][1::6] *= -1.0
+        d["m"][3::10] = 1e-310
     elif what == "subnormal":
         d["m"][::3] = 1e-310
     elif what == "outlier":
