@@ -87,7 +87,7 @@ __global__ void kick_kick_drift_kernel(double* __restrict__ vx, double* __restri
 // Bodies in rows of 128 targets; a row's units are its tiles of sources up to the diagonal, and
 // the units of all rows form one sequence that the CTAs split into equal contiguous ranges, so the
 // triangle's rows of unequal length load the SMs evenly. 1/r comes from the fixed point of
-// nb_fix.cuh (within one rounding of exact); of a pair's work only the sum, m_i * (1/r), is on the
+// nb_fix.cuh (within one rounding of exact); of a pair's work only the sum, G m_i * (1/r), is on the
 // FP64 pipe. Pairs the fixed point cannot hold (closer than 2^(K-29), or coordinates beyond its
 // exponent range) take the FP64 expression.
 //  Bound: dispatch of 107 instructions per unordered pair, half of them 64-bit (issue 58%, integer
@@ -105,7 +105,7 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
               const double* __restrict__ vx, const double* __restrict__ vy,
               const double* __restrict__ vz, uint32_t n, double G, uint32_t tile, uint64_t units,
               const uint32_t* __restrict__ k_part, uint32_t k_words, double2* __restrict__ part) {
-    __shared__ nbfix::FixRec src[EN_THREADS];  // positions; the mass as a double in (mh, ml)
+    __shared__ nbfix::FixRec src[EN_THREADS];  // positions; G times the mass as a double in (mh, ml)
     __shared__ double red_k[EN_THREADS / 32], red_p[EN_THREADS / 32];
     const uint32_t tid = threadIdx.x;
     const int K = nbfix::block_scale(x, y, z, n, k_part, k_words);
@@ -144,7 +144,7 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
             const uint32_t i = i0 + tid;
             nbfix::Fix3 c;
             nbfix::split3(x[i], y[i], z[i], K, c);
-            const double mi = m[i];
+            const double mi = G * m[i];  // first: m / r may overflow where G m m / r does not
             src[tid] = nbfix::FixRec{c.x2, c.y2, c.z2, (uint32_t)__double2hiint(mi),
                                      c.x1, c.y1, c.z1, (uint32_t)__double2loint(mi),
                                      c.x0, c.y0, c.z0, 0};
@@ -169,7 +169,7 @@ energy_kernel(const double* __restrict__ m, const double* __restrict__ x,
             acc = fma(__hiloint2double((int)f.mh, (int)f.ml), inv, acc);
         }
         if (++t == q * (row + 1) || u + 1 == u1) {  // the row (or the CTA's range) ends
-            if (paired) ep = fma(G * mj, acc, ep);  // without pairs a mass of infinity adds nothing
+            if (paired) ep = fma(mj, acc, ep);  // without pairs a mass of infinity adds nothing
             t = 0;
             ++row;
             load = true;

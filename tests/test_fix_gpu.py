@@ -381,3 +381,27 @@ def test_symmetric_pairs_outside_the_fixed_point(ctx, what):
     ref = naive(ctx, d, eps2, "f64_ieee")
     for g, r, b in zip(got, ref, bound):
         assert np.isfinite(r).all() and (np.abs(g - r) <= b).all()
+
+
+@pytest.mark.parametrize("G,heavy", [(1e-7, 1e307), (1e-200, 1e300), (1e200, 1e-250)])
+def test_energy_of_extreme_masses(ctx, G, heavy):
+    """G m_i first, as the reference multiplies: m_i / r alone leaves the doubles' range."""
+    import oracle
+    import torch
+    d = bodies("plummer", 300, seed=12)
+    for k in "xyz":
+        d[k] = d[k] * 1e-3
+    d["m"] = d["m"] * 1e-5
+    d["m"][::7] = heavy
+    if heavy > 1:
+        d["m"][7::7] = 1e-5
+    for k in ("vx", "vy", "vz"):
+        d[k] = d[k] * 1e-3
+    keys = ("m", "x", "y", "z", "vx", "vy", "vz")
+    out = torch.zeros(4, dtype=torch.float64, device="cuda")
+    ctx.energy(*[dev(d[k]) for k in keys], G, out)
+    ctx.sync()
+    o = oracle.energy(*[d[k] for k in keys], G)
+    assert np.isfinite(o["potential"]) and o["potential"] != 0
+    assert abs(out[1].item() - o["potential"]) <= 1e-12 * abs(o["potential"])
+    assert abs(out[0].item() - o["kinetic"]) <= 1e-12 * abs(o["kinetic"])
